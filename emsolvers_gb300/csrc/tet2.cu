@@ -29,11 +29,15 @@
 //   mass inverse the drift applies q(M) P, the degree-m Chebyshev polynomial
 //                of the mass preconditioned by its 2 x 2 edge and face
 //                blocks, on the element bounds of the preconditioned
-//                spectrum; one entity pass per iteration: each edge or face
-//                forms its two mass rows from the iterate of its (up to six)
-//                tetrahedra in a fixed order (no atomics, no per-tetrahedron
-//                array), applies the block inverse and the Chebyshev update,
-//                and writes the next iterate to the other of two buffers.
+//                spectrum.  All tetrahedra share one element mass.  An
+//                iteration sums, per edge or face, the values of its (up to
+//                six) tetrahedra in a fixed order (no atomics), applies the
+//                block inverse and the Chebyshev update: FP32 runs in a
+//                kernel that marches tiles up z or, on small meshes, one
+//                thread per edge or face, the iterates alternating between
+//                two buffers; FP64 runs in an element pass (the mass split
+//                into two 10 x 10 halves by the vertex reversal) and an
+//                entity pass.
 //   time loop    one CUDA graph per step, replayed; a device step counter
 //                indexes the source table and the receiver samples.
 // Units are normalised (cube edge 1, c0 = 1); the API converts.
@@ -360,6 +364,7 @@ __constant__ float c2_M32[6][400];
 __constant__ double c2_C[6][20][12];
 __constant__ float c2_C32[6][20][12];   // the same, exact in FP32 (dyadic)
 __constant__ int c2_ninc[kEnt], c2_inc[kEnt][kMaxInc], c2_axes[kEnt];
+__constant__ int c2_massslot[20];       // local function -> place in the mass element values (mass_slot)
 
 struct T2Shot {
     int n[3];
@@ -385,7 +390,6 @@ template <> __device__ __forceinline__ double mref<double>(int p, int a, int b) 
 template <> __device__ __forceinline__ float mref<float>(int p, int a, int b) { return c2_M32[p][20 * a + b]; }
 
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 
@@ -413,45 +417,6 @@ __device__ __forceinline__ TetAddr tet_addr(const T2Shot &S, unsigned long long 
     ta.nnode = S.nnode;
     ta.dof0 = S.dof0;
     return ta;
-}
-
-// Mass element pass: Yt[a][t] = eps_t (Mref_p x_t)_a (the two-pass
-// iteration: this pass, then the entity pass sums the values of an
-// entity's tetrahedra).  The type p is dispatched to a compile-time
-// constant (tetrahedra are type-major, so a warp holds one type), so the
-// reference entries are constant operands of the multiply-adds.
-template <class T, int P> __device__ __forceinline__ void mass_elem_body(const TetAddr &ta, unsigned long long NT, unsigned long long t, T e,
-                                                                         const T *__restrict__ x, T *__restrict__ Yt)
-{
-    T xv[20];
-#pragma unroll
-    for (int b = 0; b < 20; ++b) xv[b] = x[ta.dof(b)];
-#pragma unroll
-    for (int a = 0; a < 20; ++a) {
-        T y = T(0);
-#pragma unroll
-        for (int b = 0; b < 20; ++b) y = fma(mref<T>(P, a, b), xv[b], y);
-        Yt[(unsigned long long)a * NT + t] = mul_rn(e, y);
-    }
-}
-
-template <class T>
-__global__ void __launch_bounds__(128) t2_mass_elem_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
-                                                          const T *__restrict__ eps, const T *__restrict__ x, T *__restrict__ Yt)
-{
-    const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-    if (t >= NT) return;
-    const T2Shot S = sh[shot_of(sh, ns, t, 0)];
-    const TetAddr ta = tet_addr(S, t - S.tet0);
-    const T e = eps[t];
-    switch (ta.p) {
-    case 0: mass_elem_body<T, 0>(ta, NT, t, e, x, Yt); break;
-    case 1: mass_elem_body<T, 1>(ta, NT, t, e, x, Yt); break;
-    case 2: mass_elem_body<T, 2>(ta, NT, t, e, x, Yt); break;
-    case 3: mass_elem_body<T, 3>(ta, NT, t, e, x, Yt); break;
-    case 4: mass_elem_body<T, 4>(ta, NT, t, e, x, Yt); break;
-    default: mass_elem_body<T, 5>(ta, NT, t, e, x, Yt); break;
-    }
 }
 
 // Stiffness element pass in FP64: vertex curls c_v = sum_a U_a C_av, the P1
@@ -570,6 +535,152 @@ __global__ void __launch_bounds__(128, 5) t2_stiff_df_kernel(unsigned long long 
     }
 }
 
+// ------------------------------------------------------- element mass
+// The six types are images of each other under axis permutations, so one
+// element mass serves all types.  The vertex reversal of a Kuhn tetrahedron
+// (v0 v1 v2 v3 -> v3 v2 v1 v0) is an isometry that maps local function a to
+// minus its mate, so the mass splits into two 10 x 10 halves on the
+// differences u and sums w of mates: 200 multiply-adds and 40 additions
+// instead of 400.  FP64 runs, bound by the FP64 pipe, take the halves; FP32
+// runs keep the full rows, whose rounding their traces were verified with.
+struct MateTab {
+    int mate[20], rep[10];
+};
+constexpr MateTab make_mate_tab()
+{
+    return MateTab{{11, 10, 8, 9, 7, 6, 5, 4, 2, 3, 1, 0, 19, 18, 17, 16, 15, 14, 13, 12}, {0, 1, 2, 3, 4, 5, 12, 13, 14, 15}};
+}
+// The mass and its halves (M_ab - M_ab') / 2 and (M_ab + M_ab') / 2 over the
+// representatives a, b (b' the mate of b) at compile time, from the
+// barycentric integrals int l^alpha = |T| 3! alpha! / 7! (|T| = 1/6).
+struct MassTab {
+    double m[400], h[2][100];
+};
+constexpr double mono4(int a, int b, int c, int d)
+{
+    int n[4] = {0, 0, 0, 0};
+    ++n[a]; ++n[b]; ++n[c]; ++n[d];
+    constexpr double f[5] = {1, 1, 2, 6, 24};
+    return f[n[0]] * f[n[1]] * f[n[2]] * f[n[3]] / 5040.0;
+}
+struct FunC {
+    double co[4];
+    int i, j;
+};
+constexpr FunC fun_c(int a)
+{
+    FunC f{};
+    if (a < 12) {
+        f.i = kEdge[a % 6][0]; f.j = kEdge[a % 6][1];
+        for (int k = 0; k < 4; ++k) f.co[k] = (k == f.i || k == f.j) ? 0.0 : kAdmix;
+        f.co[a < 6 ? f.i : f.j] = 1.0;
+    } else {
+        const int v = (a - 12) / 2;
+        if ((a - 12) % 2 == 0) { f.co[kFace[v][2]] = 1.0; f.i = kFace[v][0]; f.j = kFace[v][1]; }
+        else { f.co[kFace[v][0]] = 1.0; f.i = kFace[v][1]; f.j = kFace[v][2]; }
+    }
+    return f;
+}
+constexpr double mass_entry(int a, int b)
+{
+    // grad l_m . grad l_n of a Kuhn tetrahedron: a path of three unit steps
+    constexpr double G[4][4] = {{1, -1, 0, 0}, {-1, 2, -1, 0}, {0, -1, 2, -1}, {0, 0, -1, 1}};
+    const FunC f = fun_c(a), g = fun_c(b);
+    double s = 0.0;
+    for (int n = 0; n < 4; ++n)
+        for (int m = 0; m < 4; ++m) {
+            if (f.co[n] == 0.0 || g.co[m] == 0.0) continue;
+            s += f.co[n] * g.co[m] *
+                 (mono4(n, m, f.i, g.i) * G[f.j][g.j] - mono4(n, m, f.i, g.j) * G[f.j][g.i] - mono4(n, m, f.j, g.i) * G[f.i][g.j] +
+                  mono4(n, m, f.j, g.j) * G[f.i][g.i]);
+        }
+    return s;
+}
+constexpr MassTab make_mass_tab()
+{
+    MassTab T{};
+    const MateTab mt = make_mate_tab();
+    for (int a = 0; a < 20; ++a)
+        for (int b = 0; b < 20; ++b) T.m[20 * a + b] = mass_entry(a, b);
+    for (int c = 0; c < 10; ++c)
+        for (int b = 0; b < 10; ++b) {
+            const double m0 = T.m[20 * mt.rep[c] + mt.rep[b]], m1 = T.m[20 * mt.rep[c] + mt.mate[mt.rep[b]]];
+            T.h[0][10 * c + b] = 0.5 * (m0 - m1);
+            T.h[1][10 * c + b] = 0.5 * (m0 + m1);
+        }
+    return T;
+}
+constexpr MassTab kMass = make_mass_tab();
+__constant__ double c2_H64[2][100];
+
+// Row A of M x in FP32.  The entries are immediate operands: read from
+// constant memory they took registers and spilled in the marching kernel
+// (50 us an iteration on 48^3 cubes against 39.5, with the halved mass).
+template <int A, int... B> __device__ __forceinline__ float mass_row(std::integer_sequence<int, B...>, const float (&x)[20])
+{
+    float r = 0.0f;
+    auto term = [&](auto b) {
+        constexpr int K = decltype(b)::value;
+        constexpr float m = (float)kMass.m[20 * A + K];
+        if constexpr (m != 0.0f) r = fmaf(m, x[K], r);
+    };
+    (term(std::integral_constant<int, B>{}), ...);
+    return r;
+}
+
+// Half H, row Q of the halved mass in FP64.
+template <int H, int Q> __device__ __forceinline__ double half_dot(const double (&u)[10])
+{
+    double s = c2_H64[H][10 * Q] * u[0];
+#pragma unroll
+    for (int b = 1; b < 10; ++b) s = fma(c2_H64[H][10 * Q + b], u[b], s);
+    return s;
+}
+constexpr int mass_slot(int a)   // place of local function a: representatives 0..9, mates 10..19
+{
+    const MateTab m = make_mate_tab();
+    for (int c = 0; c < 10; ++c) {
+        if (m.rep[c] == a) return c;
+        if (m.mate[m.rep[c]] == a) return 10 + c;
+    }
+    return -1;
+}
+
+// Mass element pass of FP64 runs: Yt[slot][t] = eps_t (M x_t), one thread per
+// tetrahedron.  Bound by the FP64 pipe (two lanes per SM and clock on GB300):
+// 270 FP64 operations per tetrahedron, 420 before the halves.  Blocks of 64
+// threads spread a small mesh over the SMs.
+template <int... Q>
+__device__ __forceinline__ void mass_elem_rows(std::integer_sequence<int, Q...>, const double (&u)[10], const double (&w)[10], double e,
+                                               double *__restrict__ y, unsigned long long NT)
+{
+    auto row = [&](auto q) {
+        constexpr int C = decltype(q)::value;
+        const double f = half_dot<0, C>(u), eh = e * half_dot<1, C>(w);
+        y[C * NT] = fma(e, f, eh);
+        y[(10 + C) * NT] = fma(-e, f, eh);
+    };
+    (row(std::integral_constant<int, Q>{}), ...);
+}
+__global__ void __launch_bounds__(64) t2_mass_elem_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
+                                                         const double *__restrict__ eps, const double *__restrict__ x,
+                                                         double *__restrict__ Yt)
+{
+    const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+    if (t >= NT) return;
+    const T2Shot S = sh[shot_of(sh, ns, t, 0)];
+    const TetAddr ta = tet_addr(S, t - S.tet0);
+    constexpr MateTab mt = make_mate_tab();
+    double u[10], w[10];
+#pragma unroll
+    for (int c = 0; c < 10; ++c) {
+        const double a = x[ta.dof(mt.rep[c])], b = x[ta.dof(mt.mate[mt.rep[c]])];
+        u[c] = a - b;
+        w[c] = a + b;
+    }
+    mass_elem_rows(std::make_integer_sequence<int, 10>{}, u, w, eps[t], Yt + t, NT);
+}
+
 enum { G_FORCE = 0, G_KICK = 1, G_CHEB0 = 2, G_CHEB = 3 };
 enum { FIN_NONE = 0, FIN_DRIFT = 1, FIN_LEAP = 2 };
 
@@ -586,8 +697,9 @@ template <class T> struct GArgs {
     const T *pinv;   // 2 x 2 block inverses, three planes over the entities
     T *U, *Uold;
     double a;        // kick: P -= a F
-    double h;        // final iteration: U += h x (drift) or U = 2U - Uold - h x (leapfrog)
-    double c0, c1, c2;   // Chebyshev: d = c1 d + c2 z (c0 = 1 / theta for the first step)
+    // scalars of the run precision: the GPU converts FP64 values at its FP64 rate
+    T h;             // final iteration: U += h x (drift) or U = 2U - Uold - h x (leapfrog)
+    T c0, c1, c2;    // Chebyshev: d = c1 d + c2 z (c0 = 1 / theta for the first step)
 };
 
 // Entity pass: one thread per edge or face of a node (both its DOFs).  Sums
@@ -637,8 +749,9 @@ __global__ void __launch_bounds__(128) t2_gather_kernel(unsigned long long NE, c
             if (ci < 0 || cj < 0 || ck < 0 || ci >= S.n[0] || cj >= S.n[1] || ck >= S.n[2]) continue;
             const unsigned long long t = S.tet0 + (unsigned long long)p * S.ncube + (unsigned long long)ci + ncx * cj + ncxy * ck;
             in[q] = true;
-            v0[q] = Y[(unsigned long long)la * g.NT + t];
-            v1[q] = Y[(unsigned long long)lb * g.NT + t];
+            const int sa = MODE == G_CHEB ? c2_massslot[la] : la, sb = MODE == G_CHEB ? c2_massslot[lb] : lb;
+            v0[q] = Y[(unsigned long long)sa * g.NT + t];
+            v1[q] = Y[(unsigned long long)sb * g.NT + t];
         }
 #pragma unroll
         for (int q = 0; q < kMaxInc; ++q)
@@ -669,22 +782,22 @@ __global__ void __launch_bounds__(128) t2_gather_kernel(unsigned long long NE, c
     const T z0 = fma(q00, r0, q01 * r1), z1 = fma(q01, r0, q11 * r1);
     T n0, n1, x0, x1;
     if (MODE == G_CHEB0) {
-        n0 = (T)g.c0 * z0; n1 = (T)g.c0 * z1;
+        n0 = g.c0 * z0; n1 = g.c0 * z1;
         x0 = n0; x1 = n1;
     } else {
-        n0 = fma((T)g.c1, g.d[d0], (T)g.c2 * z0);
-        n1 = fma((T)g.c1, g.d[d1], (T)g.c2 * z1);
+        n0 = fma(g.c1, g.d[d0], g.c2 * z0);
+        n1 = fma(g.c1, g.d[d1], g.c2 * z1);
         x0 = g.xin[d0] + n0; x1 = g.xin[d1] + n1;   // the two-pass iteration reads and writes the same buffer
     }
     g.d[d0] = n0; g.d[d1] = n1;
     g.x[d0] = x0; g.x[d1] = x1;
     if (FIN == FIN_DRIFT) {
-        g.U[d0] = fma((T)g.h, x0, g.U[d0]);
-        g.U[d1] = fma((T)g.h, x1, g.U[d1]);
+        g.U[d0] = fma(g.h, x0, g.U[d0]);
+        g.U[d1] = fma(g.h, x1, g.U[d1]);
     } else if (FIN == FIN_LEAP) {
         const T u0 = g.U[d0], u1 = g.U[d1];
-        g.U[d0] = fma(-(T)g.h, x0, T(2) * u0 - g.Uold[d0]);
-        g.U[d1] = fma(-(T)g.h, x1, T(2) * u1 - g.Uold[d1]);
+        g.U[d0] = fma(-g.h, x0, T(2) * u0 - g.Uold[d0]);
+        g.U[d1] = fma(-g.h, x1, T(2) * u1 - g.Uold[d1]);
         g.Uold[d0] = u0; g.Uold[d1] = u1;
     }
 }
@@ -771,25 +884,19 @@ constexpr IncTab make_inc_tab()
 constexpr IncTab kInc = make_inc_tab();
 static_assert(kInc.n[6] == 6 && kInc.n[7] == 2, "Kuhn split: the body diagonal lies in six tetrahedra, a face in two");
 
-// The two mass rows of entity type ET at node (i,j,k): sum over its
-// tetrahedra of eps_t (Mref_p x_t) at the entity's local DOFs, every table
-// entry a compile-time constant (the reference entries are constant-bank
-// operands, the DOF offsets plane * nnode + vertex offset).
-// r0 += Mref_p[LA][b] x_b, r1 += Mref_p[LB][b] x_b over b in order, the DOF
-// offset of b (plane * nnode + vertex offset) formed from compile-time parts
-template <class T, int P, int LA, int LB, int B>
-__device__ __forceinline__ void cheb_term(const T *__restrict__ xs, unsigned nn, unsigned nx1, unsigned nxy, T &r0, T &r1)
+// The two mass rows of entity type ET at node (i,j,k): the sum over its
+// tetrahedra of e M x at the entity's local DOFs, every table entry a
+// compile-time constant.
+template <class T, int P, int B> __device__ __forceinline__ T cheb_value(const T *__restrict__ xs, unsigned nn, unsigned nx1, unsigned nxy)
 {
     constexpr int PL = kInc.plane[P][B], VO = kInc.vo[P][B];
-    const T xb = xs[(unsigned)PL * nn + (VO & 1) + ((VO >> 1) & 1) * nx1 + ((VO >> 2) & 1) * nxy];
-    r0 = fma(mref<T>(P, LA, B), xb, r0);
-    r1 = fma(mref<T>(P, LB, B), xb, r1);
+    return xs[(unsigned)PL * nn + (VO & 1) + ((VO >> 1) & 1) * nx1 + ((VO >> 2) & 1) * nxy];
 }
-template <class T, int P, int LA, int LB, int... B>
-__device__ __forceinline__ void cheb_terms(std::integer_sequence<int, B...>, const T *__restrict__ xs, unsigned nn, unsigned nx1,
-                                           unsigned nxy, T &r0, T &r1)
+template <class T, int P, int... B>
+__device__ __forceinline__ void cheb_load(std::integer_sequence<int, B...>, const T *__restrict__ xs, unsigned nn, unsigned nx1, unsigned nxy,
+                                          T (&x)[20])
 {
-    (cheb_term<T, P, LA, LB, B>(xs, nn, nx1, nxy, r0, r1), ...);
+    ((x[B] = cheb_value<T, P, B>(xs, nn, nx1, nxy)), ...);
 }
 
 template <class T, int ET, int Q>
@@ -797,18 +904,16 @@ __device__ __forceinline__ void cheb_rows_inc(const T *__restrict__ xs, const T 
                                               unsigned ncube, unsigned nn, unsigned nx1, unsigned nxy, unsigned ncx, unsigned ncxy,
                                               const int (&n)[3], int i, int j, int k, T &y0, T &y1)
 {
-    constexpr int P = kInc.p[ET][Q], OB = kInc.ob[ET][Q], LA = kInc.la[ET][Q], LB = kInc.lb[ET][Q];
+    constexpr int P = kInc.p[ET][Q], OB = kInc.ob[ET][Q];
     const int ci = i - (OB & 1), cj = j - ((OB >> 1) & 1), ck = k - ((OB >> 2) & 1);
     if (ci < 0 || cj < 0 || ck < 0 || ci >= n[0] || cj >= n[1] || ck >= n[2]) return;
     const unsigned v0 = (unsigned)ci + nx1 * cj + nxy * ck;
-    T r0 = T(0), r1 = T(0);
-    cheb_terms<T, P, LA, LB>(std::make_integer_sequence<int, 20>{}, xs + v0, nn, nx1, nxy, r0, r1);
-    // the rounded product, then the rounded sum: the two-pass form stores
-    // e * r and sums the stored values in the same order, so both forms give
-    // the same bits
+    T x[20];
+    cheb_load<T, P>(std::make_integer_sequence<int, 20>{}, xs + v0, nn, nx1, nxy, x);
+    // the rounded product, then the rounded sum, as the marching kernel
     const T e = eps[tet0 + (unsigned long long)P * ncube + (unsigned)ci + ncx * cj + ncxy * ck];
-    y0 = add_rn(y0, mul_rn(e, r0));
-    y1 = add_rn(y1, mul_rn(e, r1));
+    y0 = add_rn(y0, mul_rn(e, mass_row<kInc.la[ET][Q]>(std::make_integer_sequence<int, 20>{}, x)));
+    y1 = add_rn(y1, mul_rn(e, mass_row<kInc.lb[ET][Q]>(std::make_integer_sequence<int, 20>{}, x)));
 }
 
 template <class T, int ET, int... Q>
@@ -878,18 +983,354 @@ __global__ void __launch_bounds__(128) t2_cheb_kernel(unsigned long long NE, con
     const T r0 = g.b[d0] - y0, r1 = g.b[d1] - y1;
     const T q00 = g.pinv[e], q01 = g.pinv[NE + e], q11 = g.pinv[2 * NE + e];
     const T z0 = fma(q00, r0, q01 * r1), z1 = fma(q01, r0, q11 * r1);
-    const T n0 = fma((T)g.c1, g.d[d0], (T)g.c2 * z0), n1 = fma((T)g.c1, g.d[d1], (T)g.c2 * z1);
+    const T n0 = fma(g.c1, g.d[d0], g.c2 * z0), n1 = fma(g.c1, g.d[d1], g.c2 * z1);
     const T x0 = g.xin[d0] + n0, x1 = g.xin[d1] + n1;
     g.d[d0] = n0; g.d[d1] = n1;
     g.x[d0] = x0; g.x[d1] = x1;
     if (FIN == FIN_DRIFT) {
-        g.U[d0] = fma((T)g.h, x0, g.U[d0]);
-        g.U[d1] = fma((T)g.h, x1, g.U[d1]);
+        g.U[d0] = fma(g.h, x0, g.U[d0]);
+        g.U[d1] = fma(g.h, x1, g.U[d1]);
     } else if (FIN == FIN_LEAP) {
         const T u0 = g.U[d0], u1 = g.U[d1];
-        g.U[d0] = fma(-(T)g.h, x0, T(2) * u0 - g.Uold[d0]);
-        g.U[d1] = fma(-(T)g.h, x1, T(2) * u1 - g.Uold[d1]);
+        g.U[d0] = fma(-g.h, x0, T(2) * u0 - g.Uold[d0]);
+        g.U[d1] = fma(-g.h, x1, T(2) * u1 - g.Uold[d1]);
         g.Uold[d0] = u0; g.Uold[d1] = u1;
+    }
+}
+
+// ------------------------------------------------- marching iteration
+// One block of the marching iteration: bx x by cube columns from (i0, j0),
+// node planes k0 .. k1 - 1 of one shot.
+struct T2Tile {
+    unsigned long long dof0, tet0, ent0;
+    int nx, ny, nz, i0, j0, k0, k1, bx, by, pad;
+};
+
+// Groups of the 38 planes in the staged iterate: the 10 whose entities do not
+// span z (a cube reads them in two layers) and the 28 that do.
+struct GroupTab {
+    int n[2], plane[2][28], grp[kPlanes], slot[kPlanes];
+};
+constexpr GroupTab make_group_tab()
+{
+    GroupTab T{};
+    for (int pl = 0; pl < kPlanes; ++pl) {
+        int ax = 0;
+        if (pl < 14) {
+            ax = kDir[pl % 7][2];
+        } else {
+            int t = 0;
+            for (int a = 1; a < 8; ++a)
+                for (int b = 1; b < 8; ++b) {
+                    if (a & b) continue;
+                    if (t++ == (pl - 14) / 2) ax = ((a | b) >> 2) & 1;
+                }
+        }
+        T.grp[pl] = ax;
+        T.slot[pl] = T.n[ax];
+        T.plane[ax][T.n[ax]++] = pl;
+    }
+    return T;
+}
+static_assert(make_group_tab().n[0] == 10 && make_group_tab().n[1] == 28, "10 planes without z, 28 with z");
+__constant__ int c2_grp[kPlanes];      // group << 8 | place in the group
+__constant__ int c2_gplane[10];        // the planes without z
+
+__device__ __forceinline__ void copy_async(float *dst, const float *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+
+// Arguments of the marching iteration.
+template <class T> struct MArgs {
+    const T *xin, *b, *pinv, *eps;
+    T *x, *d, *U, *Uold;
+    T c1, c2, h;
+    unsigned long long NE;
+};
+
+// One column's view of a layer for the update of its entities.
+template <class T> struct MarchCol {
+    const T *Y[4];            // the element values of the columns at 0, -x, -y, -x-y
+    const T *xa, *xb;         // the staged iterate of the layer (planes without and with z)
+    unsigned nn, v;           // nodes of the shot, this node
+    unsigned long long dof0, ent0;
+    int dead;                 // axes at whose near face the node lies
+};
+template <class T> struct MarchOps {
+    T b0, b1, d0, d1, q00, q01, q11;   // operands of an entity's update
+    T low[6];                          // its values from the layer below
+};
+constexpr int ent_axes(int et)
+{
+    if (et < 7) return kDir[et][0] | (kDir[et][1] << 1) | (kDir[et][2] << 2);
+    int t = 0;
+    for (int a = 1; a < 8; ++a)
+        for (int b = 1; b < 8; ++b) {
+            if (a & b) continue;
+            if (t++ == et - 7) return a | b;
+        }
+    return 0;
+}
+template <class T, int ET> __device__ __forceinline__ void march_prefetch(const MArgs<T> &g, const MarchCol<T> &c, MarchOps<T> &m)
+{
+    if (c.dead & ~ent_axes(ET)) return;
+    constexpr unsigned pl0 = ET < 7 ? ET : 2 * ET, pl1 = ET < 7 ? ET + 7 : pl0 + 1;
+    const unsigned o0 = pl0 * c.nn + c.v, o1 = pl1 * c.nn + c.v;
+    const T *pv = g.pinv + c.ent0 + (ET * c.nn + c.v);
+    m.b0 = (g.b + c.dof0)[o0]; m.b1 = (g.b + c.dof0)[o1];
+    m.d0 = (g.d + c.dof0)[o0]; m.d1 = (g.d + c.dof0)[o1];
+    m.q00 = pv[0]; m.q01 = pv[g.NE]; m.q11 = pv[2 * g.NE];
+}
+
+// The tetrahedra of entity ET in the layer below come from the registers that
+// the march keeps (low_at: the place of term Q among them).
+constexpr int low_at(int et, int q)
+{
+    int n = 0;
+    for (int r = 0; r < q; ++r) n += kInc.ob[et][r] >> 2;
+    return n;
+}
+static_assert(low_at(0, kInc.n[0]) == 3 && low_at(1, kInc.n[1]) == 3 && low_at(3, kInc.n[3]) <= 3, "at most three tetrahedra below");
+template <class T, int COLS, int ET, int Q> __device__ __forceinline__ void march_value(const MarchCol<T> &c, T &a, T &b)
+{
+    constexpr int ob = kInc.ob[ET][Q], ia = (kInc.p[ET][Q] * 20 + kInc.la[ET][Q]) * COLS, ib = (kInc.p[ET][Q] * 20 + kInc.lb[ET][Q]) * COLS;
+    a = c.Y[ob & 3][ia];
+    b = c.Y[ob & 3][ib];
+}
+template <class T, int COLS, int ET, int Q>
+__device__ __forceinline__ void march_term(const MarchCol<T> &c, const MarchOps<T> &m, T &y0, T &y1)
+{
+    T a, b;
+    if constexpr (kInc.ob[ET][Q] & 4) {
+        a = m.low[2 * low_at(ET, Q)];
+        b = m.low[2 * low_at(ET, Q) + 1];
+    } else {
+        march_value<T, COLS, ET, Q>(c, a, b);
+    }
+    y0 = add_rn(y0, a);
+    y1 = add_rn(y1, b);
+}
+template <class T, int COLS, int ET, int Q> __device__ __forceinline__ void march_keep(const MarchCol<T> &c, MarchOps<T> &m)
+{
+    if constexpr (kInc.ob[ET][Q] & 4) march_value<T, COLS, ET, Q>(c, m.low[2 * low_at(ET, Q)], m.low[2 * low_at(ET, Q) + 1]);
+}
+// The sum over the tetrahedra of the entity in ascending type, then the
+// values that its node one layer up will need.
+template <class T, int COLS, int ET, int... Q>
+__device__ __forceinline__ void march_sum(std::integer_sequence<int, Q...>, const MarchCol<T> &c, MarchOps<T> &m, T &y0, T &y1)
+{
+    (march_term<T, COLS, ET, Q>(c, m, y0, y1), ...);
+    (march_keep<T, COLS, ET, Q>(c, m), ...);
+}
+template <class T, int FIN, int COLS, int NC, int ET>
+__device__ __forceinline__ void march_update(const MArgs<T> &g, const MarchCol<T> &c, MarchOps<T> &m, bool store)
+{
+    constexpr int S = ent_axes(ET);
+    if (c.dead & ~S & 3) return;
+    T y0 = T(0), y1 = T(0);
+    march_sum<T, COLS, ET>(std::make_integer_sequence<int, kInc.n[ET]>{}, c, m, y0, y1);
+    if (!store || (c.dead & ~S)) return;
+    constexpr unsigned pl0 = ET < 7 ? ET : 2 * ET, pl1 = ET < 7 ? ET + 7 : pl0 + 1;
+    constexpr GroupTab gt = make_group_tab();
+    constexpr int s0 = gt.slot[pl0] * NC, s1 = gt.slot[pl1] * NC;
+    const T *xo = (S & 4) ? c.xb : c.xa;
+    const T r0 = m.b0 - y0, r1 = m.b1 - y1;
+    const T z0 = fma(m.q00, r0, m.q01 * r1), z1 = fma(m.q01, r0, m.q11 * r1);
+    const T e0 = fma(g.c1, m.d0, g.c2 * z0), e1 = fma(g.c1, m.d1, g.c2 * z1);
+    const T x0 = xo[s0] + e0, x1 = xo[s1] + e1;
+    const unsigned o0 = pl0 * c.nn + c.v, o1 = pl1 * c.nn + c.v;
+    (g.d + c.dof0)[o0] = e0; (g.d + c.dof0)[o1] = e1;
+    (g.x + c.dof0)[o0] = x0; (g.x + c.dof0)[o1] = x1;
+    if (FIN == FIN_DRIFT) {
+        T *U = g.U + c.dof0;
+        U[o0] = fma(g.h, x0, U[o0]);
+        U[o1] = fma(g.h, x1, U[o1]);
+    } else if (FIN == FIN_LEAP) {
+        T *U = g.U + c.dof0, *V = g.Uold + c.dof0;
+        const T u0 = U[o0], u1 = U[o1];
+        U[o0] = fma(-g.h, x0, T(2) * u0 - V[o0]);
+        U[o1] = fma(-g.h, x1, T(2) * u1 - V[o1]);
+        V[o0] = u0; V[o1] = u1;
+    }
+}
+// The entities of a warp: types P, P + 6, P + 12 and, for P = 0, 18.
+template <class T, int P> __device__ __forceinline__ void march_prefetch_all(const MArgs<T> &g, const MarchCol<T> &c, MarchOps<T> (&m)[4])
+{
+    march_prefetch<T, P>(g, c, m[0]);
+    march_prefetch<T, P + 6>(g, c, m[1]);
+    march_prefetch<T, P + 12>(g, c, m[2]);
+    if constexpr (P == 0) march_prefetch<T, 18>(g, c, m[3]);
+}
+template <class T, int FIN, int COLS, int NC, int P>
+__device__ __forceinline__ void march_update_all(const MArgs<T> &g, const MarchCol<T> &c, MarchOps<T> (&m)[4], bool store)
+{
+    march_update<T, FIN, COLS, NC, P>(g, c, m[0], store);
+    march_update<T, FIN, COLS, NC, P + 6>(g, c, m[1], store);
+    march_update<T, FIN, COLS, NC, P + 12>(g, c, m[2], store);
+    if constexpr (P == 0) march_update<T, FIN, COLS, NC, 18>(g, c, m[3], store);
+}
+
+template <class T, int COLS, int... A>
+__device__ __forceinline__ void march_rows(std::integer_sequence<int, A...>, const T (&x)[20], T e, T *yc)
+{
+    ((yc[A * COLS] = mul_rn(e, mass_row<A>(std::make_integer_sequence<int, 20>{}, x))), ...);
+}
+
+// The copy of one layer's planes by a warp: planes P, P + 6, ... of the list
+// (10 without z, of layer ka, then 28 with z, of layer kb).
+template <class T, int NC, int M>
+__device__ __forceinline__ void march_copy(const T *xa, const T *xb, T *da, T *db, unsigned nn, unsigned vin, unsigned ved, int cin, int ced,
+                                           bool inside, bool edge)
+{
+    if constexpr (M < 38) {
+        constexpr GroupTab gt = make_group_tab();
+        constexpr int gr = M < 10 ? 0 : 1, slot = M < 10 ? M : M - 10;
+        constexpr unsigned pl = gt.plane[gr][slot];
+        const T *src = (gr ? xb : xa) + pl * (unsigned long long)nn;
+        T *dst = (gr ? db : da) + slot * NC;
+        if (inside) copy_async(dst + cin, src + vin);
+        if (edge) copy_async(dst + ced, src + ved);
+    }
+}
+template <class T, int NC, int P, int... S, class... A>
+__device__ __forceinline__ void march_copies(std::integer_sequence<int, S...>, A... a)
+{
+    (march_copy<T, NC, P + 6 * S>(a...), ...);
+}
+
+// One Chebyshev iteration on tiles of cube columns marched up z.  Per layer
+// the iterate is staged by asynchronous copies one layer ahead, each warp
+// forms the element values of one tetrahedron type for 32 columns into
+// shared memory, and after a barrier each warp updates the entity types it
+// owns, whose operands were loaded before the element products; the sums of
+// entities without z pass to the next layer in registers.  So the iterate,
+// right-hand side, step and block inverses cross DRAM once and no
+// per-tetrahedron array exists.  Nodes on the far faces carry no live DOF, so
+// the columns of cubes are the columns of live nodes; a tile after the first
+// repeats a column along x and y, a chunk after the first the layer below.
+// Dead DOFs are not written: every iterate buffer keeps zeros there.  One
+// body of code serves the six types (the types' element masses are equal;
+// where the values lie comes from a table).  Bound by issue (2.3 of 4
+// instructions per clock, 24 warps per SM) and the two barriers per layer.
+// Per iteration on GB300, against the better of the two forms before it
+// (element pass and entity pass through a per-tetrahedron array; one thread
+// per edge or face): 48^3 cubes 44.7 us against 67, five shots of 12..40
+// cubes 63 against 100, thirteen shots of 22..40 cubes 227 against 345.
+template <class T, int FIN, int COLS, int NC>
+__global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *__restrict__ tiles, MArgs<T> g)
+{
+    constexpr int NT = 6 * COLS, G = COLS / 32;   // a warp: one tetrahedron type of 32 columns
+    extern __shared__ __align__(16) unsigned char t2_sm[];
+    T *sa = reinterpret_cast<T *>(t2_sm);   // [3][10][NC]: layers k, k + 1 and the one on its way
+    T *sb = sa + 30 * NC;                   // [2][28][NC]: layer k and the one on its way
+    T *Y = sb + 56 * NC;                    // [6][20][COLS]: e M x of the layer's tetrahedra
+    int *xoff = reinterpret_cast<int *>(Y + 120 * COLS);   // [6 layers][6 types][20]: byte offsets of a tetrahedron's staged values
+    const T2Tile t = tiles[blockIdx.x];
+    const int tid = threadIdx.x, warp = tid >> 5, p = warp / G, col = (warp - p * G) * 32 + (tid & 31);
+    const int rw = t.bx + 1;
+    for (int n = tid; n < 720; n += NT) {
+        const int ph = n / 120, q = n % 20, d = c2_dof[(n / 20) % 6][q], pl = d & 255, o = d >> 8;
+        const int gr = c2_grp[pl], at = (gr & 255) * NC + (o & 1) + ((o >> 1) & 1) * rw;
+        xoff[n] = (int)sizeof(T) * ((gr >> 8) ? 30 * NC + (ph & 1) * (28 * NC) + at : ((ph + (o >> 2)) % 3) * (10 * NC) + at);
+    }
+    const int ty = col / t.bx, tx = col - ty * t.bx;
+    const int i = t.i0 + tx, j = t.j0 + ty;
+    const bool active = ty < t.by && i < t.nx && j < t.ny;
+    const bool own = active && (tx > 0 || t.i0 == 0) && (ty > 0 || t.j0 == 0);
+    const unsigned nx1 = t.nx + 1, nxy = nx1 * (t.ny + 1);
+    MarchCol<T> c;
+    c.nn = nxy * (t.nz + 1);
+    c.dof0 = t.dof0;
+    c.ent0 = t.ent0;
+    c.dead = (i == 0 ? 1 : 0) | (j == 0 ? 2 : 0);
+    c.Y[0] = Y + col; c.Y[1] = Y + col - 1; c.Y[2] = Y + col - t.bx; c.Y[3] = Y + col - t.bx - 1;
+    const int mycol = ty * rw + tx;   // this column in the staged tile
+    // the copy of a layer: each warp takes every sixth plane of its column
+    // group, and of the columns beyond the last row and column
+    const T *xs = g.xin + t.dof0;
+    const bool inside = ty < t.by && i <= t.nx && j <= t.ny;
+    const int ex0 = col < t.by ? t.bx : col - t.by, ey0 = col < t.by ? col : t.by;
+    const bool edge_in = col <= t.bx + t.by && t.i0 + ex0 <= t.nx && t.j0 + ey0 <= t.ny;
+    const int ecol = ey0 * rw + ex0;
+    const unsigned vcol = (unsigned)i + nx1 * j, vedge = (unsigned)(t.i0 + ex0) + nx1 * (t.j0 + ey0);
+    auto fetch = [&](int ka, int kz) {
+        const T *xa = xs + (unsigned long long)nxy * ka, *xb = xs + (unsigned long long)nxy * kz;
+        T *da = sa + (ka % 3) * (10 * NC), *db = sb + (kz & 1) * (28 * NC);
+        auto go = [&](auto w) {
+            march_copies<T, NC, decltype(w)::value>(std::make_integer_sequence<int, 7>{}, xa, xb, da, db, c.nn, vcol, vedge, mycol, ecol,
+                                                    inside, edge_in);
+        };
+        switch (p) {
+        case 0: go(std::integral_constant<int, 0>{}); break;
+        case 1: go(std::integral_constant<int, 1>{}); break;
+        case 2: go(std::integral_constant<int, 2>{}); break;
+        case 3: go(std::integral_constant<int, 3>{}); break;
+        case 4: go(std::integral_constant<int, 4>{}); break;
+        default: go(std::integral_constant<int, 5>{}); break;
+        }
+    };
+    const int kb = t.k0 > 0 ? t.k0 - 1 : 0;
+    for (int q = p; q < 10; q += 6) {   // the first layer's planes without z
+        const T *src = xs + ((unsigned)c2_gplane[q] * c.nn + nxy * kb);
+        T *d = sa + (kb % 3) * (10 * NC) + q * NC;
+        if (inside) copy_async(d + mycol, src + vcol);
+        if (edge_in) copy_async(d + ecol, src + vedge);
+    }
+    fetch(kb + 1, kb);
+    MarchOps<T> m[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int q = 0; q < 6; ++q) m[r].low[q] = T(0);
+    const T *ep = g.eps + t.tet0 + (unsigned)p * ((unsigned)t.nx * t.ny * t.nz) + (unsigned)i + t.nx * j;
+    for (int k = kb; k < t.k1; ++k) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();   // layer k has arrived, and layer k - 1's buffers are free
+        if (k + 1 < t.k1) fetch(k + 2, k + 1);
+        // the operands of this layer's updates, on their way during the element products
+        c.v = vcol + nxy * k;
+        c.dead = (c.dead & 3) | (k == 0 ? 4 : 0);
+        const bool store = own && k >= t.k0;
+        if (store) {
+            switch (p) {
+            case 0: march_prefetch_all<T, 0>(g, c, m); break;
+            case 1: march_prefetch_all<T, 1>(g, c, m); break;
+            case 2: march_prefetch_all<T, 2>(g, c, m); break;
+            case 3: march_prefetch_all<T, 3>(g, c, m); break;
+            case 4: march_prefetch_all<T, 4>(g, c, m); break;
+            default: march_prefetch_all<T, 5>(g, c, m); break;
+            }
+        }
+        if (active) {
+            const T e = ep[(unsigned)t.nx * t.ny * k];
+            const int4 *xo = reinterpret_cast<const int4 *>(xoff + (k % 6) * 120 + p * 20);
+            const char *xc = reinterpret_cast<const char *>(sa + mycol);
+            int o[20];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                const int4 w = xo[q];
+                o[4 * q] = w.x; o[4 * q + 1] = w.y; o[4 * q + 2] = w.z; o[4 * q + 3] = w.w;
+            }
+            T x[20];
+#pragma unroll
+            for (int q = 0; q < 20; ++q) x[q] = *reinterpret_cast<const T *>(xc + o[q]);
+            T *yc = Y + p * (20 * COLS) + col;
+            march_rows<T, COLS>(std::make_integer_sequence<int, 20>{}, x, e, yc);
+        }
+        __syncthreads();
+        if (own) {
+            c.xa = sa + (k % 3) * (10 * NC) + mycol;
+            c.xb = sb + (k & 1) * (28 * NC) + mycol;
+            switch (p) {
+            case 0: march_update_all<T, FIN, COLS, NC, 0>(g, c, m, store); break;
+            case 1: march_update_all<T, FIN, COLS, NC, 1>(g, c, m, store); break;
+            case 2: march_update_all<T, FIN, COLS, NC, 2>(g, c, m, store); break;
+            case 3: march_update_all<T, FIN, COLS, NC, 3>(g, c, m, store); break;
+            case 4: march_update_all<T, FIN, COLS, NC, 4>(g, c, m, store); break;
+            default: march_update_all<T, FIN, COLS, NC, 5>(g, c, m, store); break;
+            }
+        }
     }
 }
 
@@ -1116,7 +1557,7 @@ struct Tet2Sim : Sim {
         d_U.alloc(ndof * w); d_Uold.alloc(ndof * w); d_P.alloc(ndof * 8);
         d_x.alloc(ndof * w); d_xs.alloc(ndof * w); d_d.alloc(ndof * w); d_b.alloc(ndof * w);
         if (!fp64) d_Pc.alloc(ndof * 4);
-        d_YtM.alloc(20 * ntet * w);
+        if (fp64) d_YtM.alloc(20 * ntet * w);
         d_YtK.alloc(20 * ntet * 8);
         d_ctl.alloc(16);
         d_part.alloc(kDotBlocks * 8);
@@ -1142,6 +1583,24 @@ struct Tet2Sim : Sim {
                 if (kInc.plane[p][a] != R.plane[p][a] || kInc.vo[p][a] != bits(k.vert[R.low[p][a]]))
                     throw Error{EMS_ERR_CUDA, "compile-time DOF table differs from the setup's"};
         }
+        // the compile-time element mass against the setup's (all types), and its
+        // symmetry under the vertex reversal
+        const MateTab mt = make_mate_tab();
+        int mslot[20], grp[kPlanes];
+        for (int a = 0; a < 20; ++a) mslot[a] = mass_slot(a);
+        for (int p = 0; p < 6; ++p)
+            for (int a = 0; a < 20; ++a)
+                for (int b = 0; b < 20; ++b) {
+                    const double m = kMass.m[20 * a + b];
+                    if (std::fabs(R.M[p][20 * a + b] - m) > 1e-15 || std::fabs(m - kMass.m[20 * mt.mate[a] + mt.mate[b]]) > 1e-15)
+                        throw Error{EMS_ERR_CUDA, "compile-time element mass differs from the setup's"};
+                }
+        EMS_CUDA(cudaMemcpyToSymbol(c2_H64, kMass.h, sizeof(kMass.h)));
+        EMS_CUDA(cudaMemcpyToSymbol(c2_massslot, mslot, sizeof(mslot)));
+        const GroupTab gt = make_group_tab();
+        for (int q = 0; q < kPlanes; ++q) grp[q] = gt.grp[q] << 8 | gt.slot[q];
+        EMS_CUDA(cudaMemcpyToSymbol(c2_grp, grp, sizeof(grp)));
+        EMS_CUDA(cudaMemcpyToSymbol(c2_gplane, gt.plane[0], sizeof(int) * 10));
         int dof[6][20];
         float m32[6][400];
         for (int p = 0; p < 6; ++p) {
@@ -1268,29 +1727,105 @@ struct Tet2Sim : Sim {
 
     // x = q(M) b; the last iteration applies FIN with factor h (to U, or to
     // `target` when given); the iterate ends in `xo` (default: the solver's
-    // x).  Two forms of an iteration, chosen per handle by timing
-    // (choose_iteration): fused, one entity pass that forms the mass rows
-    // from the previous iterate and writes the next one to the other of two
-    // buffers (the iterates alternate, starting where the last lands in
-    // xo); or two-pass, the mass element pass into the per-tetrahedron
-    // array, then the entity pass updating x in place.
-    // 0: two-pass, 1: fused (one thread per edge or face).  A third form,
-    // one thread per node forming all 38 rows from its 18 tetrahedra (each
-    // tetrahedron's iterate loaded once, 118 registers), measured 77 us
-    // against 68 us (fused) at 48^3 and 30 against 9 us at 16^3; not kept.
-    int cheb_form = 0;
-    template <class T, int FIN> void launch_fused_iteration(const GArgs<T> &g)
+    // x).  FP64: element pass and entity pass, the iterate updated in place.
+    // FP32: one launch per iteration, the iterates alternating between two
+    // buffers (starting where the last lands in xo): tiles marched up z, or
+    // on small meshes one thread per edge or face, chosen per handle by
+    // timing (choose_iteration).  All forms give the same bits.
+    enum { FORM_TWOPASS, FORM_FUSED, FORM_MARCH };
+    int cheb_form = FORM_TWOPASS;
+    // Tiles of the marching iteration: per shot the width bx (by = COLS / bx)
+    // that covers its columns with the fewest tiles, and one chunk length
+    // for all shots: the one whose waves of blocks (one per SM) times layers
+    // (the chunk, the repeated layer and about one more of start-up) is least.
+    static constexpr int kCols = 128, kStage = 168;
+    static constexpr size_t kMarchSmem = sizeof(float) * (86 * kStage + 120 * kCols) + sizeof(int) * 720;
+    DevBuf d_tiles;
+    unsigned ntiles = 0;
+    void build_tiles()
     {
-        t2_cheb_kernel<T, FIN><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), (int)shots.size(), g);
+        if (ntiles) return;
+        int dev = 0, nsm = 1;
+        EMS_CUDA(cudaGetDevice(&dev));
+        EMS_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        // tiles of b columns that cover n, each after the first repeating one
+        auto count = [](long n, long b) { return b >= n ? 1 : b < 2 ? n * n + n : 1 + (n - 2) / (b - 1); };
+        struct Plan {
+            int bx, by;
+            long tx, ty;
+        };
+        std::vector<Plan> plan;
+        int nzmax = 1;
+        for (const ShotH &S : shots) {
+            Plan best{0, 0, 0, 0};
+            for (int bx = 1; bx <= std::min(S.n[0], kCols); ++bx) {
+                int by = std::min(kCols / bx, S.n[1]);
+                while (by > 1 && (bx + 1) * (by + 1) > kStage) --by;
+                if ((bx + 1) * (by + 1) > kStage) break;
+                const long tx = count(S.n[0], bx), ty = count(S.n[1], by);
+                if (!best.bx || tx * ty <= best.tx * best.ty) best = {bx, by, tx, ty};
+            }
+            plan.push_back(best);
+            nzmax = std::max(nzmax, S.n[2]);
+        }
+        long bestc = -1;
+        int L = 1;
+        for (int l = 1; l <= nzmax; ++l) {
+            long nb = 0;
+            for (size_t s = 0; s < shots.size(); ++s) nb += plan[s].tx * plan[s].ty * ((shots[s].n[2] + l - 1) / l);
+            const long cost = ((nb + nsm - 1) / nsm) * (l + 2);
+            if (bestc < 0 || cost < bestc) { bestc = cost; L = l; }
+        }
+        std::vector<T2Tile> tiles;
+        for (size_t s = 0; s < shots.size(); ++s) {
+            const ShotH &S = shots[s];
+            const int nch = (S.n[2] + L - 1) / L;
+            for (int c = 0; c < nch; ++c)
+                for (int y = 0; y < plan[s].ty; ++y)
+                    for (int x = 0; x < plan[s].tx; ++x) {
+                        T2Tile t{};
+                        t.dof0 = S.dof0; t.tet0 = S.tet0; t.ent0 = S.ent0;
+                        t.nx = S.n[0]; t.ny = S.n[1]; t.nz = S.n[2];
+                        t.bx = plan[s].bx; t.by = plan[s].by;
+                        t.i0 = x * (t.bx - 1); t.j0 = y * (t.by - 1);
+                        t.k0 = (int)((long)S.n[2] * c / nch); t.k1 = (int)((long)S.n[2] * (c + 1) / nch);
+                        tiles.push_back(t);
+                    }
+        }
+        d_tiles.ensure(tiles.size() * sizeof(T2Tile));
+        EMS_CUDA(cudaMemcpy(d_tiles.p, tiles.data(), tiles.size() * sizeof(T2Tile), cudaMemcpyHostToDevice));
+        auto wide = [](auto k) { EMS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMarchSmem)); };
+        wide(t2_march_kernel<float, FIN_NONE, kCols, kStage>);
+        wide(t2_march_kernel<float, FIN_DRIFT, kCols, kStage>);
+        wide(t2_march_kernel<float, FIN_LEAP, kCols, kStage>);
+        ntiles = (unsigned)tiles.size();
+    }
+    // One iteration from g.xin to g.x; the number of launches.
+    template <class T, int FIN> int launch_iteration(const GArgs<T> &g)
+    {
+        const int ns = (int)shots.size();
+        if constexpr (sizeof(T) == 4) {
+            if (cheb_form == FORM_MARCH) {
+                const MArgs<T> a{g.xin, g.b, g.pinv, g.eps, g.x, g.d, g.U, g.Uold, g.c1, g.c2, g.h, nent};
+                t2_march_kernel<T, FIN, kCols, kStage><<<ntiles, 6 * kCols, kMarchSmem, stream>>>(d_tiles.as<T2Tile>(), a);
+            } else {
+                t2_cheb_kernel<T, FIN><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+            }
+            return 1;
+        } else {
+            t2_mass_elem_kernel<<<blocks(ntet, 64), 64, 0, stream>>>(ntet, d_shots.as<T2Shot>(), ns, d_eps.as<T>(), g.xin, d_YtM.as<T>());
+            t2_gather_kernel<T, T, G_CHEB, FIN><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+            return 2;
+        }
     }
     template <class T, int FIN> int enqueue_solve(const T *b, double h, T *xo = nullptr, T *target = nullptr)
     {
         const int ns = (int)shots.size();
-        const bool fused = cheb_form != 0;
+        const bool fused = cheb_form != FORM_TWOPASS;   // two buffers
         GArgs<T> g = gargs<T>();
         g.b = b;
-        g.c0 = cheb_c0;
-        g.h = h;
+        g.c0 = (T)cheb_c0;
+        g.h = (T)h;
         g.eps = d_eps.as<T>();
         g.Yt = d_YtM.p;
         if (!xo) xo = d_x.as<T>();
@@ -1308,20 +1843,9 @@ struct Tet2Sim : Sim {
             g.xin = buf[cur];
             cur ^= fused ? 1 : 0;
             g.x = buf[cur];
-            g.c1 = cheb_c1[k];
-            g.c2 = cheb_c2[k];
-            const bool last = k + 1 == mass_iters;
-            if (fused) {
-                if (last) launch_fused_iteration<T, FIN>(g);
-                else launch_fused_iteration<T, FIN_NONE>(g);
-                ++nl;
-            } else {
-                t2_mass_elem_kernel<T><<<blocks(ntet, 128), 128, 0, stream>>>(ntet, d_shots.as<T2Shot>(), ns, d_eps.as<T>(), g.xin,
-                                                                              d_YtM.as<T>());
-                if (last) t2_gather_kernel<T, T, G_CHEB, FIN><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
-                else t2_gather_kernel<T, T, G_CHEB, FIN_NONE><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
-                nl += 2;
-            }
+            g.c1 = (T)cheb_c1[k];
+            g.c2 = (T)cheb_c2[k];
+            nl += k + 1 == mass_iters ? launch_iteration<T, FIN>(g) : launch_iteration<T, FIN_NONE>(g);
         }
         return nl;
     }
@@ -1330,26 +1854,19 @@ struct Tet2Sim : Sim {
     // b are scratch here); ms per iteration.
     template <class T> double time_iterations(int n)
     {
-        const int ns = (int)shots.size();
         GArgs<T> g = gargs<T>();
         g.b = d_b.as<T>();
         g.eps = d_eps.as<T>();
         g.Yt = d_YtM.p;
-        g.c1 = 0.5; g.c2 = 0.1;
-        T *buf[2] = {d_x.as<T>(), cheb_form ? d_xs.as<T>() : d_x.as<T>()};
+        g.c1 = T(0.5); g.c2 = T(0.1);
+        T *buf[2] = {d_x.as<T>(), cheb_form != FORM_TWOPASS ? d_xs.as<T>() : d_x.as<T>()};
         cudaGraph_t gr = nullptr;
         cudaGraphExec_t ex = nullptr;
         EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         for (int k = 0; k < n; ++k) {
             g.xin = buf[k & 1];
             g.x = buf[(k + 1) & 1];
-            if (cheb_form) {
-                launch_fused_iteration<T, FIN_NONE>(g);
-            } else {
-                t2_mass_elem_kernel<T><<<blocks(ntet, 128), 128, 0, stream>>>(ntet, d_shots.as<T2Shot>(), ns, d_eps.as<T>(), g.xin,
-                                                                              d_YtM.as<T>());
-                t2_gather_kernel<T, T, G_CHEB, FIN_NONE><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
-            }
+            launch_iteration<T, FIN_NONE>(g);
         }
         cudaError_t ce = cudaStreamEndCapture(stream, &gr);
         if (ce != cudaSuccess) throw Error{EMS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce)};
@@ -1373,27 +1890,34 @@ struct Tet2Sim : Sim {
         return best / n;
     }
 
-    // The faster form of the Chebyshev iteration on this handle's meshes
-    // (EMS_TET2_ITERATION=twopass|fused forces one; EMS_TET2_TUNE_LOG prints
-    // the times); the forms give the same bits, so the choice changes no result.
+    // FP32: the faster form of the Chebyshev iteration on this handle's meshes
+    // (EMS_TET2_ITERATION=fused|march forces one; EMS_TET2_TUNE_LOG prints
+    // the times); the forms give the same bits, so the choice changes no
+    // result.  12x13x9 cubes: fused 5.9 us, march 11.7; 24x22x23: 13.3 and 12.0;
+    // 48^3: 70 and 44.7.  FP64 keeps two passes: the FP64 pipe bounds every form,
+    // and a tile's repeated columns and layers would add to its work.
     template <class T> void choose_iteration()
     {
-        static const char *names[2] = {"twopass", "fused"};
+        cheb_form = FORM_TWOPASS;
+        if (sizeof(T) == 8) return;
+        build_tiles();
+        static const char *names[3] = {"twopass", "fused", "march"};
         if (const char *force = std::getenv("EMS_TET2_ITERATION"))
-            for (int f = 0; f < 2; ++f)
+            for (int f = FORM_FUSED; f <= FORM_MARCH; ++f)
                 if (!std::strcmp(force, names[f])) { cheb_form = f; return; }
         d_x.zero(stream); d_xs.zero(stream); d_d.zero(stream); d_b.zero(stream);
-        int best = 0;
-        for (int f = 0; f < 2; ++f) {
+        int best = FORM_FUSED;
+        for (int f = FORM_FUSED; f <= FORM_MARCH; ++f) {
             cheb_form = f;
             iter_ms[f] = time_iterations<T>(8);
             if (iter_ms[f] < iter_ms[best]) best = f;
         }
         cheb_form = best;
         if (std::getenv("EMS_TET2_TUNE_LOG"))   // diagnostic: the forms' times per iteration
-            std::fprintf(stderr, "tet2 iteration (us): twopass %.2f fused %.2f\n", 1e3 * iter_ms[0], 1e3 * iter_ms[1]);
+            std::fprintf(stderr, "tet2 iteration (us): fused %.2f march %.2f (%u blocks)\n", 1e3 * iter_ms[FORM_FUSED],
+                         1e3 * iter_ms[FORM_MARCH], ntiles);
     }
-    double iter_ms[2] = {0.0, 0.0};
+    double iter_ms[3] = {0.0, 0.0, 0.0};
 
     double dot_host(const void *x, const void *y)
     {
@@ -1423,6 +1947,7 @@ struct Tet2Sim : Sim {
         EMS_CUDA(cudaMemcpy(d_x.p, x0.data(), ndof * sizeof(T), cudaMemcpyHostToDevice));
         T *x = d_x.as<T>(), *pb = d_b.as<T>(), *z = d_Uold.as<T>();
         enqueue_force<T>(x, pb);                    // p = K x0
+        d_x.zero(stream);                           // the iterates hold zeros at dead DOFs
         enqueue_solve<T, FIN_NONE>(pb, 0.0);        // x = q(M) p
         double lam = 0.0;
         for (int it = 0; it < iters; ++it) {
@@ -1825,7 +2350,7 @@ struct Tet2Sim : Sim {
         *ms = fp64 ? time_iterations<double>(std::max(launches, 1)) : time_iterations<float>(std::max(launches, 1));
         *bytes = (double)(fp64 ? 8 : 4) * (5.0 * ndof + ntet + 3.0 * nent);
         y_valid = false;
-        static const char *kern[2] = {"t2_mass_elem_kernel + t2_gather_kernel<", "t2_cheb_kernel<"};
+        static const char *kern[3] = {"t2_mass_elem_kernel + t2_gather_kernel<", "t2_cheb_kernel<", "t2_march_kernel<"};
         *name = std::string(kern[cheb_form]) + (fp64 ? "double>" : "float>");
     }
 
@@ -1971,6 +2496,7 @@ template <class T> void Tet2Sim::backward_t(const double *tg, double *grad)
     EMS_CUDA(cudaMemcpyAsync(keepU.p, d_U.p, w, cudaMemcpyDeviceToDevice, stream));
     EMS_CUDA(cudaMemcpyAsync(keepP.p, d_P.p, ndof * 8, cudaMemcpyDeviceToDevice, stream));
     Ub.zero(stream); Pb.zero(stream); gd.zero(stream);
+    Ys.zero(stream);   // the marching iteration leaves dead DOFs alone
     if (Ubc.p) Ubc.zero(stream);
     T *Ubr = fp64 ? Ub.as<T>() : Ubc.as<T>();   // Ubar in the run precision (right-hand side of the solves)
     int nseg0 = 0;   // first step of the segment being reversed
