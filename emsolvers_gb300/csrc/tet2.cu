@@ -361,8 +361,6 @@ const Ref &ref()
 __constant__ int c2_dof[6][20];          // plane | vertex offset bits << 8
 __constant__ double c2_M64[6][400];
 __constant__ float c2_M32[6][400];
-__constant__ double c2_C[6][20][12];
-__constant__ float c2_C32[6][20][12];   // the same, exact in FP32 (dyadic)
 __constant__ int c2_ninc[kEnt], c2_inc[kEnt][kMaxInc], c2_axes[kEnt];
 __constant__ int c2_massslot[20];       // local function -> place in the mass element values (mass_slot)
 
@@ -395,144 +393,30 @@ __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(
 
 // DOF addressing of flat tetrahedron tl of a shot: DOF a is
 // dof0 + plane * nnode + v0 + the vertex offset of its lowest vertex
+// (offsets within a shot fit 32 bits)
 struct TetAddr {
     int p;
-    unsigned long long v0, nx1, nxy, nnode, dof0;
+    unsigned v0, nx1, nxy, nnode;
+    unsigned long long dof0;
     __device__ __forceinline__ unsigned long long dof(int a) const
     {
         const int d = c2_dof[p][a], ob = d >> 8;
-        return dof0 + (unsigned long long)(d & 255) * nnode + v0 + (ob & 1) + ((ob >> 1) & 1) * nx1 + ((ob >> 2) & 1) * nxy;
+        return dof0 + ((unsigned)(d & 255) * nnode + v0 + (ob & 1) + ((ob >> 1) & 1) * nx1 + ((ob >> 2) & 1) * nxy);
     }
 };
 __device__ __forceinline__ TetAddr tet_addr(const T2Shot &S, unsigned long long tl)
 {
     TetAddr ta;
-    ta.p = (int)(tl / S.ncube);
-    const unsigned long long cube = tl - (unsigned long long)ta.p * S.ncube;
-    const unsigned long long i = cube % S.n[0], r = cube / S.n[0];
-    const unsigned long long j = r % S.n[1], k = r / S.n[1];
+    const unsigned t32 = (unsigned)tl, nc = (unsigned)S.ncube, nx = S.n[0], ny = S.n[1];
+    ta.p = (int)(t32 / nc);
+    const unsigned cube = t32 - (unsigned)ta.p * nc;
+    const unsigned r = cube / nx, i = cube - r * nx, k = r / ny, j = r - k * ny;
     ta.nx1 = S.n[0] + 1;
     ta.nxy = ta.nx1 * (S.n[1] + 1);
     ta.v0 = i + ta.nx1 * j + ta.nxy * k;
-    ta.nnode = S.nnode;
+    ta.nnode = (unsigned)S.nnode;
     ta.dof0 = S.dof0;
     return ta;
-}
-
-// Stiffness element pass in FP64: vertex curls c_v = sum_a U_a C_av, the P1
-// mass h_v = (c_v + sum_w c_w) / 120, Yt[a][t] = sum_v C_av . h_v.
-template <class TI>
-__global__ void __launch_bounds__(128) t2_stiff_elem_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
-                                                           const TI *__restrict__ U, double *__restrict__ Yt)
-{
-    const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-    if (t >= NT) return;
-    const T2Shot S = sh[shot_of(sh, ns, t, 0)];
-    const TetAddr ta = tet_addr(S, t - S.tet0);
-    const int p = ta.p;
-    double c[12];
-#pragma unroll
-    for (int q = 0; q < 12; ++q) c[q] = 0.0;
-#pragma unroll 2
-    for (int a = 0; a < 20; ++a) {
-        const double u = (double)U[ta.dof(a)];
-#pragma unroll
-        for (int q = 0; q < 12; ++q) c[q] = fma(c2_C[p][a][q], u, c[q]);
-    }
-    double h[12];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        const double s = c[q] + c[3 + q] + c[6 + q] + c[9 + q];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) h[3 * v + q] = (c[3 * v + q] + s) * (1.0 / 120.0);
-    }
-#pragma unroll 2
-    for (int a = 0; a < 20; ++a) {
-        double f = 0.0;
-#pragma unroll
-        for (int q = 0; q < 12; ++q) f = fma(c2_C[p][a][q], h[q], f);
-        Yt[(unsigned long long)a * NT + t] = f;
-    }
-}
-
-// Stiffness element pass of FP32 runs in double-float arithmetic: the same
-// vertex curls, P1 mass and transposed curl, each sum a compensated dot
-// product (Ogita, Rump and Oishi 2005, Dot2: products split exactly by FMA,
-// sums by two-sum, the errors accumulated alongside), so the element values
-// carry about twice the FP32 precision at FP32 throughput.  The curl
-// coefficients are dyadic (exact in FP32); zero coefficients are skipped
-// (the type p is uniform across a warp).
-__device__ __forceinline__ void dot2_add(float a, float b, float &s, float &c)
-{
-    const float p = __fmul_rn(a, b);
-    const float ep = fmaf(a, b, -p);
-    const float t = __fadd_rn(s, p);
-    const float bb = __fsub_rn(t, s);
-    const float es = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(p, bb));
-    s = t;
-    c = __fadd_rn(c, __fadd_rn(ep, es));
-}
-
-template <int P> __device__ __forceinline__ void stiff_df_body(const TetAddr &ta, unsigned long long NT, unsigned long long t,
-                                                               const float *__restrict__ U, double *__restrict__ Yt)
-{
-    float cs[12], cc[12];
-#pragma unroll
-    for (int q = 0; q < 12; ++q) { cs[q] = 0.0f; cc[q] = 0.0f; }
-#pragma unroll
-    for (int a = 0; a < 20; ++a) {
-        const float u = U[ta.dof(a)];
-#pragma unroll
-        for (int q = 0; q < 12; ++q) {
-            const float co = c2_C32[P][a][q];
-            if (co != 0.0f) dot2_add(co, u, cs[q], cc[q]);
-        }
-    }
-    // P1 mass in FP64 (12 values), split again into hi + lo
-    double c[12];
-#pragma unroll
-    for (int q = 0; q < 12; ++q) c[q] = (double)cs[q] + (double)cc[q];
-    float hh[12], hl[12];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        const double sm = c[q] + c[3 + q] + c[6 + q] + c[9 + q];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const double h = (c[3 * v + q] + sm) * (1.0 / 120.0);
-            hh[3 * v + q] = (float)h;
-            hl[3 * v + q] = (float)(h - (double)hh[3 * v + q]);
-        }
-    }
-#pragma unroll
-    for (int a = 0; a < 20; ++a) {
-        float fs = 0.0f, fc = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 12; ++q) {
-            const float co = c2_C32[P][a][q];
-            if (co != 0.0f) {
-                dot2_add(co, hh[q], fs, fc);
-                fc = fmaf(co, hl[q], fc);
-            }
-        }
-        Yt[(unsigned long long)a * NT + t] = (double)fs + (double)fc;
-    }
-}
-
-__global__ void __launch_bounds__(128, 5) t2_stiff_df_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
-                                                         const float *__restrict__ U, double *__restrict__ Yt)
-{
-    const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-    if (t >= NT) return;
-    const T2Shot S = sh[shot_of(sh, ns, t, 0)];
-    const TetAddr ta = tet_addr(S, t - S.tet0);
-    switch (ta.p) {
-    case 0: stiff_df_body<0>(ta, NT, t, U, Yt); break;
-    case 1: stiff_df_body<1>(ta, NT, t, U, Yt); break;
-    case 2: stiff_df_body<2>(ta, NT, t, U, Yt); break;
-    case 3: stiff_df_body<3>(ta, NT, t, U, Yt); break;
-    case 4: stiff_df_body<4>(ta, NT, t, U, Yt); break;
-    default: stiff_df_body<5>(ta, NT, t, U, Yt); break;
-    }
 }
 
 // ------------------------------------------------------- element mass
@@ -712,11 +596,11 @@ __global__ void __launch_bounds__(128) t2_gather_kernel(unsigned long long NE, c
     const unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (e >= NE) return;
     const T2Shot S = sh[shot_of(sh, ns, e, 1)];
-    const unsigned long long el = e - S.ent0;
-    const int et = (int)(el / S.nnode);
-    const unsigned long long v = el - (unsigned long long)et * S.nnode;
-    const int nx1 = S.n[0] + 1, ny1 = S.n[1] + 1;
-    const int i = (int)(v % nx1), j = (int)((v / nx1) % ny1), k = (int)(v / ((unsigned long long)nx1 * ny1));
+    const unsigned nn = (unsigned)S.nnode, el = (unsigned)(e - S.ent0);
+    const int et = (int)(el / nn);
+    const unsigned v = el - (unsigned)et * nn;
+    const unsigned nx1 = S.n[0] + 1, ny1 = S.n[1] + 1, vr = v / nx1;
+    const int i = (int)(v - vr * nx1), k = (int)(vr / ny1), j = (int)(vr - (unsigned)k * ny1);
     const int x3[3] = {i, j, k};
     const int ax = c2_axes[et];
     bool dead = false;
@@ -884,9 +768,7 @@ constexpr IncTab make_inc_tab()
 constexpr IncTab kInc = make_inc_tab();
 static_assert(kInc.n[6] == 6 && kInc.n[7] == 2, "Kuhn split: the body diagonal lies in six tetrahedra, a face in two");
 
-// The two mass rows of entity type ET at node (i,j,k): the sum over its
-// tetrahedra of e M x at the entity's local DOFs, every table entry a
-// compile-time constant.
+// The 20 values of tetrahedron type P of the cube at xs.
 template <class T, int P, int B> __device__ __forceinline__ T cheb_value(const T *__restrict__ xs, unsigned nn, unsigned nx1, unsigned nxy)
 {
     constexpr int PL = kInc.plane[P][B], VO = kInc.vo[P][B];
@@ -899,6 +781,207 @@ __device__ __forceinline__ void cheb_load(std::integer_sequence<int, B...>, cons
     ((x[B] = cheb_value<T, P, B>(xs, nn, nx1, nxy)), ...);
 }
 
+// --------------------------------------------------------- stiffness passes
+// The curl coefficients of the 20 functions at the four vertices, per type,
+// at compile time (see curls(): dyadic, exact in FP32).
+struct CurlTab {
+    float c[6][20][12];
+};
+constexpr CurlTab make_curl_tab()
+{
+    CurlTab T{};
+    for (int p = 0; p < 6; ++p) {
+        double g[4][3] = {};
+        const int a = kPerm[p][0], b = kPerm[p][1], c = kPerm[p][2];
+        g[0][a] = -1; g[1][a] = 1; g[1][b] = -1; g[2][b] = 1; g[2][c] = -1; g[3][c] = 1;
+        for (int f = 0; f < 20; ++f) {
+            const FunC F = fun_c(f);
+            double G[3] = {};   // gradient of the linear factor
+            for (int q = 0; q < 3; ++q)
+                for (int n = 0; n < 4; ++n) G[q] += F.co[n] * g[n][q];
+            for (int v = 0; v < 4; ++v)
+                for (int q = 0; q < 3; ++q) {
+                    const int q1 = (q + 1) % 3, q2 = (q + 2) % 3;
+                    const double gij = g[F.i][q1] * g[F.j][q2] - g[F.i][q2] * g[F.j][q1];
+                    const double Gj = G[q1] * g[F.j][q2] - G[q2] * g[F.j][q1], Gi = G[q1] * g[F.i][q2] - G[q2] * g[F.i][q1];
+                    T.c[p][f][3 * v + q] = (float)(2.0 * F.co[v] * gij + (v == F.i ? Gj : 0.0) - (v == F.j ? Gi : 0.0));
+                }
+        }
+    }
+    return T;
+}
+constexpr CurlTab kCurl = make_curl_tab();
+
+// Stiffness element pass in FP64: vertex curls c_v = sum_a U_a C_av, the P1
+// mass h_v = (c_v + sum_w c_w) / 120, Yt[a][t] = sum_v C_av . h_v.  The FP64
+// pipe bounds it; half of the coefficients are zero and left out.
+template <int P, int A, int Q> __device__ __forceinline__ void curl_fma(double x, double &s)
+{
+    constexpr double K = kCurl.c[P][A][Q];
+    if constexpr (K != 0.0) s = fma(K, x, s);
+}
+template <int P, int A, int... Q> __device__ __forceinline__ void curl_fmas(std::integer_sequence<int, Q...>, double u, double (&c)[12])
+{
+    (curl_fma<P, A, Q>(u, c[Q]), ...);
+}
+template <int P, int A, int... Q>
+__device__ __forceinline__ double curl_dot(std::integer_sequence<int, Q...>, const double (&h)[12])
+{
+    double f = 0.0;
+    (curl_fma<P, A, Q>(h[Q], f), ...);
+    return f;
+}
+template <int P, int... A>
+__device__ __forceinline__ void stiff_body(std::integer_sequence<int, A...>, const TetAddr &ta, unsigned long long NT, unsigned long long t,
+                                           const double *__restrict__ U, double *__restrict__ Yt)
+{
+    double u[20], c[12], h[12];
+    cheb_load<double, P>(std::make_integer_sequence<int, 20>{}, U + ta.dof0 + ta.v0, ta.nnode, ta.nx1, ta.nxy, u);
+#pragma unroll
+    for (int q = 0; q < 12; ++q) c[q] = 0.0;
+    (curl_fmas<P, A>(std::make_integer_sequence<int, 12>{}, u[A], c), ...);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double s = c[q] + c[3 + q] + c[6 + q] + c[9 + q];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) h[3 * v + q] = (c[3 * v + q] + s) * (1.0 / 120.0);
+    }
+    ((Yt[A * NT + t] = curl_dot<P, A>(std::make_integer_sequence<int, 12>{}, h)), ...);
+}
+__global__ void __launch_bounds__(64) t2_stiff_elem_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
+                                                          const double *__restrict__ U, double *__restrict__ Yt)
+{
+    const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+    if (t >= NT) return;
+    const T2Shot S = sh[shot_of(sh, ns, t, 0)];
+    const TetAddr ta = tet_addr(S, t - S.tet0);
+    constexpr auto all = std::make_integer_sequence<int, 20>{};
+    switch (ta.p) {
+    case 0: stiff_body<0>(all, ta, NT, t, U, Yt); break;
+    case 1: stiff_body<1>(all, ta, NT, t, U, Yt); break;
+    case 2: stiff_body<2>(all, ta, NT, t, U, Yt); break;
+    case 3: stiff_body<3>(all, ta, NT, t, U, Yt); break;
+    case 4: stiff_body<4>(all, ta, NT, t, U, Yt); break;
+    default: stiff_body<5>(all, ta, NT, t, U, Yt); break;
+    }
+}
+
+// s + c += K x as a compensated dot product (Ogita, Rump and Oishi 2005,
+// Dot2: the product split exactly by FMA, the sum by two-sum, the errors
+// accumulated in c).  K is a compile-time coefficient: nothing for zero, no
+// product error for a power of two.
+constexpr bool pow2(float k)
+{
+    k = k < 0.0f ? -k : k;
+    for (float t = 0.25f; t <= 4.0f; t *= 2.0f)
+        if (k == t) return true;
+    return false;
+}
+template <int P, int A, int Q> __device__ __forceinline__ void dot2_add(float x, float &s, float &c)
+{
+    constexpr float K = kCurl.c[P][A][Q], a = K < 0.0f ? -K : K;
+    if constexpr (K != 0.0f) {
+        const float m = __fmul_rn(a, x), p = K < 0.0f ? -m : m;
+        const float t = __fadd_rn(s, p);
+        const float bb = __fsub_rn(t, s);
+        const float es = __fadd_rn(__fsub_rn(s, __fsub_rn(t, bb)), __fsub_rn(p, bb));
+        s = t;
+        if constexpr (pow2(a)) {
+            c = __fadd_rn(c, es);
+        } else {
+            const float e = fmaf(a, x, -m);
+            c = __fadd_rn(c, __fadd_rn(K < 0.0f ? -e : e, es));
+        }
+    }
+}
+template <int P, int A, int... Q>
+__device__ __forceinline__ void stiff_curl(std::integer_sequence<int, Q...>, float u, float (&cs)[12], float (&cc)[12])
+{
+    (dot2_add<P, A, Q>(u, cs[Q], cc[Q]), ...);
+}
+template <int P, int... A>
+__device__ __forceinline__ void stiff_curls(std::integer_sequence<int, A...>, const float (&u)[20], float (&cs)[12], float (&cc)[12])
+{
+    (stiff_curl<P, A>(std::make_integer_sequence<int, 12>{}, u[A], cs, cc), ...);
+}
+template <int P, int A, int Q> __device__ __forceinline__ void stiff_term(float hh, float hl, float &s, float &c)
+{
+    constexpr float K = kCurl.c[P][A][Q];
+    if constexpr (K != 0.0f) {
+        dot2_add<P, A, Q>(hh, s, c);
+        c = fmaf(K, hl, c);
+    }
+}
+template <int P, int A, int... Q>
+__device__ __forceinline__ void stiff_value(std::integer_sequence<int, Q...>, const float (&hh)[12], const float (&hl)[12], double *y)
+{
+    float s = 0.0f, c = 0.0f;
+    (stiff_term<P, A, Q>(hh[Q], hl[Q], s, c), ...);
+    *y = (double)s + (double)c;
+}
+template <int P, int... A>
+__device__ __forceinline__ void stiff_values(std::integer_sequence<int, A...>, const float (&hh)[12], const float (&hl)[12], double *y,
+                                             unsigned long long NT)
+{
+    (stiff_value<P, A>(std::make_integer_sequence<int, 12>{}, hh, hl, y + A * NT), ...);
+}
+
+// Stiffness element pass of FP32 runs in double-float arithmetic: vertex
+// curls, P1 mass and transposed curl as the FP64 pass, each sum a compensated
+// dot product, so the element values carry about twice the FP32 precision at
+// FP32 throughput.  A body per type; the tetrahedra are type-major, so the
+// blocks in flight share one.  Bound by the FP64 pipe (86% busy: 77 sums and
+// 100 conversions per tetrahedron at two lanes per SM and clock).  With the
+// coefficients read from constant memory it ran 5,500 instructions per warp
+// and waited for them and for the instruction cache: 425 us on 48^3 cubes,
+// 226 us now.
+template <int P> __device__ __forceinline__ void stiff_df_body(const TetAddr &ta, unsigned long long NT, unsigned long long t,
+                                                               const float *__restrict__ U, double *__restrict__ Yt)
+{
+    float u[20], cs[12], cc[12];
+    cheb_load<float, P>(std::make_integer_sequence<int, 20>{}, U + ta.dof0 + ta.v0, ta.nnode, ta.nx1, ta.nxy, u);
+#pragma unroll
+    for (int q = 0; q < 12; ++q) { cs[q] = 0.0f; cc[q] = 0.0f; }
+    stiff_curls<P>(std::make_integer_sequence<int, 20>{}, u, cs, cc);
+    // P1 mass in FP64 (12 values), split again into hi + lo
+    double c[12];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) c[q] = (double)cs[q] + (double)cc[q];
+    float hh[12], hl[12];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double sm = c[q] + c[3 + q] + c[6 + q] + c[9 + q];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const double h = (c[3 * v + q] + sm) * (1.0 / 120.0);
+            hh[3 * v + q] = (float)h;
+            hl[3 * v + q] = (float)(h - (double)hh[3 * v + q]);
+        }
+    }
+    stiff_values<P>(std::make_integer_sequence<int, 20>{}, hh, hl, Yt + t, NT);
+}
+
+__global__ void __launch_bounds__(128) t2_stiff_df_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
+                                                         const float *__restrict__ U, double *__restrict__ Yt)
+{
+    const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+    if (t >= NT) return;
+    const T2Shot S = sh[shot_of(sh, ns, t, 0)];
+    const TetAddr ta = tet_addr(S, t - S.tet0);
+    switch (ta.p) {
+    case 0: stiff_df_body<0>(ta, NT, t, U, Yt); break;
+    case 1: stiff_df_body<1>(ta, NT, t, U, Yt); break;
+    case 2: stiff_df_body<2>(ta, NT, t, U, Yt); break;
+    case 3: stiff_df_body<3>(ta, NT, t, U, Yt); break;
+    case 4: stiff_df_body<4>(ta, NT, t, U, Yt); break;
+    default: stiff_df_body<5>(ta, NT, t, U, Yt); break;
+    }
+}
+
+
+// The two mass rows of entity type ET at node (i,j,k): the sum over its
+// tetrahedra of e M x at the entity's local DOFs, every table entry a
+// compile-time constant.
 template <class T, int ET, int Q>
 __device__ __forceinline__ void cheb_rows_inc(const T *__restrict__ xs, const T *__restrict__ eps, unsigned long long tet0,
                                               unsigned ncube, unsigned nn, unsigned nx1, unsigned nxy, unsigned ncx, unsigned ncxy,
@@ -1611,15 +1694,10 @@ struct Tet2Sim : Sim {
         EMS_CUDA(cudaMemcpyToSymbol(c2_dof, dof, sizeof(dof)));
         EMS_CUDA(cudaMemcpyToSymbol(c2_M64, R.M, sizeof(R.M)));
         EMS_CUDA(cudaMemcpyToSymbol(c2_M32, m32, sizeof(m32)));
-        EMS_CUDA(cudaMemcpyToSymbol(c2_C, R.C, sizeof(R.C)));
-        float c32[6][20][12];
         for (int p = 0; p < 6; ++p)
             for (int a = 0; a < 20; ++a)
-                for (int q = 0; q < 12; ++q) {
-                    c32[p][a][q] = (float)R.C[p][a][q];
-                    if ((double)c32[p][a][q] != R.C[p][a][q]) throw Error{EMS_ERR_CUDA, "curl coefficient not exact in FP32"};
-                }
-        EMS_CUDA(cudaMemcpyToSymbol(c2_C32, c32, sizeof(c32)));
+                for (int q = 0; q < 12; ++q)
+                    if ((double)kCurl.c[p][a][q] != R.C[p][a][q]) throw Error{EMS_ERR_CUDA, "compile-time curl differs from the setup's"};
         EMS_CUDA(cudaMemcpyToSymbol(c2_ninc, R.ninc, sizeof(R.ninc)));
         EMS_CUDA(cudaMemcpyToSymbol(c2_inc, R.inc, sizeof(R.inc)));
         EMS_CUDA(cudaMemcpyToSymbol(c2_axes, R.axes, sizeof(R.axes)));
@@ -1705,12 +1783,10 @@ struct Tet2Sim : Sim {
     // Stiffness element pass into d_YtK: FP64 for FP64 runs, double-float for FP32
     template <class T> void enqueue_stiff(const T *u)
     {
-        if (std::is_same<T, float>::value)
-            t2_stiff_df_kernel<<<blocks(ntet, 128), 128, 0, stream>>>(ntet, d_shots.as<T2Shot>(), (int)shots.size(),
-                                                                      reinterpret_cast<const float *>(u), d_YtK.as<double>());
+        if constexpr (std::is_same<T, float>::value)
+            t2_stiff_df_kernel<<<blocks(ntet, 128), 128, 0, stream>>>(ntet, d_shots.as<T2Shot>(), (int)shots.size(), u, d_YtK.as<double>());
         else
-            t2_stiff_elem_kernel<T><<<blocks(ntet, 128), 128, 0, stream>>>(ntet, d_shots.as<T2Shot>(), (int)shots.size(), u,
-                                                                           d_YtK.as<double>());
+            t2_stiff_elem_kernel<<<blocks(ntet, 64), 64, 0, stream>>>(ntet, d_shots.as<T2Shot>(), (int)shots.size(), u, d_YtK.as<double>());
     }
 
     // f = K u (element pass + entity pass), u and out device vectors

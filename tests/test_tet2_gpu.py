@@ -319,3 +319,16 @@ def test_marching_iteration_equals_the_entity_iteration_bitwise(cells, monkeypat
         for q in range(2):
             assert np.array_equal(out["fused", integ][q], out["march", integ][q])
     assert np.linalg.norm(out["march", ems.SYMP2][0]) > 0 or max(max(c) for c in cells) == 1
+
+
+@pytest.mark.parametrize("n", [(1, 1, 1), (2, 3, 1), (5, 4, 7)])
+def test_double_float_stiffness_matches_oracle(n):
+    """The FP32 handle's stiffness on FP32-exact values: element values good to
+    about 2^-45, summed in FP64, so only the rounding of the FP32 result (a
+    relative 2^-24 per value) separates it from the FP64 oracle."""
+    _, ndof, _ = oracle.tet2_sizes(n)
+    rng = np.random.default_rng(43)
+    U = np.where(oracle.tet2_pec_mask(n), 0.0, rng.standard_normal(ndof).astype(np.float32).astype(np.float64))
+    s = ems.TetFemSimulation(n, H, 2, ems.SYMP4, ems.FP32, dt=0.05 * TS)
+    f, ref = from_api(n, s.apply_stiffness(to_api(n, U))), oracle.tet2_apply(n, U, True)
+    assert np.linalg.norm(f - ref) <= 2.0 ** -24 * np.linalg.norm(ref)
