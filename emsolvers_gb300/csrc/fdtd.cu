@@ -1,7 +1,13 @@
 // Yee FDTD on one GPU: the reference time loop of fdtd/fdtd_simulation.cpp
 // (H from curl E 119-169, E from curl H 170-220, sources 222-239, receivers
-// 261-303) on the reference's padded field layout (55-88), extended with
-// per-cell materials and a convolutional PML.
+// 261-303), extended with per-cell materials and a convolutional PML.
+//
+// The API shows the reference's padded field layout (55-88).  On the device
+// all fields share one pitched layout, so one offset addresses them all and a
+// thread moves 16 bytes (4 FP32 or 2 FP64 cells along x) per access: rows of
+// `pitch` values, planes of ny + 2 rows, and the components that the
+// reference pads in x (Ey, Ez) stored one column to the left, next to the H
+// cell that reads them.
 //
 // Arithmetic is written with explicitly rounded operations (no contraction
 // into fused multiply-adds) in the reference's operand order, so the FP64
@@ -30,16 +36,13 @@ __device__ __forceinline__ float radd(float a, float b) { return __fadd_rn(a, b)
 __device__ __forceinline__ float rsub(float a, float b) { return __fsub_rn(a, b); }
 __device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
 
-// CPML coefficient profile along one axis, sampled at the derivative positions.
+// CPML coefficient profile along one axis, sampled at the derivative
+// positions; the layer is off for lo <= s < hi.  (The x profile of the E-type
+// derivatives starts at s = 1, as the columns of Ey and Ez do.)
 template <class T> struct Prof {
     const T *b, *a, *kinv;
-    const unsigned char *on;
-};
-
-// Row (y) and plane (z) strides of the padded arrays and of the material
-// grid, in elements (all arrays hold fewer than 2^32 elements).
-struct FdtdStrides {
-    unsigned ex_y, ex_z, ey_y, ey_z, ez_y, ez_z, hx_y, hx_z, hy_y, hy_z, hz_y, hz_z, m_y, m_z;
+    int lo, hi;
+    __device__ __forceinline__ bool on(int s) const { return s < lo || s >= hi; }
 };
 
 // (ca, cb) of one material, loaded as one vector.
@@ -48,126 +51,224 @@ template <class T> struct alignas(2 * sizeof(T)) CaCb {
 };
 
 template <class T> struct FdtdArgs {
-    T *Ex, *Ey, *Ez, *Hx, *Hy, *Hz;
+    T *Ex, *Ey, *Ez, *Hx, *Hy, *Hz;   // the first column of row 0, plane 0
     int nx, ny, nz;
-    FdtdStrides st;
+    // threads per row (V cells each): [g0, g1) touch no x layer and run in the
+    // first blocks of a launch, the gr others in the blocks behind them
+    int g0, g1, gr;
+    unsigned magic[2], shift[2];   // t / (g1 - g0) and t / gr as (t * magic) >> shift (see divider)
+    unsigned pitch;                // values per row
+    size_t plane;                  // values per plane
     T ch, ce;                      // uniform update coefficients dt/mu/h, dt/eps/h
-    const uint16_t *mat;           // per-cell material id (MAT)
+    const uint16_t *mat;           // per-cell material id (MAT), rows of mpitch, the last column repeated
+    unsigned mpitch;
     const CaCb<T> *cab;            // per-material E coefficients (MAT)
     Prof<T> pe[3], ph[3];          // CPML profiles for E- and H-type derivatives (PML)
-    T *psiE[3][2], *psiH[3][2];    // CPML auxiliary fields, full field size (PML)
-    int in_lo[3], in_hi[3];        // per axis, the indices [lo, hi) where no profile is on (PML)
+    T *psiE[3][2], *psiH[3][2];    // CPML auxiliary fields in the fields' layout (PML)
 };
 
-// Cells per thread along z (planes kFdtdKZ * blockIdx.z ...).  One: two
-// cells per thread raised the E kernel's registers from 32 to 58 and its
-// time at 512^3 from 1.76 to 2.93 ms.
-constexpr int kFdtdKZ = 1;
-
-// True when no thread of this block touches a CPML slab (the same for every
-// thread of the block, so the slab tests and their flag loads are skipped
-// uniformly; blocks that touch a slab test per thread as before).
-template <class T> __device__ __forceinline__ bool block_outside_slabs(const FdtdArgs<T> &a)
+// 16 bytes of consecutive cells.
+template <class T> struct Vec {
+    static constexpr int V = 16 / sizeof(T);
+    T v[V];
+};
+__device__ __forceinline__ void vload(Vec<float> &r, const float *p)
 {
-    const int i0 = blockIdx.x * blockDim.x, j0 = blockIdx.y * blockDim.y, k0 = blockIdx.z * kFdtdKZ;
-    return i0 >= a.in_lo[0] && i0 + (int)blockDim.x <= a.in_hi[0] && j0 >= a.in_lo[1] &&
-           j0 + (int)blockDim.y <= a.in_hi[1] && k0 >= a.in_lo[2] && k0 + kFdtdKZ <= a.in_hi[2];
+    const float4 t = *reinterpret_cast<const float4 *>(p);
+    r.v[0] = t.x; r.v[1] = t.y; r.v[2] = t.z; r.v[3] = t.w;
+}
+__device__ __forceinline__ void vload(Vec<double> &r, const double *p)
+{
+    const double2 t = *reinterpret_cast<const double2 *>(p);
+    r.v[0] = t.x; r.v[1] = t.y;
+}
+// the n first values (all of them in one store)
+__device__ __forceinline__ void vstore(float *p, const Vec<float> &r, int n)
+{
+    if (n >= 4) {
+        *reinterpret_cast<float4 *>(p) = make_float4(r.v[0], r.v[1], r.v[2], r.v[3]);
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+        if (q < n) p[q] = r.v[q];
+}
+__device__ __forceinline__ void vstore(double *p, const Vec<double> &r, int n)
+{
+    if (n >= 2) *reinterpret_cast<double2 *>(p) = make_double2(r.v[0], r.v[1]);
+    else if (n == 1) p[0] = r.v[0];
+}
+__device__ __forceinline__ void mload(unsigned (&m)[4], const uint16_t *p)
+{
+    const ushort4 t = *reinterpret_cast<const ushort4 *>(p);
+    m[0] = t.x; m[1] = t.y; m[2] = t.z; m[3] = t.w;
+}
+__device__ __forceinline__ void mload(unsigned (&m)[2], const uint16_t *p)
+{
+    const ushort2 t = *reinterpret_cast<const ushort2 *>(p);
+    m[0] = t.x; m[1] = t.y;
 }
 
-#define IEX(i, j, k) ((size_t)(i) + (size_t)(j) * (a.nx + 1) + (size_t)(k) * (a.nx + 1) * (a.ny + 2))
-#define IEY(i, j, k) ((size_t)(i) + (size_t)(j) * (a.nx + 2) + (size_t)(k) * (a.nx + 2) * (a.ny + 1))
-#define IEZ(i, j, k) ((size_t)(i) + (size_t)(j) * (a.nx + 2) + (size_t)(k) * (a.nx + 2) * (a.ny + 2))
-#define IHX(i, j, k) ((size_t)(i) + (size_t)(j) * a.nx + (size_t)(k) * a.nx * (a.ny + 1))
-#define IHY(i, j, k) ((size_t)(i) + (size_t)(j) * (a.nx + 1) + (size_t)(k) * (a.nx + 1) * a.ny)
-#define IHZ(i, j, k) ((size_t)(i) + (size_t)(j) * (a.nx + 1) + (size_t)(k) * (a.nx + 1) * (a.ny + 1))
+// Sources and receiver samples that the E kernel serves itself: the entries
+// of plane k are list[plane[k]] .. list[plane[k + 1] - 1], sources in
+// insertion order, then samples.  A launch belongs to step *base + step.
+struct FdtdPoint {
+    long long off;  // offset in the component's array
+    int comp;       // component, + 4 for a receiver sample
+    int idx;        // source number, or place of the sample in a row of samp
+};
+struct FdtdPoints {
+    const int *plane;        // null: no points
+    const FdtdPoint *list;
+    const double *vals;      // [step - 1][ns] source values
+    double *samp;            // [row][nsm] sampled values
+    const int *base;
+    int step, ns, nsm, tf;
+};
 
 // d = ((p - q) - r) + s, the reference's evaluation order of a curl difference.
 template <class T> __device__ __forceinline__ T curl4(T p, T q, T r, T s) { return radd(rsub(rsub(p, q), r), s); }
 
-// One CPML-stretched update value: kinv1*d1 - kinv2*d2 + psi1 - psi2 with the
-// auxiliary recursions psi = b psi + a d (oracle/orc_fdtd.c order).
+// The CPML along one axis on the cells of a thread: t = kinv d and the new
+// psi = b psi + a d; without a layer (kind 0) t = d and nothing moves.  kind 1:
+// all cells at position s; kind 2: the cells run along the axis from s.
 template <class T>
-__device__ __forceinline__ T pml_curl(T d1, T d2, const Prof<T> &p1, int s1, const Prof<T> &p2, int s2, T *psi1, T *psi2)
+__device__ __forceinline__ void layer(int kind, const Vec<T> &d, const Prof<T> &p, int s, T *psi, Vec<T> &t, Vec<T> &q)
 {
-    T q1 = radd(rmul(p1.b[s1], *psi1), rmul(p1.a[s1], d1));
-    T q2 = radd(rmul(p2.b[s2], *psi2), rmul(p2.a[s2], d2));
-    *psi1 = q1;
-    *psi2 = q2;
-    return rsub(radd(rsub(rmul(p1.kinv[s1], d1), rmul(p2.kinv[s2], d2)), q1), q2);
-}
-
-// H from curl E at cell (i,j,k): fdtd_simulation.cpp:119-169.  Offsets are
-// 32-bit, formed once per array and moved by the strides; E values shared
-// by two components are loaded once.  Every load of the cell is issued
-// before its first store (the three read-modify-writes touch distinct
-// arrays and no other thread writes them), so a thread waits for one round
-// of memory latency instead of one per component.
-template <class T, bool PML>
-__device__ __forceinline__ void fdtd_h_cell(const FdtdArgs<T> &a, int i, int j, int k, bool slab)
-{
-    const FdtdStrides &st = a.st;
-    const unsigned oEx = i + j * st.ex_y + k * st.ex_z, oEy = i + j * st.ey_y + k * st.ey_z;
-    const unsigned oEz = i + j * st.ez_y + k * st.ez_z;
-    const unsigned px = i + j * st.hx_y + k * st.hx_z, py = i + j * st.hy_y + k * st.hy_z;
-    const unsigned pz = i + j * st.hz_y + k * st.hz_z;
-    const bool hx = i < a.nx, hy = j < a.ny, hz = k < a.nz;
-    T ez11 = 0, ey1k = 0, ex1k = 0;   // Ez(i+1,j+1,k), Ey(i+1,j,k+1), Ex(i,j+1,k+1)
-    T ez1 = 0, ey1 = 0, ex1 = 0, ez0 = 0, ey0 = 0, ex0 = 0, hx0 = 0, hy0 = 0, hz0 = 0;
-    if (hx || hy) ez11 = __ldg(a.Ez + oEz + 1 + st.ez_y);
-    if (hx || hz) ey1k = __ldg(a.Ey + oEy + 1 + st.ey_z);
-    if (hy || hz) ex1k = __ldg(a.Ex + oEx + st.ex_y + st.ex_z);
-    if (hx) {
-        hx0 = a.Hx[px];
-        ez1 = __ldg(a.Ez + oEz + 1);
-        ey1 = __ldg(a.Ey + oEy + 1);
-    }
-    if (hy) {
-        hy0 = a.Hy[py];
-        ex1 = __ldg(a.Ex + oEx + st.ex_y);
-        ez0 = __ldg(a.Ez + oEz + st.ez_y);
-    }
-    if (hz) {
-        hz0 = a.Hz[pz];
-        ey0 = __ldg(a.Ey + oEy + st.ey_z);
-        ex0 = __ldg(a.Ex + oEx + st.ex_z);
-    }
-    if (hx) {
-        if (slab && (a.ph[1].on[j] | a.ph[2].on[k])) {
-            T c = pml_curl(rsub(ez11, ez1), rsub(ey1k, ey1), a.ph[1], j, a.ph[2], k, &a.psiH[0][0][px], &a.psiH[0][1][px]);
-            a.Hx[px] = rsub(hx0, rmul(a.ch, c));
-        } else {
-            a.Hx[px] = rsub(hx0, rmul(a.ch, curl4(ez11, ez1, ey1k, ey1)));
-        }
-    }
-    if (hy) {
-        if (slab && (a.ph[2].on[k] | a.ph[0].on[i])) {
-            T c = pml_curl(rsub(ex1k, ex1), rsub(ez11, ez0), a.ph[2], k, a.ph[0], i, &a.psiH[1][0][py], &a.psiH[1][1][py]);
-            a.Hy[py] = rsub(hy0, rmul(a.ch, c));
-        } else {
-            a.Hy[py] = rsub(hy0, rmul(a.ch, curl4(ex1k, ex1, ez11, ez0)));
-        }
-    }
-    if (hz) {
-        if (slab && (a.ph[0].on[i] | a.ph[1].on[j])) {
-            T c = pml_curl(rsub(ey1k, ey0), rsub(ex1k, ex0), a.ph[0], i, a.ph[1], j, &a.psiH[2][0][pz], &a.psiH[2][1][pz]);
-            a.Hz[pz] = rsub(hz0, rmul(a.ch, c));
-        } else {
-            a.Hz[pz] = rsub(hz0, rmul(a.ch, curl4(ey1k, ey0, ex1k, ex0)));
-        }
-    }
-}
-
-template <class T, bool PML>
-__global__ void __launch_bounds__(256) fdtd_h_kernel(FdtdArgs<T> a)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i > a.nx || j > a.ny) return;
-    const bool slab = PML && !block_outside_slabs(a);
+    constexpr int V = Vec<T>::V;
+    if (kind == 0) {
 #pragma unroll
-    for (int kk = 0; kk < kFdtdKZ; ++kk) {
-        const int k = blockIdx.z * kFdtdKZ + kk;
-        if (k <= a.nz) fdtd_h_cell<T, PML>(a, i, j, k, slab);
+        for (int v = 0; v < V; ++v) { t.v[v] = d.v[v]; q.v[v] = T(0); }
+        return;
+    }
+    Vec<T> b, a, k;
+    vload(q, psi);
+    if (kind == 2) {
+        vload(b, p.b + s);
+        vload(a, p.a + s);
+        vload(k, p.kinv + s);
+    } else {
+        b.v[0] = p.b[s]; a.v[0] = p.a[s]; k.v[0] = p.kinv[s];
+#pragma unroll
+        for (int v = 1; v < V; ++v) { b.v[v] = b.v[0]; a.v[v] = a.v[0]; k.v[v] = k.v[0]; }
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        q.v[v] = radd(rmul(b.v[v], q.v[v]), rmul(a.v[v], d.v[v]));
+        t.v[v] = rmul(k.v[v], d.v[v]);
+    }
+    vstore(psi, q, V);
+}
+
+// Curl differences of the cells of a thread: ((p - q) - r) + s, or in a layer
+// of either axis kinv1 d1 - kinv2 d2 + psi1 - psi2 with d1 = p - q, d2 = r - s
+// (oracle/orc_fdtd.c order; the auxiliary value of an axis without a layer
+// is zero and is not touched).  xm: the cells inside the x layer.
+template <class T, bool PML>
+__device__ __forceinline__ Vec<T> curl_vec(const Vec<T> &p, const Vec<T> &q, const Vec<T> &r, const Vec<T> &s, int k1, const Prof<T> &p1, int s1,
+                                           T *psi1, int k2, const Prof<T> &p2, int s2, T *psi2, unsigned xm)
+{
+    constexpr int V = Vec<T>::V;
+    Vec<T> c;
+#pragma unroll
+    for (int v = 0; v < V; ++v) c.v[v] = curl4(p.v[v], q.v[v], r.v[v], s.v[v]);
+    if (PML && (k1 | k2)) {
+        Vec<T> d1, d2, t1, t2, q1, q2;
+#pragma unroll
+        for (int v = 0; v < V; ++v) { d1.v[v] = rsub(p.v[v], q.v[v]); d2.v[v] = rsub(r.v[v], s.v[v]); }
+        layer(k1, d1, p1, s1, psi1, t1, q1);
+        layer(k2, d2, p2, s2, psi2, t2, q2);
+        const bool all = k1 == 1 || k2 == 1;
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            if (all || ((xm >> v) & 1)) c.v[v] = rsub(radd(rsub(t1.v[v], t2.v[v]), q1.v[v]), q2.v[v]);
+    }
+    return c;
+}
+
+// Bits of the cells i .. i + V - 1 inside the x layer.
+template <class T> __device__ __forceinline__ unsigned x_bits(const Prof<T> &p, int i)
+{
+    unsigned m = 0;
+#pragma unroll
+    for (int v = 0; v < Vec<T>::V; ++v)
+        if (p.on(i + v)) m |= 1u << v;
+    return m;
+}
+// The cells of a thread: V columns from i of row j, plane k (false: none).
+// Threads run through the rows of a plane without a break, so short rows fill
+// the warps too.  The columns near an x layer (xl) have blocks of their own:
+// in one warp with the others they made nearly every warp of a row of 400
+// cells run the layer's code (400 x 384 x 368 FP32: 72.0 ms for 60 steps).
+template <class T>
+__device__ __forceinline__ bool fdtd_cells(const FdtdArgs<T> &a, int kz, unsigned mblocks, int &i, int &j, int &k, size_t &o, bool &xl)
+{
+    xl = blockIdx.x >= mblocks;
+    const unsigned t = (blockIdx.x - (xl ? mblocks : 0)) * (blockDim.x * blockDim.y) + threadIdx.y * blockDim.x + threadIdx.x;
+    const unsigned row = (unsigned)(((unsigned long long)t * a.magic[xl]) >> a.shift[xl]);
+    int g = (int)(t - row * (xl ? a.gr : a.g1 - a.g0));
+    if (!xl) g += a.g0;
+    else if (g >= a.g0) g += a.g1 - a.g0;
+    j = (int)row;
+    i = g * Vec<T>::V;
+    k = kz + blockIdx.z;
+    o = (size_t)k * a.plane + (size_t)row * a.pitch + i;
+    return j <= a.ny;
+}
+
+// H from curl E: fdtd_simulation.cpp:119-169.  Every load of the thread is
+// issued before its first store.  Bound by DRAM on large grids: per cell and
+// step 18 values of E and H move, 9 of them here.
+template <class T, bool PML>
+__global__ void __launch_bounds__(256) fdtd_h_kernel(FdtdArgs<T> a, int kz, unsigned mblocks, int *ctr, int inc)
+{
+    constexpr int V = Vec<T>::V;
+    // the step counter of a replayed graph, moved on by its first launch (the H kernels do not read it)
+    if (ctr && blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0) *ctr += inc;
+    int i, j, k;
+    size_t o;
+    bool xl;
+    if (!fdtd_cells(a, kz, mblocks, i, j, k, o, xl)) return;
+    const size_t oy = o + a.pitch, oz = o + a.plane;
+    const bool hy = j < a.ny, hz = k < a.nz;
+    const int nx = min(V, a.nx - i), n = min(V, a.nx + 1 - i);   // valid cells of Hx, and of Hy and Hz
+    Vec<T> z11, z1, y1k, y1, x1k, x1, x0, h0, h1, h2, z0, y0;
+    vload(z11, a.Ez + oy);                 // Ez(i+1, j+1, k)
+    vload(z1, a.Ez + o);                   // Ez(i+1, j, k)
+    vload(y1k, a.Ey + oz);                 // Ey(i+1, j, k+1)
+    vload(y1, a.Ey + o);                   // Ey(i+1, j, k)
+    vload(x1k, a.Ex + oz + a.pitch);       // Ex(i, j+1, k+1)
+    vload(x1, a.Ex + oy);                  // Ex(i, j+1, k)
+    vload(x0, a.Ex + oz);                  // Ex(i, j, k+1)
+    z0.v[0] = a.Ez[(ptrdiff_t)oy - 1];     // Ez(i, j+1, k)
+    y0.v[0] = a.Ey[(ptrdiff_t)oz - 1];     // Ey(i, j, k+1)
+    vload(h0, a.Hx + o);
+    vload(h1, a.Hy + o);
+    vload(h2, a.Hz + o);
+#pragma unroll
+    for (int v = 1; v < V; ++v) {
+        z0.v[v] = z11.v[v - 1];
+        y0.v[v] = y1k.v[v - 1];
+    }
+    const unsigned xm = PML && xl ? x_bits(a.ph[0], i) : 0;
+    const int kx = xm ? 2 : 0, ky = PML && a.ph[1].on(j) ? 1 : 0, kk = PML && a.ph[2].on(k) ? 1 : 0;
+    if (nx > 0) {
+        const Vec<T> c = curl_vec<T, PML>(z11, z1, y1k, y1, ky, a.ph[1], j, a.psiH[0][0] + o, kk, a.ph[2], k, a.psiH[0][1] + o, 0);
+#pragma unroll
+        for (int v = 0; v < V; ++v) h0.v[v] = rsub(h0.v[v], rmul(a.ch, c.v[v]));
+        vstore(a.Hx + o, h0, nx);
+    }
+    if (hy) {
+        const Vec<T> c = curl_vec<T, PML>(x1k, x1, z11, z0, kk, a.ph[2], k, a.psiH[1][0] + o, kx, a.ph[0], i, a.psiH[1][1] + o, xm);
+#pragma unroll
+        for (int v = 0; v < V; ++v) h1.v[v] = rsub(h1.v[v], rmul(a.ch, c.v[v]));
+        vstore(a.Hy + o, h1, n);
+    }
+    if (hz) {
+        const Vec<T> c = curl_vec<T, PML>(y1k, y0, x1k, x0, kx, a.ph[0], i, a.psiH[2][0] + o, ky, a.ph[1], j, a.psiH[2][1] + o, xm);
+#pragma unroll
+        for (int v = 0; v < V; ++v) h2.v[v] = rsub(h2.v[v], rmul(a.ch, c.v[v]));
+        vstore(a.Hz + o, h2, n);
     }
 }
 
@@ -183,268 +284,137 @@ __device__ __forceinline__ CaCb<double> load_cab(const CaCb<double> *p)
     return {v.x, v.y};
 }
 
-// E from curl H at (i,j,k): fdtd_simulation.cpp:170-220, E = ca E + cb curl
-// (ca, cb of the cell's material; uniform: E += ce curl).  As in the H
-// update, all loads of the cell (fields, material ids, then their (ca, cb))
-// are issued before the first store.
-template <class T, bool MAT, bool PML>
-__device__ __forceinline__ void fdtd_e_cell(const FdtdArgs<T> &a, int i, int j, int k, bool slab)
+// ca E + cb c with the cells' materials, or E + ce c without (ca = 1 multiplies exactly)
+template <class T, bool MAT>
+__device__ __forceinline__ void e_update(const FdtdArgs<T> &a, Vec<T> &e, const Vec<T> &c, const CaCb<T> (&m)[Vec<T>::V])
 {
-    const int nx = a.nx, ny = a.ny, nz = a.nz;
-    const FdtdStrides &st = a.st;
-    const unsigned oHx = i + j * st.hx_y + k * st.hx_z, oHy = i + j * st.hy_y + k * st.hy_z;
-    const unsigned oHz = i + j * st.hz_y + k * st.hz_z;
-    const unsigned px = i + j * st.ex_y + k * st.ex_z, py = i + j * st.ey_y + k * st.ey_z;
-    const unsigned pz = i + j * st.ez_y + k * st.ez_z;
-    const bool ex = j >= 1 && k >= 1, ey = i >= 1 && k >= 1, ez = i >= 1 && j >= 1;
-    T hz_k = 0, hy_j = 0, hx_i = 0;   // Hz(i,j,k-1), Hy(i,j-1,k), Hx(i-1,j,k)
-    T hz_jk = 0, hy_jk = 0, hx_ik = 0, hz_ik = 0, hy_ij = 0, hx_ij = 0, ex0 = 0, ey0 = 0, ez0 = 0;
-    unsigned m0 = 0, m1 = 0, m2 = 0;
-    if (ex || ey) hz_k = __ldg(a.Hz + oHz - st.hz_z);
-    if (ex || ez) hy_j = __ldg(a.Hy + oHy - st.hy_y);
-    if (ey || ez) hx_i = __ldg(a.Hx + oHx - 1);
-    if (ex) {  // Ex, i in [0,nx]
-        ex0 = a.Ex[px];
-        hz_jk = __ldg(a.Hz + oHz - st.hz_y - st.hz_z);
-        hy_jk = __ldg(a.Hy + oHy - st.hy_y - st.hy_z);
-        if (MAT) m0 = __ldg(a.mat + (unsigned)(i < nx ? i : nx - 1) + (unsigned)(j - 1) * st.m_y + (unsigned)(k - 1) * st.m_z);
+#pragma unroll
+    for (int v = 0; v < Vec<T>::V; ++v)
+        e.v[v] = MAT ? radd(rmul(m[v].ca, e.v[v]), rmul(m[v].cb, c.v[v])) : radd(e.v[v], rmul(a.ce, c.v[v]));
+}
+// The coefficients of the cells with ids at p; mostly one material, loaded once.
+template <class T> __device__ __forceinline__ void e_material(const FdtdArgs<T> &a, const uint16_t *p, CaCb<T> (&m)[Vec<T>::V])
+{
+    unsigned id[Vec<T>::V];
+    mload(id, p);
+#pragma unroll
+    for (int v = 0; v < Vec<T>::V; ++v) m[v] = load_cab(a.cab + id[v]);
+}
+
+// E from curl H: fdtd_simulation.cpp:170-220.  As in the H update, all loads
+// of the thread are issued before the first store.  The plane's points then
+// act on the updated values before they are stored: a launch for the sources
+// and one for the receivers would cost more than a small grid's updates
+// (64^3 FP64: 44.1 us a step with them, 30.5 without).
+template <class T, bool MAT, bool PML>
+__global__ void __launch_bounds__(256) fdtd_e_kernel(FdtdArgs<T> a, FdtdPoints pt, int kz, unsigned mblocks)
+{
+    constexpr int V = Vec<T>::V;
+    int i, j, k;
+    size_t o;
+    bool xl;
+    if (!fdtd_cells(a, kz, mblocks, i, j, k, o, xl)) return;
+    const bool jn = j >= 1, kn = k >= 1;
+    const size_t py = a.pitch, pz = a.plane;
+    const int n = min(V, a.nx + 1 - i), nyz = min(V, a.nx - i);   // valid cells of Ex, and of Ey and Ez
+    const bool ex = jn && kn, ey = kn && nyz > 0, ez = jn && nyz > 0;
+    Vec<T> e0{}, e1{}, e2{}, zk{}, zjk{}, yj{}, yjk{}, xi{}, xik{}, xij{}, zk1{}, yj1{};
+    CaCb<T> c0[V], c1[V], c2[V];
+    if (kn) {
+        vload(zk, a.Hz + o - pz);                       // Hz(i, j, k-1)
+        vload(xik, a.Hx + o - pz);                      // Hx(i, j, k-1)
+        zk1.v[V - 1] = a.Hz[o - pz + V];
     }
-    if (ey) {  // Ey, j in [0,ny]
-        ey0 = a.Ey[py];
-        hx_ik = __ldg(a.Hx + oHx - 1 - st.hx_z);
-        hz_ik = __ldg(a.Hz + oHz - 1 - st.hz_z);
-        if (MAT) m1 = __ldg(a.mat + (unsigned)(i - 1) + (unsigned)(j < ny ? j : ny - 1) * st.m_y + (unsigned)(k - 1) * st.m_z);
+    if (jn) {
+        vload(yj, a.Hy + o - py);                       // Hy(i, j-1, k)
+        vload(xij, a.Hx + o - py);                      // Hx(i, j-1, k)
+        yj1.v[V - 1] = a.Hy[o - py + V];
     }
-    if (ez) {  // Ez, k in [0,nz]
-        ez0 = a.Ez[pz];
-        hy_ij = __ldg(a.Hy + oHy - 1 - st.hy_y);
-        hx_ij = __ldg(a.Hx + oHx - 1 - st.hx_y);
-        if (MAT) m2 = __ldg(a.mat + (unsigned)(i - 1) + (unsigned)(j - 1) * st.m_y + (unsigned)(k < nz ? k : nz - 1) * st.m_z);
-    }
-    CaCb<T> c0{1, 0}, c1{1, 0}, c2{1, 0};
-    if (MAT) {
-        if (ex) c0 = load_cab(a.cab + m0);
-        if (ey) c1 = load_cab(a.cab + m1);
-        if (ez) c2 = load_cab(a.cab + m2);
-    }
-    // ca E + cb c, or E + ce c without materials (ca = 1 multiplies exactly)
-    auto upd = [&](T e, const CaCb<T> &m, T c) { return MAT ? radd(rmul(m.ca, e), rmul(m.cb, c)) : radd(e, rmul(a.ce, c)); };
+    vload(xi, a.Hx + o);                                // Hx(i, j, k)
     if (ex) {
-        if (slab && (a.pe[1].on[j] | a.pe[2].on[k])) {
-            T c = pml_curl(rsub(hz_k, hz_jk), rsub(hy_j, hy_jk), a.pe[1], j, a.pe[2], k, &a.psiE[0][0][px], &a.psiE[0][1][px]);
-            a.Ex[px] = upd(ex0, c0, c);
-        } else {
-            a.Ex[px] = upd(ex0, c0, curl4(hz_k, hz_jk, hy_j, hy_jk));
-        }
+        vload(zjk, a.Hz + o - py - pz);
+        vload(yjk, a.Hy + o - py - pz);
+        vload(e0, a.Ex + o);
+    }
+    if (ey) vload(e1, a.Ey + o);
+    if (ez) vload(e2, a.Ez + o);
+    if (MAT) {   // Ex(i,j,k) -> cell (min(i,nx-1), j-1, k-1), Ey -> (i-1, min(j,ny-1), k-1), Ez -> (i-1, j-1, min(k,nz-1))
+        const size_t mrow = a.mpitch, mpl = mrow * a.ny;
+        if (ex) e_material(a, a.mat + (j - 1) * mrow + (k - 1) * mpl + i, c0);
+        if (ey) e_material(a, a.mat + min(j, a.ny - 1) * mrow + (k - 1) * mpl + i, c1);
+        if (ez) e_material(a, a.mat + (j - 1) * mrow + min(k, a.nz - 1) * mpl + i, c2);
+    }
+#pragma unroll
+    for (int v = 0; v < V - 1; ++v) {
+        zk1.v[v] = zk.v[v + 1];                         // Hz(i+1, j, k-1)
+        yj1.v[v] = yj.v[v + 1];                         // Hy(i+1, j-1, k)
+    }
+    const unsigned xm = PML && xl ? x_bits(a.pe[0], i) : 0;
+    const int kx = xm ? 2 : 0, ky = PML && a.pe[1].on(j) ? 1 : 0, kk = PML && a.pe[2].on(k) ? 1 : 0;
+    if (ex) {
+        const Vec<T> c = curl_vec<T, PML>(zk, zjk, yj, yjk, ky, a.pe[1], j, a.psiE[0][0] + o, kk, a.pe[2], k, a.psiE[0][1] + o, 0);
+        e_update<T, MAT>(a, e0, c, c0);
     }
     if (ey) {
-        if (slab && (a.pe[2].on[k] | a.pe[0].on[i])) {
-            T c = pml_curl(rsub(hx_i, hx_ik), rsub(hz_k, hz_ik), a.pe[2], k, a.pe[0], i, &a.psiE[1][0][py], &a.psiE[1][1][py]);
-            a.Ey[py] = upd(ey0, c1, c);
-        } else {
-            a.Ey[py] = upd(ey0, c1, curl4(hx_i, hx_ik, hz_k, hz_ik));
-        }
+        const Vec<T> c = curl_vec<T, PML>(xi, xik, zk1, zk, kk, a.pe[2], k, a.psiE[1][0] + o, kx, a.pe[0], i, a.psiE[1][1] + o, xm);
+        e_update<T, MAT>(a, e1, c, c1);
     }
     if (ez) {
-        if (slab && (a.pe[0].on[i] | a.pe[1].on[j])) {
-            T c = pml_curl(rsub(hy_j, hy_ij), rsub(hx_i, hx_ij), a.pe[0], i, a.pe[1], j, &a.psiE[2][0][pz], &a.psiE[2][1][pz]);
-            a.Ez[pz] = upd(ez0, c2, c);
-        } else {
-            a.Ez[pz] = upd(ez0, c2, curl4(hy_j, hy_ij, hx_i, hx_ij));
-        }
+        const Vec<T> c = curl_vec<T, PML>(yj1, yj, xi, xij, kx, a.pe[0], i, a.psiE[2][0] + o, ky, a.pe[1], j, a.psiE[2][1] + o, xm);
+        e_update<T, MAT>(a, e2, c, c2);
     }
-}
-
-template <class T, bool MAT, bool PML>
-__global__ void __launch_bounds__(256) fdtd_e_kernel(FdtdArgs<T> a)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i > a.nx || j > a.ny) return;
-    const bool slab = PML && !block_outside_slabs(a);
+    if (pt.plane) {
+        const int q1 = __ldg(pt.plane + k + 1);
+        for (int q = __ldg(pt.plane + k); q < q1; ++q) {
+            const FdtdPoint r = pt.list[q];
+            const long long at = r.off - (long long)o;
+            const int comp = r.comp & 3;
+            if (at < 0 || at >= V || !(comp == 0 ? ex : comp == 1 ? ey : ez)) continue;
+            const int step = pt.step + (pt.base ? *pt.base : 0);
+            const bool sample = r.comp >= 4, keep = sample && step % pt.tf == 0;
+            const T src = sample ? T(0) : (T)pt.vals[(size_t)(step - 1) * pt.ns + r.idx];
 #pragma unroll
-    for (int kk = 0; kk < kFdtdKZ; ++kk) {
-        const int k = blockIdx.z * kFdtdKZ + kk;
-        if (k <= a.nz) fdtd_e_cell<T, MAT, PML>(a, i, j, k, slab);
+            for (int v = 0; v < V; ++v) {
+                if (v != at) continue;
+                const T e = comp == 0 ? e0.v[v] : comp == 1 ? e1.v[v] : e2.v[v];
+                if (keep) pt.samp[(size_t)(step / pt.tf) * pt.nsm + r.idx] = (double)e;
+                if (sample) continue;
+                if (comp == 0) e0.v[v] = rsub(e, src);
+                else if (comp == 1) e1.v[v] = rsub(e, src);
+                else e2.v[v] = rsub(e, src);
+            }
+        }
     }
+    if (ex) vstore(a.Ex + o, e0, n);
+    if (ey) vstore(a.Ey + o, e1, nyz);
+    if (ez) vstore(a.Ez + o, e2, nyz);
 }
 
-// ------------------------------------------------------------- fused step
-// One pass per step: H^{n+1/2} and then E^{n+1} plane by plane along z.  A
-// block owns a 31 x 7 tile of (i, j) columns and a chunk of kFusedKZ planes;
-// its 32 x 8 threads also compute H on the tile's -x and -y halo columns
-// (and the plane below the chunk), whose E update needs them, instead of
-// waiting for the neighbouring blocks.  So every block reads only old
-// values: E, H and the H-type CPML auxiliaries are double-buffered (read
-// from the old copy, the owner writes the new one; halo values are formed
-// and dropped), E's auxiliaries are read and written by their owner only.
-// The new H of two planes sits in shared memory for the E update.  Per cell
-// the arithmetic is that of fdtd_h_cell / fdtd_e_cell, so results are the
-// bits of the two-kernel step.  Traffic: E and H read once, written once
-// (12 words per cell) instead of 18.  Opt-in (EMS_FDTD_FUSED=1): on the
-// 512^3 CPML workload the plane march, two barriers per plane, ran 3.42 ms
-// per step against 2.39 ms for the two kernels, latency-bound at 4 blocks
-// of 256 threads per SM.
-constexpr int kFusedKZ = 32, kFusedBX = 32, kFusedBY = 8;
-
-template <class T> struct FusedArgs {
-    FdtdArgs<T> a;                  // old fields (Ex..Hz) and the shared data
-    T *Exn, *Eyn, *Ezn, *Hxn, *Hyn, *Hzn;   // new fields
-    T *psiHn[3][2];                 // new H-type CPML auxiliaries (a.psiH: the old ones)
-};
-
-// psi recursion with separate read and write copies (write == nullptr: form only)
-template <class T>
-__device__ __forceinline__ T pml_curl_rw(T d1, T d2, const Prof<T> &p1, int s1, const Prof<T> &p2, int s2, const T *r1,
-                                         const T *r2, T *w1, T *w2)
+// One component between the device layout and the API's array (rows of w
+// values, ah rows per plane): out in the run precision, in from FP64.
+template <class T, class A, bool GET>
+__global__ void fdtd_field_kernel(T *f, A *api, size_t cnt, int w, int ah, size_t pitch, size_t plane, int shift)
 {
-    T q1 = radd(rmul(p1.b[s1], *r1), rmul(p1.a[s1], d1));
-    T q2 = radd(rmul(p2.b[s2], *r2), rmul(p2.a[s2], d2));
-    if (w1) { *w1 = q1; *w2 = q2; }
-    return rsub(radd(rsub(rmul(p1.kinv[s1], d1), rmul(p2.kinv[s2], d2)), q1), q2);
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= cnt) return;
+    const size_t r = t / w;
+    const ptrdiff_t o = (ptrdiff_t)((r / ah) * plane + (r % ah) * pitch + t % w) - shift;
+    if (GET) api[t] = (A)f[o];
+    else f[o] = (T)api[t];
 }
-
-template <class T, bool MAT, bool PML>
-__global__ void __launch_bounds__(kFusedBX * kFusedBY, 4) fdtd_fused_kernel(FusedArgs<T> f)
+// Material ids into rows of mpitch, the last column repeated, zero behind it.
+__global__ void fdtd_mat_kernel(const uint16_t *id, uint16_t *mat, size_t cnt, unsigned mpitch, int nx)
 {
-    const FdtdArgs<T> &a = f.a;
-    const FdtdStrides &st = a.st;
-    __shared__ T sH[2][3][kFusedBY][kFusedBX];   // new H of planes k (parity) for the tile and its halo
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int i = (int)blockIdx.x * (kFusedBX - 1) + tx - 1, j = (int)blockIdx.y * (kFusedBY - 1) + ty - 1;
-    const int kb = (int)blockIdx.z * kFusedKZ, ke = min(kb + kFusedKZ, a.nz + 1);
-    const bool col = i >= 0 && j >= 0 && i <= a.nx && j <= a.ny;   // an H column of the grid
-    const bool own = col && tx > 0 && ty > 0;                       // a column of the tile (E and the stored H)
-    bool slab = false;
-    if (PML) {
-        const int i0 = (int)blockIdx.x * (kFusedBX - 1) - 1, j0 = (int)blockIdx.y * (kFusedBY - 1) - 1;
-        slab = !(i0 >= a.in_lo[0] && i0 + kFusedBX <= a.in_hi[0] && j0 >= a.in_lo[1] && j0 + kFusedBY <= a.in_hi[1] &&
-                 kb - 1 >= a.in_lo[2] && ke <= a.in_hi[2]);
-    }
-    for (int k = max(kb - 1, 0); k < ke; ++k) {
-        const int pk = k & 1;
-        // ---- the E update's own loads (old E, material coefficients), issued
-        // before the H update so that their latency overlaps it and the barrier
-        const bool edo = own && k >= kb;
-        const bool ex = edo && j >= 1 && k >= 1, ey = edo && i >= 1 && k >= 1, ez = edo && i >= 1 && j >= 1;
-        const unsigned qx = i + j * st.ex_y + k * st.ex_z, qy = i + j * st.ey_y + k * st.ey_z;
-        const unsigned qz = i + j * st.ez_y + k * st.ez_z;
-        T ex0 = 0, ey0 = 0, ez0 = 0;
-        CaCb<T> c0{1, 0}, c1{1, 0}, c2{1, 0};
-        {
-            const int nx = a.nx, ny = a.ny, nz = a.nz;
-            unsigned m0 = 0, m1 = 0, m2 = 0;
-            if (ex) {
-                ex0 = __ldg(a.Ex + qx);
-                if (MAT) m0 = __ldg(a.mat + (unsigned)(i < nx ? i : nx - 1) + (unsigned)(j - 1) * st.m_y + (unsigned)(k - 1) * st.m_z);
-            }
-            if (ey) {
-                ey0 = __ldg(a.Ey + qy);
-                if (MAT) m1 = __ldg(a.mat + (unsigned)(i - 1) + (unsigned)(j < ny ? j : ny - 1) * st.m_y + (unsigned)(k - 1) * st.m_z);
-            }
-            if (ez) {
-                ez0 = __ldg(a.Ez + qz);
-                if (MAT) m2 = __ldg(a.mat + (unsigned)(i - 1) + (unsigned)(j - 1) * st.m_y + (unsigned)(k < nz ? k : nz - 1) * st.m_z);
-            }
-            if (MAT) {
-                if (ex) c0 = load_cab(a.cab + m0);
-                if (ey) c1 = load_cab(a.cab + m1);
-                if (ez) c2 = load_cab(a.cab + m2);
-            }
-        }
-        // ---- H^{n+1/2} at (i, j, k) from the old E (fdtd_h_cell)
-        T hxv = 0, hyv = 0, hzv = 0;
-        if (col) {
-            const bool store = own && k >= kb;
-            const unsigned oEx = i + j * st.ex_y + k * st.ex_z, oEy = i + j * st.ey_y + k * st.ey_z;
-            const unsigned oEz = i + j * st.ez_y + k * st.ez_z;
-            const unsigned px = i + j * st.hx_y + k * st.hx_z, py = i + j * st.hy_y + k * st.hy_z;
-            const unsigned pz = i + j * st.hz_y + k * st.hz_z;
-            const bool hx = i < a.nx, hy = j < a.ny, hz = k < a.nz;
-            T ez11 = 0, ey1k = 0, ex1k = 0, ez1 = 0, ey1 = 0, ex1 = 0, ez0 = 0, ey0 = 0, ex0 = 0, hx0 = 0, hy0 = 0, hz0 = 0;
-            if (hx || hy) ez11 = __ldg(a.Ez + oEz + 1 + st.ez_y);
-            if (hx || hz) ey1k = __ldg(a.Ey + oEy + 1 + st.ey_z);
-            if (hy || hz) ex1k = __ldg(a.Ex + oEx + st.ex_y + st.ex_z);
-            if (hx) { hx0 = __ldg(a.Hx + px); ez1 = __ldg(a.Ez + oEz + 1); ey1 = __ldg(a.Ey + oEy + 1); }
-            if (hy) { hy0 = __ldg(a.Hy + py); ex1 = __ldg(a.Ex + oEx + st.ex_y); ez0 = __ldg(a.Ez + oEz + st.ez_y); }
-            if (hz) { hz0 = __ldg(a.Hz + pz); ey0 = __ldg(a.Ey + oEy + st.ey_z); ex0 = __ldg(a.Ex + oEx + st.ex_z); }
-            if (hx) {
-                T c;
-                if (PML && slab && (a.ph[1].on[j] | a.ph[2].on[k]))
-                    c = pml_curl_rw(rsub(ez11, ez1), rsub(ey1k, ey1), a.ph[1], j, a.ph[2], k, &a.psiH[0][0][px], &a.psiH[0][1][px],
-                                    store ? &f.psiHn[0][0][px] : nullptr, store ? &f.psiHn[0][1][px] : nullptr);
-                else
-                    c = curl4(ez11, ez1, ey1k, ey1);
-                hxv = rsub(hx0, rmul(a.ch, c));
-                if (store) f.Hxn[px] = hxv;
-            }
-            if (hy) {
-                T c;
-                if (PML && slab && (a.ph[2].on[k] | a.ph[0].on[i]))
-                    c = pml_curl_rw(rsub(ex1k, ex1), rsub(ez11, ez0), a.ph[2], k, a.ph[0], i, &a.psiH[1][0][py], &a.psiH[1][1][py],
-                                    store ? &f.psiHn[1][0][py] : nullptr, store ? &f.psiHn[1][1][py] : nullptr);
-                else
-                    c = curl4(ex1k, ex1, ez11, ez0);
-                hyv = rsub(hy0, rmul(a.ch, c));
-                if (store) f.Hyn[py] = hyv;
-            }
-            if (hz) {
-                T c;
-                if (PML && slab && (a.ph[0].on[i] | a.ph[1].on[j]))
-                    c = pml_curl_rw(rsub(ey1k, ey0), rsub(ex1k, ex0), a.ph[0], i, a.ph[1], j, &a.psiH[2][0][pz], &a.psiH[2][1][pz],
-                                    store ? &f.psiHn[2][0][pz] : nullptr, store ? &f.psiHn[2][1][pz] : nullptr);
-                else
-                    c = curl4(ey1k, ey0, ex1k, ex0);
-                hzv = rsub(hz0, rmul(a.ch, c));
-                if (store) f.Hzn[pz] = hzv;
-            }
-        }
-        sH[pk][0][ty][tx] = hxv;
-        sH[pk][1][ty][tx] = hyv;
-        sH[pk][2][ty][tx] = hzv;
-        __syncthreads();
-        // ---- E^{n+1} at (i, j, k) from the new H (fdtd_e_cell)
-        if (edo) {
-            const int q = pk ^ 1;
-            const unsigned px = qx, py = qy, pz = qz;
-            // H(i,j,k-1), H(i,j-1,k), H(i-1,j,k) and the diagonal neighbours, from shared memory
-            const T hz_k = sH[q][2][ty][tx], hy_j = sH[pk][1][ty - 1][tx], hx_i = sH[pk][0][ty][tx - 1];
-            const T hz_jk = sH[q][2][ty - 1][tx], hy_jk = sH[q][1][ty - 1][tx];
-            const T hx_ik = sH[q][0][ty][tx - 1], hz_ik = sH[q][2][ty][tx - 1];
-            const T hy_ij = sH[pk][1][ty - 1][tx - 1], hx_ij = sH[pk][0][ty - 1][tx - 1];
-            auto upd = [&](T e, const CaCb<T> &m, T c) { return MAT ? radd(rmul(m.ca, e), rmul(m.cb, c)) : radd(e, rmul(a.ce, c)); };
-            if (ex) {
-                T c;
-                if (PML && slab && (a.pe[1].on[j] | a.pe[2].on[k]))
-                    c = pml_curl(rsub(hz_k, hz_jk), rsub(hy_j, hy_jk), a.pe[1], j, a.pe[2], k, &a.psiE[0][0][px], &a.psiE[0][1][px]);
-                else
-                    c = curl4(hz_k, hz_jk, hy_j, hy_jk);
-                f.Exn[px] = upd(ex0, c0, c);
-            }
-            if (ey) {
-                T c;
-                if (PML && slab && (a.pe[2].on[k] | a.pe[0].on[i]))
-                    c = pml_curl(rsub(hx_i, hx_ik), rsub(hz_k, hz_ik), a.pe[2], k, a.pe[0], i, &a.psiE[1][0][py], &a.psiE[1][1][py]);
-                else
-                    c = curl4(hx_i, hx_ik, hz_k, hz_ik);
-                f.Eyn[py] = upd(ey0, c1, c);
-            }
-            if (ez) {
-                T c;
-                if (PML && slab && (a.pe[0].on[i] | a.pe[1].on[j]))
-                    c = pml_curl(rsub(hy_j, hy_ij), rsub(hx_i, hx_ij), a.pe[0], i, a.pe[1], j, &a.psiE[2][0][pz], &a.psiE[2][1][pz]);
-                else
-                    c = curl4(hy_j, hy_ij, hx_i, hx_ij);
-                f.Ezn[pz] = upd(ez0, c2, c);
-            }
-        }
-        __syncthreads();
-    }
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= cnt) return;
+    const size_t r = t / mpitch;
+    const int i = (int)(t - r * mpitch);
+    mat[t] = i <= nx ? id[r * nx + min(i, nx - 1)] : (uint16_t)0;
 }
 
 // Point sources in insertion order: E[src] -= v (fdtd_simulation.cpp:222-239).
 template <class T>
-__global__ void fdtd_source_kernel(T *Ex, T *Ey, T *Ez, const int *comp, const size_t *off, const double *vals, int nsrc)
+__global__ void fdtd_source_kernel(T *Ex, T *Ey, T *Ez, const int *comp, const long long *off, const double *vals, int nsrc)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     for (int s = 0; s < nsrc; ++s) {
@@ -457,7 +427,7 @@ __global__ void fdtd_source_kernel(T *Ex, T *Ey, T *Ez, const int *comp, const s
 // summing its listed samples in order, then dividing by the count.
 template <class T>
 __global__ void fdtd_receiver_kernel(const T *Ex, const T *Ey, const T *Ez, int nobs, const int *cnt,
-                                     const int *start, const size_t *off, double *trace_row, int nsamp)
+                                     const int *start, const long long *off, double *trace_row, int nsamp)
 {
     int o = blockIdx.x * blockDim.x + threadIdx.x;
     if (o >= nobs) return;
@@ -468,6 +438,23 @@ __global__ void fdtd_receiver_kernel(const T *Ex, const T *Ey, const T *Ez, int 
         int n = cnt[3 * o + c];
         double acc = out[c];
         for (int r = 0; r < n; ++r, ++q) acc = __dadd_rn(acc, (double)f[off[q]]);
+        out[c] = acc / (double)n;
+    }
+}
+
+// The same averages from the values that the E kernel sampled: one thread per
+// receiver and sampled step (row 0, the start, stays zero).
+__global__ void fdtd_trace_kernel(const double *samp, int nsm, int nobs, const int *cnt, const int *start, double *traces, int nsamp)
+{
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int row = (int)(t % nsamp), o = (int)(t / nsamp);
+    if (o >= nobs || row == 0) return;
+    const double *v = samp + (size_t)row * nsm + start[o];
+    double *out = traces + ((size_t)o * nsamp + row) * 3;
+    for (int c = 0; c < 3; ++c) {
+        const int n = cnt[3 * o + c];
+        double acc = 0.0;
+        for (int r = 0; r < n; ++r) acc = __dadd_rn(acc, *v++);
         out[c] = acc / (double)n;
     }
 }
@@ -486,7 +473,7 @@ struct FdtdSource {
     int ijk[3];
     int kind;
     double f0, amp;
-    size_t off;
+    long long off;
 };
 
 struct FdtdSim : Sim {
@@ -494,22 +481,27 @@ struct FdtdSim : Sim {
     int nx, ny, nz;
     bool fp64;
     size_t n[6];
+    // device layout (see the head of the file): each array `lead` values in
+    int V, lead;
+    size_t pitch, plane, total, mpitch;
+    int g0, g1;                 // threads of a row [g0, g1) that touch no x layer
     DevBuf F[6];
-    DevBuf G[6];                // the other copy of the fields (the fused step writes it; swapped after each step)
-    bool fused = false;         // one fused H+E pass per step (EMS_FDTD_FUSED=1; default: the H and E kernels)
+    mutable DevBuf d_stage;     // a component in the API's layout
     // materials
     std::vector<uint16_t> mat_host;
     std::vector<double> mat_eps, mat_sigma;
     DevBuf d_mat, d_cab;
     // CPML
-    DevBuf d_prof[2][3][4];   // [E/H][axis][b,a,kinv,on]
+    DevBuf d_prof[2][3][3];   // [E/H][axis][b,a,kinv]
     std::vector<unsigned char> pml_on[2][3];   // host copies of the "on" flags
-    DevBuf d_psiE[3][2], d_psiH[3][2], d_psiH2[3][2];
+    int off_lo[2][3], off_hi[2][3];            // the index range between the layers
+    DevBuf d_psiE[3][2], d_psiH[3][2];
     // sources, receivers
     std::vector<FdtdSource> srcs;
     std::vector<std::vector<std::array<int, 3>>> obs_lists;   // 3 per receiver
     std::vector<int> obs_n;
     DevBuf d_src_comp, d_src_off, d_src_vals, d_obs_cnt, d_obs_start, d_obs_off, d_traces;
+    DevBuf d_pt_plane, d_pt_list, d_samp, d_step;
     bool dirty = true;
 
     explicit FdtdSim(const ems_fdtd_params *p) : Sim(Kind::FDTD), P(*p)
@@ -535,12 +527,23 @@ struct FdtdSim : Sim {
         n[4] = (size_t)(nx + 1) * ny * (nz + 1);
         n[5] = (size_t)(nx + 1) * (ny + 1) * nz;
         init_stream();
-        size_t w = fp64 ? 8 : 4;
-        if (const char *env = std::getenv("EMS_FDTD_FUSED")) fused = std::strcmp(env, "1") == 0;
-        for (int q = 0; q < 6; ++q) { F[q].alloc(n[q] * w); F[q].zero(stream); }
-        if (fused)
-            for (int q = 0; q < 6; ++q) { G[q].alloc(n[q] * w); G[q].zero(stream); }
-        if (P.pml_cells > 0) setup_pml();
+        const size_t w = fp64 ? 8 : 4;
+        V = (int)(16 / w);
+        lead = V;
+        auto up = [](size_t x, size_t m) { return (x + m - 1) / m * m; };
+        pitch = up(nx + 2 + lead, 32 / w);
+        plane = pitch * (ny + 2);
+        total = plane * (nz + 2) + lead + V;   // one more vector behind the last row is read
+        mpitch = up(nx + 1 + V, 4);
+        for (int q = 0; q < 6; ++q) { F[q].alloc(total * w); F[q].zero(stream); }
+        g0 = 0;
+        g1 = (nx + V) / V;
+        if (P.pml_cells > 0) {
+            setup_pml();
+            const int lo = std::max(off_lo[0][0] - 1, off_lo[1][0]), hi = std::min(off_hi[0][0] - 1, off_hi[1][0]);
+            g0 = std::min((lo + V - 1) / V, g1);
+            g1 = std::max(std::min(hi / V, g1), g0);
+        }
         EMS_CUDA(cudaStreamSynchronize(stream));
     }
 
@@ -569,19 +572,29 @@ struct FdtdSim : Sim {
                     kinv[s] = 1.0 / kap;
                     on[s] = 1;
                 }
+                // (whole vectors of the x profile are read)
+                for (std::vector<double> *v : {&b, &av, &kinv}) {
+                    if (eh == 0 && d == 0) v->erase(v->begin());   // from s = 1, the first column of Ey and Ez
+                    v->resize(cnt + V, v == &kinv ? 1.0 : 0.0);
+                }
                 upload_real(d_prof[eh][d][0], b);
                 upload_real(d_prof[eh][d][1], av);
                 upload_real(d_prof[eh][d][2], kinv);
-                d_prof[eh][d][3].alloc(cnt);
-                EMS_CUDA(cudaMemcpyAsync(d_prof[eh][d][3].p, on.data(), cnt, cudaMemcpyHostToDevice, stream));
                 pml_on[eh][d] = on;
+                // the index range between the two layers
+                int lo = 0, hi = cnt;
+                while (lo < hi && on[lo]) ++lo;
+                while (hi > lo && on[hi - 1]) --hi;
+                for (int q = lo; q < hi; ++q)
+                    if (on[q]) throw Error{EMS_ERR_STATE, "CPML profile is not two slabs"};
+                off_lo[eh][d] = lo;
+                off_hi[eh][d] = hi;
             }
         size_t w = fp64 ? 8 : 4;
         for (int c = 0; c < 3; ++c)
             for (int r = 0; r < 2; ++r) {
-                d_psiE[c][r].alloc(n[c] * w); d_psiE[c][r].zero(stream);
-                d_psiH[c][r].alloc(n[3 + c] * w); d_psiH[c][r].zero(stream);
-                if (fused) { d_psiH2[c][r].alloc(n[3 + c] * w); d_psiH2[c][r].zero(stream); }
+                d_psiE[c][r].alloc(total * w); d_psiE[c][r].zero(stream);
+                d_psiH[c][r].alloc(total * w); d_psiH[c][r].zero(stream);
             }
         EMS_CUDA(cudaStreamSynchronize(stream));
     }
@@ -599,11 +612,10 @@ struct FdtdSim : Sim {
         EMS_CUDA(cudaStreamSynchronize(stream));
     }
 
-    size_t ex_index(int c, const int *q) const
+    // offset of a padded index in the device layout (Ey, Ez: one column to the left)
+    long long ex_index(int c, const int *q) const
     {
-        if (c == 0) return (size_t)q[0] + (size_t)q[1] * (nx + 1) + (size_t)q[2] * (nx + 1) * (ny + 2);
-        if (c == 1) return (size_t)q[0] + (size_t)q[1] * (nx + 2) + (size_t)q[2] * (nx + 2) * (ny + 1);
-        return (size_t)q[0] + (size_t)q[1] * (nx + 2) + (size_t)q[2] * (nx + 2) * (ny + 2);
+        return (long long)q[0] - (c > 0 ? 1 : 0) + (long long)q[1] * (long long)pitch + (long long)q[2] * (long long)plane;
     }
     bool in_e(int c, const int *q) const
     {
@@ -649,56 +661,72 @@ struct FdtdSim : Sim {
             ca[m] = (1.0 - s) / (1.0 + s);
             cb[m] = P.dt / mat_eps[m] / P.h / (1.0 + s);
         }
-        d_mat.alloc(nc * 2);
-        EMS_CUDA(cudaMemcpyAsync(d_mat.p, mat_host.data(), nc * 2, cudaMemcpyHostToDevice, stream));
+        const size_t cnt = (size_t)ny * nz * mpitch;
+        d_mat.ensure(cnt * 2 + 16);
+        d_stage.ensure(nc * 2);
+        EMS_CUDA(cudaMemcpyAsync(d_stage.p, mat_host.data(), nc * 2, cudaMemcpyHostToDevice, stream));
+        fdtd_mat_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(d_stage.as<uint16_t>(), d_mat.as<uint16_t>(), cnt, (unsigned)mpitch, nx);
         std::vector<double> cab(2 * ca.size());
         for (size_t m = 0; m < ca.size(); ++m) { cab[2 * m] = ca[m]; cab[2 * m + 1] = cb[m]; }
         upload_real(d_cab, cab);
     }
 
+    // x / d = (x * magic) >> shift for x < 2^31: magic = ceil(2^shift / d) with
+    // 2^shift >= 2^31 d, so the error x (magic d - 2^shift) / 2^shift stays
+    // below 1; magic < 2^32
+    static void divider(unsigned d, unsigned &magic, unsigned &shift)
+    {
+        unsigned l = 0;
+        while ((1ull << l) < d) ++l;
+        shift = 31 + l;
+        magic = (unsigned)(((1ull << shift) + d - 1) / d);
+    }
+
     template <class T> FdtdArgs<T> args() const
     {
         FdtdArgs<T> a{};
-        a.Ex = F[0].as<T>(); a.Ey = F[1].as<T>(); a.Ez = F[2].as<T>();
-        a.Hx = F[3].as<T>(); a.Hy = F[4].as<T>(); a.Hz = F[5].as<T>();
+        T **f[6] = {&a.Ex, &a.Ey, &a.Ez, &a.Hx, &a.Hy, &a.Hz};
+        for (int q = 0; q < 6; ++q) *f[q] = F[q].as<T>() + lead;
         a.nx = nx; a.ny = ny; a.nz = nz;
-        const unsigned X = nx, Y = ny;
-        a.st = FdtdStrides{X + 1, (X + 1) * (Y + 2), X + 2, (X + 2) * (Y + 1), X + 2, (X + 2) * (Y + 2),
-                           X, X * (Y + 1), X + 1, (X + 1) * Y, X + 1, (X + 1) * (Y + 1), X, X * Y};
+        a.g0 = g0; a.g1 = g1; a.gr = (nx + V) / V - (g1 - g0);
+        divider(std::max(g1 - g0, 1), a.magic[0], a.shift[0]);
+        divider(std::max(a.gr, 1), a.magic[1], a.shift[1]);
+        a.pitch = (unsigned)pitch;
+        a.plane = plane;
+        a.mpitch = (unsigned)mpitch;
         a.ch = (T)(P.dt / P.permeability / P.h);
         a.ce = (T)(P.dt / P.permittivity / P.h);
         a.mat = d_mat.as<uint16_t>();
         a.cab = d_cab.as<CaCb<T>>();
         if (P.pml_cells > 0)
             for (int d = 0; d < 3; ++d) {
-                // the index range between the slabs, where neither profile is on
-                const auto &oe = pml_on[0][d], &oh = pml_on[1][d];
-                int lo = 0, hi = (int)oe.size();
-                while (lo < hi && (oe[lo] | oh[lo])) ++lo;
-                while (hi > lo && (oe[hi - 1] | oh[hi - 1])) --hi;
-                for (int q = lo; q < hi; ++q)
-                    if (oe[q] | oh[q]) throw Error{EMS_ERR_STATE, "CPML profile is not two slabs"};
-                a.in_lo[d] = lo;
-                a.in_hi[d] = hi;
-                a.pe[d] = Prof<T>{d_prof[0][d][0].as<T>(), d_prof[0][d][1].as<T>(), d_prof[0][d][2].as<T>(), d_prof[0][d][3].as<unsigned char>()};
-                a.ph[d] = Prof<T>{d_prof[1][d][0].as<T>(), d_prof[1][d][1].as<T>(), d_prof[1][d][2].as<T>(), d_prof[1][d][3].as<unsigned char>()};
-                for (int r = 0; r < 2; ++r) { a.psiE[d][r] = d_psiE[d][r].as<T>(); a.psiH[d][r] = d_psiH[d][r].as<T>(); }
+                const int s0 = d == 0 ? 1 : 0;   // the E-type x profile starts at s = 1
+                a.pe[d] = Prof<T>{d_prof[0][d][0].as<T>(), d_prof[0][d][1].as<T>(), d_prof[0][d][2].as<T>(), off_lo[0][d] - s0,
+                                  off_hi[0][d] - s0};
+                a.ph[d] = Prof<T>{d_prof[1][d][0].as<T>(), d_prof[1][d][1].as<T>(), d_prof[1][d][2].as<T>(), off_lo[1][d], off_hi[1][d]};
+                for (int r = 0; r < 2; ++r) {
+                    a.psiE[d][r] = d_psiE[d][r].as<T>() + lead;
+                    a.psiH[d][r] = d_psiH[d][r].as<T>() + lead;
+                }
             }
         return a;
     }
 
-    // Launch shape of the H and E kernels (x, y threads; one z plane per
-    // block row), chosen by tune_shape on the handle's first run of at least
-    // kTuneMinSteps steps.  Every cell is one thread whatever the shape, so
-    // the shape changes no result.
+    // Launch shape of the H and E kernels (x times y threads, each V cells
+    // along x; one z plane per block row), chosen on the handle's first run
+    // of at least kTuneMinSteps steps.  Every cell belongs to one thread
+    // whatever the shape, so the shape changes no result.
     dim3 blk{32, 8, 1};
     bool tuned = false;
     dim3 block() const { return blk; }
     void launch_shape(int b[3]) override { b[0] = (int)blk.x; b[1] = (int)blk.y; b[2] = 1; }
-    dim3 grid() const
+    unsigned blocks_of(int groups) const   // blocks that cover `groups` threads of every row
     {
-        return dim3((nx + 1 + blk.x - 1) / blk.x, (ny + 1 + blk.y - 1) / blk.y, (nz + 1 + kFdtdKZ - 1) / kFdtdKZ);
+        const size_t t = (size_t)groups * (ny + 1), b = (size_t)blk.x * blk.y;
+        return (unsigned)((t + b - 1) / b);
     }
+    unsigned main_blocks() const { return blocks_of(g1 - g0); }
+    dim3 grid(int planes) const { return dim3(main_blocks() + blocks_of((nx + V) / V - (g1 - g0)), 1, planes); }
 
     static constexpr int kShapes = 6, kTuneSteps = 3, kTuneMinSteps = 24;
     static constexpr unsigned kShape[kShapes][2] = {{32, 8}, {32, 4}, {64, 4}, {128, 2}, {256, 1}, {64, 2}};
@@ -720,44 +748,105 @@ struct FdtdSim : Sim {
         return nsteps >= kTuneMinSteps ? kShapes * kTuneSteps : 0;
     }
 
-    template <class T> void launch_h(const FdtdArgs<T> &a)
+    // H update of planes [k0, k1)
+    template <class T> void launch_h(const FdtdArgs<T> &a, int k0, int k1, int *ctr = nullptr, int inc = 0)
     {
-        if (P.pml_cells > 0) fdtd_h_kernel<T, true><<<grid(), block(), 0, stream>>>(a);
-        else fdtd_h_kernel<T, false><<<grid(), block(), 0, stream>>>(a);
+        if (P.pml_cells > 0) fdtd_h_kernel<T, true><<<grid(k1 - k0), block(), 0, stream>>>(a, k0, main_blocks(), ctr, inc);
+        else fdtd_h_kernel<T, false><<<grid(k1 - k0), block(), 0, stream>>>(a, k0, main_blocks(), ctr, inc);
     }
-    // The fused step: reads F (and the old H auxiliaries), writes G (and the
-    // new ones), then the copies are swapped.
-    template <class T> void launch_fused(const FdtdArgs<T> &a)
+    // E update of planes [k0, k1) with the planes' points
+    template <class T> void launch_e(const FdtdArgs<T> &a, int k0, int k1, const FdtdPoints &pt)
     {
-        FusedArgs<T> f;
-        f.a = a;
-        f.Exn = G[0].as<T>(); f.Eyn = G[1].as<T>(); f.Ezn = G[2].as<T>();
-        f.Hxn = G[3].as<T>(); f.Hyn = G[4].as<T>(); f.Hzn = G[5].as<T>();
-        for (int c = 0; c < 3; ++c)
-            for (int r = 0; r < 2; ++r) f.psiHn[c][r] = P.pml_cells > 0 ? d_psiH2[c][r].as<T>() : nullptr;
-        const dim3 blk(kFusedBX, kFusedBY, 1);
-        const dim3 grd((nx + 1 + kFusedBX - 2) / (kFusedBX - 1), (ny + 1 + kFusedBY - 2) / (kFusedBY - 1),
-                       (nz + 1 + kFusedKZ - 1) / kFusedKZ);
         const bool mat = !mat_host.empty(), pml = P.pml_cells > 0;
-        if (mat && pml) fdtd_fused_kernel<T, true, true><<<grd, blk, 0, stream>>>(f);
-        else if (mat) fdtd_fused_kernel<T, true, false><<<grd, blk, 0, stream>>>(f);
-        else if (pml) fdtd_fused_kernel<T, false, true><<<grd, blk, 0, stream>>>(f);
-        else fdtd_fused_kernel<T, false, false><<<grd, blk, 0, stream>>>(f);
+        const dim3 g = grid(k1 - k0);
+        if (mat && pml) fdtd_e_kernel<T, true, true><<<g, block(), 0, stream>>>(a, pt, k0, main_blocks());
+        else if (mat) fdtd_e_kernel<T, true, false><<<g, block(), 0, stream>>>(a, pt, k0, main_blocks());
+        else if (pml) fdtd_e_kernel<T, false, true><<<g, block(), 0, stream>>>(a, pt, k0, main_blocks());
+        else fdtd_e_kernel<T, false, false><<<g, block(), 0, stream>>>(a, pt, k0, main_blocks());
     }
-    void swap_copies()
+
+    // The sources and receiver samples as the E kernel's point lists; false
+    // where the kernels after the E update have to serve them: a point in the
+    // padding that no thread of the E kernel updates, more than 64 points in
+    // one plane (every thread of the plane looks through them), or more than
+    // 256 MB of samples.
+    static constexpr int kMaxPlanePoints = 64;
+    bool fold_points(int nsamp_run, FdtdPoints &pt)
     {
-        for (int q = 0; q < 6; ++q) std::swap(F[q].p, G[q].p);
-        if (P.pml_cells > 0)
-            for (int c = 0; c < 3; ++c)
-                for (int r = 0; r < 2; ++r) std::swap(d_psiH[c][r].p, d_psiH2[c][r].p);
+        struct Item {
+            int k;
+            FdtdPoint p;
+        };
+        std::vector<Item> items;
+        auto add = [&](int comp, const int *q, int tag, int idx) {
+            const int lo[3] = {comp == 0 ? 0 : 1, comp == 1 ? 0 : 1, comp == 2 ? 0 : 1};
+            if (q[0] < lo[0] || q[1] < lo[1] || q[2] < lo[2] || q[0] > nx || q[1] > ny || q[2] > nz) return false;
+            items.push_back({q[2], {ex_index(comp, q), comp + tag, idx}});
+            return true;
+        };
+        for (size_t s = 0; s < srcs.size(); ++s)
+            if (!add(srcs[s].comp, srcs[s].ijk, 0, (int)s)) return false;
+        int nsm = 0;
+        for (size_t l = 0; l < obs_lists.size(); ++l)
+            for (auto &q : obs_lists[l])
+                if (!add((int)(l % 3), q.data(), 4, nsm++)) return false;
+        if ((double)nsm * nsamp_run * 8.0 > 256e6) return false;
+        std::stable_sort(items.begin(), items.end(), [](const Item &x, const Item &y) { return x.k < y.k; });
+        std::vector<int> plane(nz + 2, 0);
+        std::vector<FdtdPoint> list(std::max<size_t>(items.size(), 1));
+        for (size_t q = 0; q < items.size(); ++q) {
+            list[q] = items[q].p;
+            ++plane[items[q].k + 1];
+        }
+        for (int k = 0; k <= nz; ++k) {
+            if (plane[k + 1] > kMaxPlanePoints) return false;
+            plane[k + 1] += plane[k];
+        }
+        d_pt_plane.ensure(plane.size() * sizeof(int));
+        d_pt_list.ensure(list.size() * sizeof(FdtdPoint));
+        d_samp.ensure((size_t)std::max(nsm, 1) * nsamp_run * 8);
+        EMS_CUDA(cudaMemcpyAsync(d_pt_plane.p, plane.data(), plane.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
+        EMS_CUDA(cudaMemcpyAsync(d_pt_list.p, list.data(), list.size() * sizeof(FdtdPoint), cudaMemcpyHostToDevice, stream));
+        EMS_CUDA(cudaStreamSynchronize(stream));   // the host vectors end here
+        pt = FdtdPoints{items.empty() ? nullptr : d_pt_plane.as<int>(), d_pt_list.as<FdtdPoint>(), d_src_vals.as<double>(),
+                        d_samp.as<double>(), nullptr, 0, (int)srcs.size(), nsm, P.time_frequency};
+        return true;
     }
-    template <class T> void launch_e(const FdtdArgs<T> &a)
+
+    // A graph of kGraphSteps steps, kept in the handle while the buffers and
+    // the launch shape stay the same.
+    static constexpr int kGraphSteps = 16;
+    cudaGraphExec_t graph = nullptr;
+    std::vector<unsigned long long> graph_key;
+    ~FdtdSim() override
     {
-        bool mat = !mat_host.empty(), pml = P.pml_cells > 0;
-        if (mat && pml) fdtd_e_kernel<T, true, true><<<grid(), block(), 0, stream>>>(a);
-        else if (mat) fdtd_e_kernel<T, true, false><<<grid(), block(), 0, stream>>>(a);
-        else if (pml) fdtd_e_kernel<T, false, true><<<grid(), block(), 0, stream>>>(a);
-        else fdtd_e_kernel<T, false, false><<<grid(), block(), 0, stream>>>(a);
+        if (graph) cudaGraphExecDestroy(graph);
+    }
+    template <class T> void make_graph(const FdtdArgs<T> &a, FdtdPoints pt)
+    {
+        std::vector<unsigned long long> key = {blk.x, blk.y, (unsigned long long)pt.ns, (unsigned long long)pt.nsm,
+                                               (unsigned long long)(pt.plane != nullptr), mat_host.empty()};
+        for (const void *q : {F[0].p, F[1].p, F[2].p, F[3].p, F[4].p, F[5].p, d_mat.p, d_cab.p, d_pt_plane.p, d_pt_list.p, d_src_vals.p,
+                              d_samp.p})
+            key.push_back((unsigned long long)reinterpret_cast<uintptr_t>(q));
+        if (graph && key == graph_key) return;
+        if (graph) {
+            cudaGraphExecDestroy(graph);
+            graph = nullptr;
+        }
+        pt.base = d_step.as<int>();
+        cudaGraph_t g = nullptr;
+        EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        for (int r = 0; r < kGraphSteps; ++r) {
+            launch_h<T>(a, 0, nz + 1, r == 0 ? d_step.as<int>() : nullptr, kGraphSteps);
+            pt.step = r + 1;
+            launch_e<T>(a, 0, nz + 1, pt);
+        }
+        EMS_CUDA(cudaStreamEndCapture(stream, &g));
+        const cudaError_t e = cudaGraphInstantiate(&graph, g, 0);
+        cudaGraphDestroy(g);
+        EMS_CUDA(e);
+        graph_key = key;
     }
 
     template <class T> void run_t(int nsteps)
@@ -791,34 +880,38 @@ struct FdtdSim : Sim {
             t += P.dt;
         }
         std::vector<int> comp(std::max(ns, 1));
-        std::vector<size_t> off(std::max(ns, 1));
+        std::vector<long long> off(std::max(ns, 1));
         for (int s = 0; s < ns; ++s) { comp[s] = srcs[s].comp; off[s] = srcs[s].off; }
-        d_src_comp.alloc(comp.size() * 4); d_src_off.alloc(off.size() * 8); d_src_vals.alloc(vals.size() * 8);
+        d_src_comp.ensure(comp.size() * 4); d_src_off.ensure(off.size() * 8); d_src_vals.ensure(vals.size() * 8);
         EMS_CUDA(cudaMemcpyAsync(d_src_comp.p, comp.data(), comp.size() * 4, cudaMemcpyHostToDevice, stream));
         EMS_CUDA(cudaMemcpyAsync(d_src_off.p, off.data(), off.size() * 8, cudaMemcpyHostToDevice, stream));
         EMS_CUDA(cudaMemcpyAsync(d_src_vals.p, vals.data(), vals.size() * 8, cudaMemcpyHostToDevice, stream));
         // receivers
         std::vector<int> start(std::max(nobs, 1), 0);
-        std::vector<size_t> roff;
+        std::vector<long long> roff;
         for (int o = 0; o < nobs; ++o) {
             start[o] = (int)roff.size();
             for (int c = 0; c < 3; ++c)
                 for (auto &q : obs_lists[3 * o + c]) roff.push_back(ex_index(c, q.data()));
         }
         if (roff.empty()) roff.push_back(0);
-        d_obs_cnt.alloc(std::max<size_t>(obs_n.size(), 1) * 4);
-        d_obs_start.alloc(start.size() * 4);
-        d_obs_off.alloc(roff.size() * 8);
+        d_obs_cnt.ensure(std::max<size_t>(obs_n.size(), 1) * 4);
+        d_obs_start.ensure(start.size() * 4);
+        d_obs_off.ensure(roff.size() * 8);
         if (!obs_n.empty()) EMS_CUDA(cudaMemcpyAsync(d_obs_cnt.p, obs_n.data(), obs_n.size() * 4, cudaMemcpyHostToDevice, stream));
         EMS_CUDA(cudaMemcpyAsync(d_obs_start.p, start.data(), start.size() * 4, cudaMemcpyHostToDevice, stream));
         EMS_CUDA(cudaMemcpyAsync(d_obs_off.p, roff.data(), roff.size() * 8, cudaMemcpyHostToDevice, stream));
         size_t ntr = (size_t)std::max(nobs, 1) * nsamp * 3;
-        d_traces.alloc(ntr * 8);
+        d_traces.ensure(ntr * 8);
+        d_step.ensure(sizeof(int));
         d_traces.zero(stream);
 
         FdtdArgs<T> a = args<T>();
         long long launches = 0;
-        const int tune = fused ? 0 : tune_steps(nsteps);
+        const int tune = tune_steps(nsteps);
+        FdtdPoints pt{};
+        const bool folded = fold_points(nsamp, pt);
+        const FdtdPoints none{};
         struct TuneEvents {   // destroyed on every exit path
             cudaEvent_t e[2 * kShapes] = {};
             ~TuneEvents()
@@ -830,30 +923,26 @@ struct FdtdSim : Sim {
         if (tune)
             for (cudaEvent_t &x : tev.e) EMS_CUDA(cudaEventCreate(&x));
         EMS_CUDA(cudaEventRecord(ev0, stream));
-        for (int step = 1; step < nsteps + 1; ++step) {
+        int step = 1;
+        const auto direct = [&](int last) {   // steps up to `last`, launch by launch
+        for (; step <= last; ++step) {
             const int ts = step - 1, c = ts / kTuneSteps, r = ts % kTuneSteps;
             if (ts < tune) {
                 blk = dim3(kShape[c][0], kShape[c][1], 1);
                 if (r == 1) EMS_CUDA(cudaEventRecord(tev.e[2 * c], stream));
             }
-            if (fused) {
-                launch_fused<T>(a);
-                swap_copies();
-                a = args<T>();
-                launches += 1;
-            } else {
-                launch_h<T>(a);
-                launch_e<T>(a);
-                launches += 2;
-            }
-            if (ns > 0) {
-                fdtd_source_kernel<T><<<1, 32, 0, stream>>>(a.Ex, a.Ey, a.Ez, d_src_comp.as<int>(), d_src_off.as<size_t>(),
+            launch_h<T>(a, 0, nz + 1);
+            pt.step = step;
+            launch_e<T>(a, 0, nz + 1, folded ? pt : none);
+            launches += 2;
+            if (ns > 0 && !folded) {
+                fdtd_source_kernel<T><<<1, 32, 0, stream>>>(a.Ex, a.Ey, a.Ez, d_src_comp.as<int>(), d_src_off.as<long long>(),
                                                            d_src_vals.as<double>() + (size_t)(step - 1) * ns, ns);
                 ++launches;
             }
-            if (nobs > 0 && step % tf == 0) {
+            if (nobs > 0 && !folded && step % tf == 0) {
                 fdtd_receiver_kernel<T><<<(nobs + 127) / 128, 128, 0, stream>>>(
-                    a.Ex, a.Ey, a.Ez, nobs, d_obs_cnt.as<int>(), d_obs_start.as<int>(), d_obs_off.as<size_t>(),
+                    a.Ex, a.Ey, a.Ez, nobs, d_obs_cnt.as<int>(), d_obs_start.as<int>(), d_obs_off.as<long long>(),
                     d_traces.as<double>() + (size_t)(step / tf) * 3, nsamp);
                 ++launches;
             }
@@ -869,6 +958,28 @@ struct FdtdSim : Sim {
                 }
                 blk = dim3(kShape[pick][0], kShape[pick][1], 1);
                 tuned = true;
+            }
+        }
+        };
+        if (!folded) {
+            direct(nsteps);
+        } else {
+            direct(std::min(tune, nsteps));
+            if (nsteps - step + 1 >= kGraphSteps) {
+                make_graph<T>(a, pt);
+                const int base = step - 1 - kGraphSteps;   // the graph's first launch moves it on
+                EMS_CUDA(cudaMemcpyAsync(d_step.p, &base, sizeof(int), cudaMemcpyHostToDevice, stream));
+                for (; step + kGraphSteps - 1 <= nsteps; step += kGraphSteps) {
+                    EMS_CUDA(cudaGraphLaunch(graph, stream));
+                    launches += 2 * kGraphSteps;
+                }
+            }
+            direct(nsteps);
+            if (nobs > 0 && nsamp > 1) {
+                const size_t nt = (size_t)nobs * nsamp;
+                fdtd_trace_kernel<<<(unsigned)((nt + 127) / 128), 128, 0, stream>>>(d_samp.as<double>(), pt.nsm, nobs, d_obs_cnt.as<int>(),
+                                                                                    d_obs_start.as<int>(), d_traces.as<double>(), nsamp);
+                ++launches;
             }
         }
         EMS_CUDA(cudaGetLastError());
@@ -887,7 +998,7 @@ struct FdtdSim : Sim {
     {
         EMS_CHECK_ARG(nsteps >= 0, "num_steps must be >= 0");
         if (fp64) run_t<double>(nsteps); else run_t<float>(nsteps);
-        check_finite({{F[0].p, n[0]}, {F[1].p, n[1]}, {F[2].p, n[2]}, {F[3].p, n[3]}, {F[4].p, n[4]}, {F[5].p, n[5]}}, fp64);
+        check_finite({{F[0].p, total}, {F[1].p, total}, {F[2].p, total}, {F[3].p, total}, {F[4].p, total}, {F[5].p, total}}, fp64);
     }
 
     size_t field_size(int which) const override
@@ -895,28 +1006,29 @@ struct FdtdSim : Sim {
         if (which < 0 || which > 5) throw Error{EMS_ERR_INVALID_ARGUMENT, "field index must be 0..5 (Ex,Ey,Ez,Hx,Hy,Hz)"};
         return n[which];
     }
+    // a component between the device layout and the API's (in d_stage)
+    template <class T, class A, bool GET> void move_field(int which) const
+    {
+        const int w[6] = {nx + 1, nx + 2, nx + 2, nx, nx + 1, nx + 1}, h[6] = {ny + 2, ny + 1, ny + 2, ny + 1, ny, ny + 1};
+        const size_t cnt = n[which];
+        fdtd_field_kernel<T, A, GET><<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(
+            F[which].as<T>() + lead, d_stage.as<A>(), cnt, w[which], h[which], pitch, plane, which == 1 || which == 2 ? 1 : 0);
+        EMS_CUDA(cudaGetLastError());
+    }
     void get_field(int which, double *out) const override
     {
-        size_t cnt = field_size(which);
-        if (fp64) {
-            EMS_CUDA(cudaMemcpy(out, F[which].p, cnt * 8, cudaMemcpyDeviceToHost));
-        } else {
-            std::vector<float> tmp(cnt);
-            EMS_CUDA(cudaMemcpy(tmp.data(), F[which].p, cnt * 4, cudaMemcpyDeviceToHost));
-            for (size_t q = 0; q < cnt; ++q) out[q] = tmp[q];
-        }
+        const size_t cnt = field_size(which);
+        d_stage.ensure(cnt * (fp64 ? 8 : 4));
+        if (fp64) move_field<double, double, true>(which); else move_field<float, float, true>(which);
+        download(out, d_stage.p, cnt, fp64);
     }
     void set_field(int which, const double *in) override
     {
-        size_t cnt = field_size(which);
-        if (fp64) {
-            EMS_CUDA(cudaMemcpy(F[which].p, in, cnt * 8, cudaMemcpyHostToDevice));
-        } else {
-            std::vector<float> tmp(in, in + cnt);
-            EMS_CUDA(cudaMemcpy(F[which].p, tmp.data(), cnt * 4, cudaMemcpyHostToDevice));
-        }
-        // the fused step never writes the boundary values of the other copy: keep them equal
-        if (fused) EMS_CUDA(cudaMemcpy(G[which].p, F[which].p, F[which].bytes, cudaMemcpyDeviceToDevice));
+        const size_t cnt = field_size(which);
+        d_stage.ensure(cnt * 8);
+        EMS_CUDA(cudaMemcpyAsync(d_stage.p, in, cnt * 8, cudaMemcpyHostToDevice, stream));
+        if (fp64) move_field<double, double, false>(which); else move_field<float, double, false>(which);
+        EMS_CUDA(cudaStreamSynchronize(stream));
     }
 
     // fdtd_simulation.cpp:308-331: results_<i>_<dt>_<h>_<N>.csv in `path`
@@ -944,13 +1056,10 @@ struct FdtdSim : Sim {
     void reset() override
     {
         for (int q = 0; q < 6; ++q) F[q].zero(stream);
-        if (fused)
-            for (int q = 0; q < 6; ++q) G[q].zero(stream);
         if (P.pml_cells > 0)
             for (int c = 0; c < 3; ++c)
                 for (int r = 0; r < 2; ++r) {
                     d_psiE[c][r].zero(stream); d_psiH[c][r].zero(stream);
-                    if (fused) d_psiH2[c][r].zero(stream);
                 }
         EMS_CUDA(cudaStreamSynchronize(stream));
     }
@@ -968,63 +1077,11 @@ struct FdtdSim : Sim {
         return (nx + 1.0) * pairs(1, ny, 2, nz) + (ny + 1.0) * pairs(2, nz, 0, nx) + (nz + 1.0) * pairs(0, nx, 1, ny);
     }
 
-    // H-type points whose update runs the CPML recursion (two psi values each).
-    double pml_h_points() const
-    {
-        if (P.pml_cells <= 0) return 0.0;
-        auto pairs = [&](int d1, int n1, int d2, int n2) {
-            double c = 0.0;
-            for (int a = 0; a <= n1; ++a)
-                for (int b = 0; b <= n2; ++b) c += (pml_on[1][d1][a] | pml_on[1][d2][b]) ? 1.0 : 0.0;
-            return c;
-        };
-        return (double)nx * pairs(1, ny, 2, nz) + (double)ny * pairs(2, nz, 0, nx) + (double)nz * pairs(0, nx, 1, ny);
-    }
-
     void time_dominant(int launches, double *ms, double *bytes, std::string *name) override
     {
         size_t w = fp64 ? 8 : 4;
         size_t cells = (size_t)nx * ny * nz;
         const double matb = mat_host.empty() ? 0.0 : 2.0 * cells;
-        if (fused) {
-            // the fused step: E and H read and written once (12 words per
-            // cell), the material id, two psi values read and written per
-            // CPML point of either type.  It reads F and writes G (and the
-            // new H auxiliaries); E's auxiliaries change in place, so they
-            // are kept and put back.
-            double b = (double)cells * 12.0 * w + matb + (pml_e_points() + pml_h_points()) * 4.0 * w;
-            DevBuf save[6];
-            if (P.pml_cells > 0)
-                for (int c = 0; c < 3; ++c)
-                    for (int r = 0; r < 2; ++r) {
-                        DevBuf &sv = save[2 * c + r];
-                        sv.alloc(d_psiE[c][r].bytes);
-                        EMS_CUDA(cudaMemcpyAsync(sv.p, d_psiE[c][r].p, d_psiE[c][r].bytes, cudaMemcpyDeviceToDevice, stream));
-                    }
-            float t = 0;
-            auto body = [&](auto tag) {
-                using T = decltype(tag);
-                auto a = args<T>();
-                launch_fused<T>(a);
-                EMS_CUDA(cudaEventRecord(ev0, stream));
-                for (int r = 0; r < launches; ++r) launch_fused<T>(a);
-                EMS_CUDA(cudaEventRecord(ev1, stream));
-            };
-            if (fp64) body(double()); else body(float());
-            EMS_CUDA(cudaStreamSynchronize(stream));
-            EMS_CUDA(cudaEventElapsedTime(&t, ev0, ev1));
-            if (P.pml_cells > 0) {
-                size_t q = 0;
-                for (int c = 0; c < 3; ++c)
-                    for (int r = 0; r < 2; ++r, ++q)
-                        EMS_CUDA(cudaMemcpyAsync(d_psiE[c][r].p, save[q].p, d_psiE[c][r].bytes, cudaMemcpyDeviceToDevice, stream));
-            }
-            EMS_CUDA(cudaStreamSynchronize(stream));
-            *ms = t / launches;
-            *bytes = b;
-            *name = fp64 ? "fdtd_fused_kernel<double>" : "fdtd_fused_kernel<float>";
-            return;
-        }
         // E update: reads H (3), reads and writes E (3), the material id, and
         // reads and writes two psi values per point inside the CPML
         double b = (double)cells * 9.0 * w + matb + pml_e_points() * 4.0 * w;
@@ -1034,8 +1091,8 @@ struct FdtdSim : Sim {
             EMS_CUDA(cudaMemcpyAsync(save[q].p, F[q].p, F[q].bytes, cudaMemcpyDeviceToDevice, stream));
         }
         float t = 0;
-        if (fp64) { auto a = args<double>(); launch_e<double>(a); EMS_CUDA(cudaEventRecord(ev0, stream)); for (int r = 0; r < launches; ++r) launch_e<double>(a); }
-        else { auto a = args<float>(); launch_e<float>(a); EMS_CUDA(cudaEventRecord(ev0, stream)); for (int r = 0; r < launches; ++r) launch_e<float>(a); }
+        if (fp64) { auto a = args<double>(); launch_e<double>(a, 0, nz + 1, {}); EMS_CUDA(cudaEventRecord(ev0, stream)); for (int r = 0; r < launches; ++r) launch_e<double>(a, 0, nz + 1, {}); }
+        else { auto a = args<float>(); launch_e<float>(a, 0, nz + 1, {}); EMS_CUDA(cudaEventRecord(ev0, stream)); for (int r = 0; r < launches; ++r) launch_e<float>(a, 0, nz + 1, {}); }
         EMS_CUDA(cudaEventRecord(ev1, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
         EMS_CUDA(cudaEventElapsedTime(&t, ev0, ev1));

@@ -258,3 +258,57 @@ def test_sphere_workload_at_full_size_bitwise_equal_to_oracle():
     np.testing.assert_array_equal(t[:, :, 2], tr_o[:, :, 2])
     for k, v in s.fields().items():
         np.testing.assert_array_equal(v, f_o[k], err_msg=k)
+
+
+@pytest.mark.parametrize("points", ["inside", "padding", "many"])
+@pytest.mark.parametrize("grid,pml", [((1, 1, 1), 0), ((3, 2, 5), 0), ((4, 4, 4), 1), ((5, 9, 3), 1), ((33, 6, 7), 2), ((31, 8, 12), 3),
+                                      ((64, 5, 5), 2)])
+def test_pitched_layout_and_served_points_bitwise_equal_to_oracle(grid, pml, points):
+    """Rows that end inside a thread's 16 bytes, random fields everywhere
+    (padding too), materials, CPML, sampling every third step over a run with
+    tuned, replayed and single steps; sources and samples that the E kernel
+    serves itself, that lie in the padding, or that are too many in a plane."""
+    nx, ny, nz = grid
+    h = 1e-3
+    dt = 0.9 * h / (2.998e8 * np.sqrt(3))
+    rng = np.random.default_rng(nx + 100 * ny)
+    ids = rng.integers(0, 3, (nz, ny, nx)).astype(np.uint16)
+    first = list(dict.fromkeys(ids.ravel().tolist()))          # library table: materials in first-occurrence order
+    te, ts = rng.uniform(1, 4, 3) * EPS0, rng.uniform(0, 0.05, 3)
+    lim = [(nx + 1, ny + 2, nz + 2), (nx + 2, ny + 1, nz + 2), (nx + 2, ny + 2, nz + 1)]
+
+    def point(c, lo):
+        top = lim[c] if lo == 0 else tuple(v + 1 for v in grid)
+        at = [int(rng.integers(0 if d == c else lo, top[d])) for d in range(3)]
+        if lo == 0:                                             # a source's material is that of its cell: keep the cell inside
+            at = [min(max(v, 0 if d == c else 1), grid[d]) for d, v in enumerate(at)]
+        return tuple(at)
+
+    srcs = [(c, point(c, 1), 1, float(rng.uniform(1e10, 4e10)), float(rng.uniform(-2, 2))) for c in (0, 1, 2, 2)]
+    srcs.append(srcs[0])                                        # twice at one place: insertion order
+    obs = [([point(0, 1)], [point(1, 1), point(1, 1)], [srcs[2][1]]) for _ in range(3)]
+    if points == "padding":
+        obs.append(([(0, 0, 0)], [(nx + 1, 0, nz + 1)], [(0, ny + 1, 0), (nx + 1, 1, nz)]))
+    if points == "many":
+        obs.append(([(0, 1, 1)] * 70, [(1, 0, 1)], [(1, 1, 0)]))
+    keys = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
+    f0 = {k: rng.standard_normal(v) for k, v in oracle.fdtd_shapes(nx, ny, nz).items()}
+    steps = 37
+    pd = dict(cells=pml, m=3.0, kmax=2.0, amax=0.02, R0=1e-5) if pml else None
+    tr_o, f_o = oracle.fdtd_run(nx, ny, nz, h, dt, EPS0, MU0, 3, steps, srcs, obs, material=(ids, te, ts), pml=pd, fields=f0)
+    s = ems.FdtdSimulation(grid, h, dt, EPS0, MU0, 3, precision=ems.FP64, pml_cells=pml, pml_kappa_max=2.0, pml_alpha_max=0.02,
+                           pml_reflection=1e-5)
+    s.set_material(te[ids], ts[ids])
+    assert len(first) <= 3
+    for c, at, kind, f, amp in srcs:
+        (s.setSource_x, s.setSource_y, s.setSource_z)[c](at, waveform=kind, f0=f, amplitude=amp)
+    for o in obs:
+        s.setObservationPoint(o)
+    for _ in range(2):                                          # the second run replays the kept graph
+        s.reset()
+        for q, k in enumerate(keys):
+            s.set_field(q, f0[k])
+        s.run(steps)
+        np.testing.assert_array_equal(s.traces(), tr_o)
+        for k, v in s.fields().items():
+            np.testing.assert_array_equal(v, f_o[k], err_msg=k)
