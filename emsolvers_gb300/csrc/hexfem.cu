@@ -11,11 +11,16 @@
 // fem_simulation.cpp:424-455 first, then inner elements) with unfused
 // operations, and the source enters between the outer and inner sweeps as in
 // the reference; the result is bit-identical to the serial reference.
+// Orders 1 and 2 run in two passes: the element values K u of every element,
+// then the DOFs, which sum theirs and take the whole update of the substep.
+// Order 3 forms the rows DOF by DOF (144 values per element do not fit the
+// registers of the element pass).
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <fstream>
 #include <iomanip>
+#include <utility>
 
 #include "ems_internal.hpp"
 
@@ -56,6 +61,19 @@ __device__ __forceinline__ bool on_pec(const HexGeom &g, int c, int ix, int iy, 
     if (c == 1) return ix == 0 || ix == g.gx || iz == 0 || iz == g.gz;
     return ix == 0 || ix == g.gx || iy == 0 || iy == g.gy;
 }
+
+// Source values of the run: entry (step, substep) of vals for every source.
+struct SrcTab {
+    int n, nsub, q;
+    int comp[kMaxSrc];
+    int idx[kMaxSrc];
+    const double *vals;
+    // steps done, counted twice: step[0] is read by the sampling and moved on
+    // by a step's last launch, step[1] by its first element pass and read by
+    // the DOF passes, so no launch reads what it writes
+    int *step;
+    bool last;
+};
 
 struct SrcList {
     int n;
@@ -147,10 +165,10 @@ __device__ __forceinline__ void dof_coords(const HexGeom &g, int c, size_t t, in
 {
     int nxc = c == 0 ? g.gx : g.gx + 1;
     int nyc = c == 1 ? g.gy : g.gy + 1;
-    ix = (int)(t % nxc);
-    size_t r = t / nxc;
-    iy = (int)(r % nyc);
+    const unsigned u = (unsigned)t, r = u / nxc;   // a component holds fewer than 2^31 values (int offsets throughout)
+    ix = (int)(u - r * nxc);
     iz = (int)(r / nyc);
+    iy = (int)(r - (unsigned)iz * nyc);
 }
 
 // Leapfrog step, one thread per DOF: E2 = (-K E1, boundary zeroed) + 2 E1 - E0,
@@ -224,12 +242,11 @@ __global__ void hex_drift_kernel(HexGeom g, T *Ux, T *Uy, T *Uz, T *Px, T *Py, T
     U[t] = u;
 }
 
-// Receivers: fem_v2/fem_simulation.cpp:1273-1312 (one thread per receiver).
+// Receivers: fem_v2/fem_simulation.cpp:1273-1312 (one thread per receiver),
+// row s of the table.
 template <class T>
-__global__ void hex_sample_kernel(HexGeom g, const T *Lx, const T *Ly, const T *Lz, int nobs, const int *obs, double *tr, int nsamp, int s)
+__device__ __forceinline__ void hex_sample(const HexGeom &g, const T *Lx, const T *Ly, const T *Lz, int o, const int *obs, double *tr, int nsamp, int s)
 {
-    int o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= nobs) return;
     const int gx = g.gx, gy = g.gy;
     int ox = obs[3 * o], oy = obs[3 * o + 1], oz = obs[3 * o + 2];
     double *out = tr + ((size_t)o * nsamp + s) * 4;
@@ -238,6 +255,268 @@ __global__ void hex_sample_kernel(HexGeom g, const T *Lx, const T *Ly, const T *
     out[1] = a / 4.0;
     out[2] = b / 4.0;
     out[3] = (double)Lz[oz];
+}
+
+template <class T>
+__global__ void hex_sample_kernel(HexGeom g, const T *Lx, const T *Ly, const T *Lz, int nobs, const int *obs, double *tr, int nsamp, int s,
+                                  const int *step, int tf)
+{
+    if (step) {   // a replayed step: the row from the step counter
+        if (*step % tf) return;
+        s = *step / tf;
+    }
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o < nobs) hex_sample<T>(g, Lx, Ly, Lz, o, obs, tr, nsamp, s);
+}
+// Sampling by the blocks behind the elements' of a leapfrog step's element
+// pass (it reads the level that is sampled).
+struct HexRec {
+    int n, nsamp, tf;
+    const int *obs;
+    double *tr;
+};
+
+// The step counter and the sampling blocks of an element pass; true for a
+// block without elements.
+template <class T>
+__device__ __forceinline__ bool hex_elem_head(const HexGeom &g, const T *Ux, const T *Uy, const T *Uz, int ne, int nt, int *step, const HexRec &rec)
+{
+    if (step && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) step[1] += 1;
+    const int first = (ne + nt - 1) / nt, b = (int)blockIdx.x - first;
+    if (b < 0) return false;
+    const int o = b * nt + threadIdx.x;
+    if (blockIdx.y == 0 && o < rec.n && step[0] % rec.tf == 0) hex_sample<T>(g, Ux, Uy, Uz, o, rec.obs, rec.tr, rec.nsamp, step[0] / rec.tf);
+    return true;
+}
+
+// Element pass: rows c D .. c D + D - 1 of K u of one element per thread
+// (component c = blockIdx.y), fe[row][element].  Each sum runs in column order
+// as dof_force's.  The element's values stay in registers, the rows of K are
+// read from shared memory, one vector for two or four rows of a column, so a
+// value of K costs a quarter to half a load instead of one per DOF and
+// element.  Order 2 on 72^3 grid cells, symp4: FP32 278 us a step in one pass DOF
+// by DOF, 95.7 in two; FP64, bound by the FP64 pipe, 2402 and 1877.  step: given to a step's first pass (see SrcTab).
+template <class T, int O, bool EXACT>
+__global__ void __launch_bounds__(128) hex_elem_kernel(HexGeom g, const T *__restrict__ K, const T *__restrict__ Ux, const T *__restrict__ Uy,
+                                                       const T *__restrict__ Uz, T *__restrict__ fe, int *step, HexRec rec)
+{
+    constexpr int D = O * (O + 1) * (O + 1), TT = 3 * D, W = 16 / (int)sizeof(T), RP = (D + W - 1) / W * W;
+    __shared__ __align__(16) T sK[TT * RP];
+    const int c = blockIdx.y;
+    const int ne = g.EX * g.EY * g.EZ, e = blockIdx.x * 128 + threadIdx.x;
+    if (hex_elem_head<T>(g, Ux, Uy, Uz, ne, 128, step, rec)) return;
+    for (int q = threadIdx.x; q < TT * D; q += 128) sK[(q % TT) * RP + q / TT] = K[(size_t)c * D * TT + q];
+    __syncthreads();
+    if (e >= ne) return;
+    const int r0 = e / g.EX, ei = e - r0 * g.EX, ek = r0 / g.EY, ej = r0 - ek * g.EY;
+    const int gx = g.gx, gy = g.gy;
+    const T *px = Ux + (O * ei + O * ej * gx + (size_t)(O * ek) * gx * (gy + 1));
+    const T *py = Uy + (O * ei + O * ej * (gx + 1) + (size_t)(O * ek) * (gx + 1) * gy);
+    const T *pz = Uz + (O * ei + O * ej * (gx + 1) + (size_t)(O * ek) * (gx + 1) * (gy + 1));
+    T u[TT];
+    int at = 0;
+#pragma unroll
+    for (int n = 0; n < O + 1; ++n)
+#pragma unroll
+        for (int m = 0; m < O + 1; ++m)
+#pragma unroll
+            for (int l = 0; l < O; ++l) u[at++] = px[l + m * gx + n * gx * (gy + 1)];
+#pragma unroll
+    for (int n = 0; n < O + 1; ++n)
+#pragma unroll
+        for (int m = 0; m < O; ++m)
+#pragma unroll
+            for (int l = 0; l < O + 1; ++l) u[at++] = py[l + m * (gx + 1) + n * (gx + 1) * gy];
+#pragma unroll
+    for (int n = 0; n < O; ++n)
+#pragma unroll
+        for (int m = 0; m < O + 1; ++m)
+#pragma unroll
+            for (int l = 0; l < O + 1; ++l) u[at++] = pz[l + m * (gx + 1) + n * (gx + 1) * (gy + 1)];
+    T f[RP];
+#pragma unroll
+    for (int r = 0; r < RP; ++r) f[r] = T(0);
+#pragma unroll
+    for (int mm = 0; mm < TT; ++mm) {
+        T k[RP];
+#pragma unroll
+        for (int r = 0; r < RP; r += W) *reinterpret_cast<int4 *>(&k[r]) = *reinterpret_cast<const int4 *>(&sK[mm * RP + r]);
+#pragma unroll
+        for (int r = 0; r < D; ++r) f[r] = EXACT ? xadd(f[r], xmul(k[r], u[mm])) : fma(k[r], u[mm], f[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < D; ++r) fe[(size_t)(c * D + r) * ne + e] = f[r];
+}
+
+// Order-1 element pass in FP64.  The entries of K have one size per class:
+// edges of one direction by how many of their two offsets differ, edges of
+// two directions by whether their offset along the third axis differs.  So a
+// column needs 5 products, not 12, and a product enters the rows with their
+// signs (exact): 204 FP64 operations per element instead of 288.  The host
+// checks the classes on the K it loaded and takes hex_elem_kernel otherwise.
+struct HexClasses {
+    double k[5];
+    unsigned sign[12];   // bit j: entry (row, j) is negative
+};
+__host__ __device__ constexpr int hex1_pos(int e, int axis)   // offset of local edge e along an axis
+{
+    const int c = e / 4, q = e % 4, lo = q & 1, hi = q >> 1;
+    return axis == c ? 0 : c == 0 ? (axis == 1 ? lo : hi) : c == 1 ? (axis == 0 ? lo : hi) : (axis == 0 ? lo : hi);
+}
+__host__ __device__ constexpr int hex1_class(int i, int j)
+{
+    const int c = i / 4, d = j / 4;
+    if (c != d) return 3 + (hex1_pos(i, 3 - c - d) != hex1_pos(j, 3 - c - d) ? 1 : 0);
+    int n = 0;
+    for (int a = 0; a < 3; ++a) n += hex1_pos(i, a) != hex1_pos(j, a) ? 1 : 0;
+    return n;
+}
+template <int J, int... I>
+__device__ __forceinline__ void hex1_column(std::integer_sequence<int, I...>, const double (&p)[5], const HexClasses &k, double (&f)[12])
+{
+    ((f[I] = __dadd_rn(f[I], __hiloint2double(__double2hiint(p[hex1_class(I, J)]) ^ (int)((k.sign[I] >> J & 1u) << 31),
+                                              __double2loint(p[hex1_class(I, J)])))), ...);
+}
+template <int... J>
+__device__ __forceinline__ void hex1_columns(std::integer_sequence<int, J...>, const double (&u)[12], const HexClasses &k, double (&f)[12])
+{
+    auto col = [&](auto j) {
+        constexpr int C = decltype(j)::value;
+        double p[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) p[q] = __dmul_rn(k.k[q], u[C]);
+        hex1_column<C>(std::make_integer_sequence<int, 12>{}, p, k, f);
+    };
+    (col(std::integral_constant<int, J>{}), ...);
+}
+__global__ void __launch_bounds__(32) hex1_elem_kernel(HexGeom g, const __grid_constant__ HexClasses k, const double *__restrict__ Ux,
+                                                       const double *__restrict__ Uy, const double *__restrict__ Uz, double *__restrict__ fe,
+                                                       int *step, HexRec rec)
+{
+    const int ne = g.EX * g.EY * g.EZ, e = blockIdx.x * 32 + threadIdx.x;
+    if (hex_elem_head<double>(g, Ux, Uy, Uz, ne, 32, step, rec) || e >= ne) return;
+    const int r0 = e / g.EX, ei = e - r0 * g.EX, ek = r0 / g.EY, ej = r0 - ek * g.EY, gx = g.gx, gy = g.gy;
+    const double *px = Ux + (ei + ej * gx + (size_t)ek * gx * (gy + 1));
+    const double *py = Uy + (ei + ej * (gx + 1) + (size_t)ek * (gx + 1) * gy);
+    const double *pz = Uz + (ei + ej * (gx + 1) + (size_t)ek * (gx + 1) * (gy + 1));
+    double u[12], f[12];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        u[q] = px[(q & 1) * gx + (q >> 1) * gx * (gy + 1)];
+        u[4 + q] = py[(q & 1) + (q >> 1) * (gx + 1) * gy];
+        u[8 + q] = pz[(q & 1) + (q >> 1) * (gx + 1)];
+    }
+#pragma unroll
+    for (int r = 0; r < 12; ++r) f[r] = 0.0;
+    hex1_columns(std::make_integer_sequence<int, 12>{}, u, k, f);
+#pragma unroll
+    for (int r = 0; r < 12; ++r) fe[(size_t)r * ne + e] = f[r];
+}
+
+// Sum of a DOF's element values with the source: dof_force's order with the
+// (at most four) elements in fixed slots, two positions along each of the two
+// axes across the edge.
+template <class T, int O, bool EXACT>
+__device__ __forceinline__ T dof_sum(const HexGeom &g, const T *__restrict__ fe, int c, int ix, int iy, int iz, T sign, bool has_src, T srcval)
+{
+    constexpr int D = O * (O + 1) * (O + 1);
+    const int pc = c == 0 ? ix : c == 1 ? iy : iz, nec = c == 0 ? g.EX : c == 1 ? g.EY : g.EZ;
+    const int pa = c == 0 ? iy : ix, na = c == 0 ? g.EY : g.EX;   // the outer of the two axes
+    const int pb = c == 2 ? iy : iz, nb = c == 2 ? g.EY : g.EZ;   // the inner one
+    const int ec = pc / O, lc = pc - O * ec, ea = pa / O, la = pa - O * ea, eb = pb / O, lb = pb - O * eb;
+    const size_t ne = (size_t)g.EX * g.EY * g.EZ;
+    T v[4];
+    int rk[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        const int sa = s >> 1, sb = s & 1;
+        const int ua = ea - sa, ub = eb - sb, fa = sa ? O : la, fb = sb ? O : lb;   // element and place along each axis
+        const bool in = ec < nec && ua >= 0 && ua < na && ub >= 0 && ub < nb && (!sa || la == 0) && (!sb || lb == 0);
+        const int ex = c == 0 ? ec : ua, ey = c == 1 ? ec : c == 0 ? ua : ub, ez = c == 2 ? ec : ub;
+        const int l = c == 0 ? lc : fa, m = c == 1 ? lc : c == 0 ? fa : fb, n = c == 2 ? lc : fb;
+        const int row = c * D + l + m * (c == 0 ? O : O + 1) + n * (c == 2 ? (O + 1) * (O + 1) : O * (O + 1));
+        v[s] = in ? fe[row * ne + (ex + g.EX * (ey + (size_t)g.EY * ez))] : T(0);
+        rk[s] = !in ? 0x7fffffff : EXACT ? elem_rank(g, ex, ey, ez) : s;
+    }
+    if (EXACT) {   // by visiting rank
+        auto order = [&](int x, int y) {
+            if (rk[x] > rk[y]) {
+                const int r = rk[x];
+                rk[x] = rk[y];
+                rk[y] = r;
+                const T t = v[x];
+                v[x] = v[y];
+                v[y] = t;
+            }
+        };
+        order(0, 1); order(2, 3); order(0, 2); order(1, 3); order(1, 2);
+    }
+    T acc = 0;
+    bool src_done = !has_src;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        if (rk[s] == 0x7fffffff) continue;
+        if (!src_done && rk[s] >= g.nouter) { acc = xadd(acc, srcval); src_done = true; }
+        acc = sign < 0 ? xsub(acc, v[s]) : xadd(acc, v[s]);
+    }
+    if (!src_done) acc = xadd(acc, srcval);
+    return acc;
+}
+
+template <class T> struct HexDofs {
+    T *a[3], *b[3], *c[3];   // leapfrog: E1, E0, E2; symplectic: U, P, F
+};
+
+// DOF pass of a leapfrog step (see hex_leapfrog_kernel).
+template <class T, int O, bool EXACT>
+__global__ void __launch_bounds__(128) hex_leap_dof_kernel(const __grid_constant__ HexGeom g, const T *__restrict__ fe, const __grid_constant__ HexDofs<T> d,
+                                                           const __grid_constant__ SrcTab src)
+{
+    const int c = blockIdx.y;
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0 && c == 0) src.step[0] += 1;
+    if (t >= g.nc[c]) return;
+    int ix, iy, iz;
+    dof_coords(g, c, t, ix, iy, iz);
+    const bool pec = on_pec(g, c, ix, iy, iz);
+    T f = 0;
+    if (!pec) f = dof_sum<T, O, EXACT>(g, fe, c, ix, iy, iz, T(-1), false, T(0));
+    T v = xadd(f, xsub(xmul(T(2), d.a[c][t]), d.b[c][t]));
+    for (int s = 0; s < src.n; ++s)
+        if (src.comp[s] == c && (size_t)src.idx[s] == t) v = xsub(v, (T)src.vals[src.step[1] - 1]);
+    if (pec) v = 0;
+    d.c[c][t] = v;
+}
+
+// DOF pass of a symplectic substep: the force (stored, as the reference keeps
+// it), the kick, the closing half drift with the PEC planes zeroed, and the
+// opening half drift of the next substep (h2 != 0; FP32 runs take both half
+// drifts as one, h1).  Drifts add (h P) / m; 1 / m is a power of two.
+template <class T, int O, bool EXACT>
+__global__ void __launch_bounds__(128) hex_kick_dof_kernel(const __grid_constant__ HexGeom g, const T *__restrict__ fe, const __grid_constant__ HexDofs<T> d,
+                                                           const __grid_constant__ SrcTab src, T dt, T h1, T h2, T rm)
+{
+    const int c = blockIdx.y;
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (src.last && t == 0 && c == 0) src.step[0] += 1;
+    if (t >= g.nc[c]) return;
+    int ix, iy, iz;
+    dof_coords(g, c, t, ix, iy, iz);
+    bool has = false;
+    T sv = 0;
+    for (int s = 0; s < src.n; ++s)
+        if (src.comp[s] == c && (size_t)src.idx[s] == t) { has = true; sv = (T)src.vals[(size_t)(src.step[1] - 1) * src.nsub + src.q]; }
+    const bool pec = on_pec(g, c, ix, iy, iz);
+    T f = 0;
+    if (!pec) f = dof_sum<T, O, EXACT>(g, fe, c, ix, iy, iz, T(1), has, sv);
+    T p = d.b[c][t], u = d.a[c][t];
+    d.c[c][t] = f;
+    p = EXACT ? xsub(p, xmul(dt, f)) : fma(-dt, f, p);
+    u = xadd(u, xmul(xmul(h1, p), rm));
+    if (pec) { u = 0; p = 0; }
+    if (h2 != T(0)) u = xadd(u, xmul(xmul(h2, p), rm));
+    d.b[c][t] = p;
+    d.a[c][t] = u;
 }
 
 static double femv2_source(double t)
@@ -261,8 +540,17 @@ struct HexFemSim : Sim {
     std::vector<std::array<int, 3>> obs_idx; // x, y, z flat indices
     std::vector<std::array<int, 3>> obs_ijk;
     int l0 = 0, l1 = 1, l2 = 2;              // leapfrog ring
+    HexClasses cls{};                        // order 1 in FP64: the sizes and signs of K's entries
+    bool classes = false;
     double cur_time = 0.0;
-    DevBuf d_obs, d_tr;
+    DevBuf d_obs, d_tr, d_fe, d_vals, d_step;
+    cudaGraphExec_t graph = nullptr;         // kGraphSteps steps, kept while the buffers stay the same
+    std::vector<unsigned long long> graph_key;
+    static constexpr int kGraphSteps = 9;    // a multiple of the three levels' ring
+    ~HexFemSim() override
+    {
+        if (graph) cudaGraphExecDestroy(graph);
+    }
 
     explicit HexFemSim(const ems_hexfem_params *p) : Sim(Kind::HEXFEM), P(*p)
     {
@@ -305,6 +593,17 @@ struct HexFemSim : Sim {
         Kh.resize((size_t)T * T);
         for (int i = 0; i < T; ++i)
             for (int j = 0; j < T; ++j) Kh[(size_t)i * T + j] = scale * M[i][j];
+        if (o == 1 && fp64) {
+            classes = true;
+            for (int i = 0; i < 12; ++i)
+                for (int j = 0; j < 12; ++j) {
+                    const double k = Kh[12 * i + j];
+                    double &size = cls.k[hex1_class(i, j)];
+                    if (size == 0.0) size = std::fabs(k);
+                    classes = classes && k != 0.0 && std::fabs(k) == size;
+                    if (k < 0.0) cls.sign[i] |= 1u << j;
+                }
+        }
         init_stream();
         size_t w = fp64 ? 8 : 4;
         for (int q = 0; q < 3; ++q) { lev[q].alloc(3 * g.nc[q] * w); lev[q].zero(stream); }
@@ -361,6 +660,131 @@ struct HexFemSim : Sim {
         return s;
     }
 
+    dim3 dof_grid() const
+    {
+        const size_t mx = std::max(g.nc[0], std::max(g.nc[1], g.nc[2]));
+        return dim3((unsigned)((mx + 127) / 128), 3);
+    }
+    int nsub() const { return P.integrator == EMS_SYMP4 ? 3 : 1; }
+    void substeps(double sub[3], double off[3]) const
+    {
+        const double x1 = 1.0 / (2.0 - std::pow(2.0, 1.0 / 3.0)), x2 = 1.0 - 2.0 * x1;
+        sub[0] = P.dt; off[0] = 0.0;
+        if (P.integrator == EMS_SYMP4) { sub[0] = x1 * P.dt; sub[1] = x2 * P.dt; off[1] = x1 * P.dt; sub[2] = x1 * P.dt; off[2] = (x1 + x2) * P.dt; }
+    }
+    // The order-1 FP64 pass with one thread per element pays where the FP64
+    // pipes are full, a warp per SM: 37x33x41 elements 28.3 us a leapfrog step
+    // against 39.8, but 8x7x6 elements 13.2 against 11.2.
+    static constexpr int kHex1MinElements = 4096;
+    // Element pass of orders 1 and 2 over the level u; samp: with the sampling blocks
+    template <class T, int O> void elements(T *const (&u)[3], bool first, bool samp)
+    {
+        constexpr bool X = sizeof(T) == 8;
+        const int ne = g.EX * g.EY * g.EZ;
+        const HexRec rec{samp ? nobs : 0, nsamp, P.time_frequency, d_obs.as<int>(), d_tr.as<double>()};
+        int *step = first ? d_step.as<int>() : nullptr;
+        if constexpr (X && O == 1)
+            if (classes && ne >= kHex1MinElements) {
+                hex1_elem_kernel<<<(ne + 31) / 32 + (rec.n + 31) / 32, 32, 0, stream>>>(g, cls, u[0], u[1], u[2], d_fe.as<T>(), step, rec);
+                return;
+            }
+        hex_elem_kernel<T, O, X><<<dim3((ne + 127) / 128 + (rec.n + 127) / 128, 3), 128, 0, stream>>>(g, dK.as<T>(), u[0], u[1], u[2],
+                                                                                                    d_fe.as<T>(), step, rec);
+    }
+    // One step of orders 1 and 2 in two passes per force; launches made.
+    template <class T, int O> int enqueue_step()
+    {
+        int n = 0;
+        const bool leap = P.integrator == EMS_LEAPFROG;
+        if (nobs > 0 && !leap) {   // the symplectic steps sample U before the step
+            hex_sample_kernel<T><<<(nobs + 63) / 64, 64, 0, stream>>>(g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(),
+                                                                      nsamp, 0, d_step.as<int>(), P.time_frequency);
+            ++n;
+        }
+        SrcTab src{};
+        src.n = (int)srcs.size();
+        src.nsub = nsub();
+        for (int q = 0; q < src.n; ++q) { src.comp[q] = srcs[q][0]; src.idx[q] = srcs[q][1]; }
+        src.vals = d_vals.as<double>();
+        src.step = d_step.as<int>();
+        constexpr bool X = sizeof(T) == 8;
+        HexDofs<T> d;
+        for (int c = 0; c < 3; ++c) {
+            d.a[c] = L<T>(c, leap ? l1 : 0);
+            d.b[c] = L<T>(c, leap ? l0 : 1);
+            d.c[c] = L<T>(c, leap ? l2 : 2);
+        }
+        if (leap) {   // fem_v2 samples E^n, which the step leaves alone
+            elements<T, O>(d.a, true, nobs > 0);
+            hex_leap_dof_kernel<T, O, X><<<dof_grid(), 128, 0, stream>>>(g, d_fe.as<T>(), d, src);
+            l0 = (l0 + 1) % 3; l1 = (l1 + 1) % 3; l2 = (l2 + 1) % 3;
+            return n + 2;
+        }
+        double sub[3], off[3];
+        substeps(sub, off);
+        const int ns = nsub();
+        launch_drift<T>((T)(0.5 * sub[0]), 0);
+        for (int q = 0; q < ns; ++q) {
+            elements<T, O>(d.a, q == 0, false);
+            const bool last = q + 1 == ns;
+            src.q = q;
+            src.last = last;
+            const T h1 = X || last ? (T)(0.5 * sub[q]) : (T)(0.5 * sub[q] + 0.5 * sub[q + 1]), h2 = X && !last ? (T)(0.5 * sub[q + 1]) : T(0);
+            hex_kick_dof_kernel<T, O, X><<<dof_grid(), 128, 0, stream>>>(g, d_fe.as<T>(), d, src, (T)sub[q], h1, h2, (T)(g.o * g.o * g.o / 8.0));
+        }
+        return n + 1 + 2 * ns;
+    }
+    template <class T, int O> long long run_two_pass(int nsteps)
+    {
+        d_fe.ensure((size_t)g.total * g.EX * g.EY * g.EZ * sizeof(T));
+        const int ns = nsub();
+        double sub[3], off[3];
+        substeps(sub, off);
+        std::vector<double> vals((size_t)std::max(nsteps, 1) * ns);
+        double t = cur_time;
+        for (int st = 0; st < nsteps; ++st) {
+            for (int q = 0; q < ns; ++q)
+                vals[(size_t)st * ns + q] = P.integrator == EMS_LEAPFROG
+                    ? femv2_source(t) * P.dt * P.dt / P.permittivity / P.h / P.h / P.h
+                    : femv2_source(t + off[q] + 0.5 * sub[q]) * 8.0 / P.permittivity / (P.h * g.o) / (P.h * g.o) / (P.h * g.o);
+            t += P.dt;
+        }
+        d_vals.ensure(vals.size() * 8);
+        d_step.ensure(2 * sizeof(int));
+        EMS_CUDA(cudaMemcpyAsync(d_vals.p, vals.data(), vals.size() * 8, cudaMemcpyHostToDevice, stream));
+        EMS_CUDA(cudaMemsetAsync(d_step.p, 0, 2 * sizeof(int), stream));
+        EMS_CUDA(cudaStreamSynchronize(stream));   // vals ends here; the run's clock starts behind the copies
+        EMS_CUDA(cudaEventRecord(ev0, stream));
+        long long launches = 0;
+        int step = 0;
+        if (nsteps >= kGraphSteps) {
+            std::vector<unsigned long long> key = {(unsigned long long)l0, (unsigned long long)nobs, (unsigned long long)nsamp, srcs.size()};
+            for (const auto &q : srcs) { key.push_back((unsigned long long)q[0]); key.push_back((unsigned long long)q[1]); }
+            for (const void *q : {d_fe.p, d_vals.p, d_step.p, d_obs.p, d_tr.p}) key.push_back((unsigned long long)reinterpret_cast<uintptr_t>(q));
+            if (!graph || key != graph_key) {
+                if (graph) {
+                    cudaGraphExecDestroy(graph);
+                    graph = nullptr;
+                }
+                cudaGraph_t gr = nullptr;
+                EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+                for (int r = 0; r < kGraphSteps; ++r) graph_launches = enqueue_step<T, O>();   // the ring ends where it began
+                EMS_CUDA(cudaStreamEndCapture(stream, &gr));
+                const cudaError_t e = cudaGraphInstantiate(&graph, gr, 0);
+                cudaGraphDestroy(gr);
+                EMS_CUDA(e);
+                graph_key = key;
+            }
+            for (; step + kGraphSteps <= nsteps; step += kGraphSteps) {
+                EMS_CUDA(cudaGraphLaunch(graph, stream));
+                launches += (long long)kGraphSteps * graph_launches;
+            }
+        }
+        for (; step < nsteps; ++step) launches += enqueue_step<T, O>();
+        return launches;
+    }
+    int graph_launches = 0;
+
     template <class T, int O> void run_o(int nsteps)
     {
         const int tf = P.time_frequency;
@@ -370,22 +794,28 @@ struct HexFemSim : Sim {
         std::vector<int> oi;
         for (auto &q : obs_idx) { oi.push_back(q[0]); oi.push_back(q[1]); oi.push_back(q[2]); }
         if (oi.empty()) oi.assign(3, 0);
-        d_obs.alloc(oi.size() * 4);
+        d_obs.ensure(oi.size() * 4);
         EMS_CUDA(cudaMemcpyAsync(d_obs.p, oi.data(), oi.size() * 4, cudaMemcpyHostToDevice, stream));
         size_t ntr = (size_t)std::max(nobs, 1) * std::max(nsamp, 1) * 4;
-        d_tr.alloc(ntr * 8);
+        d_tr.ensure(ntr * 8);
         d_tr.zero(stream);
         std::vector<double> times(std::max(nsamp, 1), 0.0);
         long long launches = 0;
-        const double x1 = 1.0 / (2.0 - std::pow(2.0, 1.0 / 3.0)), x2 = 1.0 - 2.0 * x1;
         const int o = g.o;
         EMS_CUDA(cudaEventRecord(ev0, stream));
+        if constexpr (O <= 2) {
+            launches = run_two_pass<T, O>(nsteps);
+            for (int step = 0; step < nsteps; ++step) {
+                if (step % tf == 0) times[step / tf] = cur_time;
+                cur_time += P.dt;
+            }
+        } else
         for (int step = 0; step < nsteps; ++step) {
             bool samp = nobs > 0 && step % tf == 0;
             if (P.integrator == EMS_LEAPFROG) {
                 // fem_v2 samples level 1 (E^n) after computing E^{n+1}; E^n is untouched by the step
                 if (samp) {
-                    hex_sample_kernel<T><<<(nobs + 63) / 64, 64, 0, stream>>>(g, L<T>(0, l1), L<T>(1, l1), L<T>(2, l1), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf);
+                    hex_sample_kernel<T><<<(nobs + 63) / 64, 64, 0, stream>>>(g, L<T>(0, l1), L<T>(1, l1), L<T>(2, l1), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf, nullptr, 1);
                     times[step / tf] = cur_time;
                     ++launches;
                 }
@@ -395,21 +825,20 @@ struct HexFemSim : Sim {
                 l0 = (l0 + 1) % 3; l1 = (l1 + 1) % 3; l2 = (l2 + 1) % 3;
             } else {
                 if (samp) {
-                    hex_sample_kernel<T><<<(nobs + 63) / 64, 64, 0, stream>>>(g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf);
+                    hex_sample_kernel<T><<<(nobs + 63) / 64, 64, 0, stream>>>(g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf, nullptr, 1);
                     times[step / tf] = cur_time;
                     ++launches;
                 }
                 double sub[3], off[3];
-                int nsub;
-                if (P.integrator == EMS_SYMP2) { nsub = 1; sub[0] = P.dt; off[0] = 0.0; }
-                else { nsub = 3; sub[0] = x1 * P.dt; off[0] = 0.0; sub[1] = x2 * P.dt; off[1] = x1 * P.dt; sub[2] = x1 * P.dt; off[2] = (x1 + x2) * P.dt; }
-                for (int q = 0; q < nsub; ++q) {
+                substeps(sub, off);
+                const int ns = nsub();
+                for (int q = 0; q < ns; ++q) {
                     double deltat = sub[q];
                     double sv = femv2_source(cur_time + off[q] + 0.5 * deltat) * 8.0 / P.permittivity / (P.h * o) / (P.h * o) / (P.h * o);
                     if (exact || q == 0) launch_drift<T>((T)(0.5 * deltat), 0), ++launches;
                     launch_kick<T, O>((T)deltat, sources(sv));
                     ++launches;
-                    if (exact || q == nsub - 1) launch_drift<T>((T)(0.5 * deltat), 1);
+                    if (exact || q == ns - 1) launch_drift<T>((T)(0.5 * deltat), 1);
                     else launch_drift<T>((T)(0.5 * deltat + 0.5 * sub[q + 1]), 1);
                     ++launches;
                 }
@@ -455,13 +884,7 @@ struct HexFemSim : Sim {
     void get_field(int which, double *out) const override
     {
         size_t cnt = field_size(which);
-        if (fp64) {
-            EMS_CUDA(cudaMemcpy(out, lev[which].p, cnt * 8, cudaMemcpyDeviceToHost));
-        } else {
-            std::vector<float> tmp(cnt);
-            EMS_CUDA(cudaMemcpy(tmp.data(), lev[which].p, cnt * 4, cudaMemcpyDeviceToHost));
-            for (size_t q = 0; q < cnt; ++q) out[q] = tmp[q];
-        }
+        download(out, lev[which].p, cnt, fp64);
     }
     void set_field(int which, const double *in) override
     {
@@ -515,6 +938,7 @@ struct HexFemSim : Sim {
             save[q].alloc(lev[q].bytes);
             EMS_CUDA(cudaMemcpyAsync(save[q].p, lev[q].p, lev[q].bytes, cudaMemcpyDeviceToDevice, stream));
         }
+        if (g.o <= 2) d_fe.ensure((size_t)g.total * g.EX * g.EY * g.EZ * w);
         auto body = [&](auto tag) {
             using T = decltype(tag);
             SrcList s = sources(0.0);
@@ -522,7 +946,13 @@ struct HexFemSim : Sim {
                 if (r == 1) EMS_CUDA(cudaEventRecord(ev0, stream));
                 auto go = [&](auto oc) {
                     constexpr int O = decltype(oc)::value;
-                    if (P.integrator == EMS_LEAPFROG) launch_leapfrog<T, O>(s); else launch_kick<T, O>((T)P.dt, s);
+                    if constexpr (O <= 2) {
+                        T *u[3];
+                        for (int c = 0; c < 3; ++c) u[c] = L<T>(c, P.integrator == EMS_LEAPFROG ? l1 : 0);
+                        elements<T, O>(u, false, false);
+                    } else {
+                        if (P.integrator == EMS_LEAPFROG) launch_leapfrog<T, O>(s); else launch_kick<T, O>((T)P.dt, s);
+                    }
                 };
                 if (g.o == 1) go(std::integral_constant<int, 1>());
                 else if (g.o == 2) go(std::integral_constant<int, 2>());
@@ -538,9 +968,11 @@ struct HexFemSim : Sim {
             EMS_CUDA(cudaMemcpyAsync(lev[q].p, save[q].p, lev[q].bytes, cudaMemcpyDeviceToDevice, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
         *ms = t / launches;
-        // leapfrog: read E^n, E^{n-1}, write E^{n+1}; kick: read U, read/write P, write F
-        *bytes = (double)ndof * w * (P.integrator == EMS_LEAPFROG ? 3.0 : 4.0);
-        *name = std::string(P.integrator == EMS_LEAPFROG ? "hex_leapfrog_kernel" : "hex_kick_kernel") + "<o=" + std::to_string(g.o) + ">";
+        // element pass: read U, write the element values; order 3 leapfrog: read E^n, E^{n-1}, write
+        // E^{n+1}; kick: read U, read/write P, write F
+        *bytes = g.o <= 2 ? w * ((double)ndof + (double)g.total * g.EX * g.EY * g.EZ) : (double)ndof * w * (P.integrator == EMS_LEAPFROG ? 3.0 : 4.0);
+        *name = std::string(g.o <= 2 ? (classes && g.EX * g.EY * g.EZ >= kHex1MinElements ? "hex1_elem_kernel" : "hex_elem_kernel") : P.integrator == EMS_LEAPFROG ? "hex_leapfrog_kernel" : "hex_kick_kernel") +
+                "<o=" + std::to_string(g.o) + ">";
     }
 };
 
