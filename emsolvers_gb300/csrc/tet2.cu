@@ -1046,6 +1046,17 @@ __global__ void __launch_bounds__(128) t2_cheb_kernel(unsigned long long NE, con
     const int pl0 = et < 7 ? et : 14 + 2 * (et - 7), pl1 = et < 7 ? et + 7 : pl0 + 1;
     const unsigned long long d0 = S.dof0 + (unsigned long long)pl0 * nn + v;
     const unsigned long long d1 = S.dof0 + (unsigned long long)pl1 * nn + v;
+    // Launched while the iteration before ends (programmatic dependent launch):
+    // the right-hand side and the block inverse do not change during a solve,
+    // everything else is read behind the wait; the next launch may start only
+    // after it, so what this one reads early is complete.
+    T b0 = T(0), b1 = T(0), q00 = T(0), q01 = T(0), q11 = T(0);
+    if (!dead) {
+        b0 = g.b[d0]; b1 = g.b[d1];
+        q00 = g.pinv[e]; q01 = g.pinv[NE + e]; q11 = g.pinv[2 * NE + e];
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");
     if (dead) {
         g.x[d0] = T(0); g.x[d1] = T(0); g.d[d0] = T(0); g.d[d1] = T(0);
         return;
@@ -1063,8 +1074,7 @@ __global__ void __launch_bounds__(128) t2_cheb_kernel(unsigned long long NE, con
         EMS_T2_ROWS(14) EMS_T2_ROWS(15) EMS_T2_ROWS(16) EMS_T2_ROWS(17) default: EMS_T2_ROWS(18)
     }
 #undef EMS_T2_ROWS
-    const T r0 = g.b[d0] - y0, r1 = g.b[d1] - y1;
-    const T q00 = g.pinv[e], q01 = g.pinv[NE + e], q11 = g.pinv[2 * NE + e];
+    const T r0 = b0 - y0, r1 = b1 - y1;
     const T z0 = fma(q00, r0, q01 * r1), z1 = fma(q01, r0, q11 * r1);
     const T n0 = fma(g.c1, g.d[d0], g.c2 * z0), n1 = fma(g.c1, g.d[d1], g.c2 * z1);
     const T x0 = g.xin[d0] + n0, x1 = g.xin[d1] + n1;
@@ -1086,8 +1096,10 @@ __global__ void __launch_bounds__(128) t2_cheb_kernel(unsigned long long NE, con
 // node planes k0 .. k1 - 1 of one shot.
 struct T2Tile {
     unsigned long long dof0, tet0, ent0;
-    int nx, ny, nz, i0, j0, k0, k1, bx, by, pad;
+    int nx, ny, nz, i0, j0, k0, k1, bx, by;
+    int table;   // which table of staged offsets (one per row width)
 };
+constexpr int kStageTable = 720;   // [6 layers][6 types][20] byte offsets of a tetrahedron's staged values
 
 // Groups of the 38 planes in the staged iterate: the 10 whose entities do not
 // span z (a cube reads them in two layers) and the 28 that do.
@@ -1116,7 +1128,6 @@ constexpr GroupTab make_group_tab()
     return T;
 }
 static_assert(make_group_tab().n[0] == 10 && make_group_tab().n[1] == 28, "10 planes without z, 28 with z");
-__constant__ int c2_grp[kPlanes];      // group << 8 | place in the group
 __constant__ int c2_gplane[10];        // the planes without z
 
 __device__ __forceinline__ void copy_async(float *dst, const float *src)
@@ -1198,12 +1209,16 @@ template <class T, int COLS, int ET, int Q> __device__ __forceinline__ void marc
 {
     if constexpr (kInc.ob[ET][Q] & 4) march_value<T, COLS, ET, Q>(c, m.low[2 * low_at(ET, Q)], m.low[2 * low_at(ET, Q) + 1]);
 }
-// The sum over the tetrahedra of the entity in ascending type, then the
-// values that its node one layer up will need.
+// The sum over the tetrahedra of the entity in ascending type, and the values
+// that its node one layer up will need.
 template <class T, int COLS, int ET, int... Q>
-__device__ __forceinline__ void march_sum(std::integer_sequence<int, Q...>, const MarchCol<T> &c, MarchOps<T> &m, T &y0, T &y1)
+__device__ __forceinline__ void march_sum(std::integer_sequence<int, Q...>, const MarchCol<T> &c, const MarchOps<T> &m, T &y0, T &y1)
 {
     (march_term<T, COLS, ET, Q>(c, m, y0, y1), ...);
+}
+template <class T, int COLS, int ET, int... Q>
+__device__ __forceinline__ void march_keeps(std::integer_sequence<int, Q...>, const MarchCol<T> &c, MarchOps<T> &m)
+{
     (march_keep<T, COLS, ET, Q>(c, m), ...);
 }
 template <class T, int FIN, int COLS, int NC, int ET>
@@ -1211,9 +1226,15 @@ __device__ __forceinline__ void march_update(const MArgs<T> &g, const MarchCol<T
 {
     constexpr int S = ent_axes(ET);
     if (c.dead & ~S & 3) return;
+    constexpr auto terms = std::make_integer_sequence<int, kInc.n[ET]>{};
+    if (!store) {   // the layer below the chunk
+        march_keeps<T, COLS, ET>(terms, c, m);
+        return;
+    }
     T y0 = T(0), y1 = T(0);
-    march_sum<T, COLS, ET>(std::make_integer_sequence<int, kInc.n[ET]>{}, c, m, y0, y1);
-    if (!store || (c.dead & ~S)) return;
+    march_sum<T, COLS, ET>(terms, c, m, y0, y1);
+    march_keeps<T, COLS, ET>(terms, c, m);
+    if (c.dead & ~S) return;
     constexpr unsigned pl0 = ET < 7 ? ET : 2 * ET, pl1 = ET < 7 ? ET + 7 : pl0 + 1;
     constexpr GroupTab gt = make_group_tab();
     constexpr int s0 = gt.slot[pl0] * NC, s1 = gt.slot[pl1] * NC;
@@ -1260,6 +1281,35 @@ __device__ __forceinline__ void march_rows(std::integer_sequence<int, A...>, con
     ((yc[A * COLS] = mul_rn(e, mass_row<A>(std::make_integer_sequence<int, 20>{}, x))), ...);
 }
 
+// The rows that the layer above needs of the layer below a chunk: entities
+// without z at the upper corners (20 of the 120 values of a cube).
+constexpr bool low_row(int p, int a)
+{
+    const int pl = kInc.plane[p][a], et = pl < 14 ? pl % 7 : 7 + (pl - 14) / 2;
+    return (kInc.vo[p][a] & 4) && !(ent_axes(et) & 4);
+}
+template <class T, int COLS, int P, int A> __device__ __forceinline__ void march_low_row(const T (&x)[20], T e, T *yc)
+{
+    if constexpr (low_row(P, A)) yc[A * COLS] = mul_rn(e, mass_row<A>(std::make_integer_sequence<int, 20>{}, x));
+}
+template <class T, int COLS, int P, int... A>
+__device__ __forceinline__ void march_low_rows(std::integer_sequence<int, A...>, const T (&x)[20], T e, T *yc)
+{
+    (march_low_row<T, COLS, P, A>(x, e, yc), ...);
+}
+template <class T, int COLS> __device__ __forceinline__ void march_low(int p, const T (&x)[20], T e, T *yc)
+{
+    constexpr auto all = std::make_integer_sequence<int, 20>{};
+    switch (p) {
+    case 0: march_low_rows<T, COLS, 0>(all, x, e, yc); break;
+    case 1: march_low_rows<T, COLS, 1>(all, x, e, yc); break;
+    case 2: march_low_rows<T, COLS, 2>(all, x, e, yc); break;
+    case 3: march_low_rows<T, COLS, 3>(all, x, e, yc); break;
+    case 4: march_low_rows<T, COLS, 4>(all, x, e, yc); break;
+    default: march_low_rows<T, COLS, 5>(all, x, e, yc); break;
+    }
+}
+
 // The copy of one layer's planes by a warp: planes P, P + 6, ... of the list
 // (10 without z, of layer ka, then 28 with z, of layer kb).
 template <class T, int NC, int M>
@@ -1301,7 +1351,7 @@ __device__ __forceinline__ void march_copies(std::integer_sequence<int, S...>, A
 // per edge or face): 48^3 cubes 44.7 us against 67, five shots of 12..40
 // cubes 63 against 100, thirteen shots of 22..40 cubes 227 against 345.
 template <class T, int FIN, int COLS, int NC>
-__global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *__restrict__ tiles, MArgs<T> g)
+__global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *__restrict__ tiles, const int *__restrict__ tables, MArgs<T> g)
 {
     constexpr int NT = 6 * COLS, G = COLS / 32;   // a warp: one tetrahedron type of 32 columns
     extern __shared__ __align__(16) unsigned char t2_sm[];
@@ -1312,11 +1362,8 @@ __global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *__r
     const T2Tile t = tiles[blockIdx.x];
     const int tid = threadIdx.x, warp = tid >> 5, p = warp / G, col = (warp - p * G) * 32 + (tid & 31);
     const int rw = t.bx + 1;
-    for (int n = tid; n < 720; n += NT) {
-        const int ph = n / 120, q = n % 20, d = c2_dof[(n / 20) % 6][q], pl = d & 255, o = d >> 8;
-        const int gr = c2_grp[pl], at = (gr & 255) * NC + (o & 1) + ((o >> 1) & 1) * rw;
-        xoff[n] = (int)sizeof(T) * ((gr >> 8) ? 30 * NC + (ph & 1) * (28 * NC) + at : ((ph + (o >> 2)) % 3) * (10 * NC) + at);
-    }
+    for (int n = tid; n < kStageTable / 4; n += NT)
+        reinterpret_cast<int4 *>(xoff)[n] = reinterpret_cast<const int4 *>(tables + t.table * kStageTable)[n];
     const int ty = col / t.bx, tx = col - ty * t.bx;
     const int i = t.i0 + tx, j = t.j0 + ty;
     const bool active = ty < t.by && i < t.nx && j < t.ny;
@@ -1399,7 +1446,8 @@ __global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *__r
 #pragma unroll
             for (int q = 0; q < 20; ++q) x[q] = *reinterpret_cast<const T *>(xc + o[q]);
             T *yc = Y + p * (20 * COLS) + col;
-            march_rows<T, COLS>(std::make_integer_sequence<int, 20>{}, x, e, yc);
+            if (k < t.k0) march_low<T, COLS>(p, x, e, yc);   // the layer below the chunk
+            else march_rows<T, COLS>(std::make_integer_sequence<int, 20>{}, x, e, yc);
         }
         __syncthreads();
         if (own) {
@@ -1669,7 +1717,7 @@ struct Tet2Sim : Sim {
         // the compile-time element mass against the setup's (all types), and its
         // symmetry under the vertex reversal
         const MateTab mt = make_mate_tab();
-        int mslot[20], grp[kPlanes];
+        int mslot[20];
         for (int a = 0; a < 20; ++a) mslot[a] = mass_slot(a);
         for (int p = 0; p < 6; ++p)
             for (int a = 0; a < 20; ++a)
@@ -1681,8 +1729,6 @@ struct Tet2Sim : Sim {
         EMS_CUDA(cudaMemcpyToSymbol(c2_H64, kMass.h, sizeof(kMass.h)));
         EMS_CUDA(cudaMemcpyToSymbol(c2_massslot, mslot, sizeof(mslot)));
         const GroupTab gt = make_group_tab();
-        for (int q = 0; q < kPlanes; ++q) grp[q] = gt.grp[q] << 8 | gt.slot[q];
-        EMS_CUDA(cudaMemcpyToSymbol(c2_grp, grp, sizeof(grp)));
         EMS_CUDA(cudaMemcpyToSymbol(c2_gplane, gt.plane[0], sizeof(int) * 10));
         int dof[6][20];
         float m32[6][400];
@@ -1813,10 +1859,10 @@ struct Tet2Sim : Sim {
     // Tiles of the marching iteration: per shot the width bx (by = COLS / bx)
     // that covers its columns with the fewest tiles, and one chunk length
     // for all shots: the one whose waves of blocks (one per SM) times layers
-    // (the chunk, the repeated layer and about one more of start-up) is least.
+    // (the chunk, and about 1.4 for the layer below it and the start) is least.
     static constexpr int kCols = 128, kStage = 168;
-    static constexpr size_t kMarchSmem = sizeof(float) * (86 * kStage + 120 * kCols) + sizeof(int) * 720;
-    DevBuf d_tiles;
+    static constexpr size_t kMarchSmem = sizeof(float) * (86 * kStage + 120 * kCols) + sizeof(int) * kStageTable;
+    DevBuf d_tiles, d_tables;
     unsigned ntiles = 0;
     void build_tiles()
     {
@@ -1849,9 +1895,26 @@ struct Tet2Sim : Sim {
         for (int l = 1; l <= nzmax; ++l) {
             long nb = 0;
             for (size_t s = 0; s < shots.size(); ++s) nb += plan[s].tx * plan[s].ty * ((shots[s].n[2] + l - 1) / l);
-            const long cost = ((nb + nsm - 1) / nsm) * (l + 2);
+            const long cost = ((nb + nsm - 1) / nsm) * (10 * l + 14);
             if (bestc < 0 || cost < bestc) { bestc = cost; L = l; }
         }
+        // staged offsets per row width: layers k and k + 1 of the planes without z, layer k of those with z
+        std::vector<int> tables, width;
+        const GroupTab gt = make_group_tab();
+        auto table = [&](int rw) {
+            for (size_t q = 0; q < width.size(); ++q)
+                if (width[q] == rw) return (int)q;
+            for (int ph = 0; ph < 6; ++ph)
+                for (int p = 0; p < 6; ++p)
+                    for (int a = 0; a < 20; ++a) {
+                        const int pl = kInc.plane[p][a], o = kInc.vo[p][a];
+                        const int at = gt.slot[pl] * kStage + (o & 1) + ((o >> 1) & 1) * rw;
+                        tables.push_back((int)sizeof(float) * (gt.grp[pl] ? 30 * kStage + (ph & 1) * (28 * kStage) + at
+                                                                         : ((ph + (o >> 2)) % 3) * (10 * kStage) + at));
+                    }
+            width.push_back(rw);
+            return (int)width.size() - 1;
+        };
         std::vector<T2Tile> tiles;
         for (size_t s = 0; s < shots.size(); ++s) {
             const ShotH &S = shots[s];
@@ -1863,6 +1926,7 @@ struct Tet2Sim : Sim {
                         t.dof0 = S.dof0; t.tet0 = S.tet0; t.ent0 = S.ent0;
                         t.nx = S.n[0]; t.ny = S.n[1]; t.nz = S.n[2];
                         t.bx = plan[s].bx; t.by = plan[s].by;
+                        t.table = table(t.bx + 1);
                         t.i0 = x * (t.bx - 1); t.j0 = y * (t.by - 1);
                         t.k0 = (int)((long)S.n[2] * c / nch); t.k1 = (int)((long)S.n[2] * (c + 1) / nch);
                         tiles.push_back(t);
@@ -1870,6 +1934,8 @@ struct Tet2Sim : Sim {
         }
         d_tiles.ensure(tiles.size() * sizeof(T2Tile));
         EMS_CUDA(cudaMemcpy(d_tiles.p, tiles.data(), tiles.size() * sizeof(T2Tile), cudaMemcpyHostToDevice));
+        d_tables.ensure(tables.size() * sizeof(int));
+        EMS_CUDA(cudaMemcpy(d_tables.p, tables.data(), tables.size() * sizeof(int), cudaMemcpyHostToDevice));
         auto wide = [](auto k) { EMS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMarchSmem)); };
         wide(t2_march_kernel<float, FIN_NONE, kCols, kStage>);
         wide(t2_march_kernel<float, FIN_DRIFT, kCols, kStage>);
@@ -1883,9 +1949,18 @@ struct Tet2Sim : Sim {
         if constexpr (sizeof(T) == 4) {
             if (cheb_form == FORM_MARCH) {
                 const MArgs<T> a{g.xin, g.b, g.pinv, g.eps, g.x, g.d, g.U, g.Uold, g.c1, g.c2, g.h, nent};
-                t2_march_kernel<T, FIN, kCols, kStage><<<ntiles, 6 * kCols, kMarchSmem, stream>>>(d_tiles.as<T2Tile>(), a);
+                t2_march_kernel<T, FIN, kCols, kStage><<<ntiles, 6 * kCols, kMarchSmem, stream>>>(d_tiles.as<T2Tile>(), d_tables.as<int>(), a);
             } else {
-                t2_cheb_kernel<T, FIN><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+                cudaLaunchConfig_t c{};
+                c.gridDim = dim3(blocks(nent, 128));
+                c.blockDim = dim3(128);
+                c.stream = stream;
+                cudaLaunchAttribute at{};
+                at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                at.val.programmaticStreamSerializationAllowed = 1;
+                c.attrs = &at;
+                c.numAttrs = 1;
+                EMS_CUDA(cudaLaunchKernelEx(&c, t2_cheb_kernel<T, FIN>, (unsigned long long)nent, (const T2Shot *)d_shots.as<T2Shot>(), ns, g));
             }
             return 1;
         } else {
