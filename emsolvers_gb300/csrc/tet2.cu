@@ -1496,6 +1496,17 @@ __global__ void __launch_bounds__(128) t2_pinv_kernel(unsigned long long NE, con
     out[2 * NE + e] = ok ? a / det : 0.0;
 }
 
+// A field from planes to the API's node-major order.
+template <class T>
+__global__ void t2_field_kernel(unsigned long long n, const T2Shot *__restrict__ sh, int ns, const T *__restrict__ x, T *__restrict__ out)
+{
+    const unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    const T2Shot S = sh[shot_of(sh, ns, e / 2, 1)];   // 38 DOFs and 19 entities per node
+    const unsigned l = (unsigned)(e - S.dof0), node = l / kPlanes, pl = l - node * kPlanes;
+    out[e] = x[S.dof0 + (unsigned long long)pl * S.nnode + node];
+}
+
 template <class T> __global__ void t2_narrow_kernel(unsigned long long n, const double *__restrict__ x, T *__restrict__ y)
 {
     const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -2421,18 +2432,18 @@ struct Tet2Sim : Sim {
     void get_field(int which, double *out) const override
     {
         field_size(which);
-        std::vector<double> tmp(ndof);
         const bool pfield = which == 1 && symp();
         const DevBuf &b = which == 0 ? d_U : (pfield ? d_P : d_Uold);
-        if (pfield || fp64) {
-            EMS_CUDA(cudaMemcpy(tmp.data(), b.p, ndof * 8, cudaMemcpyDeviceToHost));
-        } else {
-            std::vector<float> f(ndof);
-            EMS_CUDA(cudaMemcpy(f.data(), b.p, ndof * 4, cudaMemcpyDeviceToHost));
-            for (size_t e = 0; e < ndof; ++e) tmp[e] = f[e];
-        }
-        for (size_t e = 0; e < ndof; ++e) out[e] = tmp[dof_index(e)];
+        auto body = [&](auto tag) {
+            using T = decltype(tag);
+            d_stage.ensure(ndof * sizeof(T));
+            t2_field_kernel<T><<<blocks(ndof, 256), 256, 0, stream>>>(ndof, d_shots.as<T2Shot>(), (int)shots.size(), b.as<T>(), d_stage.as<T>());
+            EMS_CUDA(cudaGetLastError());
+            download(out, d_stage.p, ndof, sizeof(T) == 8);
+        };
+        if (pfield || fp64) body(double()); else body(float());
     }
+    mutable DevBuf d_stage;   // a field in the API's order
     void set_field(int which, const double *in) override
     {
         field_size(which);

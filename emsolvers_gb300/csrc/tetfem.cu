@@ -1420,53 +1420,109 @@ __global__ void __launch_bounds__(128) tet_grad_accumulate_kernel(size_t nnode, 
     for (int p = 0; p < 28; ++p) qv[p] += 0.5 * acc[p];
 }
 
-// Receiver adjoint of one sample, in two launches.  The receivers' edge
-// slots are listed once each: tet_receiver_gather_kernel gathers w * r over
-// each slot's receiver terms (a, also added to Wbar); then every node
-// holding such a slot gets the half drift that the merged loop folded into
-// the sampling, Pbar += cc Minv a, Q += cc sym((Minv a) z^T), one thread per
-// node in tet_receiver_drift_kernel.  (On one block the node part was
-// bound by a single SM's FP64 rate: about 37 us per sample for 512
-// receivers.)
+// Receiver adjoint of one sample.  The receivers' edge
+// slots are listed once each, by node: eight lanes take a node, lane d < 7
+// gathers w * r over the receiver terms of the node's slot d (a, also added to
+// Wbar); then the node gets the half drift that the merged loop folded into
+// the sampling, Pbar += cc Minv a, Q += cc sym((Minv a) z^T), lane d its row.
+// A launch of a few thousand threads per sample, bound by latency: with one
+// thread per slot and then one per node the two launches of 64 receivers took
+// 5.9 and 14.9 us.
 template <class T>
-__global__ void __launch_bounds__(256) tet_receiver_gather_kernel(int nsl, const int *__restrict__ sl_slot,
-                                                                  const int *__restrict__ sl_ptr, const int *__restrict__ term_rc,
-                                                                  const double *__restrict__ term_w, const double *__restrict__ r,
-                                                                  double *__restrict__ a_scr, T *__restrict__ Wb, size_t nnode)
+__global__ void __launch_bounds__(128) tet_receiver_adjoint_kernel(int nnd, const int *__restrict__ nd_node, const int *__restrict__ nd_map,
+                                                                   const int *__restrict__ sl_ptr, const int *__restrict__ term_rc,
+                                                                   const double *__restrict__ term_w, const double *__restrict__ r,
+                                                                   T *__restrict__ Wb, T *__restrict__ Pb, const T *__restrict__ minv,
+                                                                   const T *__restrict__ z, double *__restrict__ Q, double cc, size_t nnode)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nsl) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, d = t & 7, i = t >> 3;
+    const bool in = i < nnd && d < 7;
+    const size_t v = i < nnd ? (size_t)nd_node[i] : 0, f = (size_t)d * nnode + v;
+    const int k = in ? nd_map[7 * i + d] : -1;
     double acc = 0.0;
-    for (int s = sl_ptr[k]; s < sl_ptr[k + 1]; ++s) acc += term_w[s] * r[term_rc[s]];
-    a_scr[k] = acc;
-    Wb[fslot((size_t)sl_slot[k], nnode)] += (T)acc;
+    if (k >= 0) {
+        for (int s = sl_ptr[k]; s < sl_ptr[k + 1]; ++s) acc += term_w[s] * r[term_rc[s]];
+        Wb[f] += (T)acc;
+    }
+    if (cc == 0.0) return;   // no drift before the sample (uniform)
+    const T x = (T)acc, zd = in ? z[f] : T(0);
+    T y = 0;
+#pragma unroll
+    for (int j = 0; j < 7; ++j) {
+        const T xj = __shfl_sync(0xffffffffu, x, j, 8);
+        if (in) y = fma(minv[fpk(v, pk7(d, j), nnode)], xj, y);
+    }
+    if (in) Pb[f] = fma((T)cc, y, Pb[f]);
+#pragma unroll
+    for (int j = 0; j < 7; ++j) {
+        const T yj = __shfl_sync(0xffffffffu, y, j, 8), zj = __shfl_sync(0xffffffffu, zd, j, 8);
+        if (in && j >= d) Q[28 * v + pk7(d, j)] += 0.5 * cc * ((double)y * (double)zj + (double)yj * (double)zd);
+    }
 }
 
-template <class T>
-__global__ void __launch_bounds__(128) tet_receiver_drift_kernel(int nnd, const int *__restrict__ nd_node,
-                                                                 const int *__restrict__ nd_map, const double *__restrict__ a_scr,
-                                                                 T *__restrict__ Pb, const T *__restrict__ minv,
-                                                                 const T *__restrict__ z, double *__restrict__ Q, double cc,
-                                                                 size_t nnode)
+// A field from the plane layout to slot order (with the compensation added).
+template <class T, class A>
+__global__ void tet_slots_kernel(size_t nslot, size_t nnode, const T *__restrict__ x, const __nv_bfloat16 *__restrict__ lo, A *__restrict__ out)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nnd) return;
-    const size_t v = (size_t)nd_node[i];
-    T x[7], y[7], zz[7];
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nslot) return;
+    const size_t f = fslot(e, nnode);
+    out[e] = (A)x[f] + (lo ? (A)__bfloat162float(lo[f]) : A(0));
+}
+
+// Loss rate of a node: rho = sum sigma w / sum eps w over the incidences of
+// its live slots, in slot and incidence order (see loss_setup).
+__global__ void __launch_bounds__(128) tet_loss_rate_kernel(size_t nnode, const unsigned char *__restrict__ pec, const int *__restrict__ inc_ptr,
+                                                            const int *__restrict__ inc, const double *__restrict__ eps,
+                                                            const double *__restrict__ sig, double *__restrict__ rho, double *__restrict__ den)
+{
+    const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nnode) return;
+    double n = 0.0, m = 0.0;
     for (int d = 0; d < 7; ++d) {
-        int k = nd_map[7 * i + d];
-        x[d] = k >= 0 ? (T)a_scr[k] : T(0);
-        zz[d] = z[(size_t)d * nnode + v];
+        const size_t e = 7 * v + d;
+        if (pec[e] & kPecBit) continue;
+        for (int q = inc_ptr[e]; q < inc_ptr[e + 1]; ++q) {
+            const int t = inc[q] >> 3, l = inc[q] & 7, p = t % 6;
+            n = __dadd_rn(n, __dmul_rn(sig[t], c_wsq[p][l]));
+            m = __dadd_rn(m, __dmul_rn(eps[t], c_wsq[p][l]));
+        }
     }
-    for (int d = 0; d < 7; ++d) {
-        T s = 0;
-        for (int j = 0; j < 7; ++j) s = fma(minv[fpk(v, pk7(d, j), nnode)], x[j], s);
-        y[d] = s;
-        Pb[(size_t)d * nnode + v] = fma((T)cc, s, Pb[(size_t)d * nnode + v]);
+    rho[v] = m > 0.0 ? n / m : 0.0;
+    den[v] = m;
+}
+
+// Loss-rate terms of the gradient (see loss_gradient): per tetrahedron its
+// six slots in ascending order, each a term of the slot's node.
+__global__ void __launch_bounds__(128) tet_loss_node_kernel(size_t nnode, double dt, const double *__restrict__ rho, double *__restrict__ zr)
+{
+    const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < nnode) zr[v] = -0.5 * dt * exp(-0.5 * dt * rho[v]) * zr[v];   // dJ/drho
+}
+__global__ void __launch_bounds__(128) tet_loss_grad_kernel(size_t ntet, const int *__restrict__ tet_edge, const unsigned char *__restrict__ pec,
+                                                            const double *__restrict__ rho, const double *__restrict__ den,
+                                                            const double *__restrict__ gr, double sig_unit, double *__restrict__ grad,
+                                                            double *__restrict__ gsig)
+{
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ntet) return;
+    double g = grad[t], gs = 0.0;
+    int done = -1;
+    for (int n = 0; n < 6; ++n) {
+        int e = 0x7fffffff, l = 0;
+        for (int q = 0; q < 6; ++q) {
+            const int x = tet_edge[6 * t + q];
+            if (x > done && x < e) { e = x; l = q; }
+        }
+        done = e;
+        const int v = e / 7;
+        if ((pec[e] & kPecBit) || !(den[v] > 0.0)) continue;
+        const double w = c_wsq[t % 6][l] / den[v];
+        gs += gr[v] * w * sig_unit;
+        g -= gr[v] * rho[v] * w;
     }
-    for (int d = 0; d < 7; ++d)
-        for (int j = d; j < 7; ++j)
-            Q[28 * v + pk7(d, j)] += 0.5 * cc * ((double)y[d] * (double)zz[j] + (double)y[j] * (double)zz[d]);
+    grad[t] = g;
+    if (gsig) gsig[t] = gs;
 }
 
 // dJ/deps contributions of node v, FP64.  With M_v = W S^+ W^T +
@@ -1878,7 +1934,8 @@ struct TetFemSim : Sim {
     // conductivity: normalised per tetrahedron (sigma h / (c0 eps0)), the
     // per-node loss rate and its denominator, and the per-node loss factor
     // of the time loop (exp(-rho dt/2) symplectic, rho dt/2 leapfrog)
-    std::vector<double> sig_h, rho_h, lden_h;
+    std::vector<double> sig_h;
+    DevBuf d_sig, d_rho, d_lden;   // conductivity, loss rate and its denominator (FP64, lossy runs)
     bool has_loss = false;
     DevBuf d_damp;
     int step_block = 64;            // threads per block of tet_step_kernel (tune_launch_shape)
@@ -2237,35 +2294,23 @@ struct TetFemSim : Sim {
     // M_sigma,v = rho_v M_eps,v and the loss term of the momentum equation
     // is rho_v P.  The symplectic loop applies its flow exp(-rho dt/2) on
     // each side of the middle kick (a time-symmetric composition, second
-    // order when sigma != 0); leapfrog takes the centred loss term.  Host
-    // FP64, O(ntet).
+    // order when sigma != 0); leapfrog takes the centred loss term.  FP64.
     void loss_setup()
     {
-        rho_h.assign(nnode, 0.0);
-        lden_h.assign(nnode, 0.0);
         if (!has_loss) { d_damp.release(); return; }
-        double wsq[6][6];
-        for (int p = 0; p < 6; ++p) {
-            const Shape sh = make_shape(p);
-            for (int l = 0; l < 6; ++l) wsq[p][l] = sh.wsq[l];
-        }
         const bool symp = schedule().symp;
+        d_sig.ensure(ntet * 8);
+        d_rho.ensure(nnode * 8);
+        d_lden.ensure(nnode * 8);
+        EMS_CUDA(cudaMemcpyAsync(d_sig.p, sig_h.data(), ntet * 8, cudaMemcpyHostToDevice, stream));
+        tet_loss_rate_kernel<<<(unsigned)((nnode + 127) / 128), 128, 0, stream>>>(nnode, d_pec.as<unsigned char>(), d_inc_ptr.as<int>(),
+                                                                                  d_inc.as<int>(), d_eps.as<double>(), d_sig.as<double>(),
+                                                                                  d_rho.as<double>(), d_lden.as<double>());
+        EMS_CUDA(cudaGetLastError());
         std::vector<double> dmp(nnode);
-        for (size_t v = 0; v < nnode; ++v) {
-            double num = 0.0, den = 0.0;
-            for (int d = 0; d < 7; ++d) {
-                const size_t e = 7 * v + d;
-                if (pec_h[e] & kPecBit) continue;
-                for (int q = inc_ptr_h[e]; q < inc_ptr_h[e + 1]; ++q) {
-                    const int t = inc_h[q] >> 3, l = inc_h[q] & 7, p = t % 6;
-                    num += sig_h[t] * wsq[p][l];
-                    den += eps_h[t] * wsq[p][l];
-                }
-            }
-            rho_h[v] = den > 0.0 ? num / den : 0.0;
-            lden_h[v] = den;
-            dmp[v] = symp ? std::exp(-0.5 * dtn * rho_h[v]) : 0.5 * dtn * rho_h[v];
-        }
+        EMS_CUDA(cudaMemcpyAsync(dmp.data(), d_rho.p, nnode * 8, cudaMemcpyDeviceToHost, stream));
+        EMS_CUDA(cudaStreamSynchronize(stream));
+        for (double &r : dmp) r = symp ? std::exp(-0.5 * dtn * r) : 0.5 * dtn * r;
         if (fp64) {
             up(d_damp, dmp);
         } else {
@@ -3034,9 +3079,9 @@ struct TetFemSim : Sim {
 
     // ---- discrete adjoint of the recorded run
     // Receiver terms grouped by edge slot and by node for
-    // tet_receiver_gather_kernel and tet_receiver_drift_kernel.
+    // tet_receiver_adjoint_kernel.
     struct RecAdj {
-        DevBuf sl_slot, sl_ptr, term_rc, term_w, nd_node, nd_map, a_scr;
+        DevBuf sl_ptr, term_rc, term_w, nd_node, nd_map;
         int nsl = 0, nnd = 0;
     };
     void build_receiver_adjoint(RecAdj &ra)
@@ -3079,9 +3124,8 @@ struct TetFemSim : Sim {
         ra.nsl = (int)sl_slot.size();
         ra.nnd = (int)nd_node.size();
         if (sl_slot.empty()) { sl_slot.push_back(0); term_rc.push_back(0); term_w.push_back(0.0); nd_node.push_back(0); nd_map.assign(7, -1); }
-        up(ra.sl_slot, sl_slot); up(ra.sl_ptr, sl_ptr); up(ra.term_rc, term_rc); up(ra.term_w, term_w);
+        up(ra.sl_ptr, sl_ptr); up(ra.term_rc, term_rc); up(ra.term_w, term_w);
         up(ra.nd_node, nd_node); up(ra.nd_map, nd_map);
-        ra.a_scr.alloc(std::max(ra.nsl, 1) * sizeof(double));
     }
 
     // dJ/deps per tetrahedron (FP64) for dJ/dtraces tg (nobs x nsamp x 4,
@@ -3163,13 +3207,10 @@ struct TetFemSim : Sim {
                 }
                 if (n % tf == 0 && n > 0 && nobs > 0 && ra.nsl > 0) {
                     const T *z = zb + (size_t)(n - n0) * nsub * nslot;
-                    tet_receiver_gather_kernel<T><<<(ra.nsl + 255) / 256, 256, 0, stream>>>(
-                        ra.nsl, ra.sl_slot.as<int>(), ra.sl_ptr.as<int>(), ra.term_rc.as<int>(), ra.term_w.as<double>(),
-                        d_rs.as<double>() + (size_t)(n / tf) * nobs * 3, ra.a_scr.as<double>(), Wb.as<T>(), nnode);
-                    if (sc.sub[nsub - 1] != 0.0 && ra.nnd > 0)
-                        tet_receiver_drift_kernel<T><<<(ra.nnd + 127) / 128, 128, 0, stream>>>(
-                            ra.nnd, ra.nd_node.as<int>(), ra.nd_map.as<int>(), ra.a_scr.as<double>(), pb, d_minv.as<T>(),
-                            z, Q.as<double>(), 0.5 * sc.sub[nsub - 1], nnode);
+                    tet_receiver_adjoint_kernel<T><<<(8 * ra.nnd + 127) / 128, 128, 0, stream>>>(
+                        ra.nnd, ra.nd_node.as<int>(), ra.nd_map.as<int>(), ra.sl_ptr.as<int>(), ra.term_rc.as<int>(), ra.term_w.as<double>(),
+                        d_rs.as<double>() + (size_t)(n / tf) * nobs * 3, Wb.as<T>(), pb, d_minv.as<T>(), z, Q.as<double>(),
+                        0.5 * sc.sub[nsub - 1], nnode);
                 }
             }
             // the drifts of this segment: y at [k], z at [k] (k = nsub (n - n0) + q)
@@ -3186,44 +3227,27 @@ struct TetFemSim : Sim {
         tet_grad_gather_kernel<<<nbt, 256, 0, stream>>>(ntet, d_tet_edge.as<int>(), d_pec.as<unsigned char>(),
                                                         d_inc_ptr.as<int>(), d_inc.as<int>(), contrib.as<double>(),
                                                         d_grad.as<double>());
+        if (has_loss) loss_gradient(zr, d_grad, grad_sigma != nullptr);
         EMS_CUDA(cudaGetLastError());
-        EMS_CUDA(cudaMemcpyAsync(grad, d_grad.p, ntet * 8, cudaMemcpyDeviceToHost, stream));
-        EMS_CUDA(cudaStreamSynchronize(stream));
-        loss_gradient(zr, grad, grad_sigma);
+        download(grad, d_grad.p, ntet, true);
+        if (grad_sigma && has_loss) download(grad_sigma, d_gsig.p, ntet, true);
+        else if (grad_sigma) std::fill(grad_sigma, grad_sigma + ntet, 0.0);
     }
 
-    // Loss-rate terms of the gradient (host, FP64): each loss factor g_v =
+    // Loss-rate terms of the gradient (FP64): each loss factor g_v =
     // exp(-rho_v dt/2) gives dJ/drho_v = -(dt/2) g_v zr_v, and rho_v =
     // sum sigma_T c_Tv / den_v (c_Tv the loss weights of T at v) gives
     // dJ/dsigma_T = sum_v dJ/drho_v c_Tv / den_v and dJ/deps_T -= sum_v
-    // dJ/drho_v rho_v c_Tv / den_v.  grad_sigma is per S/m.
-    void loss_gradient(const DevBuf &zr, double *grad, double *grad_sigma)
+    // dJ/drho_v rho_v c_Tv / den_v.  d_gsig is per S/m.
+    DevBuf d_gsig;
+    void loss_gradient(const DevBuf &zr, const DevBuf &d_grad, bool with_sigma)
     {
-        if (grad_sigma)
-            for (size_t t = 0; t < ntet; ++t) grad_sigma[t] = 0.0;
-        if (!has_loss) return;
-        std::vector<double> z(nnode);
-        EMS_CUDA(cudaMemcpy(z.data(), zr.p, nnode * 8, cudaMemcpyDeviceToHost));
-        double wsq[6][6];
-        for (int p = 0; p < 6; ++p) {
-            const Shape sh = make_shape(p);
-            for (int l = 0; l < 6; ++l) wsq[p][l] = sh.wsq[l];
-        }
         const double sig_unit = tscale / kEps0;   // d sigma_normalised / d sigma
-        for (size_t v = 0; v < nnode; ++v) {
-            if (lden_h[v] <= 0.0) continue;
-            const double gr = -0.5 * dtn * std::exp(-0.5 * dtn * rho_h[v]) * z[v];
-            for (int d = 0; d < 7; ++d) {
-                const size_t e = 7 * v + d;
-                if (pec_h[e] & kPecBit) continue;
-                for (int q = inc_ptr_h[e]; q < inc_ptr_h[e + 1]; ++q) {
-                    const int t = inc_h[q] >> 3, l = inc_h[q] & 7, p = t % 6;
-                    const double wv = wsq[p][l] / lden_h[v];
-                    if (grad_sigma) grad_sigma[t] += gr * wv * sig_unit;
-                    grad[t] -= gr * rho_h[v] * wv;
-                }
-            }
-        }
+        if (with_sigma) d_gsig.ensure(ntet * 8);
+        tet_loss_node_kernel<<<(unsigned)((nnode + 127) / 128), 128, 0, stream>>>(nnode, dtn, d_rho.as<double>(), zr.as<double>());
+        tet_loss_grad_kernel<<<(unsigned)((ntet + 127) / 128), 128, 0, stream>>>(ntet, d_tet_edge.as<int>(), d_pec.as<unsigned char>(),
+                                                                                 d_rho.as<double>(), d_lden.as<double>(), zr.as<double>(), sig_unit,
+                                                                                 d_grad.as<double>(), with_sigma ? d_gsig.as<double>() : nullptr);
     }
 
     // Discrete energy H = 1/2 P.Minv P + 1/2 U.K U of the current
@@ -3288,16 +3312,19 @@ struct TetFemSim : Sim {
     // Fields cross the API in slot order (e = 7 node + d) and live on the
     // device in the plane layout (fslot).  With a compensation plane lo
     // (FP32 symplectic handles) the value is hi + lo, split again on upload.
+    mutable DevBuf d_slots;
     template <class T> void download_slots(const DevBuf &b, double *out, const __nv_bfloat16 *lo = nullptr) const
     {
-        std::vector<T> tmp(nslot);
-        EMS_CUDA(cudaMemcpy(tmp.data(), b.p, nslot * sizeof(T), cudaMemcpyDeviceToHost));
-        std::vector<uint16_t> lw(lo ? nslot : 0);
-        if (lo) EMS_CUDA(cudaMemcpy(lw.data(), lo, nslot * 2, cudaMemcpyDeviceToHost));
-        for (size_t e = 0; e < nslot; ++e) {
-            const size_t f = fslot(e, nnode);
-            out[e] = (double)tmp[f] + (lo ? (double)bf16_to_float(lw[f]) : 0.0);
+        const unsigned nb = (unsigned)((nslot + 255) / 256);
+        if (lo) {   // hi + lo in FP64
+            d_slots.ensure(nslot * 8);
+            tet_slots_kernel<T, double><<<nb, 256, 0, stream>>>(nslot, nnode, b.as<T>(), lo, d_slots.as<double>());
+        } else {
+            d_slots.ensure(nslot * sizeof(T));
+            tet_slots_kernel<T, T><<<nb, 256, 0, stream>>>(nslot, nnode, b.as<T>(), nullptr, d_slots.as<T>());
         }
+        EMS_CUDA(cudaGetLastError());
+        download(out, d_slots.p, nslot, lo || sizeof(T) == 8);
     }
     template <class T> void upload_slots(DevBuf &b, const double *in, __nv_bfloat16 *lo = nullptr) const
     {
@@ -3313,13 +3340,6 @@ struct TetFemSim : Sim {
     }
     // bfloat16 <-> float on the host: the upper half of the binary32
     // pattern, rounded to nearest even on the way down (NaN kept quiet).
-    static float bf16_to_float(uint16_t h)
-    {
-        const uint32_t u = (uint32_t)h << 16;
-        float f;
-        std::memcpy(&f, &u, 4);
-        return f;
-    }
     static uint16_t float_to_bf16(float f)
     {
         uint32_t u;
