@@ -2127,11 +2127,11 @@ struct Tet2Sim : Sim {
         return lam;
     }
 
-    void setup()
+    // The stability limit (the power iteration is a hundred mass solves): for
+    // the automatic time step, and when it is asked for.
+    void find_limit()
     {
-        cheb_coefficients();
-        if (fp64) launch_pinv_and_eps<double>(); else launch_pinv_and_eps<float>();
-        if (fp64) choose_iteration<double>(); else choose_iteration<float>();
+        if (limit_known) return;
         // the power iteration uses the solver's scratch; the state (U, Uold, P) is kept
         DevBuf keep;
         keep.alloc(ndof * (fp64 ? 8 : 4));
@@ -2139,7 +2139,26 @@ struct Tet2Sim : Sim {
         lambda_max = fp64 ? lambda_max_t<double>(100) : lambda_max_t<float>(100);
         EMS_CUDA(cudaMemcpy(d_Uold.p, keep.p, keep.bytes, cudaMemcpyDeviceToDevice));
         dt_lim_n = tet_stability_constant(P.integrator) / std::sqrt(lambda_max);
-        dtn = P.dt > 0 ? P.dt / tscale : P.cfl_fraction * dt_lim_n;
+        limit_known = true;
+        y_valid = false;   // it was in the scratch
+    }
+    bool chosen = false, limit_known = false;
+
+    void setup()
+    {
+        cheb_coefficients();
+        if (fp64) launch_pinv_and_eps<double>(); else launch_pinv_and_eps<float>();
+        if (!chosen) {   // the form depends on the meshes alone
+            if (fp64) choose_iteration<double>(); else choose_iteration<float>();
+            chosen = true;
+        }
+        limit_known = false;
+        if (P.dt > 0) {
+            dtn = P.dt / tscale;
+        } else {
+            find_limit();
+            dtn = P.cfl_fraction * dt_lim_n;
+        }
         ready = true;
         y_valid = false;
     }
@@ -2759,6 +2778,7 @@ void tet2_time_step(const Sim *s, double *dt, double *lim)
 {
     auto *f = const_cast<Tet2Sim *>(static_cast<const Tet2Sim *>(s));
     if (!f->ready) f->setup();
+    if (lim) f->find_limit();
     if (dt) *dt = f->dtn * f->tscale;
     if (lim) *lim = f->dt_lim_n * f->tscale;
 }

@@ -1940,11 +1940,13 @@ struct TetFemSim : Sim {
     DevBuf d_damp;
     int step_block = 64;            // threads per block of tet_step_kernel (tune_launch_shape)
     bool slot_split = true;         // symplectic lossless steps by tet_slot_kernel (tune_launch_shape)
-    // Until a run tunes the shape (recorded runs do not), the slot-split
-    // kernel serves meshes that fit in L2, the node kernel larger ones (on
-    // the 64-shot batch and the 16-shot 48^3 inversion the node kernel is
-    // the faster, bandwidth-bound one).
-    static constexpr size_t kSlotDefaultMaxNodes = 262144;
+    // Until a run tunes the shape (recorded runs do not): in FP32 the
+    // slot-split kernel on meshes of up to 100,000 nodes (us a launch, slot-split
+    // against node kernel: 36k nodes 5.3 and 7.6, 69k 7.9 and 9.2, 98k 10.1 and 9.9,
+    // 118k 11.5 and 8.2), in FP64 of up to 12,000 nodes (9k 7.6 and 11.6, 16k 12.5 and
+    // 11.8, 49k 29.5 and 22.6): the node kernel forms every curl once, and the FP64
+    // pipe is soon full.
+    static constexpr size_t kSlotMaxNodes32 = 100000, kSlotMaxNodes64 = 12000;
     bool step_tuned = false;        // the block size depends on the mesh only: tuned once per handle
     // the persistent step (tet_persist_kernel, a tuner candidate): its grid
     // barrier's counter and error word, the resident-block capacity of its
@@ -2024,7 +2026,8 @@ struct TetFemSim : Sim {
         EMS_CHECK_ARG(ntet < (size_t)1 << 28, "mesh too large for 28-bit element indices");
         EMS_CHECK_ARG(nslot < (size_t)1 << 31, "mesh too large for 32-bit slot indices");
         build_mesh();
-        slot_split = nnode <= kSlotDefaultMaxNodes;
+        slot_split = nnode <= (fp64 ? kSlotMaxNodes64 : kSlotMaxNodes32);
+        step_block = fp64 ? 32 : 128;
         eps_h.assign(ntet, 1.0);
         init_stream();
         upload_tables();
@@ -2224,8 +2227,7 @@ struct TetFemSim : Sim {
     // loop runs them, twice over, and the fastest is kept for the rest of
     // the run and later ones.  (Timed on idle steps outside a run, the
     // candidates ranked differently from the loop.)  Before that the
-    // slot-split kernel runs on meshes of up to kSlotDefaultMaxNodes nodes
-    // and the 64-thread node kernel on larger ones.  The environment
+    // default above runs.  The environment
     // variable EMS_TET_STEP_BLOCK (32, 64, 128, 256, slot or persist) forces
     // one; EMS_TET_TUNE_LOG prints the candidates' times to stderr.
     static constexpr int kShapes = 6, kTuneRounds = 2, kShapeSlot = 4, kShapePersist = 5;
