@@ -195,9 +195,8 @@ template <class T> __device__ __forceinline__ unsigned x_bits(const Prof<T> &p, 
         if (p.on(i + v)) m |= 1u << v;
     return m;
 }
-// Programmatic dependent launch: the next kernel's blocks may be scheduled;
-// everything the last kernel wrote may be read from here on.
-__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+// Programmatic dependent launch: everything the last kernel wrote may be read
+// from here on.
 __device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // The cells of a thread: V columns from i of row j, plane k (false: none).
@@ -228,7 +227,6 @@ template <class T, bool PML>
 __global__ void __launch_bounds__(256) fdtd_h_kernel(FdtdArgs<T> a, int kz, unsigned mblocks, int *ctr, int inc)
 {
     constexpr int V = Vec<T>::V;
-    next_may_start();
     wait_for_last();
     // the step counter of a replayed graph, moved on by its first launch (the H kernels do not read it)
     if (ctr && blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0) *ctr += inc;
@@ -317,7 +315,6 @@ template <class T, bool MAT, bool PML>
 __global__ void __launch_bounds__(256) fdtd_e_kernel(FdtdArgs<T> a, FdtdPoints pt, int kz, unsigned mblocks)
 {
     constexpr int V = Vec<T>::V;
-    next_may_start();
     int i, j, k;
     size_t o;
     bool xl;
@@ -328,12 +325,6 @@ __global__ void __launch_bounds__(256) fdtd_e_kernel(FdtdArgs<T> a, FdtdPoints p
     const bool ex = jn && kn, ey = kn && nyz > 0, ez = jn && nyz > 0;
     Vec<T> e0{}, e1{}, e2{}, zk{}, zjk{}, yj{}, yjk{}, xi{}, xik{}, xij{}, zk1{}, yj1{};
     CaCb<T> c0[V], c1[V], c2[V];
-    if (MAT) {   // Ex(i,j,k) -> cell (min(i,nx-1), j-1, k-1), Ey -> (i-1, min(j,ny-1), k-1), Ez -> (i-1, j-1, min(k,nz-1))
-        const size_t mrow = a.mpitch, mpl = mrow * a.ny;
-        if (ex) e_material(a, a.mat + (j - 1) * mrow + (k - 1) * mpl + i, c0);
-        if (ey) e_material(a, a.mat + min(j, a.ny - 1) * mrow + (k - 1) * mpl + i, c1);
-        if (ez) e_material(a, a.mat + (j - 1) * mrow + min(k, a.nz - 1) * mpl + i, c2);
-    }
     wait_for_last();
     if (kn) {
         vload(zk, a.Hz + o - pz);                       // Hz(i, j, k-1)
@@ -353,6 +344,12 @@ __global__ void __launch_bounds__(256) fdtd_e_kernel(FdtdArgs<T> a, FdtdPoints p
     }
     if (ey) vload(e1, a.Ey + o);
     if (ez) vload(e2, a.Ez + o);
+    if (MAT) {   // Ex(i,j,k) -> cell (min(i,nx-1), j-1, k-1), Ey -> (i-1, min(j,ny-1), k-1), Ez -> (i-1, j-1, min(k,nz-1))
+        const size_t mrow = a.mpitch, mpl = mrow * a.ny;
+        if (ex) e_material(a, a.mat + (j - 1) * mrow + (k - 1) * mpl + i, c0);
+        if (ey) e_material(a, a.mat + min(j, a.ny - 1) * mrow + (k - 1) * mpl + i, c1);
+        if (ez) e_material(a, a.mat + (j - 1) * mrow + min(k, a.nz - 1) * mpl + i, c2);
+    }
 #pragma unroll
     for (int v = 0; v < V - 1; ++v) {
         zk1.v[v] = zk.v[v + 1];                         // Hz(i+1, j, k-1)
@@ -757,10 +754,12 @@ struct FdtdSim : Sim {
         return nsteps >= kTuneMinSteps ? kShapes * kTuneSteps : 0;
     }
 
-    // A launch whose blocks may start while the kernel before it ends: index
-    // arithmetic and the material loads overlap it, everything else waits for
-    // it (64^3 FP64 25.7 -> 24.5 us a step, 141x117x93 FP32 with CPML 29.9 -> 28.2,
-    // large grids unchanged).
+    // A launch that is set up while the kernel before it runs; its blocks start
+    // as that one ends and wait for its writes (24x20x16 FP64 7.9 -> 6.8 us a
+    // step, 64^3 FP64 25.0 -> 24.2, 141x117x93 FP32 with CPML 29.2 -> 28.3, large
+    // grids unchanged).  An early trigger in the kernels gave less, and so did
+    // material loads ahead of the wait (400x384x368: 54.4 ms for 60 steps, 52.5
+    // with the field loads first).
     template <class K, class... A> void launch(K k, dim3 g, A... args)
     {
         cudaLaunchConfig_t c{};
