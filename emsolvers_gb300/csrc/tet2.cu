@@ -904,6 +904,23 @@ __device__ __forceinline__ void stiff_curls(std::integer_sequence<int, A...>, co
 {
     (stiff_curl<P, A>(std::make_integer_sequence<int, 12>{}, u[A], cs, cc), ...);
 }
+// (double)x by integer operations: GB300 converts at its FP64 rate, two lanes
+// per SM and clock, and half of the pass's FP64 work was conversions.  For
+// infinities and NaN rare is set and the caller converts again (denormals fill
+// the fringe of every growing field, so they belong to this path).  (A conversion behind a predicate per value took
+// the pipe's time all the same.)
+template <bool CONVERT> __device__ __forceinline__ double widen(float x, bool &rare)
+{
+    if constexpr (CONVERT) {
+        return (double)x;
+    } else {
+        const unsigned m0 = __float_as_uint(x) & 0x7fffffffu;
+        rare = rare || m0 >= 0x7f800000u;
+        const bool den = m0 < 0x00800000u;   // scaled by 2^64 first (exact)
+        const unsigned u = __float_as_uint(den ? x * 0x1p64f : x), m = u & 0x7fffffffu;
+        return __hiloint2double((int)((m ? (m >> 3) + (den ? 0x38000000u - (64u << 20) : 0x38000000u) : 0u) | (u & 0x80000000u)), (int)(u << 29));
+    }
+}
 template <int P, int A, int Q> __device__ __forceinline__ void stiff_term(float hh, float hl, float &s, float &c)
 {
     constexpr float K = kCurl.c[P][A][Q];
@@ -912,29 +929,46 @@ template <int P, int A, int Q> __device__ __forceinline__ void stiff_term(float 
         c = fmaf(K, hl, c);
     }
 }
-template <int P, int A, int... Q>
-__device__ __forceinline__ void stiff_value(std::integer_sequence<int, Q...>, const float (&hh)[12], const float (&hl)[12], double *y)
+template <int P, bool CONVERT, int A, int... Q>
+__device__ __forceinline__ void stiff_value(std::integer_sequence<int, Q...>, const float (&hh)[12], const float (&hl)[12], double *y, bool &rare)
 {
     float s = 0.0f, c = 0.0f;
     (stiff_term<P, A, Q>(hh[Q], hl[Q], s, c), ...);
-    *y = (double)s + (double)c;
+    *y = widen<CONVERT>(s, rare) + widen<CONVERT>(c, rare);
 }
-template <int P, int... A>
+template <int P, bool CONVERT, int... A>
 __device__ __forceinline__ void stiff_values(std::integer_sequence<int, A...>, const float (&hh)[12], const float (&hl)[12], double *y,
-                                             unsigned long long NT)
+                                             unsigned long long NT, bool &rare)
 {
-    (stiff_value<P, A>(std::make_integer_sequence<int, 12>{}, hh, hl, y + A * NT), ...);
+    (stiff_value<P, CONVERT, A>(std::make_integer_sequence<int, 12>{}, hh, hl, y + A * NT, rare), ...);
+}
+// P1 mass of the vertex curls cs + cc in FP64 (12 values), split again into hi + lo.
+template <bool CONVERT>
+__device__ __forceinline__ void stiff_mass(const float (&cs)[12], const float (&cc)[12], float (&hh)[12], float (&hl)[12], bool &rare)
+{
+    double c[12];
+#pragma unroll
+    for (int q = 0; q < 12; ++q) c[q] = widen<CONVERT>(cs[q], rare) + widen<CONVERT>(cc[q], rare);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double sm = c[q] + c[3 + q] + c[6 + q] + c[9 + q];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const double h = (c[3 * v + q] + sm) * (1.0 / 120.0);
+            hh[3 * v + q] = (float)h;
+            hl[3 * v + q] = (float)(h - widen<CONVERT>(hh[3 * v + q], rare));
+        }
+    }
 }
 
 // Stiffness element pass of FP32 runs in double-float arithmetic: vertex
 // curls, P1 mass and transposed curl as the FP64 pass, each sum a compensated
 // dot product, so the element values carry about twice the FP32 precision at
 // FP32 throughput.  A body per type; the tetrahedra are type-major, so the
-// blocks in flight share one.  Bound by the FP64 pipe (86% busy: 77 sums and
-// 100 conversions per tetrahedron at two lanes per SM and clock).  With the
-// coefficients read from constant memory it ran 5,500 instructions per warp
-// and waited for them and for the instruction cache: 425 us on 48^3 cubes,
-// 226 us now.
+// blocks in flight share one.  Bound by the FP64 pipe (64% busy: 77 sums and
+// 24 conversions per tetrahedron at two lanes per SM and clock) and the
+// instruction cache.  On 48^3 cubes 425 us with the coefficients read from
+// constant memory, 226 us with 100 conversions on the FP64 pipe, 176 us now.
 template <int P> __device__ __forceinline__ void stiff_df_body(const TetAddr &ta, unsigned long long NT, unsigned long long t,
                                                                const float *__restrict__ U, double *__restrict__ Yt)
 {
@@ -943,22 +977,15 @@ template <int P> __device__ __forceinline__ void stiff_df_body(const TetAddr &ta
 #pragma unroll
     for (int q = 0; q < 12; ++q) { cs[q] = 0.0f; cc[q] = 0.0f; }
     stiff_curls<P>(std::make_integer_sequence<int, 20>{}, u, cs, cc);
-    // P1 mass in FP64 (12 values), split again into hi + lo
-    double c[12];
-#pragma unroll
-    for (int q = 0; q < 12; ++q) c[q] = (double)cs[q] + (double)cc[q];
     float hh[12], hl[12];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        const double sm = c[q] + c[3 + q] + c[6 + q] + c[9 + q];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const double h = (c[3 * v + q] + sm) * (1.0 / 120.0);
-            hh[3 * v + q] = (float)h;
-            hl[3 * v + q] = (float)(h - (double)hh[3 * v + q]);
-        }
+    constexpr auto all = std::make_integer_sequence<int, 20>{};
+    bool rare = false;
+    stiff_mass<false>(cs, cc, hh, hl, rare);
+    if (!rare) stiff_values<P, false>(all, hh, hl, Yt + t, NT, rare);
+    if (rare) {
+        stiff_mass<true>(cs, cc, hh, hl, rare);
+        stiff_values<P, true>(all, hh, hl, Yt + t, NT, rare);
     }
-    stiff_values<P>(std::make_integer_sequence<int, 20>{}, hh, hl, Yt + t, NT);
 }
 
 __global__ void __launch_bounds__(128) t2_stiff_df_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,

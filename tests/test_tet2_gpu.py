@@ -332,3 +332,31 @@ def test_double_float_stiffness_matches_oracle(n):
     s = ems.TetFemSimulation(n, H, 2, ems.SYMP4, ems.FP32, dt=0.05 * TS)
     f, ref = from_api(n, s.apply_stiffness(to_api(n, U))), oracle.tet2_apply(n, U, True)
     assert np.linalg.norm(f - ref) <= 2.0 ** -24 * np.linalg.norm(ref)
+
+
+def test_double_float_stiffness_of_tiny_and_huge_values():
+    """Values whose conversions leave the integer path (denormals in the
+    products, infinities) next to ordinary ones: far parts of the field give
+    what the same field alone gives, an infinity stays in its elements."""
+    n = (6, 2, 2)
+    nnode, ndof, _ = oracle.tet2_sizes(n)
+    rng = np.random.default_rng(47)
+    x = np.tile(np.arange(nnode) % 7, 38)
+    pec = oracle.tet2_pec_mask(n)
+    base = np.where(pec, 0.0, rng.standard_normal(ndof).astype(np.float32).astype(np.float64))
+    s = ems.TetFemSimulation(n, H, 2, ems.SYMP4, ems.FP32, dt=0.05 * TS)
+
+    def apply(u):
+        return from_api(n, s.apply_stiffness(to_api(n, u)))
+
+    near = np.where(x <= 1, base, 0.0)
+    ref = oracle.tet2_apply(n, near, True)
+    tiny = near + np.where(x >= 4, base * 1e-40, 0.0)          # FP32 denormals from x = 4 on
+    f = apply(tiny)
+    assert np.linalg.norm(f - ref) <= 2.0 ** -24 * np.linalg.norm(ref)
+    huge = near.copy()
+    at = int(np.flatnonzero((x == 5) & ~pec)[0])
+    huge[at] = np.inf
+    f = apply(huge)
+    assert not np.isfinite(f[x >= 4]).all()
+    assert np.linalg.norm((f - ref)[x <= 2]) <= 2.0 ** -24 * np.linalg.norm(ref)
