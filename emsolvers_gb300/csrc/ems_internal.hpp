@@ -153,6 +153,28 @@ void trace_misfit(int kind, int nobs, int nsamp, const double *traces, const dou
 // Source waveforms evaluated on the host in FP64.
 double fdtd_source_value(int kind, double f0, double t, double h);
 
+#ifdef __CUDACC__
+// Launch of a kernel that waits (wait_for_last, before its first access) for
+// the kernel before it in the stream: its blocks are set up while that one
+// runs and start as it ends.
+template <class... P, class... A> void launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... a)
+{
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    EMS_CUDA(cudaLaunchKernelEx(&c, k, static_cast<P>(a)...));
+}
+// Everything the kernel before this one wrote may be read from here on.
+__device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 }  // namespace ems
 
 struct ems_sim {

@@ -195,10 +195,6 @@ template <class T> __device__ __forceinline__ unsigned x_bits(const Prof<T> &p, 
         if (p.on(i + v)) m |= 1u << v;
     return m;
 }
-// Programmatic dependent launch: everything the last kernel wrote may be read
-// from here on.
-__device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // The cells of a thread: V columns from i of row j, plane k (false: none).
 // Threads run through the rows of a plane without a break, so short rows fill
 // the warps too.  The columns near an x layer (xl) have blocks of their own:
@@ -754,30 +750,16 @@ struct FdtdSim : Sim {
         return nsteps >= kTuneMinSteps ? kShapes * kTuneSteps : 0;
     }
 
-    // A launch that is set up while the kernel before it runs; its blocks start
-    // as that one ends and wait for its writes (24x20x16 FP64 7.9 -> 6.8 us a
+    // The H and E launches are set up ahead (launch_after: 24x20x16 FP64 7.9 -> 6.8 us a
     // step, 64^3 FP64 25.0 -> 24.2, 141x117x93 FP32 with CPML 29.2 -> 28.3, large
     // grids unchanged).  An early trigger in the kernels gave less, and so did
     // material loads ahead of the wait (400x384x368: 54.4 ms for 60 steps, 52.5
     // with the field loads first).
-    template <class K, class... A> void launch(K k, dim3 g, A... args)
-    {
-        cudaLaunchConfig_t c{};
-        c.gridDim = g;
-        c.blockDim = blk;
-        c.stream = stream;
-        cudaLaunchAttribute at{};
-        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at.val.programmaticStreamSerializationAllowed = 1;
-        c.attrs = &at;
-        c.numAttrs = 1;
-        EMS_CUDA(cudaLaunchKernelEx(&c, k, args...));
-    }
     // H update of planes [k0, k1)
     template <class T> void launch_h(const FdtdArgs<T> &a, int k0, int k1, int *ctr = nullptr, int inc = 0)
     {
         auto k = P.pml_cells > 0 ? fdtd_h_kernel<T, true> : fdtd_h_kernel<T, false>;
-        launch(k, grid(k1 - k0), a, k0, main_blocks(), ctr, inc);
+        launch_after(k, grid(k1 - k0), blk, 0, stream, a, k0, main_blocks(), ctr, inc);
     }
     // E update of planes [k0, k1) with the planes' points
     template <class T> void launch_e(const FdtdArgs<T> &a, int k0, int k1, const FdtdPoints &pt)
@@ -785,7 +767,7 @@ struct FdtdSim : Sim {
         const bool mat = !mat_host.empty(), pml = P.pml_cells > 0;
         auto k = mat ? (pml ? fdtd_e_kernel<T, true, true> : fdtd_e_kernel<T, true, false>)
                      : (pml ? fdtd_e_kernel<T, false, true> : fdtd_e_kernel<T, false, false>);
-        launch(k, grid(k1 - k0), a, pt, k0, main_blocks());
+        launch_after(k, grid(k1 - k0), blk, 0, stream, a, pt, k0, main_blocks());
     }
 
     // The sources and receiver samples as the E kernel's point lists; false

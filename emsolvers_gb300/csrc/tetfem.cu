@@ -752,6 +752,7 @@ __global__ void __launch_bounds__(kStepBlockMax) tet_step_kernel(size_t nnode, c
                                                        const T *__restrict__ damp, T *__restrict__ ppre, T *__restrict__ pmid,
                                                        RecArgs<T> rec, Comp cmp)
 {
+    wait_for_last();
     static_assert(!COMP || (MODE == 0 && std::is_same<T, float>::value), "compensated updates: FP32 symplectic steps");
     constexpr StepTab tab = make_step_tab();
     // the first rec.nsb blocks sample the receivers when this launch does
@@ -1019,6 +1020,7 @@ __global__ void __launch_bounds__(kSlotThreads, sizeof(T) == 4 ? 8 : 1) tet_slot
                                                                 const T *__restrict__ Uin, T *__restrict__ Uout, T a, T c,
                                                                 SrcArgs src, T *__restrict__ zout, RecArgs<T> rec, Comp cmp)
 {
+    wait_for_last();
     constexpr StepTab tab = make_step_tab();
     const int nb = (int)blockIdx.x - rec.nsb;
     if (nb < 0) {   // the leading blocks sample the receivers (no barrier below is reached)
@@ -2558,8 +2560,8 @@ struct TetFemSim : Sim {
                 const unsigned nbs = (unsigned)((nnode + kSlotNodes - 1) / kSlotNodes) + (unsigned)rec.nsb;
                 const dim3 blk(kSlotNodes, 7);
                 auto go = [&](auto kern) {
-                    kern<<<nbs, blk, 0, stream>>>(nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), d_minv.as<T>(), Pio,
-                                                  Uin, Uout, a, c, sa, zout, rec, cm);
+                    launch_after(kern, dim3(nbs), blk, 0, stream, nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), d_minv.as<T>(), Pio,
+                                 Uin, Uout, a, c, sa, zout, rec, cm);
                     return 1;
                 };
                 const bool comp32 = std::is_same<T, float>::value && cm.p;
@@ -2571,8 +2573,8 @@ struct TetFemSim : Sim {
         const unsigned nbv = (unsigned)((nnode + step_block - 1) / step_block) + (unsigned)rec.nsb;
         const T *dm = DAMP ? d_damp.as<T>() : nullptr;
         auto go = [&](auto kern) {
-            kern<<<nbv, step_block, 0, stream>>>(nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), d_minv.as<T>(), Pio, Uin,
-                                                 Uout, Uold, a, c, sa, zout, dm, ppre, pmid, rec, cm);
+            launch_after(kern, dim3(nbv), dim3(step_block), 0, stream, nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), d_minv.as<T>(), Pio,
+                         Uin, Uout, Uold, a, c, sa, zout, dm, ppre, pmid, rec, cm);
             return 1;
         };
         if constexpr (MODE == 0 && std::is_same<T, float>::value) {
