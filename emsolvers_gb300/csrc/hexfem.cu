@@ -228,6 +228,7 @@ __global__ void __launch_bounds__(128) hex_kick_kernel(HexGeom g, const T *__res
 template <class T, bool EXACT>
 __global__ void hex_drift_kernel(HexGeom g, T *Ux, T *Uy, T *Uz, T *Px, T *Py, T *Pz, T coef, T m, int pec)
 {
+    wait_for_last();
     const int c = blockIdx.y;
     size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.nc[c]) return;
@@ -261,6 +262,7 @@ template <class T>
 __global__ void hex_sample_kernel(HexGeom g, const T *Lx, const T *Ly, const T *Lz, int nobs, const int *obs, double *tr, int nsamp, int s,
                                   const int *step, int tf)
 {
+    wait_for_last();
     if (step) {   // a replayed step: the row from the step counter
         if (*step % tf) return;
         s = *step / tf;
@@ -300,6 +302,7 @@ template <class T, int O, bool EXACT>
 __global__ void __launch_bounds__(128) hex_elem_kernel(HexGeom g, const T *__restrict__ K, const T *__restrict__ Ux, const T *__restrict__ Uy,
                                                        const T *__restrict__ Uz, T *__restrict__ fe, int *step, HexRec rec)
 {
+    wait_for_last();
     constexpr int D = O * (O + 1) * (O + 1), TT = 3 * D, W = 16 / (int)sizeof(T), RP = (D + W - 1) / W * W;
     __shared__ __align__(16) T sK[TT * RP];
     const int c = blockIdx.y;
@@ -393,6 +396,7 @@ __global__ void __launch_bounds__(32) hex1_elem_kernel(HexGeom g, const __grid_c
                                                        const double *__restrict__ Uy, const double *__restrict__ Uz, double *__restrict__ fe,
                                                        int *step, HexRec rec)
 {
+    wait_for_last();
     const int ne = g.EX * g.EY * g.EZ, e = blockIdx.x * 32 + threadIdx.x;
     if (hex_elem_head<double>(g, Ux, Uy, Uz, ne, 32, step, rec) || e >= ne) return;
     const int r0 = e / g.EX, ei = e - r0 * g.EX, ek = r0 / g.EY, ej = r0 - ek * g.EY, gx = g.gx, gy = g.gy;
@@ -472,6 +476,7 @@ template <class T, int O, bool EXACT>
 __global__ void __launch_bounds__(128) hex_leap_dof_kernel(const __grid_constant__ HexGeom g, const T *__restrict__ fe, const __grid_constant__ HexDofs<T> d,
                                                            const __grid_constant__ SrcTab src)
 {
+    wait_for_last();
     const int c = blockIdx.y;
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0 && c == 0) src.step[0] += 1;
@@ -496,6 +501,7 @@ template <class T, int O, bool EXACT>
 __global__ void __launch_bounds__(128) hex_kick_dof_kernel(const __grid_constant__ HexGeom g, const T *__restrict__ fe, const __grid_constant__ HexDofs<T> d,
                                                            const __grid_constant__ SrcTab src, T dt, T h1, T h2, T rm)
 {
+    wait_for_last();
     const int c = blockIdx.y;
     const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (src.last && t == 0 && c == 0) src.step[0] += 1;
@@ -649,7 +655,7 @@ struct HexFemSim : Sim {
         dim3 grid((unsigned)((mx + 255) / 256), 3);
         T m = (T)(8.0 / g.o / g.o / g.o);
         auto k = exact ? hex_drift_kernel<T, true> : hex_drift_kernel<T, false>;
-        k<<<grid, 256, 0, stream>>>(g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), L<T>(0, 1), L<T>(1, 1), L<T>(2, 1), coef, m, pec);
+        launch_after(k, grid, dim3(256), 0, stream, g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), L<T>(0, 1), L<T>(1, 1), L<T>(2, 1), coef, m, pec);
     }
 
     SrcList sources(double val) const
@@ -685,10 +691,10 @@ struct HexFemSim : Sim {
         int *step = first ? d_step.as<int>() : nullptr;
         if constexpr (X && O == 1)
             if (classes && ne >= kHex1MinElements) {
-                hex1_elem_kernel<<<(ne + 31) / 32 + (rec.n + 31) / 32, 32, 0, stream>>>(g, cls, u[0], u[1], u[2], d_fe.as<T>(), step, rec);
+                launch_after(hex1_elem_kernel, dim3((ne + 31) / 32 + (rec.n + 31) / 32), dim3(32), 0, stream, g, cls, u[0], u[1], u[2], d_fe.as<T>(), step, rec);
                 return;
             }
-        hex_elem_kernel<T, O, X><<<dim3((ne + 127) / 128 + (rec.n + 127) / 128, 3), 128, 0, stream>>>(g, dK.as<T>(), u[0], u[1], u[2],
+        launch_after(hex_elem_kernel<T, O, X>, dim3((ne + 127) / 128 + (rec.n + 127) / 128, 3), dim3(128), 0, stream, g, dK.as<T>(), u[0], u[1], u[2],
                                                                                                     d_fe.as<T>(), step, rec);
     }
     // One step of orders 1 and 2 in two passes per force; launches made.
@@ -697,7 +703,7 @@ struct HexFemSim : Sim {
         int n = 0;
         const bool leap = P.integrator == EMS_LEAPFROG;
         if (nobs > 0 && !leap) {   // the symplectic steps sample U before the step
-            hex_sample_kernel<T><<<(nobs + 63) / 64, 64, 0, stream>>>(g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(),
+            launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(),
                                                                       nsamp, 0, d_step.as<int>(), P.time_frequency);
             ++n;
         }
@@ -716,7 +722,7 @@ struct HexFemSim : Sim {
         }
         if (leap) {   // fem_v2 samples E^n, which the step leaves alone
             elements<T, O>(d.a, true, nobs > 0);
-            hex_leap_dof_kernel<T, O, X><<<dof_grid(), 128, 0, stream>>>(g, d_fe.as<T>(), d, src);
+            launch_after(hex_leap_dof_kernel<T, O, X>, dof_grid(), dim3(128), 0, stream, g, d_fe.as<T>(), d, src);
             l0 = (l0 + 1) % 3; l1 = (l1 + 1) % 3; l2 = (l2 + 1) % 3;
             return n + 2;
         }
@@ -730,7 +736,7 @@ struct HexFemSim : Sim {
             src.q = q;
             src.last = last;
             const T h1 = X || last ? (T)(0.5 * sub[q]) : (T)(0.5 * sub[q] + 0.5 * sub[q + 1]), h2 = X && !last ? (T)(0.5 * sub[q + 1]) : T(0);
-            hex_kick_dof_kernel<T, O, X><<<dof_grid(), 128, 0, stream>>>(g, d_fe.as<T>(), d, src, (T)sub[q], h1, h2, (T)(g.o * g.o * g.o / 8.0));
+            launch_after(hex_kick_dof_kernel<T, O, X>, dof_grid(), dim3(128), 0, stream, g, d_fe.as<T>(), d, src, (T)sub[q], h1, h2, (T)(g.o * g.o * g.o / 8.0));
         }
         return n + 1 + 2 * ns;
     }
@@ -815,7 +821,7 @@ struct HexFemSim : Sim {
             if (P.integrator == EMS_LEAPFROG) {
                 // fem_v2 samples level 1 (E^n) after computing E^{n+1}; E^n is untouched by the step
                 if (samp) {
-                    hex_sample_kernel<T><<<(nobs + 63) / 64, 64, 0, stream>>>(g, L<T>(0, l1), L<T>(1, l1), L<T>(2, l1), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf, nullptr, 1);
+                    launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, l1), L<T>(1, l1), L<T>(2, l1), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf, nullptr, 1);
                     times[step / tf] = cur_time;
                     ++launches;
                 }
@@ -825,7 +831,7 @@ struct HexFemSim : Sim {
                 l0 = (l0 + 1) % 3; l1 = (l1 + 1) % 3; l2 = (l2 + 1) % 3;
             } else {
                 if (samp) {
-                    hex_sample_kernel<T><<<(nobs + 63) / 64, 64, 0, stream>>>(g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf, nullptr, 1);
+                    launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf, nullptr, 1);
                     times[step / tf] = cur_time;
                     ++launches;
                 }

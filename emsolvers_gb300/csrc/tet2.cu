@@ -550,6 +550,7 @@ __global__ void __launch_bounds__(64) t2_mass_elem_kernel(unsigned long long NT,
                                                          const double *__restrict__ eps, const double *__restrict__ x,
                                                          double *__restrict__ Yt)
 {
+    wait_for_last();
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (t >= NT) return;
     const T2Shot S = sh[shot_of(sh, ns, t, 0)];
@@ -593,6 +594,7 @@ template <class T> struct GArgs {
 template <class T, class TY, int MODE, int FIN>
 __global__ void __launch_bounds__(128) t2_gather_kernel(unsigned long long NE, const T2Shot *__restrict__ sh, int ns, GArgs<T> g)
 {
+    wait_for_last();
     const unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (e >= NE) return;
     const T2Shot S = sh[shot_of(sh, ns, e, 1)];
@@ -851,6 +853,7 @@ __device__ __forceinline__ void stiff_body(std::integer_sequence<int, A...>, con
 __global__ void __launch_bounds__(64) t2_stiff_elem_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
                                                           const double *__restrict__ U, double *__restrict__ Yt)
 {
+    wait_for_last();
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (t >= NT) return;
     const T2Shot S = sh[shot_of(sh, ns, t, 0)];
@@ -991,6 +994,7 @@ template <int P> __device__ __forceinline__ void stiff_df_body(const TetAddr &ta
 __global__ void __launch_bounds__(128) t2_stiff_df_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
                                                          const float *__restrict__ U, double *__restrict__ Yt)
 {
+    wait_for_last();
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (t >= NT) return;
     const T2Shot S = sh[shot_of(sh, ns, t, 0)];
@@ -1073,17 +1077,15 @@ __global__ void __launch_bounds__(128) t2_cheb_kernel(unsigned long long NE, con
     const int pl0 = et < 7 ? et : 14 + 2 * (et - 7), pl1 = et < 7 ? et + 7 : pl0 + 1;
     const unsigned long long d0 = S.dof0 + (unsigned long long)pl0 * nn + v;
     const unsigned long long d1 = S.dof0 + (unsigned long long)pl1 * nn + v;
-    // Launched while the iteration before ends (programmatic dependent launch):
-    // the right-hand side and the block inverse do not change during a solve,
-    // everything else is read behind the wait; the next launch may start only
-    // after it, so what this one reads early is complete.
+    // Set up while the iteration before runs (launch_after): the right-hand
+    // side and the block inverse are older than that one, everything else is
+    // read behind the wait.
     T b0 = T(0), b1 = T(0), q00 = T(0), q01 = T(0), q11 = T(0);
     if (!dead) {
         b0 = g.b[d0]; b1 = g.b[d1];
         q00 = g.pinv[e]; q01 = g.pinv[NE + e]; q11 = g.pinv[2 * NE + e];
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;");
+    wait_for_last();
     if (dead) {
         g.x[d0] = T(0); g.x[d1] = T(0); g.d[d0] = T(0); g.d[d1] = T(0);
         return;
@@ -1391,6 +1393,7 @@ __global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *__r
     const int rw = t.bx + 1;
     for (int n = tid; n < kStageTable / 4; n += NT)
         reinterpret_cast<int4 *>(xoff)[n] = reinterpret_cast<const int4 *>(tables + t.table * kStageTable)[n];
+    wait_for_last();   // tiles and tables do not change
     const int ty = col / t.bx, tx = col - ty * t.bx;
     const int i = t.i0 + tx, j = t.j0 + ty;
     const bool active = ty < t.by && i < t.nx && j < t.ny;
@@ -1542,6 +1545,7 @@ template <class T> __global__ void t2_narrow_kernel(unsigned long long n, const 
 
 template <class T> __global__ void t2_axpy_kernel(unsigned long long n, T *__restrict__ U, const T *__restrict__ x, double h)
 {
+    wait_for_last();
     const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (i < n) U[i] = fma((T)h, x[i], U[i]);
 }
@@ -1555,6 +1559,7 @@ __global__ void t2_source_kernel(int n, const unsigned long long *__restrict__ d
                                  const int *__restrict__ ctl, int nsub, int q, int nd, double s, double *__restrict__ P,
                                  T *__restrict__ vec)
 {
+    wait_for_last();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const double *g = gt + ((size_t)ctl[0] * nsub + q) * nd;
@@ -1576,6 +1581,7 @@ template <class T>
 __global__ void t2_sample_kernel(int nrec, const unsigned long long *__restrict__ rdof, const double *__restrict__ rw,
                                  const T *__restrict__ U, const int *__restrict__ ctl, int tf, int nsamp, double *__restrict__ tr)
 {
+    wait_for_last();
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), l = threadIdx.x & 31;
     const int step = ctl[0];
     if (r >= nrec || step % tf != 0 || step / tf >= nsamp) return;
@@ -1593,13 +1599,14 @@ __global__ void t2_sample_kernel(int nrec, const unsigned long long *__restrict_
     }
 }
 
-__global__ void t2_advance_kernel(int *ctl) { ctl[0] += 1; }
+__global__ void t2_advance_kernel(int *ctl) { wait_for_last(); ctl[0] += 1; }
 
 // Block partial sums of x . y (fixed grid, fixed order); the host adds them.
 template <class T>
 __global__ void __launch_bounds__(256) t2_dot_kernel(unsigned long long n, const T *__restrict__ x, const T *__restrict__ y,
                                                     double *__restrict__ part)
 {
+    wait_for_last();
     __shared__ double sm[256];
     double s = 0.0;
     for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < n; i += 256ull * gridDim.x) s += (double)x[i] * (double)y[i];
@@ -1614,6 +1621,7 @@ __global__ void __launch_bounds__(256) t2_dot_kernel(unsigned long long n, const
 
 template <class T> __global__ void t2_scale_kernel(unsigned long long n, T *__restrict__ x, double s)
 {
+    wait_for_last();
     const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (i < n) x[i] = (T)((double)x[i] * s);
 }
@@ -1625,6 +1633,7 @@ __global__ void __launch_bounds__(128) t2_grad_kernel(unsigned long long NT, con
                                                      const T *__restrict__ Z, const T *__restrict__ Y, double c,
                                                      double *__restrict__ grad)
 {
+    wait_for_last();
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (t >= NT) return;
     const T2Shot S = sh[shot_of(sh, ns, t, 0)];
@@ -1644,7 +1653,7 @@ __global__ void __launch_bounds__(128) t2_grad_kernel(unsigned long long NT, con
     grad[t] += c * (double)s;
 }
 
-__global__ void t2_set_kernel(int *p, int v) { *p = v; }
+__global__ void t2_set_kernel(int *p, int v) { wait_for_last(); *p = v; }
 
 constexpr int kDotBlocks = 512;
 
@@ -1868,9 +1877,9 @@ struct Tet2Sim : Sim {
     template <class T> void enqueue_stiff(const T *u)
     {
         if constexpr (std::is_same<T, float>::value)
-            t2_stiff_df_kernel<<<blocks(ntet, 128), 128, 0, stream>>>(ntet, d_shots.as<T2Shot>(), (int)shots.size(), u, d_YtK.as<double>());
+            launch_after(t2_stiff_df_kernel, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(), (int)shots.size(), u, d_YtK.as<double>());
         else
-            t2_stiff_elem_kernel<<<blocks(ntet, 64), 64, 0, stream>>>(ntet, d_shots.as<T2Shot>(), (int)shots.size(), u, d_YtK.as<double>());
+            launch_after(t2_stiff_elem_kernel, dim3(blocks(ntet, 64)), dim3(64), 0, stream, ntet, d_shots.as<T2Shot>(), (int)shots.size(), u, d_YtK.as<double>());
     }
 
     // f = K u (element pass + entity pass), u and out device vectors
@@ -1880,7 +1889,7 @@ struct Tet2Sim : Sim {
         GArgs<T> g = gargs<T>();
         g.Yt = d_YtK.p;
         g.out = out;
-        t2_gather_kernel<T, double, G_FORCE, FIN_NONE><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(),
+        launch_after(t2_gather_kernel<T, double, G_FORCE, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(),
                                                                                              (int)shots.size(), g);
         return 2;
     }
@@ -1987,23 +1996,14 @@ struct Tet2Sim : Sim {
         if constexpr (sizeof(T) == 4) {
             if (cheb_form == FORM_MARCH) {
                 const MArgs<T> a{g.xin, g.b, g.pinv, g.eps, g.x, g.d, g.U, g.Uold, g.c1, g.c2, g.h, nent};
-                t2_march_kernel<T, FIN, kCols, kStage><<<ntiles, 6 * kCols, kMarchSmem, stream>>>(d_tiles.as<T2Tile>(), d_tables.as<int>(), a);
+                launch_after(t2_march_kernel<T, FIN, kCols, kStage>, dim3(ntiles), dim3(6 * kCols), kMarchSmem, stream, d_tiles.as<T2Tile>(), d_tables.as<int>(), a);
             } else {
-                cudaLaunchConfig_t c{};
-                c.gridDim = dim3(blocks(nent, 128));
-                c.blockDim = dim3(128);
-                c.stream = stream;
-                cudaLaunchAttribute at{};
-                at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                at.val.programmaticStreamSerializationAllowed = 1;
-                c.attrs = &at;
-                c.numAttrs = 1;
-                EMS_CUDA(cudaLaunchKernelEx(&c, t2_cheb_kernel<T, FIN>, (unsigned long long)nent, (const T2Shot *)d_shots.as<T2Shot>(), ns, g));
+                launch_after(t2_cheb_kernel<T, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
             }
             return 1;
         } else {
-            t2_mass_elem_kernel<<<blocks(ntet, 64), 64, 0, stream>>>(ntet, d_shots.as<T2Shot>(), ns, d_eps.as<T>(), g.xin, d_YtM.as<T>());
-            t2_gather_kernel<T, T, G_CHEB, FIN><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+            launch_after(t2_mass_elem_kernel, dim3(blocks(ntet, 64)), dim3(64), 0, stream, ntet, d_shots.as<T2Shot>(), ns, d_eps.as<T>(), g.xin, d_YtM.as<T>());
+            launch_after(t2_gather_kernel<T, T, G_CHEB, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
             return 2;
         }
     }
@@ -2023,10 +2023,10 @@ struct Tet2Sim : Sim {
         int cur = fused ? (mass_iters - 1) % 2 : 0;   // buffer of the first iterate
         g.x = buf[cur];
         if (mass_iters == 1) {
-            t2_gather_kernel<T, T, G_CHEB0, FIN><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+            launch_after(t2_gather_kernel<T, T, G_CHEB0, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
             return 1;
         }
-        t2_gather_kernel<T, T, G_CHEB0, FIN_NONE><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+        launch_after(t2_gather_kernel<T, T, G_CHEB0, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
         int nl = 1;
         for (int k = 1; k < mass_iters; ++k) {
             g.xin = buf[cur];
@@ -2110,8 +2110,8 @@ struct Tet2Sim : Sim {
 
     double dot_host(const void *x, const void *y)
     {
-        if (fp64) t2_dot_kernel<double><<<kDotBlocks, 256, 0, stream>>>(ndof, (const double *)x, (const double *)y, d_part.as<double>());
-        else t2_dot_kernel<float><<<kDotBlocks, 256, 0, stream>>>(ndof, (const float *)x, (const float *)y, d_part.as<double>());
+        if (fp64) launch_after(t2_dot_kernel<double>, dim3(kDotBlocks), dim3(256), 0, stream, ndof, (const double *)x, (const double *)y, d_part.as<double>());
+        else launch_after(t2_dot_kernel<float>, dim3(kDotBlocks), dim3(256), 0, stream, ndof, (const float *)x, (const float *)y, d_part.as<double>());
         std::vector<double> part(kDotBlocks);
         EMS_CUDA(cudaMemcpyAsync(part.data(), d_part.p, kDotBlocks * 8, cudaMemcpyDeviceToHost, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
@@ -2146,8 +2146,8 @@ struct Tet2Sim : Sim {
             EMS_CUDA(cudaMemcpyAsync(pb, z, ndof * sizeof(T), cudaMemcpyDeviceToDevice, stream));
             enqueue_solve<T, FIN_NONE>(pb, 0.0);
             const double nrm = 1.0 / std::sqrt(dot_host(x, x));
-            t2_scale_kernel<T><<<blocks(ndof, 256), 256, 0, stream>>>(ndof, x, nrm);
-            t2_scale_kernel<T><<<blocks(ndof, 256), 256, 0, stream>>>(ndof, pb, nrm);
+            launch_after(t2_scale_kernel<T>, dim3(blocks(ndof, 256)), dim3(256), 0, stream, ndof, x, nrm);
+            launch_after(t2_scale_kernel<T>, dim3(blocks(ndof, 256)), dim3(256), 0, stream, ndof, pb, nrm);
         }
         EMS_CUDA(cudaGetLastError());
         EMS_CUDA(cudaStreamSynchronize(stream));
@@ -2362,7 +2362,7 @@ struct Tet2Sim : Sim {
         int nl = 0;
         const int nd = (int)std::max<size_t>(dips.size(), 1);
         if (sample && nobs > 0) {
-            t2_sample_kernel<T><<<blocks((unsigned long long)nobs * 32, 128), 128, 0, stream>>>(
+            launch_after(t2_sample_kernel<T>, dim3(blocks((unsigned long long)nobs * 32, 128)), dim3(128), 0, stream, 
                 nobs, d_rec_dof.as<unsigned long long>(), d_rec_w.as<double>(), d_U.as<T>(), d_ctl.as<int>(), P.time_frequency,
                 nsamp, d_tr.as<double>());
             ++nl;
@@ -2371,17 +2371,17 @@ struct Tet2Sim : Sim {
             double sub[3], off[3];
             substeps(sub, off);
             const int nq = nsub();
-            t2_axpy_kernel<T><<<blocks(ndof, 256), 256, 0, stream>>>(ndof, d_U.as<T>(), d_x.as<T>(), 0.5 * sub[0]);
+            launch_after(t2_axpy_kernel<T>, dim3(blocks(ndof, 256)), dim3(256), 0, stream, ndof, d_U.as<T>(), d_x.as<T>(), 0.5 * sub[0]);
             ++nl;
             for (int q = 0; q < nq; ++q) {
                 enqueue_stiff<T>(d_U.as<T>());
                 GArgs<T> g = gargs<T>();
                 g.Yt = d_YtK.p;
                 g.a = sub[q];
-                t2_gather_kernel<T, double, G_KICK, FIN_NONE><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
                 nl += 2;
                 if (nsrc > 0) {
-                    t2_source_kernel<T, 0><<<blocks(nsrc, 128), 128, 0, stream>>>(
+                    launch_after(t2_source_kernel<T, 0>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, 
                         nsrc, d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(), d_src_coef.as<double>(),
                         d_src_g.as<double>(), d_ctl.as<int>(), nq, q, nd, sub[q], d_P.as<double>(), fp64 ? nullptr : d_Pc.as<T>());
                     ++nl;
@@ -2392,14 +2392,14 @@ struct Tet2Sim : Sim {
         } else {
             nl += enqueue_force<T>(d_U.as<T>(), d_b.as<T>());
             if (nsrc > 0) {
-                t2_source_kernel<T, 1><<<blocks(nsrc, 128), 128, 0, stream>>>(
+                launch_after(t2_source_kernel<T, 1>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, 
                     nsrc, d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(), d_src_coef.as<double>(),
                     d_src_g.as<double>(), d_ctl.as<int>(), 1, 0, nd, 1.0, nullptr, d_b.as<T>());
                 ++nl;
             }
             nl += enqueue_solve<T, FIN_LEAP>(d_b.as<T>(), dtn * dtn);
         }
-        t2_advance_kernel<<<1, 1, 0, stream>>>(d_ctl.as<int>());
+        launch_after(t2_advance_kernel, dim3(1), dim3(1), 0, stream, d_ctl.as<int>());
         return nl + 1;
     }
 
@@ -2726,30 +2726,30 @@ template <class T> void Tet2Sim::backward_t(const double *tg, double *grad)
         EMS_CUDA(cudaMemcpyAsync(d_P.p, sb + w, ndof * 8, cudaMemcpyDeviceToDevice, stream));
         narrowP();
         enqueue_solve<T, FIN_NONE>(rhs_P<T>(), 0.0, Y(n0, 0));
-        t2_set_kernel<<<1, 1, 0, stream>>>(ctl, n0);
+        launch_after(t2_set_kernel, dim3(1), dim3(1), 0, stream, ctl, n0);
         for (int n = n0; n < n1; ++n) {
-            t2_axpy_kernel<T><<<blocks(ndof, 256), 256, 0, stream>>>(ndof, d_U.as<T>(), Y(n, 0), 0.5 * sub[0]);
+            launch_after(t2_axpy_kernel<T>, dim3(blocks(ndof, 256)), dim3(256), 0, stream, ndof, d_U.as<T>(), Y(n, 0), 0.5 * sub[0]);
             for (int q = 0; q < nq; ++q) {
                 enqueue_stiff<T>(d_U.as<T>());
                 GArgs<T> g = gargs<T>();
                 g.Yt = d_YtK.p;
                 g.a = sub[q];
-                t2_gather_kernel<T, double, G_KICK, FIN_NONE><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
                 if (nsrc > 0)
-                    t2_source_kernel<T, 0><<<blocks(nsrc, 128), 128, 0, stream>>>(
+                    launch_after(t2_source_kernel<T, 0>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, 
                         nsrc, d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(), d_src_coef.as<double>(),
                         d_src_g.as<double>(), ctl, nq, q, nd, sub[q], d_P.as<double>(), fp64 ? nullptr : d_Pc.as<T>());
                 enqueue_solve<T, FIN_DRIFT>(rhs_P<T>(), hq[q], Y(n, q + 1));
             }
-            t2_advance_kernel<<<1, 1, 0, stream>>>(ctl);
+            launch_after(t2_advance_kernel, dim3(1), dim3(1), 0, stream, ctl);
         }
         // reversed steps
         for (int n = n1 - 1; n >= n0; --n) {
-            t2_set_kernel<<<1, 1, 0, stream>>>(ctl, n);
+            launch_after(t2_set_kernel, dim3(1), dim3(1), 0, stream, ctl, n);
             // adjoint of the substages
             for (int q = nq - 1; q >= 0; --q) {
                 enqueue_solve<T, FIN_DRIFT>(Ubr, hq[q], d_x.as<T>(), Pb.as<T>());
-                t2_grad_kernel<T><<<blocks(ntet, 128), 128, 0, stream>>>(ntet, d_shots.as<T2Shot>(), ns, d_x.as<T>(), Y(n, q + 1),
+                launch_after(t2_grad_kernel<T>, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(), ns, d_x.as<T>(), Y(n, q + 1),
                                                                          -hq[q], gd.as<double>());
                 enqueue_stiff<T>(Pb.as<T>());
                 GArgs<T> g = gargs<T>();
@@ -2757,13 +2757,13 @@ template <class T> void Tet2Sim::backward_t(const double *tg, double *grad)
                 g.a = sub[q];
                 g.P = Ub.as<double>();
                 g.Pc = fp64 ? nullptr : Ubc.as<T>();
-                t2_gather_kernel<T, double, G_KICK, FIN_NONE><<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), ns, g);
+                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
             }
             enqueue_solve<T, FIN_DRIFT>(Ubr, 0.5 * sub[0], d_x.as<T>(), Pb.as<T>());
-            t2_grad_kernel<T><<<blocks(ntet, 128), 128, 0, stream>>>(ntet, d_shots.as<T2Shot>(), ns, d_x.as<T>(), Y(n, 0),
+            launch_after(t2_grad_kernel<T>, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(), ns, d_x.as<T>(), Y(n, 0),
                                                                      -0.5 * sub[0], gd.as<double>());
             if (nrd > 0 && n % tf == 0)
-                t2_source_kernel<T, 0><<<blocks(nrd, 128), 128, 0, stream>>>(
+                launch_after(t2_source_kernel<T, 0>, dim3(blocks(nrd, 128)), dim3(128), 0, stream, 
                     nrd, a_dof.as<unsigned long long>(), a_ptr.as<int>(), a_idx.as<int>(), a_coef.as<double>(), a_g.as<double>(),
                     ctl, 1, 0, nd3, 1.0, Ub.as<double>(), fp64 ? nullptr : Ubc.as<T>());
             EMS_CUDA(cudaGetLastError());

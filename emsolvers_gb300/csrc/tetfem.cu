@@ -1311,6 +1311,7 @@ __global__ void __launch_bounds__(128) tet_loss_adjoint_kernel(size_t nnode, con
                                                                const T *__restrict__ pmid, const T *__restrict__ ppre,
                                                                double *__restrict__ zr)
 {
+    wait_for_last();
     const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nnode) return;
     const T g = damp[v];
@@ -1437,6 +1438,7 @@ __global__ void __launch_bounds__(128) tet_receiver_adjoint_kernel(int nnd, cons
                                                                    T *__restrict__ Wb, T *__restrict__ Pb, const T *__restrict__ minv,
                                                                    const T *__restrict__ z, double *__restrict__ Q, double cc, size_t nnode)
 {
+    wait_for_last();
     const int t = blockIdx.x * blockDim.x + threadIdx.x, d = t & 7, i = t >> 3;
     const bool in = i < nnd && d < 7;
     const size_t v = i < nnd ? (size_t)nd_node[i] : 0, f = (size_t)d * nnode + v;
@@ -1784,6 +1786,7 @@ __global__ void __launch_bounds__(256) scale_kernel(size_t n, double *__restrict
                                                     const double *__restrict__ nrm_base, const int *__restrict__ jp,
                                                     float *__restrict__ x32, float *__restrict__ kz)
 {
+    wait_for_last();
     const double s = 1.0 / sqrt(nrm_base[jp ? 2 * *jp : 0]);
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const double xs = x[i] * s;
@@ -1811,6 +1814,7 @@ __global__ void __launch_bounds__(128) lanczos_minv_kernel(size_t nnode, const d
                                                            double *__restrict__ part, unsigned *__restrict__ ticket,
                                                            double *__restrict__ alpha, int *__restrict__ jp)
 {
+    wait_for_last();
     if (jp && blockIdx.x == 0 && threadIdx.x == 0) *jp += 1;
     double acc = 0.0;
     for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nnode; v += (size_t)gridDim.x * blockDim.x) {
@@ -1854,6 +1858,7 @@ __global__ void __launch_bounds__(256) lanczos_step_kernel(size_t n, double *__r
                                                            unsigned *__restrict__ ticket, double *__restrict__ cf, int j0,
                                                            const int *__restrict__ jp)
 {
+    wait_for_last();
     const int j = jp ? *jp : j0;
     const double al = *alpha, be = vp ? sqrt(cf[2 * j - 1]) : 0.0;
     if (blockIdx.x == 0 && threadIdx.x == 0) cf[2 * j] = al;
@@ -2351,11 +2356,11 @@ struct TetFemSim : Sim {
                       DevBuf &part, unsigned *ticket, double *alpha, int *jp, int max_blocks)
     {
         const unsigned nbv = (unsigned)((nnode + step_block - 1) / step_block);
-        tet_step_kernel<float, 0, 0><<<nbv, step_block, 0, stream>>>(nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), nullptr,
+        launch_after(tet_step_kernel<float, 0, 0>, dim3(nbv), dim3(step_block), 0, stream, nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), nullptr,
                                                               kv32.as<float>(), x32.as<float>(), nullptr, nullptr, -1.0f, 0.0f,
                                                               SrcArgs{}, nullptr, nullptr, nullptr, nullptr, RecArgs<float>{}, Comp{});
         const int nb = (int)std::min<size_t>((nnode + 127) / 128, max_blocks);
-        lanczos_minv_kernel<<<nb, 128, 0, stream>>>(nnode, minv_d.as<double>(), kv32.as<float>(), vcur.as<double>(),
+        launch_after(lanczos_minv_kernel, dim3(nb), dim3(128), 0, stream, nnode, minv_d.as<double>(), kv32.as<float>(), vcur.as<double>(),
                                                     Mz.as<double>(), z.as<double>(), part.as<double>(), ticket, alpha, jp);
     }
 
@@ -2403,7 +2408,7 @@ struct TetFemSim : Sim {
         applyMinvK32(w.v32, w.kv32, minv_d, vb[0], mb[1], vb[1], w.part, tk, alpha, nullptr, nbl);
         dot_partial_kernel<<<512, 256, 0, stream>>>(nslot, vb[1].as<double>(), mb[1].as<double>(), w.part.as<double>());
         dot_finish_kernel<<<1, 512, 0, stream>>>(512, w.part.as<double>(), nrm0);
-        scale_kernel<<<nbl, 256, 0, stream>>>(nslot, vb[1].as<double>(), mb[1].as<double>(), nrm0, nullptr, w.v32.as<float>(),
+        launch_after(scale_kernel, dim3(nbl), dim3(256), 0, stream, nslot, vb[1].as<double>(), mb[1].as<double>(), nrm0, nullptr, w.v32.as<float>(),
                                               w.kv32.as<float>());
         int prev = -1, cur = 1, nxt = 2;
         // one iteration: apply (+ alpha), three-term step (+ beta^2),
@@ -2411,11 +2416,11 @@ struct TetFemSim : Sim {
         // (advanced by the apply)
         auto iteration = [&](int jj, int *jp) {
             applyMinvK32(w.v32, w.kv32, minv_d, vb[cur], mb[nxt], vb[nxt], w.part, tk, alpha, jp, nbl);
-            lanczos_step_kernel<<<nbl, 256, 0, stream>>>(nslot, vb[nxt].as<double>(), mb[nxt].as<double>(), vb[cur].as<double>(),
+            launch_after(lanczos_step_kernel, dim3(nbl), dim3(256), 0, stream, nslot, vb[nxt].as<double>(), mb[nxt].as<double>(), vb[cur].as<double>(),
                                                          mb[cur].as<double>(), prev >= 0 ? vb[prev].as<double>() : nullptr,
                                                          prev >= 0 ? mb[prev].as<double>() : nullptr, alpha,
                                                          w.part.as<double>(), tk + 1, cf, jj, jp);
-            scale_kernel<<<nbl, 256, 0, stream>>>(nslot, vb[nxt].as<double>(), mb[nxt].as<double>(),
+            launch_after(scale_kernel, dim3(nbl), dim3(256), 0, stream, nslot, vb[nxt].as<double>(), mb[nxt].as<double>(),
                                                   jp ? cf + 1 : cf + 2 * jj + 1, jp, w.v32.as<float>(), w.kv32.as<float>());
             const int t = prev < 0 ? 0 : prev;
             prev = cur; cur = nxt; nxt = t;
@@ -3199,7 +3204,7 @@ struct TetFemSim : Sim {
                         // the lossy middle kick: Pbar = g Pbar before the
                         // adjoint kick, Pbar = g Pbar + c Minv Wbar after it
                         const T *pp = pstore.as<T>() + (size_t)(n - n0) * 2 * nslot;
-                        tet_loss_adjoint_kernel<T><<<nbv2, 128, 0, stream>>>(nnode, d_damp.as<T>(), pb, pp + nslot, pp,
+                        launch_after(tet_loss_adjoint_kernel<T>, dim3(nbv2), dim3(128), 0, stream, nnode, d_damp.as<T>(), pb, pp + nslot, pp,
                                                                             zr.as<double>());
                         substep<T, 0, 2>(pb, pb2, Wb.as<T>(), nullptr, (T)sc.sub[q], (T)c, SrcArgs{}, y, nullptr, nullptr,
                                          RecArgs<T>{}, cadj);
@@ -3211,7 +3216,7 @@ struct TetFemSim : Sim {
                 }
                 if (n % tf == 0 && n > 0 && nobs > 0 && ra.nsl > 0) {
                     const T *z = zb + (size_t)(n - n0) * nsub * nslot;
-                    tet_receiver_adjoint_kernel<T><<<(8 * ra.nnd + 127) / 128, 128, 0, stream>>>(
+                    launch_after(tet_receiver_adjoint_kernel<T>, dim3((8 * ra.nnd + 127) / 128), dim3(128), 0, stream, 
                         ra.nnd, ra.nd_node.as<int>(), ra.nd_map.as<int>(), ra.sl_ptr.as<int>(), ra.term_rc.as<int>(), ra.term_w.as<double>(),
                         d_rs.as<double>() + (size_t)(n / tf) * nobs * 3, Wb.as<T>(), pb, d_minv.as<T>(), z, Q.as<double>(),
                         0.5 * sc.sub[nsub - 1], nnode);
