@@ -35,9 +35,24 @@ __device__ __forceinline__ float xmul(float a, float b) { return __fmul_rn(a, b)
 
 constexpr int kMaxSrc = 8;
 
+// Division of a value below 2^31 by a divisor known to the host, as a product
+// and a shift: m = floor(2^s / d) + 1 with s = 31 + ceil(log2 d).
+struct HexDiv {
+    unsigned m;
+    int s;
+    __device__ __forceinline__ unsigned operator()(unsigned t) const { return (unsigned)((unsigned long long)t * m >> s); }
+};
+static HexDiv hex_div(int d)
+{
+    int l = 0;
+    while ((1ll << l) < d) ++l;
+    return l ? HexDiv{(unsigned)((1ull << (31 + l)) / (unsigned)d + 1), 31 + l} : HexDiv{1u, 0};
+}
+
 struct HexGeom {
     int o, gx, gy, gz, EX, EY, EZ, nouter, dof, total;
     size_t nc[3];
+    HexDiv row[2], col[2];   // by gx, gx + 1 and gy, gy + 1
 };
 
 // Rank of element (i,j,k) in the reference's visiting order.
@@ -165,9 +180,9 @@ __device__ __forceinline__ void dof_coords(const HexGeom &g, int c, size_t t, in
 {
     int nxc = c == 0 ? g.gx : g.gx + 1;
     int nyc = c == 1 ? g.gy : g.gy + 1;
-    const unsigned u = (unsigned)t, r = u / nxc;   // a component holds fewer than 2^31 values (int offsets throughout)
+    const unsigned u = (unsigned)t, r = c == 0 ? g.row[0](u) : g.row[1](u);   // a component holds fewer than 2^31 values (int offsets throughout)
     ix = (int)(u - r * nxc);
-    iz = (int)(r / nyc);
+    iz = (int)(c == 1 ? g.col[0](r) : g.col[1](r));
     iy = (int)(r - (unsigned)iz * nyc);
 }
 
@@ -224,9 +239,10 @@ __global__ void __launch_bounds__(128) hex_kick_kernel(HexGeom g, const T *__res
 
 // Drift U += coef * P / m (symplectic_2/fem_simulation.cpp:583-601, 647-668);
 // coef = 0.5*deltat, inv_m = 8/o^3 as in the reference's operand order; with
-// `pec` set, U and P are zeroed on the boundary afterwards (1132-1276).
-template <class T, bool EXACT>
-__global__ void hex_drift_kernel(HexGeom g, T *Ux, T *Uy, T *Uz, T *Px, T *Py, T *Pz, T coef, T m, int pec)
+// `pec` set, U and P are zeroed on the boundary afterwards (1132-1276).  MUL:
+// m is a power of two and comes as 1 / m, the same value without the division.
+template <class T, bool EXACT, bool MUL>
+__global__ void hex_drift_kernel(const __grid_constant__ HexGeom g, T *Ux, T *Uy, T *Uz, T *Px, T *Py, T *Pz, T coef, T m, int pec)
 {
     wait_for_last();
     const int c = blockIdx.y;
@@ -234,7 +250,8 @@ __global__ void hex_drift_kernel(HexGeom g, T *Ux, T *Uy, T *Uz, T *Px, T *Py, T
     if (t >= g.nc[c]) return;
     T *U = c == 0 ? Ux : c == 1 ? Uy : Uz;
     T *P = c == 0 ? Px : c == 1 ? Py : Pz;
-    T u = EXACT ? xadd(U[t], (T)(xmul(coef, P[t]) / m)) : U[t] + coef * P[t] / m;
+    const T v = MUL ? xmul(xmul(coef, P[t]), m) : (T)(xmul(coef, P[t]) / m);
+    T u = xadd(U[t], v);
     if (pec) {
         int ix, iy, iz;
         dof_coords(g, c, t, ix, iy, iz);
@@ -294,22 +311,23 @@ __device__ __forceinline__ bool hex_elem_head(const HexGeom &g, const T *Ux, con
 // Element pass: rows c D .. c D + D - 1 of K u of one element per thread
 // (component c = blockIdx.y), fe[row][element].  Each sum runs in column order
 // as dof_force's.  The element's values stay in registers, the rows of K are
-// read from shared memory, one vector for two or four rows of a column, so a
+// read from shared memory (laid out by column on the host), one vector for two or four rows of a column, so a
 // value of K costs a quarter to half a load instead of one per DOF and
 // element.  Order 2 on 72^3 grid cells, symp4: FP32 278 us a step in one pass DOF
-// by DOF, 95.7 in two; FP64, bound by the FP64 pipe, 2402 and 1877.  step: given to a step's first pass (see SrcTab).
+// by DOF, 69.3 in two; FP64, bound by the FP64 pipe, 2402 and 1857.  step: given to a step's first pass (see SrcTab).
 template <class T, int O, bool EXACT>
 __global__ void __launch_bounds__(128) hex_elem_kernel(HexGeom g, const T *__restrict__ K, const T *__restrict__ Ux, const T *__restrict__ Uy,
                                                        const T *__restrict__ Uz, T *__restrict__ fe, int *step, HexRec rec)
 {
-    wait_for_last();
     constexpr int D = O * (O + 1) * (O + 1), TT = 3 * D, W = 16 / (int)sizeof(T), RP = (D + W - 1) / W * W;
     __shared__ __align__(16) T sK[TT * RP];
     const int c = blockIdx.y;
     const int ne = g.EX * g.EY * g.EZ, e = blockIdx.x * 128 + threadIdx.x;
-    if (hex_elem_head<T>(g, Ux, Uy, Uz, ne, 128, step, rec)) return;
-    for (int q = threadIdx.x; q < TT * D; q += 128) sK[(q % TT) * RP + q / TT] = K[(size_t)c * D * TT + q];
+    const int4 *k4 = reinterpret_cast<const int4 *>(K + (size_t)c * TT * RP);   // does not change: ahead of the wait
+    for (int q = threadIdx.x; q < TT * RP / W; q += 128) reinterpret_cast<int4 *>(sK)[q] = k4[q];
     __syncthreads();
+    wait_for_last();
+    if (hex_elem_head<T>(g, Ux, Uy, Uz, ne, 128, step, rec)) return;
     if (e >= ne) return;
     const int r0 = e / g.EX, ei = e - r0 * g.EX, ek = r0 / g.EY, ej = r0 - ek * g.EY;
     const int gx = g.gx, gy = g.gy;
@@ -417,51 +435,69 @@ __global__ void __launch_bounds__(32) hex1_elem_kernel(HexGeom g, const __grid_c
     for (int r = 0; r < 12; ++r) fe[(size_t)r * ne + e] = f[r];
 }
 
-// Sum of a DOF's element values with the source: dof_force's order with the
-// (at most four) elements in fixed slots, two positions along each of the two
-// axes across the edge.
-template <class T, int O, bool EXACT>
-__device__ __forceinline__ T dof_sum(const HexGeom &g, const T *__restrict__ fe, int c, int ix, int iy, int iz, T sign, bool has_src, T srcval)
+// Sum of an inner DOF's element values with the source, in dof_force's order.
+// Its (at most four) elements are the one at its place and the ones below it
+// along the two axes across the edge, a and b, present where it lies on their
+// common face; the values of those are a fixed distance away in fe.
+template <class T, int O, bool EXACT, int C>
+__device__ __forceinline__ T dof_sum(const HexGeom &g, const T *__restrict__ fe, int ix, int iy, int iz, T sign, bool has_src, T srcval)
 {
     constexpr int D = O * (O + 1) * (O + 1);
-    const int pc = c == 0 ? ix : c == 1 ? iy : iz, nec = c == 0 ? g.EX : c == 1 ? g.EY : g.EZ;
-    const int pa = c == 0 ? iy : ix, na = c == 0 ? g.EY : g.EX;   // the outer of the two axes
-    const int pb = c == 2 ? iy : iz, nb = c == 2 ? g.EY : g.EZ;   // the inner one
-    const int ec = pc / O, lc = pc - O * ec, ea = pa / O, la = pa - O * ea, eb = pb / O, lb = pb - O * eb;
-    const size_t ne = (size_t)g.EX * g.EY * g.EZ;
-    T v[4];
+    constexpr int RX = 1, RY = C == 0 ? O : O + 1, RZ = C == 2 ? (O + 1) * (O + 1) : O * (O + 1);   // rows of K along the axes
+    const int ex = ix / O, ey = iy / O, ez = iz / O, l = ix - O * ex, m = iy - O * ey, n = iz - O * ez;
+    const long long ne = (long long)g.EX * g.EY * g.EZ;
+    // a grid that is no whole number of elements has DOFs behind the last one
+    const bool in = ex < g.EX + (C != 0) && ey < g.EY + (C != 1) && ez < g.EZ + (C != 2);
+    const bool a0 = in && (C == 0 ? ey < g.EY : ex < g.EX), b0 = in && (C == 2 ? ey < g.EY : ez < g.EZ);
+    const bool a1 = in && (C == 0 ? m : l) == 0, b1 = in && (C == 2 ? m : n) == 0;
+    const bool p[4] = {a0 && b0, a0 && b1, a1 && b0, a1 && b1};
+    const long long da = O * (C == 0 ? RY : RX) * ne - (C == 0 ? g.EX : 1), db = O * (C == 2 ? RY : RZ) * ne - (C == 2 ? g.EX : g.EX * g.EY);
+    const T *f = fe + ((C * D + l * RX + m * RY + n * RZ) * ne + (ex + g.EX * (ey + (long long)g.EY * ez)));
+    T v[4] = {};
+#pragma unroll
+    for (int s = 0; s < 4; ++s)
+        if (p[s]) v[s] = f[(s >> 1) * da + (s & 1) * db];
+    T acc = 0;
+    auto add = [&](T x) { acc = sign < 0 ? xsub(acc, x) : xadd(acc, x); };
+    if (!EXACT) {   // element by element, the source behind them
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            if (p[s]) add(v[s]);
+        return has_src ? xadd(acc, srcval) : acc;
+    }
+    const int xl = ex - (C != 0 && a1), yl = ey - (C == 0 ? a1 : C == 2 && b1), zl = ez - (C != 2 && b1);   // lowest element
+    if (xl > 0 && yl > 0 && zl > 0 && ex < g.EX - 1 && ey < g.EY - 1 && ez < g.EZ - 1) {
+        // only inner elements: visited behind the source, in index order
+        if (has_src) acc = xadd(acc, srcval);
+        if (p[3]) add(v[3]);
+        if (p[1]) add(v[1]);
+        if (p[2]) add(v[2]);
+        add(v[0]);
+        return acc;
+    }
     int rk[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         const int sa = s >> 1, sb = s & 1;
-        const int ua = ea - sa, ub = eb - sb, fa = sa ? O : la, fb = sb ? O : lb;   // element and place along each axis
-        const bool in = ec < nec && ua >= 0 && ua < na && ub >= 0 && ub < nb && (!sa || la == 0) && (!sb || lb == 0);
-        const int ex = c == 0 ? ec : ua, ey = c == 1 ? ec : c == 0 ? ua : ub, ez = c == 2 ? ec : ub;
-        const int l = c == 0 ? lc : fa, m = c == 1 ? lc : c == 0 ? fa : fb, n = c == 2 ? lc : fb;
-        const int row = c * D + l + m * (c == 0 ? O : O + 1) + n * (c == 2 ? (O + 1) * (O + 1) : O * (O + 1));
-        v[s] = in ? fe[row * ne + (ex + g.EX * (ey + (size_t)g.EY * ez))] : T(0);
-        rk[s] = !in ? 0x7fffffff : EXACT ? elem_rank(g, ex, ey, ez) : s;
+        rk[s] = !p[s] ? 0x7fffffff : elem_rank(g, ex - (C != 0 ? sa : 0), ey - (C == 0 ? sa : C == 2 ? sb : 0), ez - (C != 2 ? sb : 0));
     }
-    if (EXACT) {   // by visiting rank
-        auto order = [&](int x, int y) {
-            if (rk[x] > rk[y]) {
-                const int r = rk[x];
-                rk[x] = rk[y];
-                rk[y] = r;
-                const T t = v[x];
-                v[x] = v[y];
-                v[y] = t;
-            }
-        };
-        order(0, 1); order(2, 3); order(0, 2); order(1, 3); order(1, 2);
-    }
-    T acc = 0;
+    auto order = [&](int x, int y) {
+        if (rk[x] > rk[y]) {
+            const int r = rk[x];
+            rk[x] = rk[y];
+            rk[y] = r;
+            const T t = v[x];
+            v[x] = v[y];
+            v[y] = t;
+        }
+    };
+    order(0, 1); order(2, 3); order(0, 2); order(1, 3); order(1, 2);
     bool src_done = !has_src;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         if (rk[s] == 0x7fffffff) continue;
         if (!src_done && rk[s] >= g.nouter) { acc = xadd(acc, srcval); src_done = true; }
-        acc = sign < 0 ? xsub(acc, v[s]) : xadd(acc, v[s]);
+        add(v[s]);
     }
     if (!src_done) acc = xadd(acc, srcval);
     return acc;
@@ -471,58 +507,77 @@ template <class T> struct HexDofs {
     T *a[3], *b[3], *c[3];   // leapfrog: E1, E0, E2; symplectic: U, P, F
 };
 
-// DOF pass of a leapfrog step (see hex_leapfrog_kernel).
+// Sources on a DOF.
+__device__ __forceinline__ int sources_at(const SrcTab &src, int c, unsigned t)
+{
+    int n = 0;
+    for (int s = 0; s < src.n; ++s) n += src.comp[s] == c && (unsigned)src.idx[s] == t;
+    return n;
+}
+
+// DOF pass of a leapfrog step (see hex_leapfrog_kernel), component C.
+template <class T, int O, bool EXACT, int C>
+__device__ __forceinline__ void leap_dof(const HexGeom &g, const T *__restrict__ fe, const HexDofs<T> &d, const SrcTab &src)
+{
+    const unsigned t = blockIdx.x * 128 + threadIdx.x;
+    if (C == 0 && t == 0) src.step[0] += 1;
+    if (t >= g.nc[C]) return;
+    int ix, iy, iz;
+    dof_coords(g, C, t, ix, iy, iz);
+    const bool pec = on_pec(g, C, ix, iy, iz);
+    const T a = d.a[C][t], b = d.b[C][t];
+    T f = 0;
+    if (!pec) f = dof_sum<T, O, EXACT, C>(g, fe, ix, iy, iz, T(-1), false, T(0));
+    T v = xadd(f, xsub(xmul(T(2), a), b));
+    for (int n = sources_at(src, C, t); n > 0; --n) v = xsub(v, (T)src.vals[src.step[1] - 1]);
+    if (pec) v = 0;
+    d.c[C][t] = v;
+}
+// The two DOF passes are bound by instructions, not by their L2 traffic: code
+// of its own per component and divisions by products took the kick of order 2
+// on 72^3 grid cells from 17.7 to 10.4 us (each launch alone).
 template <class T, int O, bool EXACT>
 __global__ void __launch_bounds__(128) hex_leap_dof_kernel(const __grid_constant__ HexGeom g, const T *__restrict__ fe, const __grid_constant__ HexDofs<T> d,
                                                            const __grid_constant__ SrcTab src)
 {
     wait_for_last();
-    const int c = blockIdx.y;
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0 && c == 0) src.step[0] += 1;
-    if (t >= g.nc[c]) return;
-    int ix, iy, iz;
-    dof_coords(g, c, t, ix, iy, iz);
-    const bool pec = on_pec(g, c, ix, iy, iz);
-    T f = 0;
-    if (!pec) f = dof_sum<T, O, EXACT>(g, fe, c, ix, iy, iz, T(-1), false, T(0));
-    T v = xadd(f, xsub(xmul(T(2), d.a[c][t]), d.b[c][t]));
-    for (int s = 0; s < src.n; ++s)
-        if (src.comp[s] == c && (size_t)src.idx[s] == t) v = xsub(v, (T)src.vals[src.step[1] - 1]);
-    if (pec) v = 0;
-    d.c[c][t] = v;
+    if (blockIdx.y == 0) leap_dof<T, O, EXACT, 0>(g, fe, d, src);
+    else if (blockIdx.y == 1) leap_dof<T, O, EXACT, 1>(g, fe, d, src);
+    else leap_dof<T, O, EXACT, 2>(g, fe, d, src);
 }
 
 // DOF pass of a symplectic substep: the force (stored, as the reference keeps
 // it), the kick, the closing half drift with the PEC planes zeroed, and the
 // opening half drift of the next substep (h2 != 0; FP32 runs take both half
 // drifts as one, h1).  Drifts add (h P) / m; 1 / m is a power of two.
+template <class T, int O, bool EXACT, int C>
+__device__ __forceinline__ void kick_dof(const HexGeom &g, const T *__restrict__ fe, const HexDofs<T> &d, const SrcTab &src, T dt, T h1, T h2, T rm)
+{
+    const unsigned t = blockIdx.x * 128 + threadIdx.x;
+    if (src.last && C == 0 && t == 0) src.step[0] += 1;
+    if (t >= g.nc[C]) return;
+    int ix, iy, iz;
+    dof_coords(g, C, t, ix, iy, iz);
+    const bool pec = on_pec(g, C, ix, iy, iz), has = sources_at(src, C, t) > 0;
+    T p = d.b[C][t], u = d.a[C][t], sv = 0, f = 0;
+    if (has) sv = (T)src.vals[(size_t)(src.step[1] - 1) * src.nsub + src.q];
+    if (!pec) f = dof_sum<T, O, EXACT, C>(g, fe, ix, iy, iz, T(1), has, sv);
+    d.c[C][t] = f;
+    p = EXACT ? xsub(p, xmul(dt, f)) : fma(-dt, f, p);
+    u = xadd(u, xmul(xmul(h1, p), rm));
+    if (pec) { u = 0; p = 0; }
+    if (h2 != T(0)) u = xadd(u, xmul(xmul(h2, p), rm));
+    d.b[C][t] = p;
+    d.a[C][t] = u;
+}
 template <class T, int O, bool EXACT>
 __global__ void __launch_bounds__(128) hex_kick_dof_kernel(const __grid_constant__ HexGeom g, const T *__restrict__ fe, const __grid_constant__ HexDofs<T> d,
                                                            const __grid_constant__ SrcTab src, T dt, T h1, T h2, T rm)
 {
     wait_for_last();
-    const int c = blockIdx.y;
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (src.last && t == 0 && c == 0) src.step[0] += 1;
-    if (t >= g.nc[c]) return;
-    int ix, iy, iz;
-    dof_coords(g, c, t, ix, iy, iz);
-    bool has = false;
-    T sv = 0;
-    for (int s = 0; s < src.n; ++s)
-        if (src.comp[s] == c && (size_t)src.idx[s] == t) { has = true; sv = (T)src.vals[(size_t)(src.step[1] - 1) * src.nsub + src.q]; }
-    const bool pec = on_pec(g, c, ix, iy, iz);
-    T f = 0;
-    if (!pec) f = dof_sum<T, O, EXACT>(g, fe, c, ix, iy, iz, T(1), has, sv);
-    T p = d.b[c][t], u = d.a[c][t];
-    d.c[c][t] = f;
-    p = EXACT ? xsub(p, xmul(dt, f)) : fma(-dt, f, p);
-    u = xadd(u, xmul(xmul(h1, p), rm));
-    if (pec) { u = 0; p = 0; }
-    if (h2 != T(0)) u = xadd(u, xmul(xmul(h2, p), rm));
-    d.b[c][t] = p;
-    d.a[c][t] = u;
+    if (blockIdx.y == 0) kick_dof<T, O, EXACT, 0>(g, fe, d, src, dt, h1, h2, rm);
+    else if (blockIdx.y == 1) kick_dof<T, O, EXACT, 1>(g, fe, d, src, dt, h1, h2, rm);
+    else kick_dof<T, O, EXACT, 2>(g, fe, d, src, dt, h1, h2, rm);
 }
 
 static double femv2_source(double t)
@@ -582,6 +637,7 @@ struct HexFemSim : Sim {
         g.nc[0] = (size_t)g.gx * (g.gy + 1) * (g.gz + 1);
         g.nc[1] = (size_t)(g.gx + 1) * g.gy * (g.gz + 1);
         g.nc[2] = (size_t)(g.gx + 1) * (g.gy + 1) * g.gz;
+        for (int q = 0; q < 2; ++q) { g.row[q] = hex_div(g.gx + q); g.col[q] = hex_div(g.gy + q); }
         fp64 = P.precision == EMS_FP64;
         exact = fp64;
         // element matrix (fem_v2/fem_simulation.cpp:458-490, symplectic_2 473)
@@ -613,14 +669,24 @@ struct HexFemSim : Sim {
         init_stream();
         size_t w = fp64 ? 8 : 4;
         for (int q = 0; q < 3; ++q) { lev[q].alloc(3 * g.nc[q] * w); lev[q].zero(stream); }
-        if (fp64) {
-            dK.alloc(Kh.size() * 8);
-            EMS_CUDA(cudaMemcpyAsync(dK.p, Kh.data(), Kh.size() * 8, cudaMemcpyHostToDevice, stream));
-        } else {
-            std::vector<float> kf(Kh.begin(), Kh.end());
-            dK.alloc(kf.size() * 4);
-            EMS_CUDA(cudaMemcpyAsync(dK.p, kf.data(), kf.size() * 4, cudaMemcpyHostToDevice, stream));
+        if (fp64) upload_matrix<double>();
+        else upload_matrix<float>();
+        EMS_CUDA(cudaStreamSynchronize(stream));
+    }
+
+    // K on the device: orders 1 and 2 column by column per component, its rows
+    // padded to 16 bytes (hex_elem_kernel); order 3 as loaded.
+    template <class T> void upload_matrix()
+    {
+        std::vector<T> k(Kh.begin(), Kh.end());
+        if (g.o < 3) {
+            const int D = g.dof, TT = g.total, W = 16 / (int)sizeof(T), RP = (D + W - 1) / W * W;
+            k.assign((size_t)3 * TT * RP, T(0));
+            for (int r = 0; r < TT; ++r)
+                for (int m = 0; m < TT; ++m) k[((size_t)(r / D) * TT + m) * RP + r % D] = (T)Kh[(size_t)r * TT + m];
         }
+        dK.alloc(k.size() * sizeof(T));
+        EMS_CUDA(cudaMemcpyAsync(dK.p, k.data(), k.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
     }
 
@@ -653,8 +719,9 @@ struct HexFemSim : Sim {
     {
         size_t mx = std::max(g.nc[0], std::max(g.nc[1], g.nc[2]));
         dim3 grid((unsigned)((mx + 255) / 256), 3);
-        T m = (T)(8.0 / g.o / g.o / g.o);
-        auto k = exact ? hex_drift_kernel<T, true> : hex_drift_kernel<T, false>;
+        const bool mul = g.o < 3;
+        const T m = mul ? (T)(g.o * g.o * g.o / 8.0) : (T)(8.0 / g.o / g.o / g.o);
+        auto k = mul ? hex_drift_kernel<T, sizeof(T) == 8, true> : hex_drift_kernel<T, sizeof(T) == 8, false>;
         launch_after(k, grid, dim3(256), 0, stream, g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), L<T>(0, 1), L<T>(1, 1), L<T>(2, 1), coef, m, pec);
     }
 
