@@ -310,22 +310,32 @@ __device__ __forceinline__ bool hex_elem_head(const HexGeom &g, const T *Ux, con
 
 // Element pass: rows c D .. c D + D - 1 of K u of one element per thread
 // (component c = blockIdx.y), fe[row][element].  Each sum runs in column order
-// as dof_force's.  The element's values stay in registers, the rows of K are
-// read from shared memory (laid out by column on the host), one vector for two or four rows of a column, so a
-// value of K costs a quarter to half a load instead of one per DOF and
-// element.  Order 2 on 72^3 grid cells, symp4: FP32 278 us a step in one pass DOF
-// by DOF, 69.3 in two; FP64, bound by the FP64 pipe, 2402 and 1857.  step: given to a step's first pass (see SrcTab).
+// as dof_force's.  K is laid out column by column, each padded to 16 bytes.
+// In FP32 it is a kernel argument, so a multiply-add takes its value from the
+// constant bank; from shared memory, one vector for four rows of a column, the
+// load pipe was the bound (14.8 us a pass against 12.9, order 2 on 72^3 grid
+// cells, each launch alone).  FP64 keeps shared memory: its pass is bound by
+// the FP64 pipe.  A symp4 step there: FP32 278 us in one pass DOF by DOF,
+// 65 in two; FP64 2402 and 1857.  step: given to a step's first pass (see SrcTab).
+template <class T, int O> struct HexRows {
+    static constexpr int D = O * (O + 1) * (O + 1), TT = 3 * D, W = 16 / (int)sizeof(T), RP = (D + W - 1) / W * W;
+};
+template <class T, int O> struct HexK { const T *k; };   // K of the element pass, [3][TT][RP]
+template <int O> struct HexK<float, O> { float k[3 * HexRows<float, O>::TT * HexRows<float, O>::RP]; };
 template <class T, int O, bool EXACT>
-__global__ void __launch_bounds__(128) hex_elem_kernel(HexGeom g, const T *__restrict__ K, const T *__restrict__ Ux, const T *__restrict__ Uy,
+__global__ void __launch_bounds__(128) hex_elem_kernel(const __grid_constant__ HexGeom g, const __grid_constant__ HexK<T, O> K, const T *__restrict__ Ux, const T *__restrict__ Uy,
                                                        const T *__restrict__ Uz, T *__restrict__ fe, int *step, HexRec rec)
 {
-    constexpr int D = O * (O + 1) * (O + 1), TT = 3 * D, W = 16 / (int)sizeof(T), RP = (D + W - 1) / W * W;
-    __shared__ __align__(16) T sK[TT * RP];
+    constexpr int D = HexRows<T, O>::D, TT = HexRows<T, O>::TT, W = HexRows<T, O>::W, RP = HexRows<T, O>::RP;
+    constexpr bool ARG = sizeof(T) == 4;
+    __shared__ __align__(16) T sK[ARG ? 1 : TT * RP];
     const int c = blockIdx.y;
     const int ne = g.EX * g.EY * g.EZ, e = blockIdx.x * 128 + threadIdx.x;
-    const int4 *k4 = reinterpret_cast<const int4 *>(K + (size_t)c * TT * RP);   // does not change: ahead of the wait
-    for (int q = threadIdx.x; q < TT * RP / W; q += 128) reinterpret_cast<int4 *>(sK)[q] = k4[q];
-    __syncthreads();
+    if constexpr (!ARG) {
+        const int4 *k4 = reinterpret_cast<const int4 *>(K.k + (size_t)c * TT * RP);   // does not change: ahead of the wait
+        for (int q = threadIdx.x; q < TT * RP / W; q += 128) reinterpret_cast<int4 *>(sK)[q] = k4[q];
+        __syncthreads();
+    }
     wait_for_last();
     if (hex_elem_head<T>(g, Ux, Uy, Uz, ne, 128, step, rec)) return;
     if (e >= ne) return;
@@ -361,7 +371,12 @@ __global__ void __launch_bounds__(128) hex_elem_kernel(HexGeom g, const T *__res
     for (int mm = 0; mm < TT; ++mm) {
         T k[RP];
 #pragma unroll
-        for (int r = 0; r < RP; r += W) *reinterpret_cast<int4 *>(&k[r]) = *reinterpret_cast<const int4 *>(&sK[mm * RP + r]);
+        for (int r = 0; r < RP; r += W) {
+            if constexpr (ARG) {
+#pragma unroll
+                for (int w = 0; w < W; ++w) k[r + w] = K.k[(c * TT + mm) * RP + r + w];
+            } else *reinterpret_cast<int4 *>(&k[r]) = *reinterpret_cast<const int4 *>(&sK[mm * RP + r]);
+        }
 #pragma unroll
         for (int r = 0; r < D; ++r) f[r] = EXACT ? xadd(f[r], xmul(k[r], u[mm])) : fma(k[r], u[mm], f[r]);
     }
@@ -562,7 +577,7 @@ __device__ __forceinline__ void kick_dof(const HexGeom &g, const T *__restrict__
     T p = d.b[C][t], u = d.a[C][t], sv = 0, f = 0;
     if (has) sv = (T)src.vals[(size_t)(src.step[1] - 1) * src.nsub + src.q];
     if (!pec) f = dof_sum<T, O, EXACT, C>(g, fe, ix, iy, iz, T(1), has, sv);
-    d.c[C][t] = f;
+    if (src.last) d.c[C][t] = f;   // the step's force is its last substep's
     p = EXACT ? xsub(p, xmul(dt, f)) : fma(-dt, f, p);
     u = xadd(u, xmul(xmul(h1, p), rm));
     if (pec) { u = 0; p = 0; }
@@ -603,6 +618,7 @@ struct HexFemSim : Sim {
     int l0 = 0, l1 = 1, l2 = 2;              // leapfrog ring
     HexClasses cls{};                        // order 1 in FP64: the sizes and signs of K's entries
     bool classes = false;
+    std::vector<float> k32;                  // orders 1 and 2 in FP32: K as the element pass takes it
     double cur_time = 0.0;
     DevBuf d_obs, d_tr, d_fe, d_vals, d_step;
     cudaGraphExec_t graph = nullptr;         // kGraphSteps steps, kept while the buffers stay the same
@@ -674,8 +690,7 @@ struct HexFemSim : Sim {
         EMS_CUDA(cudaStreamSynchronize(stream));
     }
 
-    // K on the device: orders 1 and 2 column by column per component, its rows
-    // padded to 16 bytes (hex_elem_kernel); order 3 as loaded.
+    // K for the kernels: orders 1 and 2 as hex_elem_kernel takes it, order 3 as loaded.
     template <class T> void upload_matrix()
     {
         std::vector<T> k(Kh.begin(), Kh.end());
@@ -685,6 +700,11 @@ struct HexFemSim : Sim {
             for (int r = 0; r < TT; ++r)
                 for (int m = 0; m < TT; ++m) k[((size_t)(r / D) * TT + m) * RP + r % D] = (T)Kh[(size_t)r * TT + m];
         }
+        if constexpr (sizeof(T) == 4)
+            if (g.o < 3) {
+                k32 = std::move(k);
+                return;
+            }
         dK.alloc(k.size() * sizeof(T));
         EMS_CUDA(cudaMemcpyAsync(dK.p, k.data(), k.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
@@ -761,7 +781,10 @@ struct HexFemSim : Sim {
                 launch_after(hex1_elem_kernel, dim3((ne + 31) / 32 + (rec.n + 31) / 32), dim3(32), 0, stream, g, cls, u[0], u[1], u[2], d_fe.as<T>(), step, rec);
                 return;
             }
-        launch_after(hex_elem_kernel<T, O, X>, dim3((ne + 127) / 128 + (rec.n + 127) / 128, 3), dim3(128), 0, stream, g, dK.as<T>(), u[0], u[1], u[2],
+        HexK<T, O> kk{};
+        if constexpr (sizeof(T) == 4) std::copy(k32.begin(), k32.end(), kk.k);
+        else kk.k = dK.as<T>();
+        launch_after(hex_elem_kernel<T, O, X>, dim3((ne + 127) / 128 + (rec.n + 127) / 128, 3), dim3(128), 0, stream, g, kk, u[0], u[1], u[2],
                                                                                                     d_fe.as<T>(), step, rec);
     }
     // One step of orders 1 and 2 in two passes per force; launches made.
