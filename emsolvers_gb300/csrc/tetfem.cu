@@ -389,17 +389,21 @@ __device__ __forceinline__ void comp_scale(float &x, float &lo, float g)
     x = p;
 }
 
-// Point-dipole loads fused into the step kernels: entry k adds
-// coef[k] * g[dip[k]] to slot[k]; g for this (step n, substep q) is read at
-// g + (n*nsub + q)*nd with n = ctl[par].  The entries are sorted by slot (entries
-// of one slot in dipole order), so a flagged slot finds its entries by
-// binary search: a linear scan of a batch's list (six entries per shot) kept
-// the few warps that hold dipole slots busy long after the rest of the grid.
+// Point-dipole loads fused into the step kernels: entry k adds coef *
+// g[dip]; g for this (step n, substep q) is read at g + (n*nsub + q)*nd with
+// n = ctl[par].  The entries are sorted by slot (entries of one slot in dipole
+// order); at[e] is the first one of slot e.  The few warps that hold dipole
+// slots end a launch last, so each dependent load counts: searching the sorted
+// slots cost a sector of L2 a probe, 9.4 us a launch against 6.7 without
+// dipoles for four shots of 28^3 cubes (7.9 this way).
+struct SrcEntry {
+    double coef;
+    int dip, more;   // more: the next entry is the same slot's
+};
 struct SrcArgs {
     int n;
-    const int *slot;
-    const double *coef;
-    const int *dip;
+    const int *at;   // per slot, read for flagged slots only; -1: no entry
+    const SrcEntry *ent;
     const double *g;
     const int *ctl;
     int nd, nsub, q;
@@ -410,13 +414,15 @@ __device__ __forceinline__ double source_load(const SrcArgs &s, size_t e)
 {
     double f = 0.0;
     if (s.n == 0) return f;
-    int lo = 0, hi = s.n;   // first entry with slot >= e
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if ((size_t)s.slot[mid] < e) lo = mid + 1; else hi = mid;
+    const int step = s.ctl[s.par];
+    int k = s.at[e];
+    if (k < 0) return f;
+    const double *g = s.g + ((size_t)step * s.nsub + s.q) * s.nd;
+    for (bool more = true; more; ++k) {
+        const int4 w = *reinterpret_cast<const int4 *>(s.ent + k);
+        f += __hiloint2double(w.y, w.x) * g[w.z];
+        more = w.w != 0;
     }
-    const double *g = s.g + ((size_t)s.ctl[s.par] * s.nsub + s.q) * s.nd;
-    for (int k = lo; k < s.n && (size_t)s.slot[k] == e; ++k) f += s.coef[k] * g[s.dip[k]];
     return f;
 }
 
@@ -741,11 +747,13 @@ __host__ __device__ constexpr int step_record_x(int sy, int mask) { return sy | 
 // candidates on the handle's own mesh (TetFemSim::force_launch_shape); small
 // meshes (a 32^3 mesh has 36k nodes) spread better over the 152 SMs in
 // small blocks.  The block size changes no arithmetic.
+// FP32 symplectic steps keep to 64 registers, four warps a scheduler at every
+// block size: 80 took the ten-shot batch of 295k nodes from 15.9 to 17.5 us.
 constexpr int kStepBlocks[4] = {32, 64, 128, 256};
 constexpr int kStepBlockMax = 256;
 
 template <class T, int MODE, int DAMP, int REC = 0, int COMP = 0>
-__global__ void __launch_bounds__(kStepBlockMax) tet_step_kernel(size_t nnode, const int2 *__restrict__ nrec,
+__global__ void __launch_bounds__(kStepBlockMax, sizeof(T) == 4 && MODE == 0 ? 4 : 1) tet_step_kernel(size_t nnode, const int2 *__restrict__ nrec,
                                                        const unsigned char *__restrict__ pec, const T *__restrict__ minv,
                                                        T *__restrict__ P, const T *__restrict__ Uin, T *__restrict__ Uout,
                                                        const T *__restrict__ Uold, T a, T c, SrcArgs src, T *__restrict__ zout,
@@ -1948,12 +1956,12 @@ struct TetFemSim : Sim {
     int step_block = 64;            // threads per block of tet_step_kernel (tune_launch_shape)
     bool slot_split = true;         // symplectic lossless steps by tet_slot_kernel (tune_launch_shape)
     // Until a run tunes the shape (recorded runs do not): in FP32 the
-    // slot-split kernel on meshes of up to 100,000 nodes (us a launch, slot-split
-    // against node kernel: 36k nodes 5.3 and 7.6, 69k 7.9 and 9.2, 98k 10.1 and 9.9,
-    // 118k 11.5 and 8.2), in FP64 of up to 12,000 nodes (9k 7.6 and 11.6, 16k 12.5 and
-    // 11.8, 49k 29.5 and 22.6): the node kernel forms every curl once, and the FP64
+    // slot-split kernel on meshes of up to 80,000 nodes (us a launch, slot-split
+    // against node kernel: 36k nodes 4.5 and 6.9, 69k 7.0 and 7.9, 98k 8.9 and 8.5,
+    // 118k 10.4 and 7.6), in FP64 of up to 12,000 nodes (9k 7.6 and 11.6, 16k 12.5 and
+    // 11.8, 49k 29.0 and 23.5): the node kernel forms every curl once, and the FP64
     // pipe is soon full.
-    static constexpr size_t kSlotMaxNodes32 = 100000, kSlotMaxNodes64 = 12000;
+    static constexpr size_t kSlotMaxNodes32 = 80000, kSlotMaxNodes64 = 12000;
     bool step_tuned = false;        // the block size depends on the mesh only: tuned once per handle
     // the persistent step (tet_persist_kernel, a tuner candidate): its grid
     // barrier's counter and error word, the resident-block capacity of its
@@ -1989,12 +1997,14 @@ struct TetFemSim : Sim {
     std::vector<Dipole> dips;
     std::vector<std::array<int, 6>> rec_edges;
     std::vector<std::array<double, 18>> rec_w;
-    DevBuf d_src_slot, d_src_coef, d_src_dip, d_src_g, d_rec_e, d_rec_w, d_rec_k, d_kslot, d_kidx, d_rz, d_tr, d_ctl;
+    DevBuf d_src_at, d_src_ent, d_src_g, d_rec_e, d_rec_w, d_rec_k, d_kslot, d_kidx, d_rz, d_tr, d_ctl;
     int nk = 0;   // distinct receiver slots
     bool ready = false;
     bool flags_dirty = false;       // pec_h gained source bits not yet on the device
     std::vector<int> rec_ks;        // receiver slots flagged in pec_h and indexed by d_kidx
     bool kidx_valid = false;        // d_kidx holds the table of rec_ks
+    std::vector<int> src_slots;     // the dipole entries' slots, sorted
+    bool src_at_valid = false;      // d_src_at holds the table of src_slots
     // recording for the adjoint: snapshots of the merged state (U, P) at the
     // start of every segment of rec_seg steps of the last run, if that run
     // started from the reset state with ckpt_nsnap > 0
@@ -2832,18 +2842,23 @@ struct TetFemSim : Sim {
         for (size_t k = 0; k < dips.size(); ++k)
             for (int l = 0; l < 6; ++l) ent.push_back({dips[k].slot[l], (int)(6 * k + l)});
         std::stable_sort(ent.begin(), ent.end(), [](const std::array<int, 2> &x, const std::array<int, 2> &y) { return x[0] < y[0]; });
-        std::vector<int> sslot, sdip;
-        std::vector<double> scoef;
-        for (auto &en : ent) {
-            sslot.push_back(en[0]);
-            sdip.push_back(en[1] / 6);
-            scoef.push_back(dips[en[1] / 6].coef[en[1] % 6]);
+        std::vector<SrcEntry> se;
+        std::vector<int> ss;
+        for (size_t k = 0; k < ent.size(); ++k) {
+            const bool more = k + 1 < ent.size() && ent[k + 1][0] == ent[k][0];
+            se.push_back({dips[ent[k][1] / 6].coef[ent[k][1] % 6], ent[k][1] / 6, more});
+            ss.push_back(ent[k][0]);
         }
-        int nsrc = (int)sslot.size();
-        if (sslot.empty()) { sslot.push_back(0); sdip.push_back(0); scoef.push_back(0.0); }
-        up(d_src_slot, sslot);
-        up(d_src_coef, scoef);
-        up(d_src_dip, sdip);
+        const int nsrc = (int)se.size();
+        if (!src_at_valid || ss != src_slots) {   // the dipoles' slots changed: slot -> first entry
+            std::vector<int> at(nslot, -1);
+            for (int k = nsrc - 1; k >= 0; --k) at[ss[k]] = k;
+            up(d_src_at, at);
+            src_slots = ss;
+            src_at_valid = true;
+        }
+        if (se.empty()) se.push_back({0.0, 0, 0});
+        up(d_src_ent, se);
         if (flags_dirty) {
             EMS_CUDA(cudaMemcpyAsync(d_pec.p, pec_h.data(), nslot, cudaMemcpyHostToDevice, stream));
             flags_dirty = false;
@@ -2865,7 +2880,7 @@ struct TetFemSim : Sim {
         up(d_src_g, gv);
         d_ctl.ensure(16);
         d_ctl.zero(stream);
-        return SrcArgs{nsrc, d_src_slot.as<int>(), d_src_coef.as<double>(), d_src_dip.as<int>(), d_src_g.as<double>(),
+        return SrcArgs{nsrc, d_src_at.as<int>(), d_src_ent.as<SrcEntry>(), d_src_g.as<double>(),
                        d_ctl.as<int>(), (int)nd, sc.nsub, 0, 0};
     }
 
