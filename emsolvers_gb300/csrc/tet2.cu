@@ -2082,8 +2082,8 @@ struct Tet2Sim : Sim {
     // FP32: the faster form of the Chebyshev iteration on this handle's meshes
     // (EMS_TET2_ITERATION=fused|march forces one; EMS_TET2_TUNE_LOG prints
     // the times); the forms give the same bits, so the choice changes no
-    // result.  12x13x9 cubes: fused 5.9 us, march 11.7; 24x22x23: 13.3 and 12.0;
-    // 48^3: 70 and 44.7.  FP64 keeps two passes: the FP64 pipe bounds every form,
+    // result.  12x13x9 cubes: fused 5.3 us, march 8.6; 24x22x23: 13.0 and 9.0;
+    // 48^3: 71 and 40.  FP64 keeps two passes: the FP64 pipe bounds every form,
     // and a tile's repeated columns and layers would add to its work.
     template <class T> void choose_iteration()
     {
