@@ -576,3 +576,37 @@ def test_analytic_cavity_mode_converges_on_the_gpu():
         errs.append(abs(_fit_omega(t, tr[ems.FP32][:, 3], w0) - w0) / w0)
     assert errs[1] < 0.004, errs
     assert errs[0] / errs[1] > 1.7, errs
+
+
+@pytest.mark.parametrize("precision", [ems.FP64, ems.FP32], ids=["fp64", "fp32"])
+def test_dipoles_added_between_runs_match_a_fresh_handle(precision):
+    # the slot -> first entry table follows the dipoles: none, one, then two
+    # in one tetrahedron; the same launches on the same tables, so the same bits
+    n = (6, 5, 5)
+    eps, dip, recs = _case(n, 23)
+    dips = [dip, (dip[0], (1.0, -0.5, 0.2), 1, 0.11, 0.7)]
+
+    def add(s, d):
+        s.add_dipole(np.array(d[0]) * H, d[1], ems.WAVE_RICKER, d[3] / TS, d[4])
+
+    def make():
+        s = ems.TetFemSimulation(n, H, 1, ems.SYMP4, precision, dt=0.01 * TS)
+        s.set_material(eps)
+        for r in recs:
+            s.add_receiver(np.array(r) * H)
+        return s
+
+    kept = make()
+    kept.run(3)
+    assert not kept.traces()[..., 1:].any()
+    for k in (1, 2):
+        add(kept, dips[k - 1])
+        kept.reset()
+        kept.run(30)
+        fresh = make()
+        for d in dips[:k]:
+            add(fresh, d)
+        fresh.run(30)
+        assert fresh.get_field(0).any()
+        np.testing.assert_array_equal(kept.get_field(0), fresh.get_field(0))
+        np.testing.assert_array_equal(kept.traces(), fresh.traces())
