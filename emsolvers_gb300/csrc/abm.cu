@@ -346,10 +346,10 @@ struct AbmSim : Sim {
         for (int l = 0; l < 4; ++l) {
             size_t dst = ((size_t)l * ntot + comp_off(c)) * w;
             if (fp64) {
-                EMS_CUDA(cudaMemcpy((char *)b.p + dst, in + (size_t)l * g.n[c], g.n[c] * 8, cudaMemcpyHostToDevice));
+                copy_in((char *)b.p + dst, in + (size_t)l * g.n[c], g.n[c] * 8);
             } else {
                 std::vector<float> tmp(in + (size_t)l * g.n[c], in + (size_t)(l + 1) * g.n[c]);
-                EMS_CUDA(cudaMemcpy((char *)b.p + dst, tmp.data(), g.n[c] * 4, cudaMemcpyHostToDevice));
+                copy_in((char *)b.p + dst, tmp.data(), g.n[c] * 4);
             }
         }
     }

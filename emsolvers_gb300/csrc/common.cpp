@@ -66,6 +66,12 @@ void Sim::init_stream()
     EMS_CUDA(cudaEventCreate(&ev1));
 }
 
+void Sim::copy_in(void *dev, const void *host, size_t bytes) const
+{
+    EMS_CUDA(cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, stream));
+    EMS_CUDA(cudaStreamSynchronize(stream));
+}
+
 void Sim::download(double *out, const void *dev, size_t cnt, bool fp64) const
 {
     const size_t w = fp64 ? 8 : 4;

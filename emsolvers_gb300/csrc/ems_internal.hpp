@@ -84,6 +84,11 @@ struct Sim {
     // element count; FP64 or FP32) holds a NaN or an Inf.
     void check_finite(std::initializer_list<std::pair<const void *, size_t>> arrays, bool fp64);
     DevBuf d_finite;
+    // Host values into a device array, on the handle's stream.  (The stream
+    // does not wait for the default one, on which cudaMemcpy would run: a small
+    // pageable copy may still be on its way when that returns, and a copy
+    // between device arrays has not even begun.)
+    void copy_in(void *dev, const void *host, size_t bytes) const;
     // cnt device values (FP64 or FP32) into a host array of doubles, through
     // two pinned buffers of kPinned values: the copy of one chunk runs while
     // the last one is converted.  (A copy into fresh pageable memory faults its

@@ -408,10 +408,10 @@ struct FemStabSim : Sim {
         for (int l = 0; l < 3; ++l) {
             char *dst = (char *)dE.p + ((size_t)l * ntot + comp_off(which)) * w;
             if (fp64) {
-                EMS_CUDA(cudaMemcpy(dst, in + (size_t)l * n, n * 8, cudaMemcpyHostToDevice));
+                copy_in(dst, in + (size_t)l * n, n * 8);
             } else {
                 std::vector<float> tmp(in + (size_t)l * n, in + (size_t)(l + 1) * n);
-                EMS_CUDA(cudaMemcpy(dst, tmp.data(), n * 4, cudaMemcpyHostToDevice));
+                copy_in(dst, tmp.data(), n * 4);
             }
         }
     }

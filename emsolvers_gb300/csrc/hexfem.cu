@@ -986,10 +986,10 @@ struct HexFemSim : Sim {
     {
         size_t cnt = field_size(which);
         if (fp64) {
-            EMS_CUDA(cudaMemcpy(lev[which].p, in, cnt * 8, cudaMemcpyHostToDevice));
+            copy_in(lev[which].p, in, cnt * 8);
         } else {
             std::vector<float> tmp(in, in + cnt);
-            EMS_CUDA(cudaMemcpy(lev[which].p, tmp.data(), cnt * 4, cudaMemcpyHostToDevice));
+            copy_in(lev[which].p, tmp.data(), cnt * 4);
         }
     }
 

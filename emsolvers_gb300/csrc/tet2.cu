@@ -1728,7 +1728,7 @@ struct Tet2Sim : Sim {
             sh[s].dof0 = shots[s].dof0; sh[s].tet0 = shots[s].tet0; sh[s].ent0 = shots[s].ent0;
         }
         d_shots.alloc(sh.size() * sizeof(T2Shot));
-        EMS_CUDA(cudaMemcpy(d_shots.p, sh.data(), sh.size() * sizeof(T2Shot), cudaMemcpyHostToDevice));
+        copy_in(d_shots.p, sh.data(), sh.size() * sizeof(T2Shot));
         for (const ShotH &S : shots)
             EMS_CHECK_ARG(kPlanes * S.nnode < ((size_t)1 << 32), "shot too large for 32-bit DOF offsets");
         const size_t w = fp64 ? 8 : 4;
@@ -1794,6 +1794,7 @@ struct Tet2Sim : Sim {
         EMS_CUDA(cudaMemcpyToSymbol(c2_ninc, R.ninc, sizeof(R.ninc)));
         EMS_CUDA(cudaMemcpyToSymbol(c2_inc, R.inc, sizeof(R.inc)));
         EMS_CUDA(cudaMemcpyToSymbol(c2_axes, R.axes, sizeof(R.axes)));
+        EMS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // these went by the default stream
     }
 
     // API position (6 * cell + p within a shot) -> type-major device order
@@ -1833,7 +1834,7 @@ struct Tet2Sim : Sim {
         DevBuf e64, p64;
         e64.alloc(ntet * 8);
         p64.alloc(3 * nent * 8);
-        EMS_CUDA(cudaMemcpy(e64.p, e.data(), ntet * 8, cudaMemcpyHostToDevice));
+        copy_in(e64.p, e.data(), ntet * 8);
         t2_pinv_kernel<<<blocks(nent, 128), 128, 0, stream>>>(nent, d_shots.as<T2Shot>(), (int)shots.size(), e64.as<double>(),
                                                               p64.as<double>());
         d_eps.ensure(ntet * sizeof(T));
@@ -1980,9 +1981,9 @@ struct Tet2Sim : Sim {
                     }
         }
         d_tiles.ensure(tiles.size() * sizeof(T2Tile));
-        EMS_CUDA(cudaMemcpy(d_tiles.p, tiles.data(), tiles.size() * sizeof(T2Tile), cudaMemcpyHostToDevice));
+        copy_in(d_tiles.p, tiles.data(), tiles.size() * sizeof(T2Tile));
         d_tables.ensure(tables.size() * sizeof(int));
-        EMS_CUDA(cudaMemcpy(d_tables.p, tables.data(), tables.size() * sizeof(int), cudaMemcpyHostToDevice));
+        copy_in(d_tables.p, tables.data(), tables.size() * sizeof(int));
         auto wide = [](auto k) { EMS_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMarchSmem)); };
         wide(t2_march_kernel<float, FIN_NONE, kCols, kStage>);
         wide(t2_march_kernel<float, FIN_DRIFT, kCols, kStage>);
@@ -2133,7 +2134,7 @@ struct Tet2Sim : Sim {
         }
         // zero the dead DOFs by one force pass on the start vector's shape: the
         // entity pass writes zeros there; the solve keeps them at zero
-        EMS_CUDA(cudaMemcpy(d_x.p, x0.data(), ndof * sizeof(T), cudaMemcpyHostToDevice));
+        copy_in(d_x.p, x0.data(), ndof * sizeof(T));
         T *x = d_x.as<T>(), *pb = d_b.as<T>(), *z = d_Uold.as<T>();
         enqueue_force<T>(x, pb);                    // p = K x0
         d_x.zero(stream);                           // the iterates hold zeros at dead DOFs
@@ -2162,9 +2163,10 @@ struct Tet2Sim : Sim {
         // the power iteration uses the solver's scratch; the state (U, Uold, P) is kept
         DevBuf keep;
         keep.alloc(ndof * (fp64 ? 8 : 4));
-        EMS_CUDA(cudaMemcpy(keep.p, d_Uold.p, keep.bytes, cudaMemcpyDeviceToDevice));
+        EMS_CUDA(cudaMemcpyAsync(keep.p, d_Uold.p, keep.bytes, cudaMemcpyDeviceToDevice, stream));
         lambda_max = fp64 ? lambda_max_t<double>(100) : lambda_max_t<float>(100);
-        EMS_CUDA(cudaMemcpy(d_Uold.p, keep.p, keep.bytes, cudaMemcpyDeviceToDevice));
+        EMS_CUDA(cudaMemcpyAsync(d_Uold.p, keep.p, keep.bytes, cudaMemcpyDeviceToDevice, stream));
+        EMS_CUDA(cudaStreamSynchronize(stream));   // keep ends here
         dt_lim_n = tet_stability_constant(P.integrator) / std::sqrt(lambda_max);
         limit_known = true;
         y_valid = false;   // it was in the scratch
@@ -2498,14 +2500,14 @@ struct Tet2Sim : Sim {
         const bool pfield = which == 1 && symp();
         DevBuf &b = which == 0 ? d_U : (pfield ? d_P : d_Uold);
         if (pfield || fp64) {
-            EMS_CUDA(cudaMemcpy(b.p, tmp.data(), ndof * 8, cudaMemcpyHostToDevice));
+            copy_in(b.p, tmp.data(), ndof * 8);
         } else {
             std::vector<float> f(tmp.begin(), tmp.end());
-            EMS_CUDA(cudaMemcpy(b.p, f.data(), ndof * 4, cudaMemcpyHostToDevice));
+            copy_in(b.p, f.data(), ndof * 4);
         }
         if (pfield && !fp64) {
             std::vector<float> f(tmp.begin(), tmp.end());
-            EMS_CUDA(cudaMemcpy(d_Pc.p, f.data(), ndof * 4, cudaMemcpyHostToDevice));
+            copy_in(d_Pc.p, f.data(), ndof * 4);
         }
         y_valid = false;
         fresh = false;
@@ -2573,7 +2575,7 @@ struct Tet2Sim : Sim {
             DevBuf a, b;
             a.alloc(ndof * sizeof(T));
             b.alloc(ndof * sizeof(T));
-            EMS_CUDA(cudaMemcpy(a.p, in.data(), ndof * sizeof(T), cudaMemcpyHostToDevice));
+            copy_in(a.p, in.data(), ndof * sizeof(T));
             enqueue_force<T>(a.as<T>(), b.as<T>());
             EMS_CUDA(cudaGetLastError());
             EMS_CUDA(cudaStreamSynchronize(stream));

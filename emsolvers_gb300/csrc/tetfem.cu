@@ -2136,6 +2136,7 @@ struct TetFemSim : Sim {
         EMS_CUDA(cudaMemcpyToSymbol(c_wsq, ws, sizeof(ws)));
         EMS_CUDA(cudaMemcpyToSymbol(c_dir, kDir, sizeof(kDir)));
         EMS_CUDA(cudaMemcpyToSymbol(c_pack, pk, sizeof(pk)));
+        EMS_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // these went by the default stream
     }
 
     template <class V> void up(DevBuf &d, const std::vector<V> &v)
@@ -3359,8 +3360,8 @@ struct TetFemSim : Sim {
             tmp[f] = (T)in[e];
             if (lo) lw[f] = float_to_bf16((float)(in[e] - (double)tmp[f]));
         }
-        EMS_CUDA(cudaMemcpy(b.p, tmp.data(), nslot * sizeof(T), cudaMemcpyHostToDevice));
-        if (lo) EMS_CUDA(cudaMemcpy(lo, lw.data(), nslot * 2, cudaMemcpyHostToDevice));
+        copy_in(b.p, tmp.data(), nslot * sizeof(T));
+        if (lo) copy_in(lo, lw.data(), nslot * 2);
     }
     // bfloat16 <-> float on the host: the upper half of the binary32
     // pattern, rounded to nearest even on the way down (NaN kept quiet).

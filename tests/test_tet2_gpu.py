@@ -360,3 +360,29 @@ def test_double_float_stiffness_of_tiny_and_huge_values():
     f = apply(huge)
     assert not np.isfinite(f[x >= 4]).all()
     assert np.linalg.norm((f - ref)[x <= 2]) <= 2.0 ** -24 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("integ", [ems.LEAPFROG, ems.SYMP4])
+@pytest.mark.parametrize("prec", [ems.FP64, ems.FP32])
+def test_asking_for_the_limit_between_runs_keeps_the_state(integ, prec):
+    """The stability limit is found when it is asked for, in the solver's
+    scratch (E^{n-1} among it): a run that goes on after time_step() gives the
+    bits of one that never asked."""
+    n = (17, 12, 14)
+    eps, dip, recs = _case(n, 23)
+    out = []
+    for ask in (False, True):
+        s = ems.TetFemSimulation(n, H, 2, integ, prec, dt=0.02 * TS)
+        s.set_material(eps)
+        s.add_dipole(np.array(dip[0]) * H, dip[1], ems.WAVE_RICKER, dip[3] / TS, dip[4])
+        for r in recs:
+            s.add_receiver(np.array(r) * H)
+        s.run(5)
+        if ask:
+            assert s.time_step()[1] > 0
+        s.run(6)
+        out.append((s.get_field(0), s.get_field(1), s.traces()))
+        s.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+    assert np.linalg.norm(out[0][0]) > 0
