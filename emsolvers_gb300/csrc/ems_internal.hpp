@@ -176,7 +176,11 @@ template <class... P, class... A> void launch_after(void (*k)(P...), dim3 grid, 
     c.numAttrs = 1;
     EMS_CUDA(cudaLaunchKernelEx(&c, k, static_cast<P>(a)...));
 }
-// Everything the kernel before this one wrote may be read from here on.
+// Everything the kernel before this one wrote may be read from here on.  The
+// operands are not read-only for the life of such a kernel, so none of its
+// parameters is __restrict__ (a const one could be read through the
+// non-coherent path, and moved ahead of the wait); outputs that loads may pass
+// are __restrict__ in an inlined function behind the wait.
 __device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
 

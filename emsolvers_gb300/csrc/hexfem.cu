@@ -323,8 +323,8 @@ template <class T, int O> struct HexRows {
 template <class T, int O> struct HexK { const T *k; };   // K of the element pass, [3][TT][RP]
 template <int O> struct HexK<float, O> { float k[3 * HexRows<float, O>::TT * HexRows<float, O>::RP]; };
 template <class T, int O, bool EXACT>
-__global__ void __launch_bounds__(128) hex_elem_kernel(const __grid_constant__ HexGeom g, const __grid_constant__ HexK<T, O> K, const T *__restrict__ Ux, const T *__restrict__ Uy,
-                                                       const T *__restrict__ Uz, T *__restrict__ fe, int *step, HexRec rec)
+__global__ void __launch_bounds__(128) hex_elem_kernel(const __grid_constant__ HexGeom g, const __grid_constant__ HexK<T, O> K, const T *Ux, const T *Uy,
+                                                       const T *Uz, T *fe, int *step, HexRec rec)
 {
     constexpr int D = HexRows<T, O>::D, TT = HexRows<T, O>::TT, W = HexRows<T, O>::W, RP = HexRows<T, O>::RP;
     constexpr bool ARG = sizeof(T) == 4;
@@ -425,8 +425,8 @@ __device__ __forceinline__ void hex1_columns(std::integer_sequence<int, J...>, c
     };
     (col(std::integral_constant<int, J>{}), ...);
 }
-__global__ void __launch_bounds__(32) hex1_elem_kernel(HexGeom g, const __grid_constant__ HexClasses k, const double *__restrict__ Ux,
-                                                       const double *__restrict__ Uy, const double *__restrict__ Uz, double *__restrict__ fe,
+__global__ void __launch_bounds__(32) hex1_elem_kernel(HexGeom g, const __grid_constant__ HexClasses k, const double *Ux,
+                                                       const double *Uy, const double *Uz, double *fe,
                                                        int *step, HexRec rec)
 {
     wait_for_last();
@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(32) hex1_elem_kernel(HexGeom g, const __grid_c
 // along the two axes across the edge, a and b, present where it lies on their
 // common face; the values of those are a fixed distance away in fe.
 template <class T, int O, bool EXACT, int C>
-__device__ __forceinline__ T dof_sum(const HexGeom &g, const T *__restrict__ fe, int ix, int iy, int iz, T sign, bool has_src, T srcval)
+__device__ __forceinline__ T dof_sum(const HexGeom &g, const T *fe, int ix, int iy, int iz, T sign, bool has_src, T srcval)
 {
     constexpr int D = O * (O + 1) * (O + 1);
     constexpr int RX = 1, RY = C == 0 ? O : O + 1, RZ = C == 2 ? (O + 1) * (O + 1) : O * (O + 1);   // rows of K along the axes
@@ -532,7 +532,7 @@ __device__ __forceinline__ int sources_at(const SrcTab &src, int c, unsigned t)
 
 // DOF pass of a leapfrog step (see hex_leapfrog_kernel), component C.
 template <class T, int O, bool EXACT, int C>
-__device__ __forceinline__ void leap_dof(const HexGeom &g, const T *__restrict__ fe, const HexDofs<T> &d, const SrcTab &src)
+__device__ __forceinline__ void leap_dof(const HexGeom &g, const T *fe, const HexDofs<T> &d, const SrcTab &src)
 {
     const unsigned t = blockIdx.x * 128 + threadIdx.x;
     if (C == 0 && t == 0) src.step[0] += 1;
@@ -552,7 +552,7 @@ __device__ __forceinline__ void leap_dof(const HexGeom &g, const T *__restrict__
 // of its own per component and divisions by products took the kick of order 2
 // on 72^3 grid cells from 17.7 to 10.4 us (each launch alone).
 template <class T, int O, bool EXACT>
-__global__ void __launch_bounds__(128) hex_leap_dof_kernel(const __grid_constant__ HexGeom g, const T *__restrict__ fe, const __grid_constant__ HexDofs<T> d,
+__global__ void __launch_bounds__(128) hex_leap_dof_kernel(const __grid_constant__ HexGeom g, const T *fe, const __grid_constant__ HexDofs<T> d,
                                                            const __grid_constant__ SrcTab src)
 {
     wait_for_last();
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(128) hex_leap_dof_kernel(const __grid_constant
 // opening half drift of the next substep (h2 != 0; FP32 runs take both half
 // drifts as one, h1).  Drifts add (h P) / m; 1 / m is a power of two.
 template <class T, int O, bool EXACT, int C>
-__device__ __forceinline__ void kick_dof(const HexGeom &g, const T *__restrict__ fe, const HexDofs<T> &d, const SrcTab &src, T dt, T h1, T h2, T rm)
+__device__ __forceinline__ void kick_dof(const HexGeom &g, const T *fe, const HexDofs<T> &d, const SrcTab &src, T dt, T h1, T h2, T rm)
 {
     const unsigned t = blockIdx.x * 128 + threadIdx.x;
     if (src.last && C == 0 && t == 0) src.step[0] += 1;
@@ -586,7 +586,7 @@ __device__ __forceinline__ void kick_dof(const HexGeom &g, const T *__restrict__
     d.a[C][t] = u;
 }
 template <class T, int O, bool EXACT>
-__global__ void __launch_bounds__(128) hex_kick_dof_kernel(const __grid_constant__ HexGeom g, const T *__restrict__ fe, const __grid_constant__ HexDofs<T> d,
+__global__ void __launch_bounds__(128) hex_kick_dof_kernel(const __grid_constant__ HexGeom g, const T *fe, const __grid_constant__ HexDofs<T> d,
                                                            const __grid_constant__ SrcTab src, T dt, T h1, T h2, T rm)
 {
     wait_for_last();

@@ -372,7 +372,7 @@ struct T2Shot {
 
 // shot holding flat index i of the per-tetrahedron (which = 0) or
 // per-entity (which = 1) ranges
-__device__ __forceinline__ int shot_of(const T2Shot *__restrict__ sh, int ns, unsigned long long i, int which)
+__device__ __forceinline__ int shot_of(const T2Shot *sh, int ns, unsigned long long i, int which)
 {
     int lo = 0, hi = ns - 1;
     while (lo < hi) {
@@ -546,9 +546,9 @@ __device__ __forceinline__ void mass_elem_rows(std::integer_sequence<int, Q...>,
     };
     (row(std::integral_constant<int, Q>{}), ...);
 }
-__global__ void __launch_bounds__(64) t2_mass_elem_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
-                                                         const double *__restrict__ eps, const double *__restrict__ x,
-                                                         double *__restrict__ Yt)
+__global__ void __launch_bounds__(64) t2_mass_elem_kernel(unsigned long long NT, const T2Shot *sh, int ns,
+                                                         const double *eps, const double *x,
+                                                         double *Yt)
 {
     wait_for_last();
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -592,7 +592,7 @@ template <class T> struct GArgs {
 // applies the mode's update.  Unused and boundary-tangential entities are
 // held at zero.
 template <class T, class TY, int MODE, int FIN>
-__global__ void __launch_bounds__(128) t2_gather_kernel(unsigned long long NE, const T2Shot *__restrict__ sh, int ns, GArgs<T> g)
+__global__ void __launch_bounds__(128) t2_gather_kernel(unsigned long long NE, const T2Shot *sh, int ns, GArgs<T> g)
 {
     wait_for_last();
     const unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -771,13 +771,13 @@ constexpr IncTab kInc = make_inc_tab();
 static_assert(kInc.n[6] == 6 && kInc.n[7] == 2, "Kuhn split: the body diagonal lies in six tetrahedra, a face in two");
 
 // The 20 values of tetrahedron type P of the cube at xs.
-template <class T, int P, int B> __device__ __forceinline__ T cheb_value(const T *__restrict__ xs, unsigned nn, unsigned nx1, unsigned nxy)
+template <class T, int P, int B> __device__ __forceinline__ T cheb_value(const T *xs, unsigned nn, unsigned nx1, unsigned nxy)
 {
     constexpr int PL = kInc.plane[P][B], VO = kInc.vo[P][B];
     return xs[(unsigned)PL * nn + (VO & 1) + ((VO >> 1) & 1) * nx1 + ((VO >> 2) & 1) * nxy];
 }
 template <class T, int P, int... B>
-__device__ __forceinline__ void cheb_load(std::integer_sequence<int, B...>, const T *__restrict__ xs, unsigned nn, unsigned nx1, unsigned nxy,
+__device__ __forceinline__ void cheb_load(std::integer_sequence<int, B...>, const T *xs, unsigned nn, unsigned nx1, unsigned nxy,
                                           T (&x)[20])
 {
     ((x[B] = cheb_value<T, P, B>(xs, nn, nx1, nxy)), ...);
@@ -835,7 +835,7 @@ __device__ __forceinline__ double curl_dot(std::integer_sequence<int, Q...>, con
 }
 template <int P, int... A>
 __device__ __forceinline__ void stiff_body(std::integer_sequence<int, A...>, const TetAddr &ta, unsigned long long NT, unsigned long long t,
-                                           const double *__restrict__ U, double *__restrict__ Yt)
+                                           const double *U, double *__restrict__ Yt)
 {
     double u[20], c[12], h[12];
     cheb_load<double, P>(std::make_integer_sequence<int, 20>{}, U + ta.dof0 + ta.v0, ta.nnode, ta.nx1, ta.nxy, u);
@@ -850,8 +850,8 @@ __device__ __forceinline__ void stiff_body(std::integer_sequence<int, A...>, con
     }
     ((Yt[A * NT + t] = curl_dot<P, A>(std::make_integer_sequence<int, 12>{}, h)), ...);
 }
-__global__ void __launch_bounds__(64) t2_stiff_elem_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
-                                                          const double *__restrict__ U, double *__restrict__ Yt)
+__global__ void __launch_bounds__(64) t2_stiff_elem_kernel(unsigned long long NT, const T2Shot *sh, int ns,
+                                                          const double *U, double *Yt)
 {
     wait_for_last();
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -973,7 +973,7 @@ __device__ __forceinline__ void stiff_mass(const float (&cs)[12], const float (&
 // instruction cache.  On 48^3 cubes 425 us with the coefficients read from
 // constant memory, 226 us with 100 conversions on the FP64 pipe, 176 us now.
 template <int P> __device__ __forceinline__ void stiff_df_body(const TetAddr &ta, unsigned long long NT, unsigned long long t,
-                                                               const float *__restrict__ U, double *__restrict__ Yt)
+                                                               const float *U, double *__restrict__ Yt)
 {
     float u[20], cs[12], cc[12];
     cheb_load<float, P>(std::make_integer_sequence<int, 20>{}, U + ta.dof0 + ta.v0, ta.nnode, ta.nx1, ta.nxy, u);
@@ -991,8 +991,8 @@ template <int P> __device__ __forceinline__ void stiff_df_body(const TetAddr &ta
     }
 }
 
-__global__ void __launch_bounds__(128) t2_stiff_df_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
-                                                         const float *__restrict__ U, double *__restrict__ Yt)
+__global__ void __launch_bounds__(128) t2_stiff_df_kernel(unsigned long long NT, const T2Shot *sh, int ns,
+                                                         const float *U, double *Yt)
 {
     wait_for_last();
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -1014,7 +1014,7 @@ __global__ void __launch_bounds__(128) t2_stiff_df_kernel(unsigned long long NT,
 // tetrahedra of e M x at the entity's local DOFs, every table entry a
 // compile-time constant.
 template <class T, int ET, int Q>
-__device__ __forceinline__ void cheb_rows_inc(const T *__restrict__ xs, const T *__restrict__ eps, unsigned long long tet0,
+__device__ __forceinline__ void cheb_rows_inc(const T *xs, const T *eps, unsigned long long tet0,
                                               unsigned ncube, unsigned nn, unsigned nx1, unsigned nxy, unsigned ncx, unsigned ncxy,
                                               const int (&n)[3], int i, int j, int k, T &y0, T &y1)
 {
@@ -1031,7 +1031,7 @@ __device__ __forceinline__ void cheb_rows_inc(const T *__restrict__ xs, const T 
 }
 
 template <class T, int ET, int... Q>
-__device__ __forceinline__ void cheb_rows_all(std::integer_sequence<int, Q...>, const T *__restrict__ xs, const T *__restrict__ eps,
+__device__ __forceinline__ void cheb_rows_all(std::integer_sequence<int, Q...>, const T *xs, const T *eps,
                                               unsigned long long tet0, unsigned ncube, unsigned nn, unsigned nx1, unsigned nxy,
                                               unsigned ncx, unsigned ncxy, const int (&n)[3], int i, int j, int k, T &y0, T &y1)
 {
@@ -1039,7 +1039,7 @@ __device__ __forceinline__ void cheb_rows_all(std::integer_sequence<int, Q...>, 
 }
 
 template <class T, int ET>
-__device__ __forceinline__ void cheb_rows(const T *__restrict__ xs, const T *__restrict__ eps, unsigned long long tet0, unsigned ncube,
+__device__ __forceinline__ void cheb_rows(const T *xs, const T *eps, unsigned long long tet0, unsigned ncube,
                                           unsigned nn, unsigned nx1, unsigned nxy, unsigned ncx, unsigned ncxy, const int (&n)[3], int i,
                                           int j, int k, T &y0, T &y1)
 {
@@ -1054,7 +1054,7 @@ __device__ __forceinline__ void cheb_rows(const T *__restrict__ xs, const T *__r
 // body compiled for its incidences (cheb_rows); the entity types are
 // plane-major, so a warp holds one type.
 template <class T, int FIN>
-__global__ void __launch_bounds__(128) t2_cheb_kernel(unsigned long long NE, const T2Shot *__restrict__ sh, int ns, GArgs<T> g)
+__global__ void __launch_bounds__(128) t2_cheb_kernel(unsigned long long NE, const T2Shot *sh, int ns, GArgs<T> g)
 {
     const unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
     if (e >= NE) return;
@@ -1380,7 +1380,7 @@ __device__ __forceinline__ void march_copies(std::integer_sequence<int, S...>, A
 // per edge or face): 48^3 cubes 44.7 us against 67, five shots of 12..40
 // cubes 63 against 100, thirteen shots of 22..40 cubes 227 against 345.
 template <class T, int FIN, int COLS, int NC>
-__global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *__restrict__ tiles, const int *__restrict__ tables, MArgs<T> g)
+__global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *tiles, const int *tables, MArgs<T> g)
 {
     constexpr int NT = 6 * COLS, G = COLS / 32;   // a warp: one tetrahedron type of 32 columns
     extern __shared__ __align__(16) unsigned char t2_sm[];
@@ -1543,7 +1543,7 @@ template <class T> __global__ void t2_narrow_kernel(unsigned long long n, const 
     if (i < n) y[i] = (T)x[i];
 }
 
-template <class T> __global__ void t2_axpy_kernel(unsigned long long n, T *__restrict__ U, const T *__restrict__ x, double h)
+template <class T> __global__ void t2_axpy_kernel(unsigned long long n, T *U, const T *x, double h)
 {
     wait_for_last();
     const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -1554,10 +1554,10 @@ template <class T> __global__ void t2_axpy_kernel(unsigned long long n, T *__res
 // symplectic P += s sum_k coef_k g_k (and the run-precision copy), leapfrog
 // b -= sum_k coef_k g_k.
 template <class T, int LEAP>
-__global__ void t2_source_kernel(int n, const unsigned long long *__restrict__ dof, const int *__restrict__ ptr,
-                                 const int *__restrict__ dip, const double *__restrict__ coef, const double *__restrict__ gt,
-                                 const int *__restrict__ ctl, int nsub, int q, int nd, double s, double *__restrict__ P,
-                                 T *__restrict__ vec)
+__global__ void t2_source_kernel(int n, const unsigned long long *dof, const int *ptr,
+                                 const int *dip, const double *coef, const double *gt,
+                                 const int *ctl, int nsub, int q, int nd, double s, double *P,
+                                 T *vec)
 {
     wait_for_last();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1578,8 +1578,8 @@ __global__ void t2_source_kernel(int n, const unsigned long long *__restrict__ d
 // Receivers: one warp each; lane a < 20 forms its function's terms, a fixed
 // shuffle tree sums them.
 template <class T>
-__global__ void t2_sample_kernel(int nrec, const unsigned long long *__restrict__ rdof, const double *__restrict__ rw,
-                                 const T *__restrict__ U, const int *__restrict__ ctl, int tf, int nsamp, double *__restrict__ tr)
+__global__ void t2_sample_kernel(int nrec, const unsigned long long *rdof, const double *rw,
+                                 const T *U, const int *ctl, int tf, int nsamp, double *tr)
 {
     wait_for_last();
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), l = threadIdx.x & 31;
@@ -1603,8 +1603,8 @@ __global__ void t2_advance_kernel(int *ctl) { wait_for_last(); ctl[0] += 1; }
 
 // Block partial sums of x . y (fixed grid, fixed order); the host adds them.
 template <class T>
-__global__ void __launch_bounds__(256) t2_dot_kernel(unsigned long long n, const T *__restrict__ x, const T *__restrict__ y,
-                                                    double *__restrict__ part)
+__global__ void __launch_bounds__(256) t2_dot_kernel(unsigned long long n, const T *x, const T *y,
+                                                    double *part)
 {
     wait_for_last();
     __shared__ double sm[256];
@@ -1619,7 +1619,7 @@ __global__ void __launch_bounds__(256) t2_dot_kernel(unsigned long long n, const
     if (threadIdx.x == 0) part[blockIdx.x] = sm[0];
 }
 
-template <class T> __global__ void t2_scale_kernel(unsigned long long n, T *__restrict__ x, double s)
+template <class T> __global__ void t2_scale_kernel(unsigned long long n, T *x, double s)
 {
     wait_for_last();
     const unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -1629,9 +1629,9 @@ template <class T> __global__ void t2_scale_kernel(unsigned long long n, T *__re
 // Gradient contraction of the adjoint: grad_t += c * Z_t . (Mref_p Y_t), the
 // element product in the run precision, the sum over time in FP64.
 template <class T>
-__global__ void __launch_bounds__(128) t2_grad_kernel(unsigned long long NT, const T2Shot *__restrict__ sh, int ns,
-                                                     const T *__restrict__ Z, const T *__restrict__ Y, double c,
-                                                     double *__restrict__ grad)
+__global__ void __launch_bounds__(128) t2_grad_kernel(unsigned long long NT, const T2Shot *sh, int ns,
+                                                     const T *Z, const T *Y, double c,
+                                                     double *grad)
 {
     wait_for_last();
     const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
