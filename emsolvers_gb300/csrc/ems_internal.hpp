@@ -179,8 +179,9 @@ template <class... P, class... A> void launch_after(void (*k)(P...), dim3 grid, 
 // Everything the kernel before this one wrote may be read from here on.  The
 // operands are not read-only for the life of such a kernel, so none of its
 // parameters is __restrict__ (a const one could be read through the
-// non-coherent path, and moved ahead of the wait); outputs that loads may pass
-// are __restrict__ in an inlined function behind the wait.
+// non-coherent path, and moved ahead of the wait).  They are in a function
+// inlined behind the wait, where loads have to pass stores (the leapfrog
+// step of 705k nodes: 39.9 us without, 26.6 us with it).
 __device__ __forceinline__ void wait_for_last() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
 

@@ -455,7 +455,7 @@ __global__ void __launch_bounds__(32) hex1_elem_kernel(HexGeom g, const __grid_c
 // along the two axes across the edge, a and b, present where it lies on their
 // common face; the values of those are a fixed distance away in fe.
 template <class T, int O, bool EXACT, int C>
-__device__ __forceinline__ T dof_sum(const HexGeom &g, const T *fe, int ix, int iy, int iz, T sign, bool has_src, T srcval)
+__device__ __forceinline__ T dof_sum(const HexGeom &g, const T *__restrict__ fe, int ix, int iy, int iz, T sign, bool has_src, T srcval)
 {
     constexpr int D = O * (O + 1) * (O + 1);
     constexpr int RX = 1, RY = C == 0 ? O : O + 1, RZ = C == 2 ? (O + 1) * (O + 1) : O * (O + 1);   // rows of K along the axes
@@ -532,7 +532,7 @@ __device__ __forceinline__ int sources_at(const SrcTab &src, int c, unsigned t)
 
 // DOF pass of a leapfrog step (see hex_leapfrog_kernel), component C.
 template <class T, int O, bool EXACT, int C>
-__device__ __forceinline__ void leap_dof(const HexGeom &g, const T *fe, const HexDofs<T> &d, const SrcTab &src)
+__device__ __forceinline__ void leap_dof(const HexGeom &g, const T *__restrict__ fe, const HexDofs<T> &d, const SrcTab &src)
 {
     const unsigned t = blockIdx.x * 128 + threadIdx.x;
     if (C == 0 && t == 0) src.step[0] += 1;
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(128) hex_leap_dof_kernel(const __grid_constant
 // opening half drift of the next substep (h2 != 0; FP32 runs take both half
 // drifts as one, h1).  Drifts add (h P) / m; 1 / m is a power of two.
 template <class T, int O, bool EXACT, int C>
-__device__ __forceinline__ void kick_dof(const HexGeom &g, const T *fe, const HexDofs<T> &d, const SrcTab &src, T dt, T h1, T h2, T rm)
+__device__ __forceinline__ void kick_dof(const HexGeom &g, const T *__restrict__ fe, const HexDofs<T> &d, const SrcTab &src, T dt, T h1, T h2, T rm)
 {
     const unsigned t = blockIdx.x * 128 + threadIdx.x;
     if (src.last && C == 0 && t == 0) src.step[0] += 1;

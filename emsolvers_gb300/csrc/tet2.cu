@@ -372,7 +372,7 @@ struct T2Shot {
 
 // shot holding flat index i of the per-tetrahedron (which = 0) or
 // per-entity (which = 1) ranges
-__device__ __forceinline__ int shot_of(const T2Shot *sh, int ns, unsigned long long i, int which)
+__device__ __forceinline__ int shot_of(const T2Shot *__restrict__ sh, int ns, unsigned long long i, int which)
 {
     int lo = 0, hi = ns - 1;
     while (lo < hi) {
@@ -771,13 +771,13 @@ constexpr IncTab kInc = make_inc_tab();
 static_assert(kInc.n[6] == 6 && kInc.n[7] == 2, "Kuhn split: the body diagonal lies in six tetrahedra, a face in two");
 
 // The 20 values of tetrahedron type P of the cube at xs.
-template <class T, int P, int B> __device__ __forceinline__ T cheb_value(const T *xs, unsigned nn, unsigned nx1, unsigned nxy)
+template <class T, int P, int B> __device__ __forceinline__ T cheb_value(const T *__restrict__ xs, unsigned nn, unsigned nx1, unsigned nxy)
 {
     constexpr int PL = kInc.plane[P][B], VO = kInc.vo[P][B];
     return xs[(unsigned)PL * nn + (VO & 1) + ((VO >> 1) & 1) * nx1 + ((VO >> 2) & 1) * nxy];
 }
 template <class T, int P, int... B>
-__device__ __forceinline__ void cheb_load(std::integer_sequence<int, B...>, const T *xs, unsigned nn, unsigned nx1, unsigned nxy,
+__device__ __forceinline__ void cheb_load(std::integer_sequence<int, B...>, const T *__restrict__ xs, unsigned nn, unsigned nx1, unsigned nxy,
                                           T (&x)[20])
 {
     ((x[B] = cheb_value<T, P, B>(xs, nn, nx1, nxy)), ...);
@@ -835,7 +835,7 @@ __device__ __forceinline__ double curl_dot(std::integer_sequence<int, Q...>, con
 }
 template <int P, int... A>
 __device__ __forceinline__ void stiff_body(std::integer_sequence<int, A...>, const TetAddr &ta, unsigned long long NT, unsigned long long t,
-                                           const double *U, double *__restrict__ Yt)
+                                           const double *__restrict__ U, double *__restrict__ Yt)
 {
     double u[20], c[12], h[12];
     cheb_load<double, P>(std::make_integer_sequence<int, 20>{}, U + ta.dof0 + ta.v0, ta.nnode, ta.nx1, ta.nxy, u);
@@ -973,7 +973,7 @@ __device__ __forceinline__ void stiff_mass(const float (&cs)[12], const float (&
 // instruction cache.  On 48^3 cubes 425 us with the coefficients read from
 // constant memory, 226 us with 100 conversions on the FP64 pipe, 176 us now.
 template <int P> __device__ __forceinline__ void stiff_df_body(const TetAddr &ta, unsigned long long NT, unsigned long long t,
-                                                               const float *U, double *__restrict__ Yt)
+                                                               const float *__restrict__ U, double *__restrict__ Yt)
 {
     float u[20], cs[12], cc[12];
     cheb_load<float, P>(std::make_integer_sequence<int, 20>{}, U + ta.dof0 + ta.v0, ta.nnode, ta.nx1, ta.nxy, u);
@@ -1014,7 +1014,7 @@ __global__ void __launch_bounds__(128) t2_stiff_df_kernel(unsigned long long NT,
 // tetrahedra of e M x at the entity's local DOFs, every table entry a
 // compile-time constant.
 template <class T, int ET, int Q>
-__device__ __forceinline__ void cheb_rows_inc(const T *xs, const T *eps, unsigned long long tet0,
+__device__ __forceinline__ void cheb_rows_inc(const T *__restrict__ xs, const T *__restrict__ eps, unsigned long long tet0,
                                               unsigned ncube, unsigned nn, unsigned nx1, unsigned nxy, unsigned ncx, unsigned ncxy,
                                               const int (&n)[3], int i, int j, int k, T &y0, T &y1)
 {
@@ -1031,7 +1031,7 @@ __device__ __forceinline__ void cheb_rows_inc(const T *xs, const T *eps, unsigne
 }
 
 template <class T, int ET, int... Q>
-__device__ __forceinline__ void cheb_rows_all(std::integer_sequence<int, Q...>, const T *xs, const T *eps,
+__device__ __forceinline__ void cheb_rows_all(std::integer_sequence<int, Q...>, const T *__restrict__ xs, const T *__restrict__ eps,
                                               unsigned long long tet0, unsigned ncube, unsigned nn, unsigned nx1, unsigned nxy,
                                               unsigned ncx, unsigned ncxy, const int (&n)[3], int i, int j, int k, T &y0, T &y1)
 {
@@ -1039,7 +1039,7 @@ __device__ __forceinline__ void cheb_rows_all(std::integer_sequence<int, Q...>, 
 }
 
 template <class T, int ET>
-__device__ __forceinline__ void cheb_rows(const T *xs, const T *eps, unsigned long long tet0, unsigned ncube,
+__device__ __forceinline__ void cheb_rows(const T *__restrict__ xs, const T *__restrict__ eps, unsigned long long tet0, unsigned ncube,
                                           unsigned nn, unsigned nx1, unsigned nxy, unsigned ncx, unsigned ncxy, const int (&n)[3], int i,
                                           int j, int k, T &y0, T &y1)
 {

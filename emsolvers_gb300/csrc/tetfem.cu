@@ -317,7 +317,7 @@ __device__ __forceinline__ int pk7(int r, int c)
 }
 
 // The packed mass block of node v (plane layout) into registers.
-template <class T> __device__ __forceinline__ void load_block(const T *minv, size_t nnode, size_t v, T (&mv)[28])
+template <class T> __device__ __forceinline__ void load_block(const T *__restrict__ minv, size_t nnode, size_t v, T (&mv)[28])
 {
     const vec4<T> *m4 = reinterpret_cast<const vec4<T> *>(minv);
 #pragma unroll
@@ -753,9 +753,10 @@ constexpr int kStepBlocks[4] = {32, 64, 128, 256};
 constexpr int kStepBlockMax = 256;
 
 template <class T, int MODE, int DAMP, int REC = 0, int COMP = 0>
-__device__ __forceinline__ void tet_step(size_t nnode, const int2 *nrec, const unsigned char *pec, const T *minv,
-                                         T *__restrict__ P, const T *Uin, T *__restrict__ Uout, const T *Uold, T a, T c,
-                                         const SrcArgs &src, T *__restrict__ zout, const T *damp, T *__restrict__ ppre,
+__device__ __forceinline__ void tet_step(size_t nnode, const int2 *__restrict__ nrec, const unsigned char *__restrict__ pec,
+                                         const T *__restrict__ minv, T *__restrict__ P, const T *__restrict__ Uin,
+                                         T *__restrict__ Uout, const T *__restrict__ Uold, T a, T c, const SrcArgs &src,
+                                         T *__restrict__ zout, const T *__restrict__ damp, T *__restrict__ ppre,
                                          T *__restrict__ pmid, const RecArgs<T> &rec, const Comp &cmp)
 {
     static_assert(!COMP || (MODE == 0 && std::is_same<T, float>::value), "compensated updates: FP32 symplectic steps");
@@ -991,7 +992,7 @@ __device__ __forceinline__ void slot_loads(T (&ue)[NU], const T *u0, I nnode, co
 
 // Row D of the node's packed mass block (plane layout), in column order.
 template <class T, int D, int... J>
-__device__ __forceinline__ void slot_mass_row(const T *minv, size_t v, size_t nnode, T (&row)[7],
+__device__ __forceinline__ void slot_mass_row(const T *__restrict__ minv, size_t v, size_t nnode, T (&row)[7],
                                               std::integer_sequence<int, J...>)
 {
     constexpr int idx[7] = {(D < J ? D * (13 - D) / 2 + J : J * (13 - J) / 2 + D)...};   // packed (D, j)
@@ -1017,7 +1018,7 @@ __device__ __forceinline__ void slot_curl(const T *u0, I nnode, const int (&off)
 // The force of slot D and row D of the node's mass block.
 template <class T, int D, int COMP>
 __device__ __forceinline__ void slot_force(const T *u0, size_t nnode, const int (&off)[13], int have, T &f, T &fl,
-                                           const T *minv, size_t v, T (&row)[7])
+                                           const T *__restrict__ minv, size_t v, T (&row)[7])
 {
     slot_mass_row<T, D>(minv, v, nnode, row, std::make_integer_sequence<int, 7>{});
     slot_curl<T, D, COMP>(u0, nnode, off, have, f, fl);
@@ -1027,9 +1028,10 @@ __device__ __forceinline__ void slot_force(const T *u0, size_t nnode, const int 
 // of the 32^3 headline mesh run in one wave (40 registers left 61 blocks
 // for a second wave; 30.7 -> 29.8 ms per 2000-step solve).
 template <class T, int REC, int COMP>
-__device__ __forceinline__ void tet_slot(size_t nnode, const int2 *nrec, const unsigned char *pec, const T *minv,
-                                         T *__restrict__ P, const T *Uin, T *__restrict__ Uout, T a, T c, const SrcArgs &src,
-                                         T *__restrict__ zout, const RecArgs<T> &rec, const Comp &cmp)
+__device__ __forceinline__ void tet_slot(size_t nnode, const int2 *__restrict__ nrec, const unsigned char *__restrict__ pec,
+                                         const T *__restrict__ minv, T *__restrict__ P, const T *__restrict__ Uin,
+                                         T *__restrict__ Uout, T a, T c, const SrcArgs &src, T *__restrict__ zout,
+                                         const RecArgs<T> &rec, const Comp &cmp)
 {
     constexpr StepTab tab = make_step_tab();
     const int nb = (int)blockIdx.x - rec.nsb;
@@ -1325,8 +1327,8 @@ __global__ void __launch_bounds__(kSlotThreads, sizeof(T) == 4 ? 8 : 1) tet_pers
 // zr_v += Pbar . Pmid + (g Pbar) . Ppre in FP64 (the sensitivity after the
 // first factor is g Pbar, the adjoint kick leaves Pbar alone), Pbar = g Pbar.
 template <class T>
-__device__ __forceinline__ void tet_loss_adjoint(size_t nnode, const T *damp, T *__restrict__ Pb, const T *pmid, const T *ppre,
-                                                 double *__restrict__ zr)
+__device__ __forceinline__ void tet_loss_adjoint(size_t nnode, const T *__restrict__ damp, T *__restrict__ Pb,
+                                                 const T *__restrict__ pmid, const T *__restrict__ ppre, double *__restrict__ zr)
 {
     const size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nnode) return;
@@ -1455,10 +1457,11 @@ __global__ void __launch_bounds__(128) tet_grad_accumulate_kernel(size_t nnode, 
 // thread per slot and then one per node the two launches of 64 receivers took
 // 5.9 and 14.9 us.
 template <class T>
-__device__ __forceinline__ void tet_receiver_adjoint(int nnd, const int *nd_node, const int *nd_map, const int *sl_ptr,
-                                                     const int *term_rc, const double *term_w, const double *r,
-                                                     T *__restrict__ Wb, T *__restrict__ Pb, const T *minv, const T *z,
-                                                     double *__restrict__ Q, double cc, size_t nnode)
+__device__ __forceinline__ void tet_receiver_adjoint(int nnd, const int *__restrict__ nd_node, const int *__restrict__ nd_map,
+                                                     const int *__restrict__ sl_ptr, const int *__restrict__ term_rc,
+                                                     const double *__restrict__ term_w, const double *__restrict__ r,
+                                                     T *__restrict__ Wb, T *__restrict__ Pb, const T *__restrict__ minv,
+                                                     const T *__restrict__ z, double *__restrict__ Q, double cc, size_t nnode)
 {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, d = t & 7, i = t >> 3;
     const bool in = i < nnd && d < 7;
@@ -1811,8 +1814,9 @@ __device__ __forceinline__ void grid_sum(double s, double *__restrict__ part, un
 // x, y *= 1 / sqrt(nrm), nrm = nrm_base[2 * *jp] with jp, else nrm_base[0];
 // x32 = (float) x afterwards and kz = 0 (the FP32 buffer the next apply
 // accumulates K x32 into).
-__device__ __forceinline__ void scale_pair(size_t n, double *__restrict__ x, double *__restrict__ y, const double *nrm_base,
-                                      const int *jp, float *__restrict__ x32, float *__restrict__ kz)
+__device__ __forceinline__ void scale_pair(size_t n, double *__restrict__ x, double *__restrict__ y,
+                                           const double *__restrict__ nrm_base, const int *__restrict__ jp,
+                                           float *__restrict__ x32, float *__restrict__ kz)
 {
     const double s = 1.0 / sqrt(nrm_base[jp ? 2 * *jp : 0]);
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -1841,9 +1845,10 @@ __global__ void narrow_kernel(size_t n, const double *__restrict__ x, float *__r
 // Kv32, w = Minv Mw (FP64 mass blocks), and *alpha = v . Mw.  With jp
 // given, the device iteration index is advanced here (no kernel of this
 // iteration has read it yet).
-__device__ __forceinline__ void lanczos_minv(size_t nnode, const double *minv, const float *kv32, const double *vcur,
-                                             double *__restrict__ Mw, double *__restrict__ w, double *__restrict__ part,
-                                             unsigned *__restrict__ ticket, double *__restrict__ alpha, int *__restrict__ jp)
+__device__ __forceinline__ void lanczos_minv(size_t nnode, const double *__restrict__ minv, const float *__restrict__ kv32,
+                                             const double *__restrict__ vcur, double *__restrict__ Mw, double *__restrict__ w,
+                                             double *__restrict__ part, unsigned *__restrict__ ticket,
+                                             double *__restrict__ alpha, int *__restrict__ jp)
 {
     if (jp && blockIdx.x == 0 && threadIdx.x == 0) *jp += 1;
     double acc = 0.0;
@@ -1887,10 +1892,12 @@ __global__ void lanczos_start_kernel(size_t nslot, size_t nnode, const unsigned 
 // (kept at cf[2j]), beta_j^2 at cf[2j - 1]; w -= alpha v + beta vp, Mw -=
 // alpha Mv + beta Mvp (vp == nullptr: no beta term), then beta_{j+1}^2 =
 // w . Mw at cf[2j + 1].  j = *jp when jp is given, else j0.
-__device__ __forceinline__ void lanczos_step(size_t n, double *__restrict__ w, double *__restrict__ Mw, const double *v,
-                                             const double *Mv, const double *vp, const double *Mvp, const double *alpha,
-                                             double *__restrict__ part, unsigned *__restrict__ ticket, double *__restrict__ cf,
-                                             int j0, const int *jp)
+__device__ __forceinline__ void lanczos_step(size_t n, double *__restrict__ w, double *__restrict__ Mw,
+                                             const double *__restrict__ v, const double *__restrict__ Mv,
+                                             const double *__restrict__ vp, const double *__restrict__ Mvp,
+                                             const double *__restrict__ alpha, double *__restrict__ part,
+                                             unsigned *__restrict__ ticket, double *__restrict__ cf, int j0,
+                                             const int *__restrict__ jp)
 {
     const int j = jp ? *jp : j0;
     const double al = *alpha, be = vp ? sqrt(cf[2 * j - 1]) : 0.0;
