@@ -1043,7 +1043,6 @@ __device__ __forceinline__ void tet_slot(size_t nnode, const int2 *__restrict__ 
     const int lane = threadIdx.x, d = threadIdx.y;
     const size_t v = (size_t)nb * kSlotNodes + lane;
     const bool valid = v < nnode;
-    if (rec.adv && v == 0 && d == 0) rec.ctl[1 - rec.par] = rec.ctl[rec.par] + 1;
     const size_t f0 = (size_t)d * nnode + v, e0 = 7 * v;
     T x = 0, u = 0, row[7] = {0, 0, 0, 0, 0, 0, 0};   // row: the mass row of slot d, loaded before the barrier
     unsigned char m = 0;
@@ -1098,6 +1097,8 @@ __device__ __forceinline__ void tet_slot(size_t nnode, const int2 *__restrict__ 
     Uout[f0] = fma(c, y, u);
     if (zout) zout[f0] = y;
     if (REC && (m & kRecBit)) rec.rz_out[rec.kidx[e0 + d]] = y;
+    // behind the loads, which may not pass this store (32^3 FP32: 4.62 us a launch ahead of them, 4.56 here)
+    if (rec.adv && v == 0 && d == 0) rec.ctl[1 - rec.par] = rec.ctl[rec.par] + 1;
 }
 template <class T, int REC, int COMP>
 __global__ void __launch_bounds__(kSlotThreads, sizeof(T) == 4 ? 8 : 1) tet_slot_kernel(size_t nnode, const int2 *nrec,
