@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <array>
 #include <cstdio>
 #include <initializer_list>
@@ -45,6 +46,7 @@ struct DevBuf {
     ~DevBuf() { release(); }
     void alloc(size_t b);
     void ensure(size_t b);   // alloc(b) unless the buffer already holds exactly b bytes
+    void grow(size_t b);     // alloc(b) unless the buffer holds b bytes or more
     void zero(cudaStream_t s);
     void release();
     template <class T> T *as() const { return static_cast<T *>(p); }
@@ -89,14 +91,25 @@ struct Sim {
     // pageable copy may still be on its way when that returns, and a copy
     // between device arrays has not even begun.)
     void copy_in(void *dev, const void *host, size_t bytes) const;
-    // cnt device values (FP64 or FP32) into a host array of doubles, through
-    // two pinned buffers of kPinned values: the copy of one chunk runs while
-    // the last one is converted.  (A copy into fresh pageable memory faults its
-    // pages in one by one: 74 MB took 55 ms.)
-    void download(double *out, const void *dev, size_t cnt, bool fp64) const;
-    static constexpr size_t kPinned = (size_t)1 << 18;
-    mutable void *pinned[2] = {nullptr, nullptr};
-    mutable cudaEvent_t pinned_ev[2] = {nullptr, nullptr};
+    // cnt device values into a host array.  Its pages are touched first: the
+    // copy engine faults fresh pages in one by one (six FP64 fields of
+    // 160x150x140 cells into fresh arrays: 137 ms, 7 so).
+    void download(double *out, const double *dev, size_t cnt) const;
+    // cnt values that pack(at, n, dst) forms in device memory, n of them from
+    // `at`, by way of a buffer of at most kStage values.
+    template <class F> void download(double *out, size_t cnt, F &&pack) const
+    {
+        const size_t piece = std::min(cnt, kStage);
+        d_stage.grow(piece * sizeof(double));
+        for (size_t at = 0; at < cnt; at += piece) {
+            const size_t n = std::min(piece, cnt - at);
+            pack(at, n, d_stage.as<double>());
+            EMS_CUDA(cudaGetLastError());
+            download(out + at, d_stage.as<double>(), n);
+        }
+    }
+    static constexpr size_t kStage = (size_t)1 << 20;
+    mutable DevBuf d_stage;
 };
 
 // CSV element matrices in the reference format (fem_v2/fem_simulation.cpp:1477-1524).

@@ -392,17 +392,17 @@ __global__ void __launch_bounds__(256) fdtd_e_kernel(FdtdArgs<T> a, FdtdPoints p
     if (ez) vstore(a.Ez + o, e2, nyz);
 }
 
-// One component between the device layout and the API's array (rows of w
-// values, ah rows per plane): out in the run precision, in from FP64.
-template <class T, class A, bool GET>
-__global__ void fdtd_field_kernel(T *f, A *api, size_t cnt, int w, int ah, size_t pitch, size_t plane, int shift)
+// n values of one component from `at` on between the device layout and the
+// API's array (rows of w values, ah rows per plane).
+template <class T, bool GET>
+__global__ void fdtd_field_kernel(T *f, double *api, size_t at, size_t n, int w, int ah, size_t pitch, size_t plane, int shift)
 {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= cnt) return;
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x, t = at + q;
+    if (q >= n) return;
     const size_t r = t / w;
     const ptrdiff_t o = (ptrdiff_t)((r / ah) * plane + (r % ah) * pitch + t % w) - shift;
-    if (GET) api[t] = (A)f[o];
-    else f[o] = (T)api[t];
+    if (GET) api[q] = (double)f[o];
+    else f[o] = (T)api[q];
 }
 // Material ids into rows of mpitch, the last column repeated, zero behind it.
 __global__ void fdtd_mat_kernel(const uint16_t *id, uint16_t *mat, size_t cnt, unsigned mpitch, int nx)
@@ -488,7 +488,6 @@ struct FdtdSim : Sim {
     size_t pitch, plane, total, mpitch;
     int g0, g1;                 // threads of a row [g0, g1) that touch no x layer
     DevBuf F[6];
-    mutable DevBuf d_stage;     // a component in the API's layout
     // materials
     std::vector<uint16_t> mat_host;
     std::vector<double> mat_eps, mat_sigma;
@@ -663,11 +662,15 @@ struct FdtdSim : Sim {
             ca[m] = (1.0 - s) / (1.0 + s);
             cb[m] = P.dt / mat_eps[m] / P.h / (1.0 + s);
         }
-        const size_t cnt = (size_t)ny * nz * mpitch;
-        d_mat.ensure(cnt * 2 + 16);
-        d_stage.ensure(nc * 2);
-        EMS_CUDA(cudaMemcpyAsync(d_stage.p, mat_host.data(), nc * 2, cudaMemcpyHostToDevice, stream));
-        fdtd_mat_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(d_stage.as<uint16_t>(), d_mat.as<uint16_t>(), cnt, (unsigned)mpitch, nx);
+        d_mat.ensure((size_t)ny * nz * mpitch * 2 + 16);
+        const size_t rows = (size_t)ny * nz, piece = std::min(rows, std::max<size_t>(kStage / nx, 1));
+        d_stage.grow(piece * nx * 2);
+        for (size_t r = 0; r < rows; r += piece) {
+            const size_t m = std::min(piece, rows - r), cnt = m * mpitch;
+            copy_in(d_stage.p, mat_host.data() + r * nx, m * nx * 2);
+            fdtd_mat_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(d_stage.as<uint16_t>(), d_mat.as<uint16_t>() + r * mpitch,
+                                                                               cnt, (unsigned)mpitch, nx);
+        }
         std::vector<double> cab(2 * ca.size());
         for (size_t m = 0; m < ca.size(); ++m) { cab[2 * m] = ca[m]; cab[2 * m + 1] = cb[m]; }
         upload_real(d_cab, cab);
@@ -1011,28 +1014,30 @@ struct FdtdSim : Sim {
         if (which < 0 || which > 5) throw Error{EMS_ERR_INVALID_ARGUMENT, "field index must be 0..5 (Ex,Ey,Ez,Hx,Hy,Hz)"};
         return n[which];
     }
-    // a component between the device layout and the API's (in d_stage)
-    template <class T, class A, bool GET> void move_field(int which) const
+    // n values of a component from `at` on between the device layout and the API's
+    template <class T, bool GET> void move_field(int which, size_t at, size_t n, double *api) const
     {
         const int w[6] = {nx + 1, nx + 2, nx + 2, nx, nx + 1, nx + 1}, h[6] = {ny + 2, ny + 1, ny + 2, ny + 1, ny, ny + 1};
-        const size_t cnt = n[which];
-        fdtd_field_kernel<T, A, GET><<<(unsigned)((cnt + 255) / 256), 256, 0, stream>>>(
-            F[which].as<T>() + lead, d_stage.as<A>(), cnt, w[which], h[which], pitch, plane, which == 1 || which == 2 ? 1 : 0);
+        fdtd_field_kernel<T, GET><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(
+            F[which].as<T>() + lead, api, at, n, w[which], h[which], pitch, plane, which == 1 || which == 2 ? 1 : 0);
         EMS_CUDA(cudaGetLastError());
     }
     void get_field(int which, double *out) const override
     {
-        const size_t cnt = field_size(which);
-        d_stage.ensure(cnt * (fp64 ? 8 : 4));
-        if (fp64) move_field<double, double, true>(which); else move_field<float, float, true>(which);
-        download(out, d_stage.p, cnt, fp64);
+        download(out, field_size(which), [&](size_t at, size_t n, double *dst) {
+            if (fp64) move_field<double, true>(which, at, n, dst); else move_field<float, true>(which, at, n, dst);
+        });
     }
     void set_field(int which, const double *in) override
     {
-        const size_t cnt = field_size(which);
-        d_stage.ensure(cnt * 8);
-        EMS_CUDA(cudaMemcpyAsync(d_stage.p, in, cnt * 8, cudaMemcpyHostToDevice, stream));
-        if (fp64) move_field<double, double, false>(which); else move_field<float, double, false>(which);
+        const size_t cnt = field_size(which), piece = std::min(cnt, kStage);
+        d_stage.grow(piece * sizeof(double));
+        for (size_t at = 0; at < cnt; at += piece) {
+            const size_t n = std::min(piece, cnt - at);
+            copy_in(d_stage.p, in + at, n * sizeof(double));
+            if (fp64) move_field<double, false>(which, at, n, d_stage.as<double>());
+            else move_field<float, false>(which, at, n, d_stage.as<double>());
+        }
         EMS_CUDA(cudaStreamSynchronize(stream));
     }
 

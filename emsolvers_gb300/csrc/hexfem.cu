@@ -595,6 +595,12 @@ __global__ void __launch_bounds__(128) hex_kick_dof_kernel(const __grid_constant
     else kick_dof<T, O, EXACT, 2>(g, fe, d, src, dt, h1, h2, rm);
 }
 
+__global__ void hex_widen_kernel(const float *x, double *y, size_t n)
+{
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < n) y[t] = (double)x[t];
+}
+
 static double femv2_source(double t)
 {
     const double freq = 1.0e9;
@@ -979,8 +985,12 @@ struct HexFemSim : Sim {
     // levels returned in the reference's storage order (ring index 0,1,2)
     void get_field(int which, double *out) const override
     {
-        size_t cnt = field_size(which);
-        download(out, lev[which].p, cnt, fp64);
+        const size_t cnt = field_size(which);
+        if (fp64) download(out, lev[which].as<double>(), cnt);
+        else
+            download(out, cnt, [&](size_t at, size_t n, double *dst) {
+                hex_widen_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(lev[which].as<float>() + at, dst, n);
+            });
     }
     void set_field(int which, const double *in) override
     {

@@ -1526,15 +1526,16 @@ __global__ void __launch_bounds__(128) t2_pinv_kernel(unsigned long long NE, con
     out[2 * NE + e] = ok ? a / det : 0.0;
 }
 
-// A field from planes to the API's node-major order.
+// m values of a field from `at` on, from planes to the API's node-major order.
 template <class T>
-__global__ void t2_field_kernel(unsigned long long n, const T2Shot *__restrict__ sh, int ns, const T *__restrict__ x, T *__restrict__ out)
+__global__ void t2_field_kernel(unsigned long long at, unsigned long long m, const T2Shot *__restrict__ sh, int ns, const T *__restrict__ x,
+                                double *__restrict__ out)
 {
-    const unsigned long long e = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-    if (e >= n) return;
+    const unsigned long long q = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x, e = at + q;
+    if (q >= m) return;
     const T2Shot S = sh[shot_of(sh, ns, e / 2, 1)];   // 38 DOFs and 19 entities per node
     const unsigned l = (unsigned)(e - S.dof0), node = l / kPlanes, pl = l - node * kPlanes;
-    out[e] = x[S.dof0 + (unsigned long long)pl * S.nnode + node];
+    out[q] = (double)x[S.dof0 + (unsigned long long)pl * S.nnode + node];
 }
 
 template <class T> __global__ void t2_narrow_kernel(unsigned long long n, const double *__restrict__ x, T *__restrict__ y)
@@ -2484,14 +2485,12 @@ struct Tet2Sim : Sim {
         const DevBuf &b = which == 0 ? d_U : (pfield ? d_P : d_Uold);
         auto body = [&](auto tag) {
             using T = decltype(tag);
-            d_stage.ensure(ndof * sizeof(T));
-            t2_field_kernel<T><<<blocks(ndof, 256), 256, 0, stream>>>(ndof, d_shots.as<T2Shot>(), (int)shots.size(), b.as<T>(), d_stage.as<T>());
-            EMS_CUDA(cudaGetLastError());
-            download(out, d_stage.p, ndof, sizeof(T) == 8);
+            download(out, ndof, [&](size_t at, size_t n, double *dst) {
+                t2_field_kernel<T><<<blocks(n, 256), 256, 0, stream>>>(at, n, d_shots.as<T2Shot>(), (int)shots.size(), b.as<T>(), dst);
+            });
         };
         if (pfield || fp64) body(double()); else body(float());
     }
-    mutable DevBuf d_stage;   // a field in the API's order
     void set_field(int which, const double *in) override
     {
         field_size(which);

@@ -1497,14 +1497,15 @@ __global__ void __launch_bounds__(128) tet_receiver_adjoint_kernel(int nnd, cons
     tet_receiver_adjoint<T>(nnd, nd_node, nd_map, sl_ptr, term_rc, term_w, r, Wb, Pb, minv, z, Q, cc, nnode);
 }
 
-// A field from the plane layout to slot order (with the compensation added).
-template <class T, class A>
-__global__ void tet_slots_kernel(size_t nslot, size_t nnode, const T *__restrict__ x, const __nv_bfloat16 *__restrict__ lo, A *__restrict__ out)
+// n values of a field from `at` on, from the plane layout to slot order (with the compensation added).
+template <class T>
+__global__ void tet_slots_kernel(size_t at, size_t n, size_t nnode, const T *__restrict__ x, const __nv_bfloat16 *__restrict__ lo,
+                                 double *__restrict__ out)
 {
-    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nslot) return;
-    const size_t f = fslot(e, nnode);
-    out[e] = (A)x[f] + (lo ? (A)__bfloat162float(lo[f]) : A(0));
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n) return;
+    const size_t f = fslot(at + q, nnode);
+    out[q] = (double)x[f] + (lo ? (double)__bfloat162float(lo[f]) : 0.0);
 }
 
 // Loss rate of a node: rho = sum sigma w / sum eps w over the incidences of
@@ -3294,8 +3295,8 @@ struct TetFemSim : Sim {
                                                         d_grad.as<double>());
         if (has_loss) loss_gradient(zr, d_grad, grad_sigma != nullptr);
         EMS_CUDA(cudaGetLastError());
-        download(grad, d_grad.p, ntet, true);
-        if (grad_sigma && has_loss) download(grad_sigma, d_gsig.p, ntet, true);
+        download(grad, d_grad.as<double>(), ntet);
+        if (grad_sigma && has_loss) download(grad_sigma, d_gsig.as<double>(), ntet);
         else if (grad_sigma) std::fill(grad_sigma, grad_sigma + ntet, 0.0);
     }
 
@@ -3377,19 +3378,11 @@ struct TetFemSim : Sim {
     // Fields cross the API in slot order (e = 7 node + d) and live on the
     // device in the plane layout (fslot).  With a compensation plane lo
     // (FP32 symplectic handles) the value is hi + lo, split again on upload.
-    mutable DevBuf d_slots;
     template <class T> void download_slots(const DevBuf &b, double *out, const __nv_bfloat16 *lo = nullptr) const
     {
-        const unsigned nb = (unsigned)((nslot + 255) / 256);
-        if (lo) {   // hi + lo in FP64
-            d_slots.ensure(nslot * 8);
-            tet_slots_kernel<T, double><<<nb, 256, 0, stream>>>(nslot, nnode, b.as<T>(), lo, d_slots.as<double>());
-        } else {
-            d_slots.ensure(nslot * sizeof(T));
-            tet_slots_kernel<T, T><<<nb, 256, 0, stream>>>(nslot, nnode, b.as<T>(), nullptr, d_slots.as<T>());
-        }
-        EMS_CUDA(cudaGetLastError());
-        download(out, d_slots.p, nslot, lo || sizeof(T) == 8);
+        download(out, nslot, [&](size_t at, size_t n, double *dst) {
+            tet_slots_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(at, n, nnode, b.as<T>(), lo, dst);
+        });
     }
     template <class T> void upload_slots(DevBuf &b, const double *in, __nv_bfloat16 *lo = nullptr) const
     {
