@@ -14,7 +14,8 @@
 // Orders 1 and 2 run in two passes: the element values K u of every element,
 // then the DOFs, which sum theirs and take the whole update of the substep.
 // Order 3 forms the rows DOF by DOF (144 values per element do not fit the
-// registers of the element pass).
+// registers of the element pass), and so do grids of 2^31 DOFs and more per
+// component.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -42,6 +43,7 @@ struct HexDiv {
     int s;
     __device__ __forceinline__ unsigned operator()(unsigned t) const { return (unsigned)((unsigned long long)t * m >> s); }
 };
+constexpr size_t kHexDivLimit = (size_t)1 << 31;
 static HexDiv hex_div(int d)
 {
     int l = 0;
@@ -176,14 +178,23 @@ __device__ T dof_force(const HexGeom &g, const T *__restrict__ K, const T *const
     return acc;
 }
 
-__device__ __forceinline__ void dof_coords(const HexGeom &g, int c, size_t t, int &ix, int &iy, int &iz)
+// Coordinates of DOF t of component c, for fewer than 2^31 of them (see HexDiv).
+__device__ __forceinline__ void dof_coords32(const HexGeom &g, int c, unsigned u, int &ix, int &iy, int &iz)
 {
-    int nxc = c == 0 ? g.gx : g.gx + 1;
-    int nyc = c == 1 ? g.gy : g.gy + 1;
-    const unsigned u = (unsigned)t, r = c == 0 ? g.row[0](u) : g.row[1](u);   // a component holds fewer than 2^31 values (int offsets throughout)
+    const int nxc = c == 0 ? g.gx : g.gx + 1, nyc = c == 1 ? g.gy : g.gy + 1;
+    const unsigned r = c == 0 ? g.row[0](u) : g.row[1](u);
     ix = (int)(u - r * nxc);
     iz = (int)(c == 1 ? g.col[0](r) : g.col[1](r));
     iy = (int)(r - (unsigned)iz * nyc);
+}
+__device__ __forceinline__ void dof_coords(const HexGeom &g, int c, size_t t, int &ix, int &iy, int &iz)
+{
+    if (g.nc[c] < kHexDivLimit) return dof_coords32(g, c, (unsigned)t, ix, iy, iz);
+    const int nxc = c == 0 ? g.gx : g.gx + 1, nyc = c == 1 ? g.gy : g.gy + 1;
+    const size_t r = t / nxc;
+    ix = (int)(t % nxc);
+    iy = (int)(r % nyc);
+    iz = (int)(r / nyc);
 }
 
 // Leapfrog step, one thread per DOF: E2 = (-K E1, boundary zeroed) + 2 E1 - E0,
@@ -538,7 +549,7 @@ __device__ __forceinline__ void leap_dof(const HexGeom &g, const T *__restrict__
     if (C == 0 && t == 0) src.step[0] += 1;
     if (t >= g.nc[C]) return;
     int ix, iy, iz;
-    dof_coords(g, C, t, ix, iy, iz);
+    dof_coords32(g, C, t, ix, iy, iz);
     const bool pec = on_pec(g, C, ix, iy, iz);
     const T a = d.a[C][t], b = d.b[C][t];
     T f = 0;
@@ -572,7 +583,7 @@ __device__ __forceinline__ void kick_dof(const HexGeom &g, const T *__restrict__
     if (src.last && C == 0 && t == 0) src.step[0] += 1;
     if (t >= g.nc[C]) return;
     int ix, iy, iz;
-    dof_coords(g, C, t, ix, iy, iz);
+    dof_coords32(g, C, t, ix, iy, iz);
     const bool pec = on_pec(g, C, ix, iy, iz), has = sources_at(src, C, t) > 0;
     T p = d.b[C][t], u = d.a[C][t], sv = 0, f = 0;
     if (has) sv = (T)src.vals[(size_t)(src.step[1] - 1) * src.nsub + src.q];
@@ -616,7 +627,8 @@ struct HexFemSim : Sim {
     HexGeom g{};
     bool fp64, exact;
     DevBuf lev[3];         // per component: 3 levels
-    DevBuf dK;
+    DevBuf dK, dKr;        // K as the element pass takes it, and row by row
+    bool one_pass = false; // the force DOF by DOF (see below)
     std::vector<double> Kh;
     std::vector<std::array<int, 4>> srcs;   // comp, flat index
     std::vector<std::array<int, 3>> obs_idx; // x, y, z flat indices
@@ -662,6 +674,8 @@ struct HexFemSim : Sim {
         for (int q = 0; q < 2; ++q) { g.row[q] = hex_div(g.gx + q); g.col[q] = hex_div(g.gy + q); }
         fp64 = P.precision == EMS_FP64;
         exact = fp64;
+        // Order 3, and grids beyond the two passes' 32-bit indices
+        one_pass = o == 3 || std::max(g.nc[0], std::max(g.nc[1], g.nc[2])) >= kHexDivLimit;
         // element matrix (fem_v2/fem_simulation.cpp:458-490, symplectic_2 473)
         std::string fn = kdir + "/" + (P.use_ofem ? std::to_string(o) : "lamped" + std::to_string(o)) + ".csv";
         auto M = load_matrix_csv(fn);
@@ -691,29 +705,34 @@ struct HexFemSim : Sim {
         init_stream();
         size_t w = fp64 ? 8 : 4;
         for (int q = 0; q < 3; ++q) { lev[q].alloc(3 * g.nc[q] * w); lev[q].zero(stream); }
-        if (fp64) upload_matrix<double>();
-        else upload_matrix<float>();
+        if (one_pass) {
+            if (fp64) matrix_rows<double>(); else matrix_rows<float>();
+        } else {
+            if (fp64) upload_matrix<double>(); else upload_matrix<float>();
+        }
         EMS_CUDA(cudaStreamSynchronize(stream));
     }
 
-    // K for the kernels: orders 1 and 2 as hex_elem_kernel takes it, order 3 as loaded.
+    template <class T> void upload(DevBuf &d, const std::vector<T> &k)
+    {
+        d.alloc(k.size() * sizeof(T));
+        copy_in(d.p, k.data(), k.size() * sizeof(T));
+    }
+    // K as hex_elem_kernel takes it (orders 1 and 2)
     template <class T> void upload_matrix()
     {
-        std::vector<T> k(Kh.begin(), Kh.end());
-        if (g.o < 3) {
-            const int D = g.dof, TT = g.total, W = 16 / (int)sizeof(T), RP = (D + W - 1) / W * W;
-            k.assign((size_t)3 * TT * RP, T(0));
-            for (int r = 0; r < TT; ++r)
-                for (int m = 0; m < TT; ++m) k[((size_t)(r / D) * TT + m) * RP + r % D] = (T)Kh[(size_t)r * TT + m];
-        }
-        if constexpr (sizeof(T) == 4)
-            if (g.o < 3) {
-                k32 = std::move(k);
-                return;
-            }
-        dK.alloc(k.size() * sizeof(T));
-        EMS_CUDA(cudaMemcpyAsync(dK.p, k.data(), k.size() * sizeof(T), cudaMemcpyHostToDevice, stream));
-        EMS_CUDA(cudaStreamSynchronize(stream));
+        const int D = g.dof, TT = g.total, W = 16 / (int)sizeof(T), RP = (D + W - 1) / W * W;
+        std::vector<T> k((size_t)3 * TT * RP, T(0));
+        for (int r = 0; r < TT; ++r)
+            for (int m = 0; m < TT; ++m) k[((size_t)(r / D) * TT + m) * RP + r % D] = (T)Kh[(size_t)r * TT + m];
+        if constexpr (sizeof(T) == 4) k32 = std::move(k);
+        else upload(dK, k);
+    }
+    // K row by row, for the one-pass kernels
+    template <class T> const T *matrix_rows()
+    {
+        if (!dKr.p) upload(dKr, std::vector<T>(Kh.begin(), Kh.end()));
+        return dKr.as<T>();
     }
 
     int flat(int c, const int *q) const
@@ -730,7 +749,7 @@ struct HexFemSim : Sim {
         size_t mx = std::max(g.nc[0], std::max(g.nc[1], g.nc[2]));
         dim3 grid((unsigned)((mx + 127) / 128), 3);
         auto k = exact ? hex_leapfrog_kernel<T, O, true> : hex_leapfrog_kernel<T, O, false>;
-        k<<<grid, 128, 0, stream>>>(g, dK.as<T>(), L<T>(0, l1), L<T>(1, l1), L<T>(2, l1), L<T>(0, l0), L<T>(1, l0), L<T>(2, l0),
+        k<<<grid, 128, 0, stream>>>(g, matrix_rows<T>(), L<T>(0, l1), L<T>(1, l1), L<T>(2, l1), L<T>(0, l0), L<T>(1, l0), L<T>(2, l0),
                                     L<T>(0, l2), L<T>(1, l2), L<T>(2, l2), s);
     }
     template <class T, int O> void launch_kick(T dt, const SrcList &s)
@@ -738,7 +757,7 @@ struct HexFemSim : Sim {
         size_t mx = std::max(g.nc[0], std::max(g.nc[1], g.nc[2]));
         dim3 grid((unsigned)((mx + 127) / 128), 3);
         auto k = exact ? hex_kick_kernel<T, O, true> : hex_kick_kernel<T, O, false>;
-        k<<<grid, 128, 0, stream>>>(g, dK.as<T>(), L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), L<T>(0, 1), L<T>(1, 1), L<T>(2, 1),
+        k<<<grid, 128, 0, stream>>>(g, matrix_rows<T>(), L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), L<T>(0, 1), L<T>(1, 1), L<T>(2, 1),
                                     L<T>(0, 2), L<T>(1, 2), L<T>(2, 2), dt, s);
     }
     template <class T> void launch_drift(T coef, int pec)
@@ -836,7 +855,7 @@ struct HexFemSim : Sim {
         }
         return n + 1 + 2 * ns;
     }
-    template <class T, int O> long long run_two_pass(int nsteps)
+    template <class T, int O> long long run_two_pass(int nsteps, std::vector<double> &times)
     {
         d_fe.ensure((size_t)g.total * g.EX * g.EY * g.EZ * sizeof(T));
         const int ns = nsub();
@@ -845,6 +864,7 @@ struct HexFemSim : Sim {
         std::vector<double> vals((size_t)std::max(nsteps, 1) * ns);
         double t = cur_time;
         for (int st = 0; st < nsteps; ++st) {
+            if (st % P.time_frequency == 0) times[st / P.time_frequency] = t;
             for (int q = 0; q < ns; ++q)
                 vals[(size_t)st * ns + q] = P.integrator == EMS_LEAPFROG
                     ? femv2_source(t) * P.dt * P.dt / P.permittivity / P.h / P.h / P.h
@@ -883,41 +903,28 @@ struct HexFemSim : Sim {
             }
         }
         for (; step < nsteps; ++step) launches += enqueue_step<T, O>();
+        cur_time = t;
         return launches;
     }
     int graph_launches = 0;
 
-    template <class T, int O> void run_o(int nsteps)
+    // Receivers from `level` into row s of the table.
+    template <class T> void sample_level(int level, int s)
     {
-        const int tf = P.time_frequency;
-        nobs = (int)obs_idx.size();
-        nsamp = nsteps > 0 ? (nsteps - 1) / tf + 1 : 0;
-        ncols = 4;
-        std::vector<int> oi;
-        for (auto &q : obs_idx) { oi.push_back(q[0]); oi.push_back(q[1]); oi.push_back(q[2]); }
-        if (oi.empty()) oi.assign(3, 0);
-        d_obs.ensure(oi.size() * 4);
-        EMS_CUDA(cudaMemcpyAsync(d_obs.p, oi.data(), oi.size() * 4, cudaMemcpyHostToDevice, stream));
-        size_t ntr = (size_t)std::max(nobs, 1) * std::max(nsamp, 1) * 4;
-        d_tr.ensure(ntr * 8);
-        d_tr.zero(stream);
-        std::vector<double> times(std::max(nsamp, 1), 0.0);
+        launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, level), L<T>(1, level), L<T>(2, level),
+                     nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, s, nullptr, 1);
+    }
+    // The run with the force DOF by DOF, launch by launch.
+    template <class T, int O> long long run_one_pass(int nsteps, std::vector<double> &times)
+    {
+        const int tf = P.time_frequency, o = g.o;
         long long launches = 0;
-        const int o = g.o;
-        EMS_CUDA(cudaEventRecord(ev0, stream));
-        if constexpr (O <= 2) {
-            launches = run_two_pass<T, O>(nsteps);
-            for (int step = 0; step < nsteps; ++step) {
-                if (step % tf == 0) times[step / tf] = cur_time;
-                cur_time += P.dt;
-            }
-        } else
         for (int step = 0; step < nsteps; ++step) {
             bool samp = nobs > 0 && step % tf == 0;
             if (P.integrator == EMS_LEAPFROG) {
                 // fem_v2 samples level 1 (E^n) after computing E^{n+1}; E^n is untouched by the step
                 if (samp) {
-                    launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, l1), L<T>(1, l1), L<T>(2, l1), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf, nullptr, 1);
+                    sample_level<T>(l1, step / tf);
                     times[step / tf] = cur_time;
                     ++launches;
                 }
@@ -927,7 +934,7 @@ struct HexFemSim : Sim {
                 l0 = (l0 + 1) % 3; l1 = (l1 + 1) % 3; l2 = (l2 + 1) % 3;
             } else {
                 if (samp) {
-                    launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, step / tf, nullptr, 1);
+                    sample_level<T>(0, step / tf);
                     times[step / tf] = cur_time;
                     ++launches;
                 }
@@ -947,6 +954,28 @@ struct HexFemSim : Sim {
             }
             cur_time += P.dt;
         }
+        return launches;
+    }
+
+    template <class T, int O> void run_o(int nsteps)
+    {
+        const int tf = P.time_frequency;
+        nobs = (int)obs_idx.size();
+        nsamp = nsteps > 0 ? (nsteps - 1) / tf + 1 : 0;
+        ncols = 4;
+        std::vector<int> oi;
+        for (auto &q : obs_idx) { oi.push_back(q[0]); oi.push_back(q[1]); oi.push_back(q[2]); }
+        if (oi.empty()) oi.assign(3, 0);
+        d_obs.ensure(oi.size() * 4);
+        EMS_CUDA(cudaMemcpyAsync(d_obs.p, oi.data(), oi.size() * 4, cudaMemcpyHostToDevice, stream));
+        size_t ntr = (size_t)std::max(nobs, 1) * std::max(nsamp, 1) * 4;
+        d_tr.ensure(ntr * 8);
+        d_tr.zero(stream);
+        std::vector<double> times(std::max(nsamp, 1), 0.0);
+        long long launches = 0;
+        EMS_CUDA(cudaEventRecord(ev0, stream));
+        if constexpr (O <= 2) launches = one_pass ? run_one_pass<T, O>(nsteps, times) : run_two_pass<T, O>(nsteps, times);
+        else launches = run_one_pass<T, O>(nsteps, times);
         EMS_CUDA(cudaGetLastError());
         EMS_CUDA(cudaEventRecord(ev1, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
@@ -1044,7 +1073,7 @@ struct HexFemSim : Sim {
             save[q].alloc(lev[q].bytes);
             EMS_CUDA(cudaMemcpyAsync(save[q].p, lev[q].p, lev[q].bytes, cudaMemcpyDeviceToDevice, stream));
         }
-        if (g.o <= 2) d_fe.ensure((size_t)g.total * g.EX * g.EY * g.EZ * w);
+        if (!one_pass) d_fe.ensure((size_t)g.total * g.EX * g.EY * g.EZ * w);
         auto body = [&](auto tag) {
             using T = decltype(tag);
             SrcList s = sources(0.0);
@@ -1052,13 +1081,14 @@ struct HexFemSim : Sim {
                 if (r == 1) EMS_CUDA(cudaEventRecord(ev0, stream));
                 auto go = [&](auto oc) {
                     constexpr int O = decltype(oc)::value;
-                    if constexpr (O <= 2) {
-                        T *u[3];
-                        for (int c = 0; c < 3; ++c) u[c] = L<T>(c, P.integrator == EMS_LEAPFROG ? l1 : 0);
-                        elements<T, O>(u, false, false);
-                    } else {
-                        if (P.integrator == EMS_LEAPFROG) launch_leapfrog<T, O>(s); else launch_kick<T, O>((T)P.dt, s);
-                    }
+                    if constexpr (O <= 2)
+                        if (!one_pass) {
+                            T *u[3];
+                            for (int c = 0; c < 3; ++c) u[c] = L<T>(c, P.integrator == EMS_LEAPFROG ? l1 : 0);
+                            elements<T, O>(u, false, false);
+                            return;
+                        }
+                    if (P.integrator == EMS_LEAPFROG) launch_leapfrog<T, O>(s); else launch_kick<T, O>((T)P.dt, s);
                 };
                 if (g.o == 1) go(std::integral_constant<int, 1>());
                 else if (g.o == 2) go(std::integral_constant<int, 2>());
@@ -1074,10 +1104,12 @@ struct HexFemSim : Sim {
             EMS_CUDA(cudaMemcpyAsync(lev[q].p, save[q].p, lev[q].bytes, cudaMemcpyDeviceToDevice, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
         *ms = t / launches;
-        // element pass: read U, write the element values; order 3 leapfrog: read E^n, E^{n-1}, write
+        // element pass: read U, write the element values; one-pass leapfrog: read E^n, E^{n-1}, write
         // E^{n+1}; kick: read U, read/write P, write F
-        *bytes = g.o <= 2 ? w * ((double)ndof + (double)g.total * g.EX * g.EY * g.EZ) : (double)ndof * w * (P.integrator == EMS_LEAPFROG ? 3.0 : 4.0);
-        *name = std::string(g.o <= 2 ? (classes && g.EX * g.EY * g.EZ >= kHex1MinElements ? "hex1_elem_kernel" : "hex_elem_kernel") : P.integrator == EMS_LEAPFROG ? "hex_leapfrog_kernel" : "hex_kick_kernel") +
+        *bytes = one_pass ? (double)ndof * w * (P.integrator == EMS_LEAPFROG ? 3.0 : 4.0)
+                          : w * ((double)ndof + (double)g.total * g.EX * g.EY * g.EZ);
+        *name = std::string(one_pass ? (P.integrator == EMS_LEAPFROG ? "hex_leapfrog_kernel" : "hex_kick_kernel")
+                                     : classes && g.EX * g.EY * g.EZ >= kHex1MinElements ? "hex1_elem_kernel" : "hex_elem_kernel") +
                 "<o=" + std::to_string(g.o) + ">";
     }
 };

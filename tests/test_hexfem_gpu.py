@@ -118,3 +118,31 @@ def test_two_pass_force_bitwise_equal_to_oracle(order, grid, integ, ofem):
     np.testing.assert_array_equal(s.traces()[:, :, 1:], t1[:, 5:, 1:])
     for q, lv in enumerate(s.levels()):
         np.testing.assert_array_equal(lv, l1[q])
+
+
+def test_grid_beyond_32_bit_dof_indices():
+    """A component of more than 2^31 DOFs (a rod of 2 x 2 x 240 million
+    elements): a wave launched just below DOF 2^31 and crossing it gives the
+    bits of the same wave in a short rod whose ends it does not reach."""
+    torch = pytest.importorskip("torch")
+    if torch.cuda.mem_get_info()[0] < 100e9:
+        pytest.skip("needs 100 GB of device memory")
+    h, eps, mu = 0.05, 8.8541878128e-12, 1.25663706212e-6
+    dt = h * np.sqrt(eps * mu / 3.0) / 2.0
+    nz, steps = 240_000_000, 24
+    top = (2 ** 31 - 1) // 9 - 2            # Ez has 3 x 3 values per layer
+    assert 9 * nz > 2 ** 31 and 9 * (top + 1) < 2 ** 31 < 9 * (top + 12)
+
+    def run(grid, z):
+        s = ems.HexFemSimulation(1, grid, h, dt, eps, mu, 1, 1, precision=ems.FP32, kmat_dir=golden_io.KMAT_DIR)
+        s.setSource_z((1, 1, z))
+        for q in (z - 5, z - 1, z):
+            s.setObservationPoint((1, 1, q))
+        s.run(steps)
+        t = s.traces()
+        s.close()
+        return t
+
+    ref, got = run((2, 2, 400), 200), run((2, 2, nz), top)
+    assert np.abs(ref[..., 1:]).max() > 0
+    np.testing.assert_array_equal(got, ref)
