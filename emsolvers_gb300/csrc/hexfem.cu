@@ -15,7 +15,7 @@
 // then the DOFs, which sum theirs and take the whole update of the substep.
 // Order 3 forms the rows DOF by DOF (144 values per element do not fit the
 // registers of the element pass), and so do grids of 2^31 DOFs and more per
-// component.
+// component and small FP64 grids of order 2.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -674,8 +674,9 @@ struct HexFemSim : Sim {
         for (int q = 0; q < 2; ++q) { g.row[q] = hex_div(g.gx + q); g.col[q] = hex_div(g.gy + q); }
         fp64 = P.precision == EMS_FP64;
         exact = fp64;
-        // Order 3, and grids beyond the two passes' 32-bit indices
-        one_pass = o == 3 || std::max(g.nc[0], std::max(g.nc[1], g.nc[2])) >= kHexDivLimit;
+        // Order 3, grids beyond the two passes' 32-bit indices, and small FP64 grids of order 2
+        one_pass = o == 3 || std::max(g.nc[0], std::max(g.nc[1], g.nc[2])) >= kHexDivLimit ||
+                   (o == 2 && fp64 && (long long)g.EX * g.EY * g.EZ < kHex2MinElements);
         // element matrix (fem_v2/fem_simulation.cpp:458-490, symplectic_2 473)
         std::string fn = kdir + "/" + (P.use_ofem ? std::to_string(o) : "lamped" + std::to_string(o)) + ".csv";
         auto M = load_matrix_csv(fn);
@@ -794,6 +795,12 @@ struct HexFemSim : Sim {
     // pipes are full, a warp per SM: 37x33x41 elements 28.3 us a leapfrog step
     // against 39.8, but 8x7x6 elements 13.2 against 11.2.
     static constexpr int kHex1MinElements = 4096;
+    // In FP64 a warp of the order-2 element pass takes 65 us for its 1944
+    // operations a thread (its quarter of the SM does one in 64 clocks), however few
+    // warps there are.  DOF by DOF a small grid has more of them: leapfrog step of
+    // 512 elements 24.6 us against 77, 2197 55 against 78, 2744 72 against 78,
+    // 3375 87 against 78.
+    static constexpr int kHex2MinElements = 3000;
     // Element pass of orders 1 and 2 over the level u; samp: with the sampling blocks
     template <class T, int O> void elements(T *const (&u)[3], bool first, bool samp)
     {

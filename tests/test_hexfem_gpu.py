@@ -146,3 +146,28 @@ def test_grid_beyond_32_bit_dof_indices():
     ref, got = run((2, 2, 400), 200), run((2, 2, nz), top)
     assert np.abs(ref[..., 1:]).max() > 0
     np.testing.assert_array_equal(got, ref)
+
+
+@pytest.mark.parametrize("grid", [(28, 28, 29), (31, 29, 30), (61, 20, 20)])
+@pytest.mark.parametrize("integ", [oracle.LEAPFROG, oracle.SYMP4])
+def test_order2_fp64_on_both_sides_of_the_one_pass_rule_bitwise_equal_to_oracle(grid, integ):
+    """FP64 of order 2 sums DOF by DOF on grids of fewer than 3000 elements
+    (2744 here) and in two passes on larger ones (3150 and 3000, odd grid lines
+    among them): the oracle's bits from either."""
+    h, eps, mu = 0.05, 8.8541878128e-12, 1.25663706212e-6
+    dt = h * np.sqrt(eps * mu / 3.0) / 2.0
+    km = oracle.load_kmat(golden_io.kmat_path(2, 1))
+    srcs = [(2, tuple(v // 2 for v in grid)), (0, (0, 1, 1))]
+    obs = [tuple(v // 2 for v in grid)]
+    steps = 12
+    tr_o, ef_o = oracle.hexfem_run(2, grid, h, dt, eps, mu, 2, integ, km, steps, srcs, obs)
+    s = ems.HexFemSimulation(2, grid, h, dt, eps, mu, 2, 1, integrator=integ, precision=ems.FP64, kmat_dir=golden_io.KMAT_DIR)
+    for c, at in srcs:
+        (s.setSource_x, s.setSource_y, s.setSource_z)[c](at)
+    s.setObservationPoint(obs[0])
+    s.run(steps)
+    np.testing.assert_array_equal(s.traces(), tr_o)
+    for q, lv in enumerate(s.levels()):
+        np.testing.assert_array_equal(lv, ef_o[q])
+    name = s.time_dominant_kernel(1)[2]
+    assert ("elem" in name) == (np.prod([v // 2 for v in grid]) >= 3000), name
