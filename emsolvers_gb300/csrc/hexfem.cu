@@ -15,7 +15,8 @@
 // then the DOFs, which sum theirs and take the whole update of the substep.
 // Order 3 forms the rows DOF by DOF (144 values per element do not fit the
 // registers of the element pass), and so do grids of 2^31 DOFs and more per
-// component and small FP64 grids of order 2.
+// component, small FP64 grids of order 2, and grids that leave no memory for
+// the element values.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -784,6 +785,18 @@ struct HexFemSim : Sim {
         const size_t mx = std::max(g.nc[0], std::max(g.nc[1], g.nc[2]));
         return dim3((unsigned)((mx + 127) / 128), 3);
     }
+    // The element values of the two passes (12 or 54 per element); a grid whose
+    // fields leave no room for them takes the one-pass kernels.
+    void make_fe()
+    {
+        if (one_pass) return;
+        try {
+            d_fe.ensure((size_t)g.total * g.EX * g.EY * g.EZ * (fp64 ? 8 : 4));
+        } catch (const Error &e) {
+            if (e.code != EMS_ERR_OUT_OF_MEMORY) throw;
+            one_pass = true;
+        }
+    }
     int nsub() const { return P.integrator == EMS_SYMP4 ? 3 : 1; }
     void substeps(double sub[3], double off[3]) const
     {
@@ -864,7 +877,6 @@ struct HexFemSim : Sim {
     }
     template <class T, int O> long long run_two_pass(int nsteps, std::vector<double> &times)
     {
-        d_fe.ensure((size_t)g.total * g.EX * g.EY * g.EZ * sizeof(T));
         const int ns = nsub();
         double sub[3], off[3];
         substeps(sub, off);
@@ -980,6 +992,7 @@ struct HexFemSim : Sim {
         d_tr.zero(stream);
         std::vector<double> times(std::max(nsamp, 1), 0.0);
         long long launches = 0;
+        make_fe();
         EMS_CUDA(cudaEventRecord(ev0, stream));
         if constexpr (O <= 2) launches = one_pass ? run_one_pass<T, O>(nsteps, times) : run_two_pass<T, O>(nsteps, times);
         else launches = run_one_pass<T, O>(nsteps, times);
@@ -1080,7 +1093,7 @@ struct HexFemSim : Sim {
             save[q].alloc(lev[q].bytes);
             EMS_CUDA(cudaMemcpyAsync(save[q].p, lev[q].p, lev[q].bytes, cudaMemcpyDeviceToDevice, stream));
         }
-        if (!one_pass) d_fe.ensure((size_t)g.total * g.EX * g.EY * g.EZ * w);
+        make_fe();
         auto body = [&](auto tag) {
             using T = decltype(tag);
             SrcList s = sources(0.0);

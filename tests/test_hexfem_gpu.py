@@ -171,3 +171,27 @@ def test_order2_fp64_on_both_sides_of_the_one_pass_rule_bitwise_equal_to_oracle(
         np.testing.assert_array_equal(lv, ef_o[q])
     name = s.time_dominant_kernel(1)[2]
     assert ("elem" in name) == (np.prod([v // 2 for v in grid]) >= 3000), name
+
+
+@pytest.mark.parametrize("integ", [ems.LEAPFROG, ems.SYMP4])
+def test_no_room_for_the_element_values(integ):
+    """A grid whose fields fit while the two passes' element values do not
+    (384 MB here, 150 MB left): the run takes the one-pass kernels and gives the
+    same bits."""
+    torch = pytest.importorskip("torch")
+    g, h, eps, mu = (200, 200, 200), 0.05, 8.8541878128e-12, 1.25663706212e-6
+    dt = h * np.sqrt(eps * mu / 3.0) / 2.0
+    out = []
+    for full in (False, True):
+        s = ems.HexFemSimulation(1, g, h, dt, eps, mu, 1, 1, integrator=integ, precision=ems.FP32, kmat_dir=golden_io.KMAT_DIR)
+        s.setSource_z((100, 100, 100))
+        s.setObservationPoint((101, 100, 100))
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (150 << 20), dtype=torch.uint8, device="cuda") if full else None
+        s.run(11)
+        out.append((s.traces(), s.get_field(2)))
+        del hog
+        torch.cuda.empty_cache()
+        s.close()
+    assert np.linalg.norm(out[0][1]) > 0
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
