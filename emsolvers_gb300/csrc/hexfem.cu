@@ -641,8 +641,13 @@ struct HexFemSim : Sim {
     double cur_time = 0.0;
     DevBuf d_obs, d_tr, d_fe, d_vals, d_step;
     cudaGraphExec_t graph = nullptr;         // kGraphSteps steps, kept while the buffers stay the same
-    std::vector<unsigned long long> graph_key;
+    std::vector<unsigned long long> graph_key, last_key;   // of the graph, of the last run
     static constexpr int kGraphSteps = 9;    // a multiple of the three levels' ring
+    // Capturing and instantiating a graph takes 60 to 170 us.  A run of this many
+    // launches earns it (leapfrog of 512 elements, a fresh handle: 16 steps 211 us
+    // with a graph and 170 before there was one, 100 steps 455 and 690), and so
+    // does a run that repeats the last one.
+    static constexpr int kGraphMinLaunches = 160;
     ~HexFemSim() override
     {
         if (graph) cudaGraphExecDestroy(graph);
@@ -898,29 +903,35 @@ struct HexFemSim : Sim {
         EMS_CUDA(cudaEventRecord(ev0, stream));
         long long launches = 0;
         int step = 0;
-        if (nsteps >= kGraphSteps) {
-            std::vector<unsigned long long> key = {(unsigned long long)l0, (unsigned long long)nobs, (unsigned long long)nsamp, srcs.size()};
-            for (const auto &q : srcs) { key.push_back((unsigned long long)q[0]); key.push_back((unsigned long long)q[1]); }
-            for (const void *q : {d_fe.p, d_vals.p, d_step.p, d_obs.p, d_tr.p}) key.push_back((unsigned long long)reinterpret_cast<uintptr_t>(q));
-            if (!graph || key != graph_key) {
-                if (graph) {
-                    cudaGraphExecDestroy(graph);
-                    graph = nullptr;
+        std::vector<unsigned long long> key = {(unsigned long long)nobs, (unsigned long long)nsamp, srcs.size()};
+        for (const auto &q : srcs) { key.push_back((unsigned long long)q[0]); key.push_back((unsigned long long)q[1]); }
+        for (const void *q : {d_fe.p, d_vals.p, d_step.p, d_obs.p, d_tr.p}) key.push_back((unsigned long long)reinterpret_cast<uintptr_t>(q));
+        const bool kept = graph && key == graph_key;
+        const int per = P.integrator == EMS_LEAPFROG ? 2 : 1 + 2 * ns + (nobs > 0);
+        if (kept || key == last_key || nsteps * per >= kGraphMinLaunches) {
+            for (; l0 != 0 && step < nsteps; ++step) launches += enqueue_step<T, O>();   // the graph's ring begins at level 0
+            if (nsteps - step >= kGraphSteps) {
+                if (!kept) {
+                    if (graph) {
+                        cudaGraphExecDestroy(graph);
+                        graph = nullptr;
+                    }
+                    cudaGraph_t gr = nullptr;
+                    EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+                    for (int r = 0; r < kGraphSteps; ++r) graph_launches = enqueue_step<T, O>();   // the ring ends where it began
+                    EMS_CUDA(cudaStreamEndCapture(stream, &gr));
+                    const cudaError_t e = cudaGraphInstantiate(&graph, gr, 0);
+                    cudaGraphDestroy(gr);
+                    EMS_CUDA(e);
+                    graph_key = key;
                 }
-                cudaGraph_t gr = nullptr;
-                EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-                for (int r = 0; r < kGraphSteps; ++r) graph_launches = enqueue_step<T, O>();   // the ring ends where it began
-                EMS_CUDA(cudaStreamEndCapture(stream, &gr));
-                const cudaError_t e = cudaGraphInstantiate(&graph, gr, 0);
-                cudaGraphDestroy(gr);
-                EMS_CUDA(e);
-                graph_key = key;
-            }
-            for (; step + kGraphSteps <= nsteps; step += kGraphSteps) {
-                EMS_CUDA(cudaGraphLaunch(graph, stream));
-                launches += (long long)kGraphSteps * graph_launches;
+                for (; step + kGraphSteps <= nsteps; step += kGraphSteps) {
+                    EMS_CUDA(cudaGraphLaunch(graph, stream));
+                    launches += (long long)kGraphSteps * graph_launches;
+                }
             }
         }
+        last_key = std::move(key);
         for (; step < nsteps; ++step) launches += enqueue_step<T, O>();
         cur_time = t;
         return launches;

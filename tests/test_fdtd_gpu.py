@@ -312,3 +312,43 @@ def test_pitched_layout_and_served_points_bitwise_equal_to_oracle(grid, pml, poi
         np.testing.assert_array_equal(s.traces(), tr_o)
         for k, v in s.fields().items():
             np.testing.assert_array_equal(v, f_o[k], err_msg=k)
+
+
+@pytest.mark.parametrize("prec", [ems.FP64, ems.FP32], ids=["fp64", "fp32"])
+def test_changes_between_runs_reach_the_replayed_steps(prec):
+    """Runs of one handle, which keeps a graph of its steps, with a material, a
+    source and a receiver added between them: each gives the bits of a new
+    handle that starts from the same fields."""
+    g, h = (13, 10, 9), 1e-3
+    dt = 0.9 * h / (2.998e8 * np.sqrt(3))
+    rng = np.random.default_rng(8)
+    keys = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
+    calls = [lambda s: s.setSource_z((6, 5, 4), waveform=ems.WAVE_RICKER, f0=2e10),
+             lambda s: s.setObservationPoint(([(5, 5, 5)], [(5, 5, 5)], [(6, 5, 4)]))]
+
+    def handle():
+        s = ems.FdtdSimulation(g, h, dt, EPS0, MU0, 1, precision=prec)
+        for c in calls:
+            c(s)
+        return s
+
+    a = handle()
+    e1, e2 = (EPS0 * rng.choice([1.0, 2.0, 3.5], g[::-1]) for _ in range(2))
+    more = [None, None, lambda s: s.set_material(e1), lambda s: s.setSource_x((4, 5, 5), waveform=ems.WAVE_RICKER, f0=3e10),
+            lambda s: s.set_material(e2), lambda s: s.setObservationPoint(([(4, 5, 5)], [], [(3, 3, 3), (6, 5, 4)]))]
+    for c in more:
+        before = a.fields()
+        if c:
+            c(a)
+            calls.append(c)
+        b = handle()
+        for q, k in enumerate(keys):
+            b.set_field(q, before[k])
+        for s in (a, b):
+            s.run(40)
+        np.testing.assert_array_equal(a.traces(), b.traces())
+        for k, v in b.fields().items():
+            np.testing.assert_array_equal(a.fields()[k], v, err_msg=k)
+        b.close()
+    assert np.nanmax(np.abs(a.traces())) > 0   # (the receiver without Ey samples averages nothing: NaN)
+    a.close()

@@ -195,3 +195,39 @@ def test_no_room_for_the_element_values(integ):
     assert np.linalg.norm(out[0][1]) > 0
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("integ", [ems.LEAPFROG, ems.SYMP2, ems.SYMP4])
+@pytest.mark.parametrize("order,prec", [(1, ems.FP64), (1, ems.FP32), (2, ems.FP32)])
+def test_replayed_steps_over_runs_equal_single_steps(order, prec, integ):
+    """Runs that begin at every position of the leapfrog ring, repeated runs that
+    replay a kept graph, and sources and receivers added between runs: the bits
+    of the same steps run one by one."""
+    g, h, eps, mu = (12, 9, 10), 0.05, 8.8541878128e-12, 1.25663706212e-6
+    dt = h * np.sqrt(eps * mu / 3.0) / 2.0
+    out = []
+    for single in (False, True):
+        s = ems.HexFemSimulation(order, g, h, dt, eps, mu, 1, 1, integrator=integ, precision=prec, kmat_dir=golden_io.KMAT_DIR)
+
+        def run(n):
+            t = []
+            for k in [1] * n if single else [n]:
+                s.run(k)
+                t.append(s.traces())
+            return np.concatenate(t, axis=1)
+
+        tr = []
+        s.setSource_z((6, 4, 5))
+        s.setObservationPoint((5, 4, 4))
+        tr += [run(17), run(17), run(17), run(100)]
+        s.setSource_x((3, 4, 5))
+        tr += [run(100), run(100)]
+        s.setObservationPoint((7, 3, 5))
+        tr += [run(100), run(17)]
+        out.append((tr, s.levels()))
+        s.close()
+    assert np.abs(out[0][0][-1][..., 1:]).max() > 0
+    for a, b in zip(out[0][0], out[1][0]):
+        np.testing.assert_array_equal(a, b)
+    for a, b in zip(out[0][1], out[1][1]):
+        np.testing.assert_array_equal(a, b)
