@@ -809,10 +809,10 @@ struct HexFemSim : Sim {
         sub[0] = P.dt; off[0] = 0.0;
         if (P.integrator == EMS_SYMP4) { sub[0] = x1 * P.dt; sub[1] = x2 * P.dt; off[1] = x1 * P.dt; sub[2] = x1 * P.dt; off[2] = (x1 + x2) * P.dt; }
     }
-    // The order-1 FP64 pass with one thread per element pays where the FP64
-    // pipes are full, a warp per SM: 37x33x41 elements 28.3 us a leapfrog step
-    // against 39.8, but 8x7x6 elements 13.2 against 11.2.
-    static constexpr int kHex1MinElements = 4096;
+    // The order-1 FP64 pass with one thread per element pays where the FP64 pipes
+    // are full.  A leapfrog step of 4096 elements 12.4 us with it and 8.1 without,
+    // 8000 12.9 and 12.0, 13824 13.6 and 15.6, 21952 15.5 and 19.8, 50061 28.0 and 35.9.
+    static constexpr int kHex1MinElements = 10000;
     // In FP64 a warp of the order-2 element pass takes 65 us for its 1944
     // operations a thread (its quarter of the SM does one in 64 clocks), however few
     // warps there are.  DOF by DOF a small grid has more of them: leapfrog step of
