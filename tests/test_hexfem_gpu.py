@@ -231,3 +231,26 @@ def test_replayed_steps_over_runs_equal_single_steps(order, prec, integ):
         np.testing.assert_array_equal(a, b)
     for a, b in zip(out[0][1], out[1][1]):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("ofem", [1, 0])
+@pytest.mark.parametrize("grid", [(21, 21, 22), (33, 31, 10), (25, 20, 20)])
+@pytest.mark.parametrize("integ", [oracle.LEAPFROG, oracle.SYMP2])
+def test_order1_fp64_element_passes_bitwise_equal_to_oracle(grid, integ, ofem):
+    """Grids of 9702, 10230 and 10000 elements, on both sides of the line from
+    which one thread takes a whole element of order 1 in FP64."""
+    h, eps, mu = 0.05, 8.8541878128e-12, 1.25663706212e-6
+    dt = h * np.sqrt(eps * mu / 3.0) / 2.0
+    km = oracle.load_kmat(golden_io.kmat_path(1, ofem))
+    srcs = [(2, tuple(v // 2 for v in grid)), (0, (0, 1, 1))]
+    obs = [tuple(v // 2 for v in grid), (1, 1, 0)]
+    tr_o, ef_o = oracle.hexfem_run(1, grid, h, dt, eps, mu, 2, integ, km, 25, srcs, obs)
+    s = ems.HexFemSimulation(1, grid, h, dt, eps, mu, 2, ofem, integrator=integ, precision=ems.FP64, kmat_dir=golden_io.KMAT_DIR)
+    for c, at in srcs:
+        (s.setSource_x, s.setSource_y, s.setSource_z)[c](at)
+    for o in obs:
+        s.setObservationPoint(o)
+    s.run(25)
+    np.testing.assert_array_equal(s.traces(), tr_o)
+    for q, lv in enumerate(s.levels()):
+        np.testing.assert_array_equal(lv, ef_o[q])
