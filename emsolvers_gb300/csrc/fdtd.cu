@@ -873,11 +873,11 @@ struct FdtdSim : Sim {
                 const FdtdSource &q = srcs[s];
                 double eps = P.permittivity, div = 1.0;
                 if (!mat_host.empty()) {
-                    int ci = q.ijk[0], cj = q.ijk[1], ck = q.ijk[2];
-                    if (q.comp == 0) { ci = ci < nx ? ci : nx - 1; cj -= 1; ck -= 1; }
-                    else if (q.comp == 1) { ci -= 1; cj = cj < ny ? cj : ny - 1; ck -= 1; }
-                    else { ci -= 1; cj -= 1; ck = ck < nz ? ck : nz - 1; }
-                    int m = mat_host[(size_t)ci + (size_t)cj * nx + (size_t)ck * nx * ny];
+                    // the cell whose material the E kernel takes at this point; the nearest one in the padding
+                    int cell[3];
+                    const int n3[3] = {nx, ny, nz};
+                    for (int d = 0; d < 3; ++d) cell[d] = std::min(std::max(q.ijk[d] - (d == q.comp ? 0 : 1), 0), n3[d] - 1);
+                    const int m = mat_host[(size_t)cell[0] + (size_t)cell[1] * nx + (size_t)cell[2] * nx * ny];
                     eps = mat_eps[m];
                     div = 1.0 + mat_sigma[m] * P.dt / (2.0 * mat_eps[m]);
                 }

@@ -352,3 +352,30 @@ def test_changes_between_runs_reach_the_replayed_steps(prec):
         b.close()
     assert np.nanmax(np.abs(a.traces())) > 0   # (the receiver without Ey samples averages nothing: NaN)
     a.close()
+
+
+@pytest.mark.parametrize("prec", [ems.FP64, ems.FP32], ids=["fp64", "fp32"])
+def test_sources_in_the_padding_of_a_grid_with_materials(prec):
+    """A source on a padded index takes the material of the nearest cell: after
+    one step from rest its point holds what the same source in a uniform grid of
+    that cell's permittivity leaves there."""
+    g, h = (6, 5, 4), 1e-3
+    nx, ny, nz = g
+    dt = 0.9 * h / (2.998e8 * np.sqrt(3))
+    eps = EPS0 * np.random.default_rng(5).uniform(1, 4, g[::-1])
+    top = [(nx, ny + 1, nz + 1), (nx + 1, ny, nz + 1), (nx + 1, ny + 1, nz)]
+    for comp in range(3):
+        for corner in range(8):
+            at = tuple(top[comp][d] if corner >> d & 1 else 0 for d in range(3))
+            cell = [min(max(at[d] - (d != comp), 0), g[d] - 1) for d in range(3)]
+            e = eps[cell[2], cell[1], cell[0]]
+            got = []
+            for uniform in (False, True):
+                s = ems.FdtdSimulation(g, h, dt, e if uniform else EPS0, MU0, 1, precision=prec)
+                if not uniform:
+                    s.set_material(eps)
+                (s.setSource_x, s.setSource_y, s.setSource_z)[comp](at, waveform=ems.WAVE_RICKER, f0=2e10)
+                s.run(1)
+                got.append(s.fields()[("Ex", "Ey", "Ez")[comp]][at[2], at[1], at[0]])
+                s.close()
+            assert got[0] == got[1] != 0
