@@ -379,3 +379,27 @@ def test_sources_in_the_padding_of_a_grid_with_materials(prec):
                 got.append(s.fields()[("Ex", "Ey", "Ez")[comp]][at[2], at[1], at[0]])
                 s.close()
             assert got[0] == got[1] != 0
+
+
+@pytest.mark.parametrize("pml", [0, 3])
+@pytest.mark.parametrize("prec", [ems.FP64, ems.FP32], ids=["fp64", "fp32"])
+def test_timing_the_dominant_kernel_keeps_the_state(prec, pml):
+    """time_dominant_kernel restores what its launches write, the CPML's
+    auxiliary fields too: the run goes on as if it had not been called."""
+    g, h = (20, 17, 13), 1e-3
+    dt = 0.9 * h / (2.998e8 * np.sqrt(3))
+    eps = EPS0 * np.random.default_rng(6).uniform(1, 4, g[::-1])
+    out = []
+    for timed in (False, True):
+        s = ems.FdtdSimulation(g, h, dt, EPS0, MU0, 1, precision=prec, pml_cells=pml, pml_kappa_max=2.0, pml_alpha_max=0.02)
+        s.set_material(eps, 0.01 * np.ones_like(eps))
+        s.setSource_z((4, 4, 4), waveform=ems.WAVE_RICKER, f0=3e10)
+        s.run(25)
+        if timed:
+            assert s.time_dominant_kernel(3)[0] > 0
+        s.run(25)
+        out.append(s.fields())
+        s.close()
+    for k in out[0]:
+        assert np.abs(out[0][k]).max() > 0
+        np.testing.assert_array_equal(out[0][k], out[1][k], err_msg=k)
