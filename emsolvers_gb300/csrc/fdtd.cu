@@ -110,8 +110,9 @@ __device__ __forceinline__ void mload(unsigned (&m)[2], const uint16_t *p)
 }
 
 // Sources and receiver samples that the E kernel serves itself: the entries
-// of plane k are list[plane[k]] .. list[plane[k + 1] - 1], sources in
-// insertion order, then samples.  A launch belongs to step *base + step.
+// of plane k are list[plane[k]] .. list[plane[k + 1] - 1] in order of their
+// offset, those of one place as they were added, sources before samples.  A
+// launch belongs to step *base + step.
 struct FdtdPoint {
     long long off;  // offset in the component's array
     int comp;       // component, + 4 for a receiver sample
@@ -367,11 +368,17 @@ __global__ void __launch_bounds__(256) fdtd_e_kernel(FdtdArgs<T> a, FdtdPoints p
     }
     if (pt.plane) {
         const int q1 = __ldg(pt.plane + k + 1);
-        for (int q = __ldg(pt.plane + k); q < q1; ++q) {
+        int q = __ldg(pt.plane + k);
+        for (int end = q1; end - q > 4;) {   // close to the first point at the thread's cells or behind them
+            const int mid = (q + end) >> 1;
+            if (pt.list[mid].off < (long long)o) q = mid + 1; else end = mid;
+        }
+        for (; q < q1; ++q) {
             const FdtdPoint r = pt.list[q];
             const long long at = r.off - (long long)o;
+            if (at >= V) break;
             const int comp = r.comp & 3;
-            if (at < 0 || at >= V || !(comp == 0 ? ex : comp == 1 ? ey : ez)) continue;
+            if (at < 0 || !(comp == 0 ? ex : comp == 1 ? ey : ez)) continue;
             const int step = pt.step + (pt.base ? *pt.base : 0);
             const bool sample = r.comp >= 4, keep = sample && step % pt.tf == 0;
             const T src = sample ? T(0) : (T)pt.vals[(size_t)(step - 1) * pt.ns + r.idx];
@@ -775,10 +782,14 @@ struct FdtdSim : Sim {
 
     // The sources and receiver samples as the E kernel's point lists; false
     // where the kernels after the E update have to serve them: a point in the
-    // padding that no thread of the E kernel updates, more than 64 points in
-    // one plane (every thread of the plane looks through them), or more than
-    // 256 MB of samples.
-    static constexpr int kMaxPlanePoints = 64;
+    // padding that no thread of the E kernel updates, more than 256 MB of
+    // samples, or in FP32 so many points in so many planes that the threads'
+    // search (each probe of a plane's list by each of its cells) takes longer
+    // than the two launches.  192^3 FP32, us a step, served by the E kernel and
+    // by the other two: 63 points in each plane (43 million probes) 94 and 93,
+    // 180 (55 million) 104 and 93, 180 in one plane 79 and 92.  In FP64, bound by
+    // the FP64 pipe, 180 in each plane 421 and 433.
+    static constexpr double kMaxProbes = 4e7;
     bool fold_points(int nsamp_run, FdtdPoints &pt)
     {
         struct Item {
@@ -799,17 +810,19 @@ struct FdtdSim : Sim {
             for (auto &q : obs_lists[l])
                 if (!add((int)(l % 3), q.data(), 4, nsm++)) return false;
         if ((double)nsm * nsamp_run * 8.0 > 256e6) return false;
-        std::stable_sort(items.begin(), items.end(), [](const Item &x, const Item &y) { return x.k < y.k; });
+        std::stable_sort(items.begin(), items.end(), [](const Item &x, const Item &y) { return x.k != y.k ? x.k < y.k : x.p.off < y.p.off; });
         std::vector<int> plane(nz + 2, 0);
         std::vector<FdtdPoint> list(std::max<size_t>(items.size(), 1));
         for (size_t q = 0; q < items.size(); ++q) {
             list[q] = items[q].p;
             ++plane[items[q].k + 1];
         }
+        double probes = 0.0;
         for (int k = 0; k <= nz; ++k) {
-            if (plane[k + 1] > kMaxPlanePoints) return false;
+            probes += std::log2(1.0 + plane[k + 1]) * (nx + 1.0) * (ny + 1.0);
             plane[k + 1] += plane[k];
         }
+        if (!fp64 && probes > kMaxProbes) return false;
         d_pt_plane.ensure(plane.size() * sizeof(int));
         d_pt_list.ensure(list.size() * sizeof(FdtdPoint));
         d_samp.ensure((size_t)std::max(nsm, 1) * nsamp_run * 8);

@@ -403,3 +403,39 @@ def test_timing_the_dominant_kernel_keeps_the_state(prec, pml):
     for k in out[0]:
         assert np.abs(out[0][k]).max() > 0
         np.testing.assert_array_equal(out[0][k], out[1][k], err_msg=k)
+
+
+@pytest.mark.parametrize("npts", [1, 4, 5, 8, 63, 300])
+def test_served_points_of_any_number_bitwise(npts):
+    """Sources and samples found by the E kernel in its plane's list: in FP64
+    against the oracle, in FP32 against the kernels behind the E update, which
+    serve a run as soon as one sample lies in the padding."""
+    g, h, steps = (33, 9, 4), 1e-3, 20
+    nx, ny, nz = g
+    dt = 0.9 * h / (2.998e8 * np.sqrt(3))
+    rng = np.random.default_rng(npts)
+
+    def points(n):
+        p = [(int(rng.integers(1, nx + 1)), int(rng.integers(1, ny + 1)), int(rng.integers(1, 3))) for _ in range(n)]
+        return p + [(1, 1, 2), (nx, ny, 2)] + p[:1]          # first and last cells of rows, a place twice
+
+    # (Ex, Ey and Ez indices that the E kernel updates all contain these)
+    srcs = [(q % 3, p, 1, 3e10, float(rng.uniform(-1, 1))) for q, p in enumerate(points(npts))]
+    obs = [([p], [p, p], [p]) for p in points(npts)]
+    tr_o, f_o = oracle.fdtd_run(nx, ny, nz, h, dt, EPS0, MU0, 1, steps, srcs, obs)
+    out = []
+    for prec, pad in ((ems.FP64, False), (ems.FP32, False), (ems.FP32, True)):
+        s = ems.FdtdSimulation(g, h, dt, EPS0, MU0, 1, precision=prec)
+        for c, at, kind, f, amp in srcs:
+            (s.setSource_x, s.setSource_y, s.setSource_z)[c](at, waveform=kind, f0=f, amplitude=amp)
+        for o in obs + ([([(0, 0, 0)], [(0, 0, 0)], [(0, 0, 0)])] if pad else []):
+            s.setObservationPoint(o)
+        s.run(steps)
+        out.append((s.traces()[:len(obs)], s.fields()))
+        s.close()
+    assert np.abs(tr_o).max() > 0
+    np.testing.assert_array_equal(out[0][0], tr_o)
+    np.testing.assert_array_equal(out[1][0], out[2][0])
+    for k in f_o:
+        np.testing.assert_array_equal(out[0][1][k], f_o[k], err_msg=k)
+        np.testing.assert_array_equal(out[1][1][k], out[2][1][k], err_msg=k)
