@@ -539,7 +539,9 @@ struct FdtdSim : Sim {
         V = (int)(16 / w);
         lead = V;
         auto up = [](size_t x, size_t m) { return (x + m - 1) / m * m; };
-        pitch = up(nx + 2 + lead, 32 / w);
+        // columns -1 .. nx, the first one at the end of the row before; whole
+        // 32-byte sectors, so that a thread's vectors never leave its row
+        pitch = up(nx + 2, 32 / w);
         plane = pitch * (ny + 2);
         total = plane * (nz + 2) + lead + V;   // one more vector behind the last row is read
         mpitch = up(nx + 1 + V, 4);

@@ -439,3 +439,53 @@ def test_served_points_of_any_number_bitwise(npts):
     for k in f_o:
         np.testing.assert_array_equal(out[0][1][k], f_o[k], err_msg=k)
         np.testing.assert_array_equal(out[1][1][k], out[2][1][k], err_msg=k)
+
+
+@pytest.mark.parametrize("points", ["inside", "padding"])
+@pytest.mark.parametrize("grid,pml", [((2, 3, 4), 0), ((6, 5, 4), 1), ((14, 6, 5), 2), ((62, 5, 5), 2)])
+def test_rows_that_fill_their_sectors_bitwise_equal_to_oracle(grid, pml, points):
+    """Grids whose nx + 2 columns are whole 32-byte sectors: a row ends where
+    the next one's first column, x = 0 of Ey and Ez, is kept."""
+    test_pitched_layout_and_served_points_bitwise_equal_to_oracle(grid, pml, points)
+
+
+@pytest.mark.parametrize("prec,bits", [(ems.FP32, np.float32), (ems.FP64, np.float64)], ids=["fp32", "fp64"])
+@pytest.mark.parametrize("nx", [1, 2, 3, 4, 5, 6, 7, 8, 14, 22, 31, 33])
+def test_uniform_steps_bitwise_equal_to_numpy(nx, prec, bits):
+    """Random fields, padding included, advanced by the update equations in numpy
+    arrays of the run's precision, operation by operation in their order."""
+    ny, nz, h, steps = 4, 3, 1e-3, 5
+    dt = 0.9 * h / (2.998e8 * np.sqrt(3))
+    rng = np.random.default_rng(nx)
+    keys = ("Ex", "Ey", "Ez", "Hx", "Hy", "Hz")
+    f = {k: rng.standard_normal(v).astype(bits) for k, v in oracle.fdtd_shapes(nx, ny, nz).items()}
+    s = ems.FdtdSimulation((nx, ny, nz), h, dt, EPS0, MU0, 1, precision=prec)
+    for q, k in enumerate(keys):
+        s.set_field(q, f[k].astype(np.float64))
+    s.run(steps)
+    ch, ce = bits(dt / MU0 / h), bits(dt / EPS0 / h)
+    Ex, Ey, Ez, Hx, Hy, Hz = (f[k] for k in keys)
+    X, Y, Z = nx, ny, nz
+    for _ in range(steps):
+        Hx -= ch * (((Ez[:, 1:, 1:X + 1] - Ez[:, :Y + 1, 1:X + 1]) - Ey[1:, :, 1:X + 1]) + Ey[:Z + 1, :, 1:X + 1])
+        Hy -= ch * (((Ex[1:, 1:Y + 1] - Ex[:Z + 1, 1:Y + 1]) - Ez[:, 1:Y + 1, 1:]) + Ez[:, 1:Y + 1, :X + 1])
+        Hz -= ch * (((Ey[1:Z + 1, :, 1:] - Ey[1:Z + 1, :, :X + 1]) - Ex[1:Z + 1, 1:]) + Ex[1:Z + 1, :Y + 1])
+        Ex[1:Z + 1, 1:Y + 1] += ce * (((Hz[:, 1:] - Hz[:, :Y]) - Hy[1:]) + Hy[:Z])
+        Ey[1:Z + 1, :, 1:X + 1] += ce * (((Hx[1:] - Hx[:Z]) - Hz[:, :, 1:]) + Hz[:, :, :X])
+        Ez[:, 1:Y + 1, 1:X + 1] += ce * (((Hy[:, :, 1:] - Hy[:, :, :X]) - Hx[:, 1:]) + Hx[:, :Y])
+    got = s.fields()
+    for k, v in zip(keys, (Ex, Ey, Ez, Hx, Hy, Hz)):
+        assert np.array_equal(got[k], v.astype(np.float64)), k
+
+
+@pytest.mark.parametrize("prec", [ems.FP64, ems.FP32], ids=["fp64", "fp32"])
+def test_thin_grids_hold_one_sector_a_row(prec):
+    """Grids one cell wide keep 32 bytes of each field and row, no more: large
+    two-dimensional grids fit the device."""
+    torch = pytest.importorskip("torch")
+    ny, nz = 1200, 1100
+    free = torch.cuda.mem_get_info()[0]
+    s = ems.FdtdSimulation((1, ny, nz), 1e-3, 1e-13, EPS0, MU0, 1, precision=prec)
+    used = free - torch.cuda.mem_get_info()[0]
+    s.close()
+    assert used <= 6 * 32 * (ny + 2) * (nz + 2) + (24 << 20)
