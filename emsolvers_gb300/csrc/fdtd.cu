@@ -784,8 +784,8 @@ struct FdtdSim : Sim {
 
     // The sources and receiver samples as the E kernel's point lists; false
     // where the kernels after the E update have to serve them: a point in the
-    // padding that no thread of the E kernel updates, more than 256 MB of
-    // samples, or in FP32 so many points in so many planes that the threads'
+    // padding that no thread of the E kernel updates, more samples than 256 MB
+    // or the free memory hold, or in FP32 so many points in so many planes that the threads'
     // search (each probe of a plane's list by each of its cells) takes longer
     // than the two launches.  192^3 FP32, us a step, served by the E kernel and
     // by the other two: 63 points in each plane (43 million probes) 94 and 93,
@@ -827,7 +827,12 @@ struct FdtdSim : Sim {
         if (!fp64 && probes > kMaxProbes) return false;
         d_pt_plane.ensure(plane.size() * sizeof(int));
         d_pt_list.ensure(list.size() * sizeof(FdtdPoint));
-        d_samp.ensure((size_t)std::max(nsm, 1) * nsamp_run * 8);
+        try {
+            d_samp.ensure((size_t)std::max(nsm, 1) * nsamp_run * 8);
+        } catch (const Error &e) {   // a grid that leaves no memory for them
+            if (e.code != EMS_ERR_OUT_OF_MEMORY) throw;
+            return false;
+        }
         EMS_CUDA(cudaMemcpyAsync(d_pt_plane.p, plane.data(), plane.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
         EMS_CUDA(cudaMemcpyAsync(d_pt_list.p, list.data(), list.size() * sizeof(FdtdPoint), cudaMemcpyHostToDevice, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));   // the host vectors end here

@@ -489,3 +489,26 @@ def test_thin_grids_hold_one_sector_a_row(prec):
     used = free - torch.cuda.mem_get_info()[0]
     s.close()
     assert used <= 6 * 32 * (ny + 2) * (nz + 2) + (24 << 20)
+
+
+def test_no_room_for_the_samples():
+    """200 MB of samples with 150 MB left on the device: the run is served by
+    the kernels behind the E update and gives the same traces."""
+    torch = pytest.importorskip("torch")
+    g, h = (24, 20, 16), 1e-3
+    dt = 0.9 * h / (2.998e8 * np.sqrt(3))
+    pts = [(i, j, k) for k in range(1, 8) for j in range(1, 20) for i in range(1, 20)]
+    out = []
+    for full in (False, True):
+        s = ems.FdtdSimulation(g, h, dt, EPS0, MU0, 1, precision=ems.FP64)
+        s.setSource_z((12, 10, 8), waveform=ems.WAVE_RICKER, f0=2e10)
+        s.setObservationPoint((pts, [], []))
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (150 << 20), dtype=torch.uint8, device="cuda") if full else None
+        s.run(10000)
+        out.append((s.traces()[..., 0], s.fields()["Ez"]))
+        del hog
+        torch.cuda.empty_cache()
+        s.close()
+    assert len(pts) * 10000 * 8 > 200e6 and np.abs(out[0][0]).max() > 0
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
