@@ -91,6 +91,23 @@ struct Sim {
     // pageable copy may still be on its way when that returns, and a copy
     // between device arrays has not even begun.)
     void copy_in(void *dev, const void *host, size_t bytes) const;
+    // The graph of what f enqueues on the handle's stream.  The capture ends on
+    // every path: a stream left capturing would fail all later calls.
+    template <class F> cudaGraph_t capture(F &&f)
+    {
+        cudaGraph_t g = nullptr;
+        EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+        try {
+            f();
+        } catch (...) {
+            cudaStreamEndCapture(stream, &g);
+            if (g) cudaGraphDestroy(g);
+            cudaGetLastError();
+            throw;
+        }
+        EMS_CUDA(cudaStreamEndCapture(stream, &g));
+        return g;
+    }
     // cnt device values into a host array.  Its pages are touched first: the
     // copy engine faults fresh pages in one by one (six FP64 fields of
     // 160x150x140 cells into fresh arrays: 137 ms, 7 so).

@@ -863,14 +863,13 @@ struct FdtdSim : Sim {
             graph = nullptr;
         }
         pt.base = d_step.as<int>();
-        cudaGraph_t g = nullptr;
-        EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int r = 0; r < kGraphSteps; ++r) {
-            launch_h<T>(a, 0, nz + 1, r == 0 ? d_step.as<int>() : nullptr, kGraphSteps);
-            pt.step = r + 1;
-            launch_e<T>(a, 0, nz + 1, pt);
-        }
-        EMS_CUDA(cudaStreamEndCapture(stream, &g));
+        const cudaGraph_t g = capture([&] {
+            for (int r = 0; r < kGraphSteps; ++r) {
+                launch_h<T>(a, 0, nz + 1, r == 0 ? d_step.as<int>() : nullptr, kGraphSteps);
+                pt.step = r + 1;
+                launch_e<T>(a, 0, nz + 1, pt);
+            }
+        });
         const cudaError_t e = cudaGraphInstantiate(&graph, g, 0);
         cudaGraphDestroy(g);
         EMS_CUDA(e);

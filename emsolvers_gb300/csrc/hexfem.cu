@@ -916,10 +916,9 @@ struct HexFemSim : Sim {
                         cudaGraphExecDestroy(graph);
                         graph = nullptr;
                     }
-                    cudaGraph_t gr = nullptr;
-                    EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-                    for (int r = 0; r < kGraphSteps; ++r) graph_launches = enqueue_step<T, O>();   // the ring ends where it began
-                    EMS_CUDA(cudaStreamEndCapture(stream, &gr));
+                    const cudaGraph_t gr = capture([&] {   // the ring ends where it began
+                        for (int r = 0; r < kGraphSteps; ++r) graph_launches = enqueue_step<T, O>();
+                    });
                     const cudaError_t e = cudaGraphInstantiate(&graph, gr, 0);
                     cudaGraphDestroy(gr);
                     EMS_CUDA(e);

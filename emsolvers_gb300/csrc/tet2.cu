@@ -2051,17 +2051,15 @@ struct Tet2Sim : Sim {
         g.Yt = d_YtM.p;
         g.c1 = T(0.5); g.c2 = T(0.1);
         T *buf[2] = {d_x.as<T>(), cheb_form != FORM_TWOPASS ? d_xs.as<T>() : d_x.as<T>()};
-        cudaGraph_t gr = nullptr;
         cudaGraphExec_t ex = nullptr;
-        EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (int k = 0; k < n; ++k) {
-            g.xin = buf[k & 1];
-            g.x = buf[(k + 1) & 1];
-            launch_iteration<T, FIN_NONE>(g);
-        }
-        cudaError_t ce = cudaStreamEndCapture(stream, &gr);
-        if (ce != cudaSuccess) throw Error{EMS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce)};
-        ce = cudaGraphInstantiate(&ex, gr, 0);
+        const cudaGraph_t gr = capture([&] {
+            for (int k = 0; k < n; ++k) {
+                g.xin = buf[k & 1];
+                g.x = buf[(k + 1) & 1];
+                launch_iteration<T, FIN_NONE>(g);
+            }
+        });
+        cudaError_t ce = cudaGraphInstantiate(&ex, gr, 0);
         if (ce != cudaSuccess) {
             cudaGraphDestroy(gr);
             throw Error{EMS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce)};
@@ -2429,10 +2427,8 @@ struct Tet2Sim : Sim {
                     if (g) cudaGraphDestroy(g);
                 }
             } G;
-            EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-            const int per = enqueue_step<T>();
-            cudaError_t ce = cudaStreamEndCapture(stream, &G.g);
-            if (ce != cudaSuccess) throw Error{EMS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce)};
+            int per = 0;
+            G.g = capture([&] { per = enqueue_step<T>(); });
             EMS_CUDA(cudaGraphInstantiate(&G.exec, G.g, 0));
             const bool record = ckpt_nsnap > 0 && symp() && cur_time == 0.0 && fresh;
             const int seg = record ? (nsteps + ckpt_nsnap - 1) / ckpt_nsnap : nsteps;

@@ -2488,11 +2488,10 @@ struct TetFemSim : Sim {
         if (!w.exec || w.block != step_block || !std::equal(reads, reads + 3, w.reads)) {
             w.drop_graph();
             EMS_CUDA(cudaStreamSynchronize(stream));
-            EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-            for (int q = 0; q < 3; ++q) iteration(0, w.jbuf.as<int>());
-            cudaError_t ce = cudaStreamEndCapture(stream, &w.g);
-            if (ce != cudaSuccess) throw Error{EMS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce)};
-            ce = cudaGraphInstantiate(&w.exec, w.g, 0);
+            w.g = capture([&] {
+                for (int q = 0; q < 3; ++q) iteration(0, w.jbuf.as<int>());
+            });
+            const cudaError_t ce = cudaGraphInstantiate(&w.exec, w.g, 0);
             if (ce != cudaSuccess) {
                 w.exec = nullptr;
                 throw Error{EMS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce)};
@@ -2997,19 +2996,8 @@ struct TetFemSim : Sim {
             G.par = par0;
             int nl = 0;
             EMS_CUDA(cudaStreamSynchronize(stream));
-            EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-            try {
-                nl += enqueue_steps<T>(kGraphSteps, u, p, o, sc, sa, par0, cm);
-            } catch (...) {   // end the capture before the error leaves
-                cudaGraph_t g = nullptr;
-                cudaStreamEndCapture(stream, &g);
-                if (g) cudaGraphDestroy(g);
-                cudaGetLastError();
-                throw;
-            }
-            cudaError_t ce = cudaStreamEndCapture(stream, &G.g);
-            if (ce != cudaSuccess) throw Error{EMS_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(ce)};
-            ce = cudaGraphInstantiate(&G.exec, G.g, 0);
+            G.g = this->capture([&] { nl += enqueue_steps<T>(kGraphSteps, u, p, o, sc, sa, par0, cm); });
+            const cudaError_t ce = cudaGraphInstantiate(&G.exec, G.g, 0);
             if (ce != cudaSuccess) throw Error{EMS_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce)};
             G.launches = nl;
         };
@@ -3499,12 +3487,10 @@ struct TetFemSim : Sim {
         const Schedule sc = schedule();
         const bool pers = persist && can_persist(sc.symp);
         const int per_graph = pers ? kLaunches * sc.nsub : kLaunches;   // substeps of one replay
-        cudaGraph_t g = nullptr;
         cudaGraphExec_t exec = nullptr;
         if (pers) EMS_CUDA(cudaMemsetAsync(d_bar.p, 0, 8, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
-        EMS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        try {
+        const cudaGraph_t g = capture([&] {
             if (pers) {
                 auto body = [&](auto tag) {
                     using T = decltype(tag);
@@ -3515,15 +3501,8 @@ struct TetFemSim : Sim {
             } else {
                 for (int r = 0; r < kLaunches; ++r) idle_step(nbv, r % 2);
             }
-        } catch (...) {
-            cudaGraph_t gg = nullptr;
-            cudaStreamEndCapture(stream, &gg);
-            if (gg) cudaGraphDestroy(gg);
-            cudaGetLastError();
-            throw;
-        }
-        cudaError_t ce = cudaStreamEndCapture(stream, &g);
-        if (ce == cudaSuccess) ce = cudaGraphInstantiate(&exec, g, 0);
+        });
+        cudaError_t ce = cudaGraphInstantiate(&exec, g, 0);
         const int reps = std::max(1, launches / per_graph);
         if (ce == cudaSuccess) ce = cudaGraphLaunch(exec, stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(ev0, stream);
@@ -3533,7 +3512,7 @@ struct TetFemSim : Sim {
         float t = 0;
         if (ce == cudaSuccess) ce = cudaEventElapsedTime(&t, ev0, ev1);
         if (exec) cudaGraphExecDestroy(exec);
-        if (g) cudaGraphDestroy(g);
+        cudaGraphDestroy(g);
         if (ce != cudaSuccess) throw Error{EMS_ERR_CUDA, std::string("dominant-kernel timing: ") + cudaGetErrorString(ce)};
         if (pers) {
             int err = 0;

@@ -42,3 +42,11 @@ def test_kernels_launched_ahead_wait_and_promise_nothing(path):
     for name, (params, body) in kernels.items():
         if "wait_for_last()" in body:
             assert "__restrict__" not in params, name
+
+
+def test_captures_end_on_every_path():
+    """Only Sim::capture begins a stream capture: it ends it also when a launch
+    inside fails, which would leave the handle's stream capturing."""
+    for path in glob.glob(os.path.join(CSRC, "*")):
+        text = open(path).read()
+        assert text.count("cudaStreamBeginCapture(") == (1 if path.endswith("ems_internal.hpp") else 0), path
