@@ -2088,12 +2088,17 @@ struct Tet2Sim : Sim {
     template <class T> void choose_iteration()
     {
         cheb_form = FORM_TWOPASS;
-        if (sizeof(T) == 8) return;
-        build_tiles();
         static const char *names[3] = {"twopass", "fused", "march"};
-        if (const char *force = std::getenv("EMS_TET2_ITERATION"))
-            for (int f = FORM_FUSED; f <= FORM_MARCH; ++f)
+        const char *force = std::getenv("EMS_TET2_ITERATION");
+        const int first = sizeof(T) == 8 ? FORM_TWOPASS : FORM_FUSED, last = sizeof(T) == 8 ? FORM_TWOPASS : FORM_MARCH;
+        if (sizeof(T) == 4) build_tiles();
+        if (force) {
+            for (int f = first; f <= last; ++f)
                 if (!std::strcmp(force, names[f])) { cheb_form = f; return; }
+            std::fprintf(stderr, "ems: EMS_TET2_ITERATION=%s is no form of the %s iteration and is ignored\n", force,
+                         sizeof(T) == 8 ? "FP64" : "FP32");
+        }
+        if (sizeof(T) == 8) return;
         d_x.zero(stream); d_xs.zero(stream); d_d.zero(stream); d_b.zero(stream);
         int best = FORM_FUSED;
         for (int f = FORM_FUSED; f <= FORM_MARCH; ++f) {

@@ -386,3 +386,24 @@ def test_asking_for_the_limit_between_runs_keeps_the_state(integ, prec):
     for a, b in zip(*out):
         assert np.array_equal(a, b)
     assert np.linalg.norm(out[0][0]) > 0
+
+
+@pytest.mark.parametrize("prec,forms", [("FP32", ("fused", "march")), ("FP64", ("twopass",))])
+def test_forms_that_a_precision_does_not_have_are_reported(prec, forms):
+    """EMS_TET2_ITERATION names a form of the iteration; a name that the run's
+    precision has no form for changes nothing and is said to be ignored."""
+    import os
+    import subprocess
+    import sys
+    code = ("import emsolvers_gb300 as ems\n"
+            f"s = ems.TetFemSimulation((3, 2, 4), {H!r}, 2, ems.SYMP2, ems.{prec}, dt=0.02 * {TS!r})\n"
+            "s.run(1)\n"
+            "print(s.time_dominant_kernel(2)[2])\n")
+    kernel = {"twopass": "t2_mass_elem_kernel", "fused": "t2_cheb_kernel", "march": "t2_march_kernel"}
+    for name in ("twopass", "fused", "march", "other"):
+        r = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, EMS_TET2_ITERATION=name), capture_output=True, text=True,
+                           timeout=300, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+        assert r.returncode == 0, r.stderr
+        assert (name in forms) == (f"EMS_TET2_ITERATION={name} is no form of the {prec} iteration" not in r.stderr)
+        if name in forms:
+            assert kernel[name] in r.stdout
