@@ -748,7 +748,9 @@ __host__ __device__ constexpr int step_record_x(int sy, int mask) { return sy | 
 // meshes (a 32^3 mesh has 36k nodes) spread better over the 152 SMs in
 // small blocks.  The block size changes no arithmetic.
 // FP32 symplectic steps keep to 64 registers, four warps a scheduler at every
-// block size: 80 took the ten-shot batch of 295k nodes from 15.9 to 17.5 us.
+// block size.  us a launch, 64 registers and the 107 it takes unheld: 69k nodes
+// 6.1 and 5.8, 104k 7.4 and 9.6, 298k (ten shots) 14.9 and 19.3, 705k 46.3 and
+// 68.6, 1.88M (sixteen shots) 112.4 and 172.
 constexpr int kStepBlocks[4] = {32, 64, 128, 256};
 constexpr int kStepBlockMax = 256;
 
@@ -2085,6 +2087,10 @@ struct TetFemSim : Sim {
         EMS_CHECK_ARG(nslot < (size_t)1 << 31, "mesh too large for 32-bit slot indices");
         build_mesh();
         slot_split = nnode <= (fp64 ? kSlotMaxNodes64 : kSlotMaxNodes32);
+        // us a launch, node kernel in blocks of 32, 64, 128 and 256 threads: FP32 104k
+        // nodes 7.6 7.7 7.6 7.4, 185k 11.5 11.4 11.2 11.7, 314k 15.5 15.3 15.2 15.5, 1.86M
+        // 112.6 112.9 113.6 115.6; FP64 16k 10.6 10.8 11.3 17.2, 118k 52.0 53.0 53.3 60.0,
+        // 705k 277 in each but the last
         step_block = fp64 ? 32 : 128;
         eps_h.assign(ntet, 1.0);
         init_stream();
