@@ -1999,12 +1999,12 @@ struct TetFemSim : Sim {
     int step_block = 64;            // threads per block of tet_step_kernel (tune_launch_shape)
     bool slot_split = true;         // symplectic lossless steps by tet_slot_kernel (tune_launch_shape)
     // Until a run tunes the shape (recorded runs do not): in FP32 the
-    // slot-split kernel on meshes of up to 80,000 nodes (us a launch, slot-split
-    // against node kernel: 36k nodes 4.5 and 6.9, 69k 7.0 and 7.9, 98k 8.9 and 8.5,
-    // 118k 10.4 and 7.6), in FP64 of up to 12,000 nodes (9k 7.6 and 11.6, 16k 12.5 and
-    // 11.8, 49k 29.0 and 23.5): the node kernel forms every curl once, and the FP64
-    // pipe is soon full.
-    static constexpr size_t kSlotMaxNodes32 = 80000, kSlotMaxNodes64 = 12000;
+    // slot-split kernel on meshes of up to 50,000 nodes (us a launch, slot-split
+    // against node kernel: 36k nodes 4.5 and 5.6, 43k 5.0 and 6.0, 51k 6.3 and 6.2,
+    // 59k 6.8 and 6.2, 69k 7.2 and 6.3), in FP64 of up to 13,000 nodes (9k 7.0 and 10.0,
+    // 12k 9.7 and 10.0, 16k 12.0 and 10.4): the node kernel forms every curl once, and
+    // the FP64 pipe is soon full.
+    static constexpr size_t kSlotMaxNodes32 = 50000, kSlotMaxNodes64 = 13000;
     bool step_tuned = false;        // the block size depends on the mesh only: tuned once per handle
     // the persistent step (tet_persist_kernel, a tuner candidate): its grid
     // barrier's counter and error word, the resident-block capacity of its
