@@ -952,41 +952,41 @@ struct FdtdSim : Sim {
         EMS_CUDA(cudaEventRecord(ev0, stream));
         int step = 1;
         const auto direct = [&](int last) {   // steps up to `last`, launch by launch
-        for (; step <= last; ++step) {
-            const int ts = step - 1, c = ts / kTuneSteps, r = ts % kTuneSteps;
-            if (ts < tune) {
-                blk = dim3(kShape[c][0], kShape[c][1], 1);
-                if (r == 1) EMS_CUDA(cudaEventRecord(tev.e[2 * c], stream));
-            }
-            launch_h<T>(a, 0, nz + 1);
-            pt.step = step;
-            launch_e<T>(a, 0, nz + 1, folded ? pt : none);
-            launches += 2;
-            if (ns > 0 && !folded) {
-                fdtd_source_kernel<T><<<1, 32, 0, stream>>>(a.Ex, a.Ey, a.Ez, d_src_comp.as<int>(), d_src_off.as<long long>(),
-                                                           d_src_vals.as<double>() + (size_t)(step - 1) * ns, ns);
-                ++launches;
-            }
-            if (nobs > 0 && !folded && step % tf == 0) {
-                fdtd_receiver_kernel<T><<<(nobs + 127) / 128, 128, 0, stream>>>(
-                    a.Ex, a.Ey, a.Ez, nobs, d_obs_cnt.as<int>(), d_obs_start.as<int>(), d_obs_off.as<long long>(),
-                    d_traces.as<double>() + (size_t)(step / tf) * 3, nsamp);
-                ++launches;
-            }
-            if (ts < tune && r == kTuneSteps - 1) EMS_CUDA(cudaEventRecord(tev.e[2 * c + 1], stream));
-            if (tune && step == tune) {   // all shapes timed: keep the fastest
-                EMS_CUDA(cudaEventSynchronize(tev.e[2 * kShapes - 1]));
-                float best = 0.0f;
-                int pick = 0;
-                for (int k = 0; k < kShapes; ++k) {
-                    float ms = 0.0f;
-                    EMS_CUDA(cudaEventElapsedTime(&ms, tev.e[2 * k], tev.e[2 * k + 1]));
-                    if (k == 0 || ms < best) { best = ms; pick = k; }
+            for (; step <= last; ++step) {
+                const int ts = step - 1, c = ts / kTuneSteps, r = ts % kTuneSteps;
+                if (ts < tune) {
+                    blk = dim3(kShape[c][0], kShape[c][1], 1);
+                    if (r == 1) EMS_CUDA(cudaEventRecord(tev.e[2 * c], stream));
                 }
-                blk = dim3(kShape[pick][0], kShape[pick][1], 1);
-                tuned = true;
+                launch_h<T>(a, 0, nz + 1);
+                pt.step = step;
+                launch_e<T>(a, 0, nz + 1, folded ? pt : none);
+                launches += 2;
+                if (ns > 0 && !folded) {
+                    fdtd_source_kernel<T><<<1, 32, 0, stream>>>(a.Ex, a.Ey, a.Ez, d_src_comp.as<int>(), d_src_off.as<long long>(),
+                                                               d_src_vals.as<double>() + (size_t)(step - 1) * ns, ns);
+                    ++launches;
+                }
+                if (nobs > 0 && !folded && step % tf == 0) {
+                    fdtd_receiver_kernel<T><<<(nobs + 127) / 128, 128, 0, stream>>>(
+                        a.Ex, a.Ey, a.Ez, nobs, d_obs_cnt.as<int>(), d_obs_start.as<int>(), d_obs_off.as<long long>(),
+                        d_traces.as<double>() + (size_t)(step / tf) * 3, nsamp);
+                    ++launches;
+                }
+                if (ts < tune && r == kTuneSteps - 1) EMS_CUDA(cudaEventRecord(tev.e[2 * c + 1], stream));
+                if (tune && step == tune) {   // all shapes timed: keep the fastest
+                    EMS_CUDA(cudaEventSynchronize(tev.e[2 * kShapes - 1]));
+                    float best = 0.0f;
+                    int pick = 0;
+                    for (int k = 0; k < kShapes; ++k) {
+                        float ms = 0.0f;
+                        EMS_CUDA(cudaEventElapsedTime(&ms, tev.e[2 * k], tev.e[2 * k + 1]));
+                        if (k == 0 || ms < best) { best = ms; pick = k; }
+                    }
+                    blk = dim3(kShape[pick][0], kShape[pick][1], 1);
+                    tuned = true;
+                }
             }
-        }
         };
         if (!folded) {
             direct(nsteps);

@@ -275,7 +275,8 @@ __global__ void hex_drift_kernel(const __grid_constant__ HexGeom g, T *Ux, T *Uy
 // Receivers: fem_v2/fem_simulation.cpp:1273-1312 (one thread per receiver),
 // row s of the table.
 template <class T>
-__device__ __forceinline__ void hex_sample(const HexGeom &g, const T *Lx, const T *Ly, const T *Lz, int o, const int *obs, double *tr, int nsamp, int s)
+__device__ __forceinline__ void hex_sample(const HexGeom &g, const T *Lx, const T *Ly, const T *Lz, int o, const int *obs, double *tr,
+                                           int nsamp, int s)
 {
     const int gx = g.gx, gy = g.gy;
     int ox = obs[3 * o], oy = obs[3 * o + 1], oz = obs[3 * o + 2];
@@ -335,8 +336,8 @@ template <class T, int O> struct HexRows {
 template <class T, int O> struct HexK { const T *k; };   // K of the element pass, [3][TT][RP]
 template <int O> struct HexK<float, O> { float k[3 * HexRows<float, O>::TT * HexRows<float, O>::RP]; };
 template <class T, int O, bool EXACT>
-__global__ void __launch_bounds__(128) hex_elem_kernel(const __grid_constant__ HexGeom g, const __grid_constant__ HexK<T, O> K, const T *Ux, const T *Uy,
-                                                       const T *Uz, T *fe, int *step, HexRec rec)
+__global__ void __launch_bounds__(128) hex_elem_kernel(const __grid_constant__ HexGeom g, const __grid_constant__ HexK<T, O> K,
+                                                       const T *Ux, const T *Uy, const T *Uz, T *fe, int *step, HexRec rec)
 {
     constexpr int D = HexRows<T, O>::D, TT = HexRows<T, O>::TT, W = HexRows<T, O>::W, RP = HexRows<T, O>::RP;
     constexpr bool ARG = sizeof(T) == 4;
@@ -755,7 +756,7 @@ struct HexFemSim : Sim {
     {
         size_t mx = std::max(g.nc[0], std::max(g.nc[1], g.nc[2]));
         dim3 grid((unsigned)((mx + 127) / 128), 3);
-        auto k = exact ? hex_leapfrog_kernel<T, O, true> : hex_leapfrog_kernel<T, O, false>;
+        auto k = hex_leapfrog_kernel<T, O, sizeof(T) == 8>;
         k<<<grid, 128, 0, stream>>>(g, matrix_rows<T>(), L<T>(0, l1), L<T>(1, l1), L<T>(2, l1), L<T>(0, l0), L<T>(1, l0), L<T>(2, l0),
                                     L<T>(0, l2), L<T>(1, l2), L<T>(2, l2), s);
     }
@@ -763,7 +764,7 @@ struct HexFemSim : Sim {
     {
         size_t mx = std::max(g.nc[0], std::max(g.nc[1], g.nc[2]));
         dim3 grid((unsigned)((mx + 127) / 128), 3);
-        auto k = exact ? hex_kick_kernel<T, O, true> : hex_kick_kernel<T, O, false>;
+        auto k = hex_kick_kernel<T, O, sizeof(T) == 8>;
         k<<<grid, 128, 0, stream>>>(g, matrix_rows<T>(), L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), L<T>(0, 1), L<T>(1, 1), L<T>(2, 1),
                                     L<T>(0, 2), L<T>(1, 2), L<T>(2, 2), dt, s);
     }
@@ -774,7 +775,8 @@ struct HexFemSim : Sim {
         const bool mul = g.o < 3;
         const T m = mul ? (T)(g.o * g.o * g.o / 8.0) : (T)(8.0 / g.o / g.o / g.o);
         auto k = mul ? hex_drift_kernel<T, sizeof(T) == 8, true> : hex_drift_kernel<T, sizeof(T) == 8, false>;
-        launch_after(k, grid, dim3(256), 0, stream, g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), L<T>(0, 1), L<T>(1, 1), L<T>(2, 1), coef, m, pec);
+        launch_after(k, grid, dim3(256), 0, stream, g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), L<T>(0, 1), L<T>(1, 1), L<T>(2, 1),
+                     coef, m, pec);
     }
 
     SrcList sources(double val) const
@@ -828,14 +830,15 @@ struct HexFemSim : Sim {
         int *step = first ? d_step.as<int>() : nullptr;
         if constexpr (X && O == 1)
             if (classes && ne >= kHex1MinElements) {
-                launch_after(hex1_elem_kernel, dim3((ne + 31) / 32 + (rec.n + 31) / 32), dim3(32), 0, stream, g, cls, u[0], u[1], u[2], d_fe.as<T>(), step, rec);
+                launch_after(hex1_elem_kernel, dim3((ne + 31) / 32 + (rec.n + 31) / 32), dim3(32), 0, stream, g, cls, u[0],
+                             u[1], u[2], d_fe.as<T>(), step, rec);
                 return;
             }
         HexK<T, O> kk{};
         if constexpr (sizeof(T) == 4) std::copy(k32.begin(), k32.end(), kk.k);
         else kk.k = dK.as<T>();
-        launch_after(hex_elem_kernel<T, O, X>, dim3((ne + 127) / 128 + (rec.n + 127) / 128, 3), dim3(128), 0, stream, g, kk, u[0], u[1], u[2],
-                                                                                                    d_fe.as<T>(), step, rec);
+        launch_after(hex_elem_kernel<T, O, X>, dim3((ne + 127) / 128 + (rec.n + 127) / 128, 3), dim3(128), 0, stream, g, kk,
+                     u[0], u[1], u[2], d_fe.as<T>(), step, rec);
     }
     // One step of orders 1 and 2 in two passes per force; launches made.
     template <class T, int O> int enqueue_step()
@@ -843,8 +846,8 @@ struct HexFemSim : Sim {
         int n = 0;
         const bool leap = P.integrator == EMS_LEAPFROG;
         if (nobs > 0 && !leap) {   // the symplectic steps sample U before the step
-            launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, 0), L<T>(1, 0), L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(),
-                                                                      nsamp, 0, d_step.as<int>(), P.time_frequency);
+            launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, 0), L<T>(1, 0),
+                         L<T>(2, 0), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, 0, d_step.as<int>(), P.time_frequency);
             ++n;
         }
         SrcTab src{};
@@ -876,7 +879,8 @@ struct HexFemSim : Sim {
             src.q = q;
             src.last = last;
             const T h1 = X || last ? (T)(0.5 * sub[q]) : (T)(0.5 * sub[q] + 0.5 * sub[q + 1]), h2 = X && !last ? (T)(0.5 * sub[q + 1]) : T(0);
-            launch_after(hex_kick_dof_kernel<T, O, X>, dof_grid(), dim3(128), 0, stream, g, d_fe.as<T>(), d, src, (T)sub[q], h1, h2, (T)(g.o * g.o * g.o / 8.0));
+            launch_after(hex_kick_dof_kernel<T, O, X>, dof_grid(), dim3(128), 0, stream, g, d_fe.as<T>(), d, src, (T)sub[q], h1,
+                         h2, (T)(g.o * g.o * g.o / 8.0));
         }
         return n + 1 + 2 * ns;
     }
@@ -940,8 +944,8 @@ struct HexFemSim : Sim {
     // Receivers from `level` into row s of the table.
     template <class T> void sample_level(int level, int s)
     {
-        launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, level), L<T>(1, level), L<T>(2, level),
-                     nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, s, nullptr, 1);
+        launch_after(hex_sample_kernel<T>, dim3((nobs + 63) / 64), dim3(64), 0, stream, g, L<T>(0, level), L<T>(1, level),
+                     L<T>(2, level), nobs, d_obs.as<int>(), d_tr.as<double>(), nsamp, s, nullptr, 1);
     }
     // The run with the force DOF by DOF, launch by launch.
     template <class T, int O> long long run_one_pass(int nsteps, std::vector<double> &times)

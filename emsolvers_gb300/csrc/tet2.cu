@@ -498,8 +498,8 @@ constexpr MassTab kMass = make_mass_tab();
 __constant__ double c2_H64[2][100];
 
 // Row A of M x in FP32.  The entries are immediate operands: read from
-// constant memory they took registers and spilled in the marching kernel
-// (50 us an iteration on 48^3 cubes against 39.5, with the halved mass).
+// constant memory they took registers and spilled in the marching kernel (a
+// quarter more time an iteration on 48^3 cubes).
 template <int A, int... B> __device__ __forceinline__ float mass_row(std::integer_sequence<int, B...>, const float (&x)[20])
 {
     float r = 0.0f;
@@ -909,9 +909,9 @@ __device__ __forceinline__ void stiff_curls(std::integer_sequence<int, A...>, co
 }
 // (double)x by integer operations: GB300 converts at its FP64 rate, two lanes
 // per SM and clock, and half of the pass's FP64 work was conversions.  For
-// infinities and NaN rare is set and the caller converts again (denormals fill
-// the fringe of every growing field, so they belong to this path).  (A conversion behind a predicate per value took
-// the pipe's time all the same.)
+// infinities and NaN rare is set and the caller converts again; a conversion
+// behind a predicate per value took the pipe's time all the same.  Denormals
+// fill the fringe of every growing field, so they belong to this path.
 template <bool CONVERT> __device__ __forceinline__ double widen(float x, bool &rare)
 {
     if constexpr (CONVERT) {
@@ -1377,8 +1377,8 @@ __device__ __forceinline__ void march_copies(std::integer_sequence<int, S...>, A
 // instructions per clock, 24 warps per SM) and the two barriers per layer.
 // Per iteration on GB300, against the better of the two forms before it
 // (element pass and entity pass through a per-tetrahedron array; one thread
-// per edge or face): 48^3 cubes 44.7 us against 67, five shots of 12..40
-// cubes 63 against 100, thirteen shots of 22..40 cubes 227 against 345.
+// per edge or face): 48^3 cubes 40.4 us against 67, five shots of 12..40
+// cubes 57.5 against 100, thirteen shots of 22..40 cubes 206 against 345.
 template <class T, int FIN, int COLS, int NC>
 __global__ void __launch_bounds__(6 * COLS, 1) t2_march_kernel(const T2Tile *tiles, const int *tables, MArgs<T> g)
 {
@@ -1879,9 +1879,11 @@ struct Tet2Sim : Sim {
     template <class T> void enqueue_stiff(const T *u)
     {
         if constexpr (std::is_same<T, float>::value)
-            launch_after(t2_stiff_df_kernel, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(), (int)shots.size(), u, d_YtK.as<double>());
+            launch_after(t2_stiff_df_kernel, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(),
+                         (int)shots.size(), u, d_YtK.as<double>());
         else
-            launch_after(t2_stiff_elem_kernel, dim3(blocks(ntet, 64)), dim3(64), 0, stream, ntet, d_shots.as<T2Shot>(), (int)shots.size(), u, d_YtK.as<double>());
+            launch_after(t2_stiff_elem_kernel, dim3(blocks(ntet, 64)), dim3(64), 0, stream, ntet, d_shots.as<T2Shot>(),
+                         (int)shots.size(), u, d_YtK.as<double>());
     }
 
     // f = K u (element pass + entity pass), u and out device vectors
@@ -1891,8 +1893,8 @@ struct Tet2Sim : Sim {
         GArgs<T> g = gargs<T>();
         g.Yt = d_YtK.p;
         g.out = out;
-        launch_after(t2_gather_kernel<T, double, G_FORCE, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(),
-                                                                                             (int)shots.size(), g);
+        launch_after(t2_gather_kernel<T, double, G_FORCE, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent,
+                     d_shots.as<T2Shot>(), (int)shots.size(), g);
         return 2;
     }
 
@@ -1998,14 +2000,18 @@ struct Tet2Sim : Sim {
         if constexpr (sizeof(T) == 4) {
             if (cheb_form == FORM_MARCH) {
                 const MArgs<T> a{g.xin, g.b, g.pinv, g.eps, g.x, g.d, g.U, g.Uold, g.c1, g.c2, g.h, nent};
-                launch_after(t2_march_kernel<T, FIN, kCols, kStage>, dim3(ntiles), dim3(6 * kCols), kMarchSmem, stream, d_tiles.as<T2Tile>(), d_tables.as<int>(), a);
+                launch_after(t2_march_kernel<T, FIN, kCols, kStage>, dim3(ntiles), dim3(6 * kCols), kMarchSmem, stream,
+                             d_tiles.as<T2Tile>(), d_tables.as<int>(), a);
             } else {
-                launch_after(t2_cheb_kernel<T, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
+                launch_after(t2_cheb_kernel<T, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(),
+                             ns, g);
             }
             return 1;
         } else {
-            launch_after(t2_mass_elem_kernel, dim3(blocks(ntet, 64)), dim3(64), 0, stream, ntet, d_shots.as<T2Shot>(), ns, d_eps.as<T>(), g.xin, d_YtM.as<T>());
-            launch_after(t2_gather_kernel<T, T, G_CHEB, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
+            launch_after(t2_mass_elem_kernel, dim3(blocks(ntet, 64)), dim3(64), 0, stream, ntet, d_shots.as<T2Shot>(), ns,
+                         d_eps.as<T>(), g.xin, d_YtM.as<T>());
+            launch_after(t2_gather_kernel<T, T, G_CHEB, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent,
+                         d_shots.as<T2Shot>(), ns, g);
             return 2;
         }
     }
@@ -2025,10 +2031,12 @@ struct Tet2Sim : Sim {
         int cur = fused ? (mass_iters - 1) % 2 : 0;   // buffer of the first iterate
         g.x = buf[cur];
         if (mass_iters == 1) {
-            launch_after(t2_gather_kernel<T, T, G_CHEB0, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
+            launch_after(t2_gather_kernel<T, T, G_CHEB0, FIN>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent,
+                         d_shots.as<T2Shot>(), ns, g);
             return 1;
         }
-        launch_after(t2_gather_kernel<T, T, G_CHEB0, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
+        launch_after(t2_gather_kernel<T, T, G_CHEB0, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent,
+                     d_shots.as<T2Shot>(), ns, g);
         int nl = 1;
         for (int k = 1; k < mass_iters; ++k) {
             g.xin = buf[cur];
@@ -2115,8 +2123,10 @@ struct Tet2Sim : Sim {
 
     double dot_host(const void *x, const void *y)
     {
-        if (fp64) launch_after(t2_dot_kernel<double>, dim3(kDotBlocks), dim3(256), 0, stream, ndof, (const double *)x, (const double *)y, d_part.as<double>());
-        else launch_after(t2_dot_kernel<float>, dim3(kDotBlocks), dim3(256), 0, stream, ndof, (const float *)x, (const float *)y, d_part.as<double>());
+        if (fp64) launch_after(t2_dot_kernel<double>, dim3(kDotBlocks), dim3(256), 0, stream, ndof, (const double *)x,
+                               (const double *)y, d_part.as<double>());
+        else launch_after(t2_dot_kernel<float>, dim3(kDotBlocks), dim3(256), 0, stream, ndof, (const float *)x,
+                          (const float *)y, d_part.as<double>());
         std::vector<double> part(kDotBlocks);
         EMS_CUDA(cudaMemcpyAsync(part.data(), d_part.p, kDotBlocks * 8, cudaMemcpyDeviceToHost, stream));
         EMS_CUDA(cudaStreamSynchronize(stream));
@@ -2368,28 +2378,31 @@ struct Tet2Sim : Sim {
         int nl = 0;
         const int nd = (int)std::max<size_t>(dips.size(), 1);
         if (sample && nobs > 0) {
-            launch_after(t2_sample_kernel<T>, dim3(blocks((unsigned long long)nobs * 32, 128)), dim3(128), 0, stream, 
-                nobs, d_rec_dof.as<unsigned long long>(), d_rec_w.as<double>(), d_U.as<T>(), d_ctl.as<int>(), P.time_frequency,
-                nsamp, d_tr.as<double>());
+            launch_after(t2_sample_kernel<T>, dim3(blocks((unsigned long long)nobs * 32, 128)), dim3(128), 0, stream, nobs,
+                         d_rec_dof.as<unsigned long long>(), d_rec_w.as<double>(), d_U.as<T>(), d_ctl.as<int>(),
+                         P.time_frequency, nsamp, d_tr.as<double>());
             ++nl;
         }
         if (symp()) {
             double sub[3], off[3];
             substeps(sub, off);
             const int nq = nsub();
-            launch_after(t2_axpy_kernel<T>, dim3(blocks(ndof, 256)), dim3(256), 0, stream, ndof, d_U.as<T>(), d_x.as<T>(), 0.5 * sub[0]);
+            launch_after(t2_axpy_kernel<T>, dim3(blocks(ndof, 256)), dim3(256), 0, stream, ndof, d_U.as<T>(), d_x.as<T>(),
+                         0.5 * sub[0]);
             ++nl;
             for (int q = 0; q < nq; ++q) {
                 enqueue_stiff<T>(d_U.as<T>());
                 GArgs<T> g = gargs<T>();
                 g.Yt = d_YtK.p;
                 g.a = sub[q];
-                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
+                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent,
+                             d_shots.as<T2Shot>(), ns, g);
                 nl += 2;
                 if (nsrc > 0) {
-                    launch_after(t2_source_kernel<T, 0>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, 
-                        nsrc, d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(), d_src_coef.as<double>(),
-                        d_src_g.as<double>(), d_ctl.as<int>(), nq, q, nd, sub[q], d_P.as<double>(), fp64 ? nullptr : d_Pc.as<T>());
+                    launch_after(t2_source_kernel<T, 0>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, nsrc,
+                                 d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(),
+                                 d_src_coef.as<double>(), d_src_g.as<double>(), d_ctl.as<int>(), nq, q, nd, sub[q],
+                                 d_P.as<double>(), fp64 ? nullptr : d_Pc.as<T>());
                     ++nl;
                 }
                 const double h = 0.5 * sub[q] + (q + 1 < nq ? 0.5 * sub[q + 1] : 0.0);
@@ -2398,9 +2411,10 @@ struct Tet2Sim : Sim {
         } else {
             nl += enqueue_force<T>(d_U.as<T>(), d_b.as<T>());
             if (nsrc > 0) {
-                launch_after(t2_source_kernel<T, 1>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, 
-                    nsrc, d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(), d_src_coef.as<double>(),
-                    d_src_g.as<double>(), d_ctl.as<int>(), 1, 0, nd, 1.0, nullptr, d_b.as<T>());
+                launch_after(t2_source_kernel<T, 1>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, nsrc,
+                             d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(),
+                             d_src_coef.as<double>(), d_src_g.as<double>(), d_ctl.as<int>(), 1, 0, nd, 1.0, nullptr,
+                             d_b.as<T>());
                 ++nl;
             }
             nl += enqueue_solve<T, FIN_LEAP>(d_b.as<T>(), dtn * dtn);
@@ -2730,17 +2744,20 @@ template <class T> void Tet2Sim::backward_t(const double *tg, double *grad)
         enqueue_solve<T, FIN_NONE>(rhs_P<T>(), 0.0, Y(n0, 0));
         launch_after(t2_set_kernel, dim3(1), dim3(1), 0, stream, ctl, n0);
         for (int n = n0; n < n1; ++n) {
-            launch_after(t2_axpy_kernel<T>, dim3(blocks(ndof, 256)), dim3(256), 0, stream, ndof, d_U.as<T>(), Y(n, 0), 0.5 * sub[0]);
+            launch_after(t2_axpy_kernel<T>, dim3(blocks(ndof, 256)), dim3(256), 0, stream, ndof, d_U.as<T>(), Y(n, 0),
+                         0.5 * sub[0]);
             for (int q = 0; q < nq; ++q) {
                 enqueue_stiff<T>(d_U.as<T>());
                 GArgs<T> g = gargs<T>();
                 g.Yt = d_YtK.p;
                 g.a = sub[q];
-                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
+                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent,
+                             d_shots.as<T2Shot>(), ns, g);
                 if (nsrc > 0)
-                    launch_after(t2_source_kernel<T, 0>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, 
-                        nsrc, d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(), d_src_coef.as<double>(),
-                        d_src_g.as<double>(), ctl, nq, q, nd, sub[q], d_P.as<double>(), fp64 ? nullptr : d_Pc.as<T>());
+                    launch_after(t2_source_kernel<T, 0>, dim3(blocks(nsrc, 128)), dim3(128), 0, stream, nsrc,
+                                 d_src_dof.as<unsigned long long>(), d_src_ptr.as<int>(), d_src_dip.as<int>(),
+                                 d_src_coef.as<double>(), d_src_g.as<double>(), ctl, nq, q, nd, sub[q], d_P.as<double>(),
+                                 fp64 ? nullptr : d_Pc.as<T>());
                 enqueue_solve<T, FIN_DRIFT>(rhs_P<T>(), hq[q], Y(n, q + 1));
             }
             launch_after(t2_advance_kernel, dim3(1), dim3(1), 0, stream, ctl);
@@ -2751,23 +2768,24 @@ template <class T> void Tet2Sim::backward_t(const double *tg, double *grad)
             // adjoint of the substages
             for (int q = nq - 1; q >= 0; --q) {
                 enqueue_solve<T, FIN_DRIFT>(Ubr, hq[q], d_x.as<T>(), Pb.as<T>());
-                launch_after(t2_grad_kernel<T>, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(), ns, d_x.as<T>(), Y(n, q + 1),
-                                                                         -hq[q], gd.as<double>());
+                launch_after(t2_grad_kernel<T>, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(), ns,
+                             d_x.as<T>(), Y(n, q + 1), -hq[q], gd.as<double>());
                 enqueue_stiff<T>(Pb.as<T>());
                 GArgs<T> g = gargs<T>();
                 g.Yt = d_YtK.p;
                 g.a = sub[q];
                 g.P = Ub.as<double>();
                 g.Pc = fp64 ? nullptr : Ubc.as<T>();
-                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent, d_shots.as<T2Shot>(), ns, g);
+                launch_after(t2_gather_kernel<T, double, G_KICK, FIN_NONE>, dim3(blocks(nent, 128)), dim3(128), 0, stream, nent,
+                             d_shots.as<T2Shot>(), ns, g);
             }
             enqueue_solve<T, FIN_DRIFT>(Ubr, 0.5 * sub[0], d_x.as<T>(), Pb.as<T>());
-            launch_after(t2_grad_kernel<T>, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(), ns, d_x.as<T>(), Y(n, 0),
-                                                                     -0.5 * sub[0], gd.as<double>());
+            launch_after(t2_grad_kernel<T>, dim3(blocks(ntet, 128)), dim3(128), 0, stream, ntet, d_shots.as<T2Shot>(), ns,
+                         d_x.as<T>(), Y(n, 0), -0.5 * sub[0], gd.as<double>());
             if (nrd > 0 && n % tf == 0)
-                launch_after(t2_source_kernel<T, 0>, dim3(blocks(nrd, 128)), dim3(128), 0, stream, 
-                    nrd, a_dof.as<unsigned long long>(), a_ptr.as<int>(), a_idx.as<int>(), a_coef.as<double>(), a_g.as<double>(),
-                    ctl, 1, 0, nd3, 1.0, Ub.as<double>(), fp64 ? nullptr : Ubc.as<T>());
+                launch_after(t2_source_kernel<T, 0>, dim3(blocks(nrd, 128)), dim3(128), 0, stream, nrd,
+                             a_dof.as<unsigned long long>(), a_ptr.as<int>(), a_idx.as<int>(), a_coef.as<double>(),
+                             a_g.as<double>(), ctl, 1, 0, nd3, 1.0, Ub.as<double>(), fp64 ? nullptr : Ubc.as<T>());
             EMS_CUDA(cudaGetLastError());
         }
     }

@@ -2414,12 +2414,12 @@ struct TetFemSim : Sim {
                       DevBuf &part, unsigned *ticket, double *alpha, int *jp, int max_blocks)
     {
         const unsigned nbv = (unsigned)((nnode + step_block - 1) / step_block);
-        launch_after(tet_step_kernel<float, 0, 0>, dim3(nbv), dim3(step_block), 0, stream, nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), nullptr,
-                                                              kv32.as<float>(), x32.as<float>(), nullptr, nullptr, -1.0f, 0.0f,
-                                                              SrcArgs{}, nullptr, nullptr, nullptr, nullptr, RecArgs<float>{}, Comp{});
+        launch_after(tet_step_kernel<float, 0, 0>, dim3(nbv), dim3(step_block), 0, stream, nnode, d_nrec.as<int2>(),
+                     d_pec.as<unsigned char>(), nullptr, kv32.as<float>(), x32.as<float>(), nullptr, nullptr, -1.0f, 0.0f,
+                     SrcArgs{}, nullptr, nullptr, nullptr, nullptr, RecArgs<float>{}, Comp{});
         const int nb = (int)std::min<size_t>((nnode + 127) / 128, max_blocks);
-        launch_after(lanczos_minv_kernel, dim3(nb), dim3(128), 0, stream, nnode, minv_d.as<double>(), kv32.as<float>(), vcur.as<double>(),
-                                                    Mz.as<double>(), z.as<double>(), part.as<double>(), ticket, alpha, jp);
+        launch_after(lanczos_minv_kernel, dim3(nb), dim3(128), 0, stream, nnode, minv_d.as<double>(), kv32.as<float>(),
+                     vcur.as<double>(), Mz.as<double>(), z.as<double>(), part.as<double>(), ticket, alpha, jp);
     }
 
     // Largest eigenvalue of Minv K by Lanczos in the M inner product.  Minv K
@@ -2466,18 +2466,18 @@ struct TetFemSim : Sim {
         applyMinvK32(w.v32, w.kv32, minv_d, vb[0], mb[1], vb[1], w.part, tk, alpha, nullptr, nbl);
         dot_partial_kernel<<<512, 256, 0, stream>>>(nslot, vb[1].as<double>(), mb[1].as<double>(), w.part.as<double>());
         dot_finish_kernel<<<1, 512, 0, stream>>>(512, w.part.as<double>(), nrm0);
-        launch_after(scale_kernel, dim3(nbl), dim3(256), 0, stream, nslot, vb[1].as<double>(), mb[1].as<double>(), nrm0, nullptr, w.v32.as<float>(),
-                                              w.kv32.as<float>());
+        launch_after(scale_kernel, dim3(nbl), dim3(256), 0, stream, nslot, vb[1].as<double>(), mb[1].as<double>(), nrm0,
+                     nullptr, w.v32.as<float>(), w.kv32.as<float>());
         int prev = -1, cur = 1, nxt = 2;
         // one iteration: apply (+ alpha), three-term step (+ beta^2),
         // normalisation; jp == nullptr: host index jj, else the device index
         // (advanced by the apply)
         auto iteration = [&](int jj, int *jp) {
             applyMinvK32(w.v32, w.kv32, minv_d, vb[cur], mb[nxt], vb[nxt], w.part, tk, alpha, jp, nbl);
-            launch_after(lanczos_step_kernel, dim3(nbl), dim3(256), 0, stream, nslot, vb[nxt].as<double>(), mb[nxt].as<double>(), vb[cur].as<double>(),
-                                                         mb[cur].as<double>(), prev >= 0 ? vb[prev].as<double>() : nullptr,
-                                                         prev >= 0 ? mb[prev].as<double>() : nullptr, alpha,
-                                                         w.part.as<double>(), tk + 1, cf, jj, jp);
+            launch_after(lanczos_step_kernel, dim3(nbl), dim3(256), 0, stream, nslot, vb[nxt].as<double>(),
+                         mb[nxt].as<double>(), vb[cur].as<double>(), mb[cur].as<double>(),
+                         prev >= 0 ? vb[prev].as<double>() : nullptr, prev >= 0 ? mb[prev].as<double>() : nullptr, alpha,
+                         w.part.as<double>(), tk + 1, cf, jj, jp);
             launch_after(scale_kernel, dim3(nbl), dim3(256), 0, stream, nslot, vb[nxt].as<double>(), mb[nxt].as<double>(),
                                                   jp ? cf + 1 : cf + 2 * jj + 1, jp, w.v32.as<float>(), w.kv32.as<float>());
             const int t = prev < 0 ? 0 : prev;
@@ -2622,8 +2622,8 @@ struct TetFemSim : Sim {
                 const unsigned nbs = (unsigned)((nnode + kSlotNodes - 1) / kSlotNodes) + (unsigned)rec.nsb;
                 const dim3 blk(kSlotNodes, 7);
                 auto go = [&](auto kern) {
-                    launch_after(kern, dim3(nbs), blk, 0, stream, nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), d_minv.as<T>(), Pio,
-                                 Uin, Uout, a, c, sa, zout, rec, cm);
+                    launch_after(kern, dim3(nbs), blk, 0, stream, nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(),
+                                 d_minv.as<T>(), Pio, Uin, Uout, a, c, sa, zout, rec, cm);
                     return 1;
                 };
                 const bool comp32 = std::is_same<T, float>::value && cm.p;
@@ -2635,8 +2635,8 @@ struct TetFemSim : Sim {
         const unsigned nbv = (unsigned)((nnode + step_block - 1) / step_block) + (unsigned)rec.nsb;
         const T *dm = DAMP ? d_damp.as<T>() : nullptr;
         auto go = [&](auto kern) {
-            launch_after(kern, dim3(nbv), dim3(step_block), 0, stream, nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(), d_minv.as<T>(), Pio,
-                         Uin, Uout, Uold, a, c, sa, zout, dm, ppre, pmid, rec, cm);
+            launch_after(kern, dim3(nbv), dim3(step_block), 0, stream, nnode, d_nrec.as<int2>(), d_pec.as<unsigned char>(),
+                         d_minv.as<T>(), Pio, Uin, Uout, Uold, a, c, sa, zout, dm, ppre, pmid, rec, cm);
             return 1;
         };
         if constexpr (MODE == 0 && std::is_same<T, float>::value) {
@@ -3255,8 +3255,8 @@ struct TetFemSim : Sim {
                         // the lossy middle kick: Pbar = g Pbar before the
                         // adjoint kick, Pbar = g Pbar + c Minv Wbar after it
                         const T *pp = pstore.as<T>() + (size_t)(n - n0) * 2 * nslot;
-                        launch_after(tet_loss_adjoint_kernel<T>, dim3(nbv2), dim3(128), 0, stream, nnode, d_damp.as<T>(), pb, pp + nslot, pp,
-                                                                            zr.as<double>());
+                        launch_after(tet_loss_adjoint_kernel<T>, dim3(nbv2), dim3(128), 0, stream, nnode, d_damp.as<T>(), pb,
+                                     pp + nslot, pp, zr.as<double>());
                         substep<T, 0, 2>(pb, pb2, Wb.as<T>(), nullptr, (T)sc.sub[q], (T)c, SrcArgs{}, y, nullptr, nullptr,
                                          RecArgs<T>{}, cadj);
                     } else {
@@ -3267,10 +3267,10 @@ struct TetFemSim : Sim {
                 }
                 if (n % tf == 0 && n > 0 && nobs > 0 && ra.nsl > 0) {
                     const T *z = zb + (size_t)(n - n0) * nsub * nslot;
-                    launch_after(tet_receiver_adjoint_kernel<T>, dim3((8 * ra.nnd + 127) / 128), dim3(128), 0, stream, 
-                        ra.nnd, ra.nd_node.as<int>(), ra.nd_map.as<int>(), ra.sl_ptr.as<int>(), ra.term_rc.as<int>(), ra.term_w.as<double>(),
-                        d_rs.as<double>() + (size_t)(n / tf) * nobs * 3, Wb.as<T>(), pb, d_minv.as<T>(), z, Q.as<double>(),
-                        0.5 * sc.sub[nsub - 1], nnode);
+                    launch_after(tet_receiver_adjoint_kernel<T>, dim3((8 * ra.nnd + 127) / 128), dim3(128), 0, stream, ra.nnd,
+                                 ra.nd_node.as<int>(), ra.nd_map.as<int>(), ra.sl_ptr.as<int>(), ra.term_rc.as<int>(),
+                                 ra.term_w.as<double>(), d_rs.as<double>() + (size_t)(n / tf) * nobs * 3, Wb.as<T>(), pb,
+                                 d_minv.as<T>(), z, Q.as<double>(), 0.5 * sc.sub[nsub - 1], nnode);
                 }
             }
             // the drifts of this segment: y at [k], z at [k] (k = nsub (n - n0) + q)
