@@ -6,6 +6,7 @@
 #include <array>
 #include <cstdio>
 #include <initializer_list>
+#include <mutex>
 #include <utility>
 #include <type_traits>
 #include <string>
@@ -113,9 +114,11 @@ struct Sim {
     // 160x150x140 cells into fresh arrays: 137 ms, 7 so).
     void download(double *out, const double *dev, size_t cnt) const;
     // cnt values that pack(at, n, dst) forms in device memory, n of them from
-    // `at`, by way of a buffer of at most kStage values.
+    // `at`, by way of a buffer of at most kStage values (the lock: fields of one
+    // handle may be read by several threads at a time).
     template <class F> void download(double *out, size_t cnt, F &&pack) const
     {
+        const std::lock_guard<std::mutex> lock(stage_lock);
         const size_t piece = std::min(cnt, kStage);
         d_stage.grow(piece * sizeof(double));
         for (size_t at = 0; at < cnt; at += piece) {
@@ -127,6 +130,7 @@ struct Sim {
     }
     static constexpr size_t kStage = (size_t)1 << 20;
     mutable DevBuf d_stage;
+    mutable std::mutex stage_lock;
 };
 
 // CSV element matrices in the reference format (fem_v2/fem_simulation.cpp:1477-1524).

@@ -48,3 +48,20 @@ def test_fields_of_several_pieces_in_bounded_memory(kind, prec):
         assert np.array_equal(got[live], vals[q][live])
     assert free - torch.cuda.mem_get_info()[0] <= SCRATCH
     s.close()
+
+
+@pytest.mark.parametrize("prec", [ems.FP64, ems.FP32], ids=["fp64", "fp32"])
+@pytest.mark.parametrize("kind", ["fdtd", "hex", "tet1", "tet2"])
+def test_threads_read_fields_of_one_handle(kind, prec):
+    """Threads that read fields of the same handle at the same time each get
+    their own field."""
+    from concurrent.futures import ThreadPoolExecutor
+    s, nf = _handle(kind, prec)
+    rng = np.random.default_rng(4)
+    for q in range(nf):
+        s.set_field(q, rng.standard_normal(s.field_size(q)))
+    ref = [s.get_field(q) for q in range(nf)]
+    with ThreadPoolExecutor(4) as ex:
+        for q, got in zip(list(range(nf)) * 6, ex.map(s.get_field, list(range(nf)) * 6)):
+            assert np.array_equal(got, ref[q])
+    s.close()
