@@ -1046,7 +1046,7 @@ __device__ __forceinline__ void tet_slot(size_t nnode, const int2 *__restrict__ 
     const size_t v = (size_t)nb * kSlotNodes + lane;
     const bool valid = v < nnode;
     const size_t f0 = (size_t)d * nnode + v, e0 = 7 * v;
-    T x = 0, u = 0, row[7] = {0, 0, 0, 0, 0, 0, 0};   // row: the mass row of slot d, loaded before the barrier
+    T x = 0, row[7] = {0, 0, 0, 0, 0, 0, 0};   // row: the mass row of slot d, loaded before the barrier
     unsigned char m = 0;
     if (valid) {
         const int2 r = __ldg(nrec + v);
@@ -1066,7 +1066,6 @@ __device__ __forceinline__ void tet_slot(size_t nnode, const int2 *__restrict__ 
         case 5: slot_force<T, 5, COMP>(u0, nnode, off, have, f, fl, minv, v, row); break;
         default: slot_force<T, 6, COMP>(u0, nnode, off, have, f, fl, minv, v, row); break;
         }
-        u = Uin[f0];
         m = pec[e0 + d];
         x = P[f0];
         // the kick of the node kernel (MODE 0, no losses)
@@ -1093,6 +1092,9 @@ __device__ __forceinline__ void tet_slot(size_t nnode, const int2 *__restrict__ 
     sx[d][lane] = x;
     __syncthreads();
     if (!valid) return;
+    // behind the barrier, where the register is free (us a step of three launches,
+    // FP32: 24^3 10.24 ahead of it and 10.43 here, 32^3 13.67 and 13.34, 40^3 21.4 and 21.2)
+    const T u = Uin[f0];
     T y = 0;
 #pragma unroll
     for (int j = 0; j < 7; ++j) y = fma(row[j], sx[j][lane], y);
